@@ -19,7 +19,7 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libdistconv_b200.so")
 
-SOURCES = ["runtime.cu", "halo.cu", "bn.cu", "conv.cu", "conv_simt.cu", "conv_tc.cu", "comm.cu", "pool.cu", "shuffle.cu"]
+SOURCES = ["runtime.cu", "halo.cu", "bn.cu", "conv.cu", "conv_simt.cu", "conv_tc.cu", "conv_tc_shift.cu", "comm.cu", "pool.cu", "shuffle.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -51,8 +51,7 @@ def sources():
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """DCB_BUILD_DEFINES (e.g. "-DDCB_SW_PROFILE=1": per-role clock accounting in
-    the sweep convolution kernel) adds compiler flags; use it with force."""
+    """DCB_BUILD_DEFINES adds compiler flags; use it with force."""
     os.makedirs(OBJ, exist_ok=True)
     extra = os.environ.get("DCB_BUILD_DEFINES", "").split()
     hdr_t = _newest_header()

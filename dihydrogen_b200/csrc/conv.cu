@@ -1,6 +1,7 @@
 // Convolution front end: plan, geometry validation, kernel selection, bias.
 #include "conv_simt.cuh"
 #include "conv_tc.cuh"
+#include "conv_tc_shift_api.cuh"
 
 using namespace dcb;
 
@@ -12,7 +13,9 @@ struct dcb_conv_plan
     float* workspace = nullptr; // backward-filter partials
     size_t workspace_bytes = 0;
     float* wflip = nullptr; // flipped/transposed filter for backward data
-    TcPlan* tc = nullptr;   // tensor-core state (packed filters), may be null
+    ShPlan* sh[2] = {nullptr, nullptr}; // tensor-core forward and backward data, may be null
+    TcPlan* tc = nullptr;   // sweep kernel and backward filter, may be null
+    int* status = nullptr;  // device word: a tensor-core kernel gave up on a wait
     int kind[3] = {0, 0, 0};
     bool bwd_data_as_fwd = false;
 };
@@ -111,40 +114,43 @@ int32_t dcb_conv_plan_create(const dcb_conv_desc* cd, const dcb_nd_desc* xd,
     for (int i = 0; i < 3; ++i)
         if (g.stride[i] != 1 || (g.f[i] - 1) * g.dil[i] - g.pad[i] < 0)
             p->bwd_data_as_fwd = false;
+    if (cd->math_mode != DCB_MATH_FP32_SIMT)
+    {
+        // Tensor-core kernels where the geometry fits; otherwise the fp32
+        // CUDA-core kernels stay selected.
+        for (int dir = 0; dir < 2; ++dir)
+        {
+            p->kind[dir] = sh_plan_create(g, dir == 1, cd->math_mode, &p->sh[dir], &st) ? 1 : 0;
+            if (st != DCB_OK)
+            {
+                dcb_conv_plan_destroy(p);
+                return st;
+            }
+        }
+        st = tc_plan_create(g, cd->math_mode, &p->tc);
+        if (st != DCB_OK)
+        {
+            dcb_conv_plan_destroy(p);
+            return st;
+        }
+        p->kind[2] = tc_has_bwd_filter(p->tc) ? 1 : 0;
+    }
     const size_t fbytes =
         (size_t) g.k * g.c * g.f[0] * g.f[1] * g.f[2] * sizeof(float);
     p->workspace_bytes = simt_conv_bwd_filter_workspace(g);
     bool ok = cudaMalloc(&p->workspace, p->workspace_bytes ? p->workspace_bytes : 16)
               == cudaSuccess;
-    ok = ok && cudaMalloc(&p->wflip, fbytes ? fbytes : 16) == cudaSuccess;
+    if (p->bwd_data_as_fwd && p->kind[1] == 0)
+        ok = ok && cudaMalloc(&p->wflip, fbytes ? fbytes : 16) == cudaSuccess;
+    if (p->kind[0] || p->kind[1] || p->kind[2])
+        ok = ok && cudaMalloc(&p->status, sizeof(int)) == cudaSuccess
+             && cudaMemset(p->status, 0, sizeof(int)) == cudaSuccess;
     if (!ok)
     {
         (void) cudaGetLastError();
         set_last_error("cudaMalloc of convolution workspace failed");
-        cudaFree(p->workspace);
-        cudaFree(p->wflip);
-        delete p;
+        dcb_conv_plan_destroy(p);
         return DCB_CUDA_ERROR;
-    }
-    if (cd->math_mode != DCB_MATH_FP32_SIMT)
-    {
-        // Tensor-core kernels where the geometry fits; otherwise the fp32
-        // CUDA-core kernels stay selected.
-        st = tc_plan_create(g, p->bwd_data_as_fwd ? bwd_as_fwd_geom(g) : g,
-                            p->bwd_data_as_fwd, cd->math_mode, &p->tc);
-        if (st != DCB_OK)
-        {
-            cudaFree(p->workspace);
-            cudaFree(p->wflip);
-            delete p;
-            return st;
-        }
-        if (p->tc)
-        {
-            p->kind[0] = tc_supports(p->tc, 0) ? 1 : 0;
-            p->kind[1] = tc_supports(p->tc, 1) ? 1 : 0;
-            p->kind[2] = tc_supports(p->tc, 2) ? 1 : 0;
-        }
     }
     *out = p;
     return DCB_OK;
@@ -154,9 +160,12 @@ int32_t dcb_conv_plan_destroy(dcb_conv_plan* p)
 {
     if (!p)
         return DCB_OK;
+    sh_plan_destroy(p->sh[0]);
+    sh_plan_destroy(p->sh[1]);
     tc_plan_destroy(p->tc);
     cudaFree(p->workspace);
     cudaFree(p->wflip);
+    cudaFree(p->status);
     delete p;
     return DCB_OK;
 }
@@ -165,7 +174,7 @@ int32_t dcb_conv_plan_status(dcb_conv_plan* p, void* stream)
 {
     DCB_REQUIRE(p, "null argument");
     DCB_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
-    int* word = tc_status_word(p->tc);
+    int* word = p->status;
     if (!word)
         return DCB_OK;
     int st = 0;
@@ -190,7 +199,9 @@ int32_t dcb_conv_plan_kernel_variant(const dcb_conv_plan* p, int32_t which)
 {
     if (!p || which < 0 || which > 2)
         return -1;
-    return p->kind[which] == 1 ? tc_variant(p->tc, which) : 0;
+    if (p->kind[which] != 1)
+        return 0;
+    return which == 2 ? 5 : (sh_two_sets(p->sh[which]) ? 4 : 3);
 }
 
 int32_t dcb_conv_fwd(dcb_conv_plan* p, double alpha, const void* x,
@@ -198,10 +209,21 @@ int32_t dcb_conv_fwd(dcb_conv_plan* p, double alpha, const void* x,
 {
     DCB_REQUIRE(p && x && w && y, "null argument");
     if (p->kind[0] == 1)
-        return tc_conv_fwd(p->tc, 0, (float) alpha,
-                           static_cast<const float*>(x),
-                           static_cast<const float*>(w), (float) beta,
-                           static_cast<float*>(y), as_stream(stream));
+    {
+        // the sweep kernel where it covers the problem and the pointers allow it
+        if (beta == 0.0)
+        {
+            const int32_t st = tc_sweep_fwd(
+                p->tc, (float) alpha, static_cast<const float*>(x),
+                static_cast<const float*>(w), static_cast<float*>(y), p->status,
+                as_stream(stream));
+            if (st != DCB_UNSUPPORTED)
+                return st;
+        }
+        return sh_conv(p->sh[0], (float) alpha, static_cast<const float*>(x),
+                       static_cast<const float*>(w), (float) beta,
+                       static_cast<float*>(y), p->status, as_stream(stream));
+    }
     return simt_conv_fwd(p->g, (float) alpha, static_cast<const float*>(x),
                          static_cast<const float*>(w), (float) beta,
                          static_cast<float*>(y), as_stream(stream));
@@ -212,12 +234,19 @@ int32_t dcb_conv_fwd_stats(dcb_conv_plan* p, double alpha, const void* x,
                            void* stream)
 {
     DCB_REQUIRE(p && x && w && y && sums && sqsums, "null argument");
-    if (p->kind[0] != 1)
+    if (p->kind[0] != 1 || p->cd.nsd != 3)
         return DCB_UNSUPPORTED;
-    return tc_conv_fwd_stats(p->tc, (float) alpha, static_cast<const float*>(x),
-                             static_cast<const float*>(w),
-                             static_cast<float*>(y), static_cast<float*>(sums),
-                             static_cast<float*>(sqsums), as_stream(stream));
+    const int32_t st = tc_sweep_fwd(
+        p->tc, (float) alpha, static_cast<const float*>(x),
+        static_cast<const float*>(w), static_cast<float*>(y), p->status,
+        as_stream(stream), static_cast<float*>(sums),
+        static_cast<float*>(sqsums));
+    if (st != DCB_UNSUPPORTED)
+        return st;
+    return sh_conv(p->sh[0], (float) alpha, static_cast<const float*>(x),
+                   static_cast<const float*>(w), 0.f, static_cast<float*>(y),
+                   p->status, as_stream(stream), static_cast<float*>(sums),
+                   static_cast<float*>(sqsums));
 }
 
 int32_t dcb_conv_bwd_data(dcb_conv_plan* p, double alpha, const void* w,
@@ -225,6 +254,10 @@ int32_t dcb_conv_bwd_data(dcb_conv_plan* p, double alpha, const void* w,
 {
     DCB_REQUIRE(p && w && dy && dx, "null argument");
     const ConvGeom& g = p->g;
+    if (p->kind[1] == 1)
+        return sh_conv(p->sh[1], (float) alpha, static_cast<const float*>(dy),
+                       static_cast<const float*>(w), (float) beta,
+                       static_cast<float*>(dx), p->status, as_stream(stream));
     if (p->bwd_data_as_fwd)
     {
         const int taps = g.f[0] * g.f[1] * g.f[2];
@@ -233,11 +266,6 @@ int32_t dcb_conv_bwd_data(dcb_conv_plan* p, double alpha, const void* w,
                                            as_stream(stream));
         if (st != DCB_OK)
             return st;
-        if (p->kind[1] == 1)
-            return tc_conv_fwd(p->tc, 1, (float) alpha,
-                               static_cast<const float*>(dy), p->wflip,
-                               (float) beta, static_cast<float*>(dx),
-                               as_stream(stream));
         return simt_conv_fwd(bwd_as_fwd_geom(g), (float) alpha,
                              static_cast<const float*>(dy), p->wflip,
                              (float) beta, static_cast<float*>(dx),
@@ -258,7 +286,7 @@ int32_t dcb_conv_bwd_filter(dcb_conv_plan* p, double alpha, const void* x,
         const int32_t st = tc_conv_bwd_filter(
             p->tc, (float) alpha, static_cast<const float*>(x),
             static_cast<const float*>(dy), (float) beta,
-            static_cast<float*>(dw), as_stream(stream));
+            static_cast<float*>(dw), p->status, as_stream(stream));
         if (st != DCB_UNSUPPORTED) // unaligned base pointers take the kernel below
             return st;
     }

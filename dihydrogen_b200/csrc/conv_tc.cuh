@@ -1,4 +1,5 @@
-// Interface of the tcgen05 / TMEM convolution kernels.
+// Interface of the tcgen05 sweep kernel (forward, few input channels) and of the
+// tcgen05 backward filter.
 #pragma once
 
 #include "conv_simt.cuh"
@@ -8,32 +9,20 @@ namespace dcb
 
 struct TcPlan;
 
-// Creates tensor-core state for the problems the kernels cover; *out stays
-// null (and DCB_OK is returned) when none of them applies.  `fwd` is the
-// forward geometry, `bwd` the forward-shaped geometry that computes backward
-// data (only meaningful when bwd_is_fwd).
-int32_t tc_plan_create(const ConvGeom& fwd, const ConvGeom& bwd,
-                       bool bwd_is_fwd, int math_mode, TcPlan** out);
+// Tensor-core state for the forward geometry `fwd` and its backward filter; *out
+// stays null (and DCB_OK is returned) when neither kernel covers the geometry.
+int32_t tc_plan_create(const ConvGeom& fwd, int math_mode, TcPlan** out);
 void tc_plan_destroy(TcPlan* p);
-// which: 0 forward, 1 backward data, 2 backward filter
-bool tc_supports(const TcPlan* p, int which);
-// The kernel the plan prefers for that pass, as dcb_conv_plan_kernel_variant
-// numbers them (1 row kernel fed by bulk copies, 2 row kernel whose converters
-// fetch their own rows, 3 sweep, 4 multi-group sweep, 5 backward filter; 0 none).
-int tc_variant(const TcPlan* p, int which);
-// slot 0 runs the forward geometry, slot 1 the backward-data one.
-int32_t tc_conv_fwd(TcPlan* p, int slot, float alpha, const float* x,
-                    const float* w, float beta, float* y, cudaStream_t stream);
-// Forward convolution (beta = 0) whose epilogue also returns, per filter, the sum
-// and the sum of squares of the outputs.  DCB_UNSUPPORTED when the plan's
-// kernel for this problem cannot do that; nothing has been launched then.
-int32_t tc_conv_fwd_stats(TcPlan* p, float alpha, const float* x,
-                          const float* w, float* y, float* sums,
-                          float* sqsums, cudaStream_t stream);
-// Device word that kernels set when a bounded wait expires (null if no plan).
-int* tc_status_word(TcPlan* p);
+bool tc_has_bwd_filter(const TcPlan* p);
+// `status`: device word that a kernel sets when a bounded wait expires.
+// y = alpha * conv(x, w), optionally with the per-filter sums and sums of squares
+// of y.  DCB_UNSUPPORTED, with nothing launched, when the kernel does not cover
+// the plan or x's alignment.
+int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w,
+                     float* y, int* status, cudaStream_t stream,
+                     float* sums = nullptr, float* sqsums = nullptr);
 int32_t tc_conv_bwd_filter(TcPlan* p, float alpha, const float* x,
                            const float* dy, float beta, float* dw,
-                           cudaStream_t stream);
+                           int* status, cudaStream_t stream);
 
 } // namespace dcb

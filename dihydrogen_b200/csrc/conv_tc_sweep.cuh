@@ -1,7 +1,7 @@
 // tcgen05 / TMEM convolution for filters with depth (fd > 1): the "sweep"
-// kernel.  Same GEMM view as conv_tc_kernel.cuh (M = 128 outputs along W, the
-// reduction runs over (c, kw) of one staged input row), but a staged row is
-// converted ONCE and serves every (kd, kh) tap:
+// kernel, forward with few input channels.  One MMA tile is 128 consecutive outputs
+// of one output row (M = 128 along W); for a staged input row the reduction index
+// runs over (c, kw).  A staged row is converted ONCE and serves every (kd, kh) tap:
 //
 //   * A CTA owns a column of the volume (th output rows x 128 outputs wide)
 //     and sweeps a segment of output planes od0..od1-1 along D, one input
@@ -50,66 +50,31 @@
 // per column under random schedules in a host-side model.
 #pragma once
 
-#include "conv_tc_kernel.cuh"
+#include "conv_simt.cuh"
+#include "conv_tc_common.cuh"
 
 namespace dcb
 {
 namespace
 {
 
-// Per-role clock accounting (a build with -DDCB_SW_PROFILE=1 only): every warp
-// adds up the clocks it spends in each phase of its loop and leaves eight
-// totals in `prof` at the end; the host prints the per-role averages.
-#ifndef DCB_SW_PROFILE
-#define DCB_SW_PROFILE 0
-#endif
-// Timing knock-outs (a build with -DDCB_SW_KNOCKOUT=1 only; results are wrong
-// with any bit set): bits of DCB_SW_DBG switch single pieces of work off so
-// that what the kernel's time depends on can be measured.
-#ifndef DCB_SW_KNOCKOUT
-#define DCB_SW_KNOCKOUT 0
-#endif
-#if DCB_SW_KNOCKOUT
-#define SW_DBG(bit) ((g.nsets >> (bit)) & 1)
-#else
-#define SW_DBG(bit) 0
-#endif
-#if DCB_SW_PROFILE
-#define SW_PROF_DECL long long pf_t = clock64(), pf_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}; const long long pf_t0 = pf_t;
-#define SW_PROF_MARK(slot)                                                                                            \
-    {                                                                                                                 \
-        const long long pf_now = clock64();                                                                           \
-        pf_acc[slot] += pf_now - pf_t;                                                                                \
-        pf_t = pf_now;                                                                                                \
-    }
-#define SW_PROF_FLUSH(prof)                                                                                           \
-    if (prof != nullptr && lane == 0)                                                                                 \
-    {                                                                                                                 \
-        pf_acc[7] = clock64() - pf_t0;                                                                                \
-        for (int pf_i = 0; pf_i < 8; ++pf_i)                                                                          \
-            prof[((size_t) blockIdx.x * 32 + warp) * 8 + pf_i] = pf_acc[pf_i];                                        \
-    }
-#else
-#define SW_PROF_DECL
-#define SW_PROF_MARK(slot)
-#define SW_PROF_FLUSH(prof)
-#endif
-
 constexpr int SW_NBK = 16; // accumulator columns per (output row, plane slot)
 
 
 struct SwGeom
 {
-    int n, c, k;    // c: input channels of one launch (a group of the filter's w_c_total)
-    int w_c_total;  // input channels of the filter
-    int w_c_off;    // first input channel of this launch's group
-    int cgroups;    // launches per convolution = w_c_total / c
+    int n, c, k;
     int in[3], out[3], f[3], pad[3];
-    int lx, rx;     // as in TcGeom: where a staged row starts, where its first tap sits
+    // A staged raw row holds the input cells from ow0 + lx on (lx a multiple of 4, what a
+    // bulk copy can start at); tap kw of output ow0 + j sits rx + kw + j cells into it.
+    // Set per launch from the input pointer's alignment (tc_row_window).
+    int lx, rx;
     long long xs_n, xs_c, xs[3];
     long long ys_n, ys_c, ys[3];
     int split;      // 1: 3xTF32, 0: single TF32 pass
-    uint32_t rnd_add, rnd_mask; // as in TcGeom
+    // rounding of the operands' hi part, (bits + rnd_add) & rnd_mask: to TF32
+    // (0x1000, 0xffffe000) or, in the bf16 mode, to bf16 (0x8000, 0xffff0000)
+    uint32_t rnd_add, rnd_mask;
     int th;         // output rows per column
     int rows;       // staged rows per step = th + fh - 1
     int crows;      // c * fw
@@ -123,7 +88,6 @@ struct SwGeom
     int tiles_w, tiles_h, nseg;
     long long units;
     int raw_slots, raw_slot_bytes, chunk_rows, chunks_pp;
-    int nsets;      // multi-group kernel: accumulator sets the channel groups are spread over
 };
 
 struct SwUnit
@@ -210,7 +174,7 @@ __global__ void sw_pack_filter_kernel(const float* __restrict__ w, float* __rest
         float val = 0.f;
         if (ko < g.k && part < 3)
         {
-            const float wv = w[((((size_t) ko * g.w_c_total + g.w_c_off + c) * fd + kd) * fh + kh) * fw + kw];
+            const float wv = w[((((size_t) ko * g.c + c) * fd + kd) * fh + kh) * fw + kw];
             const float hi = __uint_as_float((__float_as_uint(wv) + g.rnd_add) & g.rnd_mask);
             val = part < 2 ? hi : __uint_as_float(tf32_rna(wv - hi));
         }
@@ -281,11 +245,6 @@ __global__ void __launch_bounds__(SW_FOLD_WARPS * 32)
 }
 
 // 4 channels x 3 taps, split: A columns 0..11 hi, 12..23 lo.
-// ROUND_LO: the lo part rounded to TF32 as well (two more instructions per tap).
-// The multi-group kernel asks for it: its accumulators take 180 and more updates
-// per output, the tensor pipe's accumulation already uses most of the 1e-5 there
-// and the unrounded remainder tipped a case over the bound.
-template <bool ROUND_LO = false>
 __device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitch, uint32_t (&v)[3][8])
 {
     uint32_t xv[12];
@@ -301,8 +260,7 @@ __device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitc
         const uint32_t hi = tf32_rna(xe);
         // x - hi is exact in fp32 and below 2^-11 |x|; the tensor pipe reads the
         // upper 19 bits of it, an error below 2^-21 |x|: no rounding of its own
-        const uint32_t lo =
-            ROUND_LO ? tf32_rna(xe - __uint_as_float(hi)) : __float_as_uint(xe - __uint_as_float(hi));
+        const uint32_t lo = __float_as_uint(xe - __uint_as_float(hi));
         v[r / 8][r % 8] = hi;
         v[(12 + r) / 8][(12 + r) % 8] = lo;
     }
@@ -318,13 +276,12 @@ __device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitc
 // lane keeps its own fp32 sums, every epilogue warp leaves 32 partials in
 // `stat_part` at the end, and sw_stats_fold_kernel adds those in a fixed order
 // in fp64.
-// BLEND: beta != 0, the old output is fetched early and blended in (plain stores).
-// EPI: epilogue warps, EPI / 4 per TMEM quadrant, each retiring every
-// (EPI / 4)-th output row.  Retiring a row costs its warp a tensor-memory load
+// SW_EPI: epilogue warps, SW_EPI / 4 per TMEM quadrant, each retiring every
+// (SW_EPI / 4)-th output row.  Retiring a row costs its warp a tensor-memory load
 // and a zeroing store back to back, well over a thousand clocks with MMAs in
 // flight, and the issuers wait for the hand-back: the more rows of a plane are
 // in retirement at once, the shorter the step.
-// Warps: converters 0..11, issuers 12..14, the copy warp 15, epilogue 16..16+EPI-1
+// Warps: converters 0..11, issuers 12..14, the copy warp 15, epilogue 16..16+SW_EPI-1
 // (warp & 3 is the TMEM quadrant).
 // XISS: the last TC_GROUPS_MAX warps are second issuers.  With two A slots per
 // converter group, issuer (q, 0) takes the group's rows that land in its first slot
@@ -335,16 +292,17 @@ __device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitc
 // (statistics, blend) are held by their epilogue warps and by registers (the extra
 // warps lower the cap to 66 per thread, their epilogues then spill): they keep
 // three issuers and one slot per group.
-__host__ __device__ constexpr int sw_threads(int epi, int xiss)
+constexpr int SW_EPI = 12;
+__host__ __device__ constexpr int sw_threads(int xiss)
 {
-    return (TC_TMA_WARP + 1 + epi + (xiss ? TC_GROUPS_MAX : 0)) * 32;
+    return (TC_TMA_WARP + 1 + SW_EPI + (xiss ? TC_GROUPS_MAX : 0)) * 32;
 }
 
-template <bool C4F3, bool STATS, bool BLEND, int EPI, int XISS>
-__global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
-    sw_conv_kernel(SwGeom g, float alpha, float beta, const float* __restrict__ bimg, float* y, int* status,
+template <bool C4F3, bool STATS, int XISS>
+__global__ void __launch_bounds__(sw_threads(XISS), 1)
+    sw_conv_kernel(SwGeom g, float alpha, const float* __restrict__ bimg, float* y, int* status,
                    const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap ymap, int use_ymap,
-                   float* __restrict__ stat_part, long long* prof)
+                   float* __restrict__ stat_part)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -368,9 +326,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int fd = g.f[0], fh = g.f[1], R = g.rows, G = g.groups;
-#if DCB_SW_PROFILE
-    __shared__ volatile long long pf_issue_end[32], pf_freed[32]; // clocks: row i issued / row j handed back
-#endif
 
     if (tid == 0)
     {
@@ -403,7 +358,7 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
     }
     // k-row table: offset of the tap inside a raw chunk row, and what the row
     // carries: 0 hi part, 1 lo part, 2 zero
-    for (int r = tid; r < g.kr; r += sw_threads(EPI, XISS))
+    for (int r = tid; r < g.kr; r += sw_threads(XISS))
     {
         const int part = r / g.crows, rem = r % g.crows;
         const int c = rem / g.f[2], kw = rem % g.f[2];
@@ -411,7 +366,7 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
         const uint32_t sel = part < (g.split ? 2 : 1) ? (uint32_t) part : 2u;
         ktab[r] = sel == 2u ? ((2u << 16) | 4u) : (off | (sel << 16));
     }
-    for (int i = tid; i < g.b_bytes / 16; i += sw_threads(EPI, XISS))
+    for (int i = tid; i < g.b_bytes / 16; i += sw_threads(XISS))
         reinterpret_cast<float4*>(b_smem)[i] = reinterpret_cast<const float4*>(bimg)[i];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
@@ -440,7 +395,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
         // this group's rows of every step: a contiguous block (see the issuers)
         const int rpg = (R + G - 1) / G;
         const int my_lo = gq * rpg, my_hi = min(R, my_lo + rpg);
-        SW_PROF_DECL
         for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x)
         {
             const SwUnit t = sw_unit(g, u);
@@ -455,11 +409,9 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                     for (int i = max(lo, my_lo); i < hi && ok; ++i)
                     {
                         const int a_slot = gq + G * lap_a;
-                        SW_PROF_MARK(4)
-                        if (!have && !SW_DBG(6))
+                        if (!have)
                             ok = mbar_wait(&raw_full[cslot], cphase, abort_flag);
                         have = true;
-                        SW_PROF_MARK(0)
                         if (!ok)
                             break;
                         const float* raw = reinterpret_cast<const float*>(raw_ring + (size_t) cslot * g.raw_slot_bytes)
@@ -469,30 +421,16 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                         if (C4F3)
                         {
                             uint32_t v[3][8];
-                            if (!SW_DBG(5))
-                                // the converter is written for taps that start 3 cells into the staged row
-                                sw_convert_c4f3(raw_s + 4u * (uint32_t) (g.rx - 3), pitch, v);
-                            else
-                            {
-#pragma unroll
-                                for (int ck = 0; ck < 3; ++ck)
-#pragma unroll
-                                    for (int e = 0; e < 8; ++e)
-                                        v[ck][e] = 0u;
-                            }
-                            SW_PROF_MARK(1)
-                            if (!a_first && !SW_DBG(10))
+                            // the converter is written for taps that start 3 cells into the staged row
+                            sw_convert_c4f3(raw_s + 4u * (uint32_t) (g.rx - 3), pitch, v);
+                            if (!a_first)
                                 ok = mbar_wait(&a_empty[a_slot], a_phase, abort_flag);
-                            SW_PROF_MARK(2)
                             if (!ok)
                                 break;
                             tc_fence_after();
-                            if (!SW_DBG(0))
-                            {
 #pragma unroll
-                                for (int ck = 0; ck < 3; ++ck)
-                                    tmem_st8(a_addr + (uint32_t) (ck * 8), v[ck]);
-                            }
+                            for (int ck = 0; ck < 3; ++ck)
+                                tmem_st8(a_addr + (uint32_t) (ck * 8), v[ck]);
                         }
                         else
                         {
@@ -513,7 +451,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                         __syncwarp();
                         if (lane == 0)
                             mbar_arrive(&a_full[a_slot]);
-                        SW_PROF_MARK(3)
                         if (++lap_a == laps_a)
                         {
                             lap_a = 0;
@@ -524,7 +461,7 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                     // every converter warp releases every chunk, and only after it
                     // has seen it arrive (a group without rows in this chunk too:
                     // no warp runs further ahead of the copies than the ring is deep)
-                    if (!have && ok && !SW_DBG(6))
+                    if (!have && ok)
                         ok = mbar_wait(&raw_full[cslot], cphase, abort_flag);
                     __syncwarp();
                     if (lane == 0)
@@ -537,7 +474,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                 }
             }
         }
-        SW_PROF_FLUSH(prof)
     }
     else if (warp == TC_TMA_WARP)
     {
@@ -548,7 +484,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
         const uint32_t bytes = (uint32_t) (g.c * g.chunk_rows) * TC_RAW_W * 4u;
         uint32_t slot = 0, empty_phase = 1;
         bool first_lap = true;
-        SW_PROF_DECL
         for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x)
         {
             const SwUnit t = sw_unit(g, u);
@@ -558,12 +493,8 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                     continue;
                 for (int ch = 0; ch < g.chunks_pp; ++ch)
                 {
-                    SW_PROF_MARK(4)
-                    if (SW_DBG(6))
-                        continue;
                     if (!first_lap)
                         ok = mbar_wait(&raw_empty[slot], empty_phase, abort_flag);
-                    SW_PROF_MARK(0)
                     if (!ok)
                         break;
                     if (lane == 0)
@@ -574,7 +505,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                                     t.oh0 - g.pad[1] + ch * g.chunk_rows, d, 0, t.n, &raw_full[slot]);
                     }
                     __syncwarp();
-                    SW_PROF_MARK(1)
                     if (++slot == (uint32_t) g.raw_slots)
                     {
                         slot = 0;
@@ -584,16 +514,15 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                 }
             }
         }
-        SW_PROF_FLUSH(prof)
     }
-    else if ((warp >= TC_MMA_WARP && warp < TC_TMA_WARP) || (XISS && warp >= TC_TMA_WARP + 1 + EPI))
+    else if ((warp >= TC_MMA_WARP && warp < TC_TMA_WARP) || (XISS && warp >= TC_TMA_WARP + 1 + SW_EPI))
     {
         // ------------------------------------------------------------------
         // MMA issue: issuer (mq, mh) takes the rows converter group mq wrote into
         // its A slot mq + G * mh.  Lane i issues staged row i (its descriptors
         // depend on i only).
         // ------------------------------------------------------------------
-        const int mq = warp < TC_TMA_WARP ? warp - TC_MMA_WARP : warp - (TC_TMA_WARP + 1 + EPI);
+        const int mq = warp < TC_TMA_WARP ? warp - TC_MMA_WARP : warp - (TC_TMA_WARP + 1 + SW_EPI);
         const int mh = warp < TC_TMA_WARP ? 0 : 1;
         if (mq < G && mh < g.a_slots / G)
         {
@@ -625,7 +554,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
             const int rpg = (R + G - 1) / G;
             const int my_lo = mq * rpg, my_hi = min(R, my_lo + rpg);
             int rot = 0; // d mod fd, kept by counting
-            SW_PROF_DECL
             for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x)
             {
                 const SwUnit t = sw_unit(g, u);
@@ -658,29 +586,20 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                         }
                         // The blocks this row adds into (output rows r_lo..r_hi) must
                         // have been retired.  Each epilogue warp of a quadrant retires
-                        // its rows in ascending order, so the top EPI / 4 rows (one per
+                        // its rows in ascending order, so the top SW_EPI / 4 rows (one per
                         // warp) stand for all of them.  Only rows
                         // this row adds into may be waited for: their next retirement
                         // needs this very row, so such a barrier cannot complete again
                         // before this wait has seen it.
                         const int r_hi = min(i, g.th - 1), r_lo = max(0, i - fh + 1);
-                        SW_PROF_MARK(4)
-                        for (int r = r_hi; r >= r_lo && r > r_hi - EPI / 4 && ok && !SW_DBG(8); --r)
+                        for (int r = r_hi; r >= r_lo && r > r_hi - SW_EPI / 4 && ok; --r)
                             ok = mbar_wait_t<0>(&row_free[r], par, abort_flag);
-                        SW_PROF_MARK(0)
-#if DCB_SW_PROFILE
-                        // how long ago the last row this one needed was handed back
-                        if (step > 2)
-                            pf_acc[5] += clock64() - pf_freed[r_hi];
-#endif
                         if (!ok)
                             break;
                         if (real)
                         {
                             const uint32_t slot = (uint32_t) (mq + G * lap_a);
-                            if (!SW_DBG(11))
-                                ok = mbar_wait_t<0>(&a_full[slot], full_phase, abort_flag);
-                            SW_PROF_MARK(1)
+                            ok = mbar_wait_t<0>(&a_full[slot], full_phase, abort_flag);
                             if (!ok)
                                 break;
                             tc_fence_after();
@@ -689,30 +608,18 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                                 const uint32_t a_base = a_ring + slot * (uint32_t) g.kr;
                                 uint32_t a_addr = a_base + 8u * (uint32_t) ks_lo;
                                 uint64_t bd = bd0 + (uint64_t) (b_kstep_units * (uint32_t) ks_lo);
-                                for (int ks = ks_lo; ks < (SW_DBG(3) ? ks_lo + 1 : ks_hi); ++ks)
+                                for (int ks = ks_lo; ks < ks_hi; ++ks)
                                 {
-                                    mma_tf32_ts(my_d, a_addr, bd, SW_DBG(4) ? ((my_idesc & ~(0x3fu << 17)) | (2u << 17)) : my_idesc);
+                                    mma_tf32_ts(my_d, a_addr, bd, my_idesc);
                                     // after the k-steps over [hi | lo] the hi parts are read again
                                     a_addr = ks + 1 == g.ks1 ? a_base : a_addr + 8;
                                     bd += b_kstep_units;
                                 }
-                                if (SW_DBG(7))
-                                {
-                                    mbar_arrive(&a_empty[slot]);
-                                    mbar_arrive(&row_done[i]);
-                                }
-                                else
-                                {
-                                    mma_commit(&a_empty[slot]);
-                                    mma_commit(&row_done[i]);
-                                }
+                                mma_commit(&a_empty[slot]);
+                                mma_commit(&row_done[i]);
                                 tc_fence_before();
-#if DCB_SW_PROFILE
-                                pf_issue_end[i] = clock64();
-#endif
                             }
                             __syncwarp();
-                            SW_PROF_MARK(2)
                             if (++lap_a == laps_a)
                             {
                                 lap_a = 0;
@@ -735,22 +642,20 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                     }
                 }
             }
-            SW_PROF_FLUSH(prof)
         }
     }
-    else if (warp >= (TC_TMA_WARP + 1) && warp < TC_TMA_WARP + 1 + EPI)
+    else if (warp >= (TC_TMA_WARP + 1) && warp < TC_TMA_WARP + 1 + SW_EPI)
     {
         // ------------------------------------------------------------------
         // epilogue: after step d retire output plane d + pad - (fd-1)
         // ------------------------------------------------------------------
         const int quad = warp & 3;
         const int ew = warp - (TC_TMA_WARP + 1); // index among the epilogue warps
-        const int half = ew >> 2, nhalf = EPI / 4;
+        const int half = ew >> 2, nhalf = SW_EPI / 4;
         const uint32_t lane_addr = tmem_base + ((uint32_t) (quad * 32) << 16);
         const int nk = g.k;
         const size_t ysc = (size_t) g.ys_c;
-        // bulk stores overwrite: the blend with the old output takes the plain path
-        const bool bulk = !BLEND && use_ymap != 0;
+        const bool bulk = use_ymap != 0;
         float* stage = stage_base + ew * (2 * SW_NBK * 32);
         uint32_t nstored = 0;
         uint64_t s1[STATS ? SW_NBK / 2 : 1], s2[STATS ? SW_NBK / 2 : 1]; // packed pairs of filters
@@ -769,7 +674,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
             for (int j = half; j < g.th; j += nhalf)
                 mbar_arrive(&row_free[j]);
         uint32_t step = 0;
-        SW_PROF_DECL
         for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x)
         {
             const SwUnit t = sw_unit(g, u);
@@ -784,30 +688,10 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                 {
                     const int oh = t.oh0 + j;
                     const bool wr = store && oh < g.out[1];
-                    // a blend with the old output: fetch it while the row is still in the works
-                    float old[BLEND ? SW_NBK : 1];
                     float* const yrow =
                         y + (size_t) t.n * g.ys_n + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1] + ow;
-                    if (BLEND && wr && ow < g.out[2])
-                    {
-#pragma unroll
-                        for (int k = 0; k < (BLEND ? SW_NBK : 1); ++k)
-                            if (k < nk)
-                                old[k] = yrow[(size_t) k * ysc];
-                    }
-                    SW_PROF_MARK(4)
-                    for (int i = j; i < j + fh && ok && !SW_DBG(9); ++i)
+                    for (int i = j; i < j + fh && ok; ++i)
                         ok = mbar_wait(&row_done[i], par, abort_flag);
-                    SW_PROF_MARK(0)
-#if DCB_SW_PROFILE
-                    if (step > 2 && sw_real(g, t, d))
-                    {
-                        long long last = 0;
-                        for (int i = j; i < j + fh; ++i)
-                            last = pf_issue_end[i] > last ? pf_issue_end[i] : last;
-                        pf_acc[5] += clock64() - last; // issue of the last row needed -> seen complete
-                    }
-#endif
                     if (!ok)
                         break;
                     tc_fence_after();
@@ -818,7 +702,6 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                         tmem_ld16(addr, v);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     }
-                    SW_PROF_MARK(1)
                     // hand the blocks back first: the issuers wait for that, nobody for the store
                     tmem_st16_zero(addr);
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -826,18 +709,13 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                     __syncwarp();
                     if (lane == 0)
                     {
-#if DCB_SW_PROFILE
-                        pf_freed[j] = clock64();
-#endif
                         mbar_arrive(&row_free[j]);
                     }
-                    SW_PROF_MARK(2)
                     if (!wr)
                         continue;
                     if (STATS && ow < g.out[2])
                     {
-                        // beta is zero whenever statistics are asked for
-#pragma unroll
+                #pragma unroll
                         // of the raw accumulators: alpha goes on at the end
                         for (int k = 0; k < (STATS ? SW_NBK / 2 : 1); ++k)
                         {
@@ -888,21 +766,17 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                         }
                         ++nstored;
-                        SW_PROF_MARK(3)
                     }
                     else if (ow < g.out[2])
                     {
 #pragma unroll
                         for (int k = 0; k < SW_NBK; ++k)
                             if (k < nk)
-                                yrow[(size_t) k * ysc] =
-                                    BLEND ? alpha * __uint_as_float(v[k]) + beta * old[BLEND ? k : 0]
-                                          : alpha * __uint_as_float(v[k]);
+                                yrow[(size_t) k * ysc] = alpha * __uint_as_float(v[k]);
                     }
                 }
             }
         }
-        SW_PROF_FLUSH(prof)
         // the staged rows must have left shared memory before the CTA does
         if (bulk && lane == 0)
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -932,7 +806,7 @@ __global__ void __launch_bounds__(sw_threads(EPI, XISS), 1)
                 if (lane == SW_NBK + k)
                     mine = alpha * alpha * b;
             }
-            stat_part[((size_t) blockIdx.x * EPI + ew) * 32 + lane] = mine;
+            stat_part[((size_t) blockIdx.x * SW_EPI + ew) * 32 + lane] = mine;
         }
     }
 

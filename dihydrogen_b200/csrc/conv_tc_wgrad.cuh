@@ -32,7 +32,8 @@
 // All waits are bounded.
 #pragma once
 
-#include "conv_tc_kernel.cuh"
+#include "conv_simt.cuh"
+#include "conv_tc_common.cuh"
 
 namespace dcb
 {

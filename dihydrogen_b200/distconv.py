@@ -1110,9 +1110,8 @@ class Convolution:
         return _abi.lib().dcb_conv_plan_kernel_kind(plan, which)
 
     def kernel_variant(self, which: int) -> int:
-        """dcb_conv_plan_kernel_variant: 0 fp32 CUDA-core, 1 / 2 tcgen05 row
-        kernel (bulk-copy fed / register fed), 3 sweep, 4 multi-group sweep,
-        5 tcgen05 backward filter."""
+        """dcb_conv_plan_kernel_variant: 0 fp32 CUDA-core; tcgen05: 3 and 4 forward
+        and backward data (4: two accumulator sets), 5 backward filter."""
         return _abi.lib().dcb_conv_plan_kernel_variant(self._plan_of(which), which)
 
     # -- halo --

@@ -559,3 +559,32 @@ def test_backward_data_full_shard_16_channels_against_fp64():
             got = dx[0, :, o0[0]:o0[0] + B, o0[1]:o0[1] + B, o0[2]:o0[2] + B].double()
             worst = max(worst, ((got - ref).abs() / (ref.abs() + ref.pow(2).mean().sqrt())).max().item())
         assert worst <= TOL, (rep, worst)
+
+
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, stride: edges of the shift kernel's tiles and tables
+    (1, 8, 8, (5, 6, 9), (3, 3, 3), 1),        # six sub-columns side by side in the 128 lanes
+    (1, 8, 8, (5, 6, 127), (3, 3, 3), 1),      # one cell short of a tile
+    (1, 8, 8, (5, 6, 129), (3, 3, 3), 1),      # one cell over: two tiles
+    (3, 9, 17, (4, 5, 31), (3, 3, 3), 1),      # a cell of one channel, 17 filters in 20 columns
+    (1, 32, 32, (9, 34, 40), (3, 3, 3), 1),    # filter images streamed per plane, channel groups
+    (2, 7, 33, (6, 7, 65), (3, 3, 3), 2),      # stride 2, filters in groups, odd extents
+    (1, 31, 31, (13, 131), (5, 5), 2),         # 2-D 5 x 5 stride 2
+    (2, 1, 4, (40, 17), (3, 3), 1),            # one channel, 2-D
+    (1, 6, 5, (4, 4, 4), (3, 3, 3), 2),        # smallest
+])
+def test_shift_kernel_tile_and_table_edges(geom):
+    N, C, K, sp, f, s = geom
+    rng = np.random.default_rng(sum(sp) + C)
+    nsd, pads, strides = len(sp), [(e - 1) // 2 for e in f], [s] * len(sp)
+    x = rng.normal(0, 1, (N, C, *sp)).astype(np.float32)
+    w = rng.normal(0, np.sqrt(2.0 / (C * np.prod(f))), (K, C, *f)).astype(np.float32)
+    dy = rng.normal(0, 1, (N, K, *[O.conv_out_extent(i, ff, p, s, 1) for i, ff, p in zip(sp, f, pads)])).astype(np.float32)
+    y0 = rng.normal(size=dy.shape).astype(np.float32)
+    dx0 = rng.normal(size=x.shape).astype(np.float32)
+    y, dx, _ = run_all(x, w, dy, pads, strides, [1] * nsd, _abi.MATH_FP32, alpha=0.5, beta=-1.0, y0=y0, dx0=dx0,
+                       dw0=np.zeros_like(w))
+    emu.assert_close(y, 0.5 * O.conv_fwd(x, w, pads, strides) - y0, TOL, "y")
+    dx_ref = np.zeros_like(x)
+    O.conv_bwd_data(w, dy, dx_ref, pads, strides)
+    emu.assert_close(dx, 0.5 * dx_ref - dx0, TOL, "dx")
