@@ -187,5 +187,13 @@ def check(status: int, where: str):
         raise DcbError(status, where, lib().dcb_last_error().decode())
 
 
+_FUNCTIONS = {}
+
+
 def call(name: str, *args):
-    check(getattr(lib(), name)(*args), name)
+    fn = _FUNCTIONS.get(name)
+    if fn is None:
+        fn = _FUNCTIONS[name] = getattr(lib(), name)
+    status = fn(*args)
+    if status != OK:
+        check(status, name)

@@ -23,6 +23,7 @@ kernel on the path is launched by the library.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 from typing import Callable, List, Optional, Sequence
 
@@ -36,13 +37,30 @@ LHS, RHS = 0, 1
 SIDES = (LHS, RHS)
 
 
-def _stream_ptr(stream=None) -> ctypes.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+def _stream_ptr(stream=None) -> int:
+    if stream is not None:
+        return stream.cuda_stream
+    # the raw handle of torch's current stream: making a Stream object of it for
+    # every launch cost 10 us a call, half the host time of a small layer
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _ptr(v) -> ctypes.c_void_p:
-    return ctypes.c_void_p(int(v))
+def _ptr(v) -> int:
+    return int(v)
+
+
+class _Geometry:
+    """What a Tensor's methods compute over and over, for one state of its
+    local shape, overlap and pitch."""
+
+    def __init__(self, t: "Tensor"):
+        self.local, self.overlap, self.pitch = list(t.local_shape), list(t.dist.overlap), t.pitch
+        self.size = math.prod(self.local)
+        self.strides = t.get_strides()
+        self.base = 4 * t.get_local_offset([0] * t.nd)
+        self.split_root = t.is_split_root()
+        self.descs = {}    # widths -> NdDesc
+        self.offsets = {}  # widths -> byte offset of the window
 
 
 def _zero_on(stream, *tensors):
@@ -239,6 +257,7 @@ class Tensor:
         real_w = self.local_shape[0] + 2 * self.dist.overlap[0]
         self.lead = (-self.dist.overlap[0]) % self.pitch_align
         self.pitch = -(-(self.lead + real_w) // self.pitch_align) * self.pitch_align
+        self._geometry: Optional[_Geometry] = None
         self.buffer: Optional[torch.Tensor] = None
         self._storage: Optional[torch.Tensor] = None
 
@@ -279,10 +298,7 @@ class Tensor:
         return [l + 2 * o for l, o in zip(self.local_shape, self.dist.overlap)]
 
     def get_local_size(self):
-        n = 1
-        for v in self.local_shape:
-            n *= v
-        return n
+        return math.prod(self.local_shape)
 
     def get_size(self):
         n = 1
@@ -316,6 +332,21 @@ class Tensor:
             idx[dim] = j * per
             off += self._local_of(idx)[dim]
         return off
+
+    def _geo(self) -> _Geometry:
+        g = self._geometry
+        if g is None or g.local != self.local_shape or g.overlap != self.dist.overlap or g.pitch != self.pitch:
+            g = self._geometry = _Geometry(self)
+        return g
+
+    def _nd(self, lo=None, hi=None):
+        """nd_desc() by reference, made once per pair of widths."""
+        descs = self._geo().descs
+        key = (tuple(lo), tuple(hi)) if lo is not None else None
+        d = descs.get(key)
+        if d is None:
+            d = descs[key] = self.nd_desc(lo, hi)
+        return ctypes.byref(d)
 
     # -- memory --
     def np_real_shape(self):
@@ -377,7 +408,7 @@ class Tensor:
         return sum((i + (0 if idx_include_halo else o)) * s for i, o, s in zip(idx, ov, st))
 
     def get_base_ptr(self) -> int:
-        return self.get_buffer() + 4 * self.get_local_offset([0] * self.nd)
+        return self.buffer.data_ptr() + self._geo().base
 
     def owned(self) -> torch.Tensor:
         sl = tuple(slice(o, o + l) for o, l in reversed(list(zip(self.dist.overlap, self.local_shape))))
@@ -426,10 +457,14 @@ class Tensor:
         return d
 
     def nd_ptr(self, widths_lo=None) -> int:
-        nsd = self.nd - 2
-        lo = list(widths_lo or [0] * nsd) + [0, 0]
-        idx = [self.dist.overlap[i] - lo[i] for i in range(self.nd)]
-        return self.get_buffer() + 4 * self.get_local_offset(idx, True)
+        offsets = self._geo().offsets
+        key = tuple(widths_lo) if widths_lo else None
+        off = offsets.get(key)
+        if off is None:
+            lo = list(widths_lo or [0] * (self.nd - 2)) + [0, 0]
+            idx = [self.dist.overlap[i] - lo[i] for i in range(self.nd)]
+            off = offsets[key] = 4 * self.get_local_offset(idx, True)
+        return self.buffer.data_ptr() + off
 
     def full_nd_desc(self) -> NdDesc:
         ov = self.dist.overlap[: self.nd - 2]
@@ -647,6 +682,8 @@ class HaloExchange:
 
     @staticmethod
     def _flags(is_reverse=False, skip_unpack=False, op="ID", clear_boundary=False):
+        if not (is_reverse or skip_unpack) and op == "ID":
+            return _abi.HALO_CLEAR_BOUNDARY | _abi.HALO_OPS["ID"] if clear_boundary else _abi.HALO_OPS["ID"]
         return (_abi.HALO_REVERSE if is_reverse else 0) | (_abi.HALO_SKIP_UNPACK if skip_unpack else 0) | \
             (_abi.HALO_CLEAR_BOUNDARY if clear_boundary else 0) | _abi.HALO_OPS[op]
 
@@ -1163,7 +1200,7 @@ class Convolution:
             self.halo_xch_input.exchange(s, clear_boundary=True)
             if prof:
                 torch.cuda.nvtx.range_pop()
-        if statistics is not None and float(beta) == 0.0 and input.is_split_root():
+        if statistics is not None and float(beta) == 0.0 and input._geo().split_root:
             st = _abi.lib().dcb_conv_fwd_stats(self._plan_fwd, float(alpha), _ptr(input.nd_ptr(self._x_lo)),
                                                _ptr(filter.data_ptr()), _ptr(output.get_base_ptr()),
                                                _ptr(statistics[0].data_ptr()), _ptr(statistics[1].data_ptr()),
@@ -1196,7 +1233,7 @@ class Convolution:
         halo-extended tensor)."""
         s = self.be.stream
         if (input.get_local_size() == 0 or d_output.get_local_size() == 0 or d_filter.numel() == 0
-                or not input.is_split_root()):
+                or not input._geo().split_root):
             _zero_on(s, d_filter)
         else:
             call("dcb_conv_bwd_filter", self._plan_wgrad, float(alpha), _ptr(input.nd_ptr(self._x_lo)),
@@ -1212,8 +1249,8 @@ class Convolution:
         """convolution.hpp:641-659."""
         if output.get_local_size() == 0:
             return 0
-        yd = output.nd_desc()
-        call("dcb_bias_fwd", float(alpha), _ptr(bias.data_ptr()), float(beta), ctypes.byref(yd),
+        yd = output._nd()
+        call("dcb_bias_fwd", float(alpha), _ptr(bias.data_ptr()), float(beta), yd,
              _ptr(output.get_base_ptr()), _stream_ptr(self.be.stream))
         return 0
 
@@ -1222,8 +1259,8 @@ class Convolution:
         if d_output.get_local_size() == 0:
             _zero_on(self.be.stream, bias_gradient)
         else:
-            yd = d_output.nd_desc()
-            call("dcb_bias_bwd", float(alpha), ctypes.byref(yd), _ptr(d_output.get_base_ptr()), float(beta),
+            yd = d_output._nd()
+            call("dcb_bias_bwd", float(alpha), yd, _ptr(d_output.get_base_ptr()), float(beta),
                  _ptr(bias_gradient.data_ptr()), _stream_ptr(self.be.stream))
         if reduce:
             self.allreduce_gradients(bias_gradient)
@@ -1253,6 +1290,7 @@ class BatchNormalization:
         self.be, self.num_dims = backend, num_dims
         self.decay, self.epsilon, self.global_stats = float(decay), float(epsilon), bool(global_stats)
         self._plans = {}
+        self._last = (None, None)
 
     def __del__(self):
         try:
@@ -1262,12 +1300,16 @@ class BatchNormalization:
             pass
 
     def _plan(self, t: Tensor):
+        geo = t._geo()
+        if geo is self._last[0]:
+            return self._last[1]
         key = (tuple(t.local_shape), tuple(t.dist.overlap))
         if key not in self._plans:
             xd = t.nd_desc()
             p = ctypes.c_void_p()
             call("dcb_bn_plan_create", ctypes.byref(xd), ctypes.byref(p))
             self._plans[key] = p
+        self._last = (geo, self._plans[key])
         return self._plans[key]
 
     # forward
@@ -1275,7 +1317,7 @@ class BatchNormalization:
         if not is_training:
             return 0
         s = self.be.stream
-        if input.get_local_size() == 0 or not input.is_split_root():
+        if input.get_local_size() == 0 or not input._geo().split_root:
             _zero_on(s, mean, var)
             return 0
         call("dcb_bn_stats", self._plan(input), _ptr(input.get_base_ptr()), _ptr(mean.data_ptr()),
@@ -1307,10 +1349,7 @@ class BatchNormalization:
         C = input.local_shape[-2]
         if is_training:
             stat_shape = input.shape if self.global_stats else input.local_shape
-            nps = 1
-            for v in stat_shape:
-                nps *= v
-            nps //= stat_shape[-2]
+            nps = math.prod(stat_shape) // stat_shape[-2]
             call("dcb_bn_finalize", C, nps, self.decay, _ptr(mean.data_ptr()), _ptr(var.data_ptr()),
                  _ptr(running_mean.data_ptr()), _ptr(running_var.data_ptr()), _stream_ptr(s))
             m, v = mean, var
@@ -1318,14 +1357,14 @@ class BatchNormalization:
             m, v = running_mean, running_var
         if input.get_local_size() == 0:
             return 0
-        xd, yd = input.nd_desc(), output.nd_desc()
+        xd, yd = input._nd(), output._nd()
         if leaky_relu_slope is not None:
-            call("dcb_bn_apply_leaky_relu", ctypes.byref(xd), _ptr(input.get_base_ptr()), _ptr(m.data_ptr()),
+            call("dcb_bn_apply_leaky_relu", xd, _ptr(input.get_base_ptr()), _ptr(m.data_ptr()),
                  _ptr(v.data_ptr()), _ptr(scale.data_ptr()), _ptr(bias.data_ptr()), self.epsilon,
-                 float(leaky_relu_slope), ctypes.byref(yd), _ptr(output.get_base_ptr()), _stream_ptr(s))
+                 float(leaky_relu_slope), yd, _ptr(output.get_base_ptr()), _stream_ptr(s))
             return 0
-        call("dcb_bn_apply", ctypes.byref(xd), _ptr(input.get_base_ptr()), _ptr(m.data_ptr()), _ptr(v.data_ptr()),
-             _ptr(scale.data_ptr()), _ptr(bias.data_ptr()), self.epsilon, ctypes.byref(yd),
+        call("dcb_bn_apply", xd, _ptr(input.get_base_ptr()), _ptr(m.data_ptr()), _ptr(v.data_ptr()),
+             _ptr(scale.data_ptr()), _ptr(bias.data_ptr()), self.epsilon, yd,
              _ptr(output.get_base_ptr()), _stream_ptr(s))
         return 0
 
@@ -1343,11 +1382,10 @@ class BatchNormalization:
     def backward_stage1(self, input: Tensor, d_output: Tensor, mean, var, scale, scale_gradient, bias_gradient,
                         mean_gradient, var_gradient):
         s = self.be.stream
-        if input.get_local_size() == 0 or not input.is_split_root():
+        if input.get_local_size() == 0 or not input._geo().split_root:
             _zero_on(s, scale_gradient, bias_gradient, mean_gradient, var_gradient)
             return 0
-        dyd = d_output.nd_desc()
-        call("dcb_bn_bwd_reduce", self._plan(input), _ptr(input.get_base_ptr()), ctypes.byref(dyd),
+        call("dcb_bn_bwd_reduce", self._plan(input), _ptr(input.get_base_ptr()), d_output._nd(),
              _ptr(d_output.get_base_ptr()), _ptr(mean.data_ptr()), _ptr(var.data_ptr()), _ptr(scale.data_ptr()),
              self.epsilon, _ptr(scale_gradient.data_ptr()), _ptr(bias_gradient.data_ptr()),
              _ptr(mean_gradient.data_ptr()), _ptr(var_gradient.data_ptr()), _stream_ptr(s))
@@ -1370,14 +1408,11 @@ class BatchNormalization:
         if input.get_local_size() == 0:
             return 0
         stat_shape = input.shape if self.global_stats else input.local_shape
-        nps = 1
-        for v in stat_shape:
-            nps *= v
-        nps //= stat_shape[-2]
-        xd, dyd, dxd = input.nd_desc(), d_output.nd_desc(), d_input.nd_desc()
-        call("dcb_bn_bwd_apply", ctypes.byref(xd), _ptr(input.get_base_ptr()), ctypes.byref(dyd),
+        nps = math.prod(stat_shape) // stat_shape[-2]
+        xd, dyd, dxd = input._nd(), d_output._nd(), d_input._nd()
+        call("dcb_bn_bwd_apply", xd, _ptr(input.get_base_ptr()), dyd,
              _ptr(d_output.get_base_ptr()), _ptr(mean.data_ptr()), _ptr(var.data_ptr()), _ptr(scale.data_ptr()),
-             _ptr(mean_gradient.data_ptr()), _ptr(var_gradient.data_ptr()), self.epsilon, nps, ctypes.byref(dxd),
+             _ptr(mean_gradient.data_ptr()), _ptr(var_gradient.data_ptr()), self.epsilon, nps, dxd,
              _ptr(d_input.get_base_ptr()), _stream_ptr(self.be.stream))
         return 0
 
@@ -1462,8 +1497,8 @@ class Pooling:
             self.halo_xch_input.exchange(s)
         if output.get_local_size() == 0:
             return 0
-        xd, yd = input.nd_desc(self._lo, self._hi), output.nd_desc()
-        call("dcb_pool_fwd", ctypes.byref(self._pd), ctypes.byref(xd), ctypes.byref(yd), float(alpha),
+        xd, yd = input._nd(self._lo, self._hi), output._nd()
+        call("dcb_pool_fwd", ctypes.byref(self._pd), xd, yd, float(alpha),
              _ptr(input.nd_ptr(self._lo)), float(beta), _ptr(output.get_base_ptr()), _stream_ptr(s))
         return 0
 
@@ -1478,14 +1513,14 @@ class Pooling:
         for dim in self._halo_dims(d_input):
             d_input.clear_halo(dim, s)
         if d_output.get_local_size() > 0:
-            xd, yd = input.nd_desc(self._lo, self._hi), output.nd_desc()
-            dxd, dyd = d_input.nd_desc(self._lo, self._hi), d_output.nd_desc()
-            assert list(xd.strides) == list(dxd.strides) and list(yd.strides) == list(dyd.strides)
+            xd, yd = input._nd(self._lo, self._hi), output._nd()
+            assert input._geo().strides[:-2] == d_input._geo().strides[:-2]
+            assert output._geo().strides[:-2] == d_output._geo().strides[:-2]
             if self._ws is None:
-                need = _abi.lib().dcb_pool_bwd_workspace_bytes(ctypes.byref(self._pd), ctypes.byref(xd),
-                                                               ctypes.byref(yd))
+                need = _abi.lib().dcb_pool_bwd_workspace_bytes(ctypes.byref(self._pd), xd,
+                                                               yd)
                 self._ws = torch.empty(max(need, 0), dtype=torch.uint8, device=d_input.buffer.device)
-            call("dcb_pool_bwd", ctypes.byref(self._pd), ctypes.byref(xd), ctypes.byref(yd), float(alpha),
+            call("dcb_pool_bwd", ctypes.byref(self._pd), xd, yd, float(alpha),
                  _ptr(output.get_base_ptr()), _ptr(d_output.get_base_ptr()), _ptr(input.nd_ptr(self._lo)),
                  float(beta), _ptr(d_input.nd_ptr(self._lo)),
                  _ptr(self._ws.data_ptr() if self._ws.numel() else 0), self._ws.numel(), _stream_ptr(s))
@@ -1506,16 +1541,16 @@ class LeakyReLU:
     def forward(self, input: Tensor, negative_slope: float, output: Tensor):
         if input.get_local_size() == 0:
             return 0
-        xd, yd = input.nd_desc(), output.nd_desc()
-        call("dcb_leaky_relu_fwd", ctypes.byref(xd), _ptr(input.get_base_ptr()), float(negative_slope),
-             ctypes.byref(yd), _ptr(output.get_base_ptr()), _stream_ptr(self.be.stream))
+        xd, yd = input._nd(), output._nd()
+        call("dcb_leaky_relu_fwd", xd, _ptr(input.get_base_ptr()), float(negative_slope),
+             yd, _ptr(output.get_base_ptr()), _stream_ptr(self.be.stream))
         return 0
 
     def backward(self, input: Tensor, d_output: Tensor, negative_slope: float, d_input: Tensor):
         if input.get_local_size() == 0:
             return 0
-        xd, dyd, dxd = input.nd_desc(), d_output.nd_desc(), d_input.nd_desc()
-        call("dcb_leaky_relu_bwd", ctypes.byref(xd), _ptr(input.get_base_ptr()), ctypes.byref(dyd),
-             _ptr(d_output.get_base_ptr()), float(negative_slope), ctypes.byref(dxd), _ptr(d_input.get_base_ptr()),
+        xd, dyd, dxd = input._nd(), d_output._nd(), d_input._nd()
+        call("dcb_leaky_relu_bwd", xd, _ptr(input.get_base_ptr()), dyd,
+             _ptr(d_output.get_base_ptr()), float(negative_slope), dxd, _ptr(d_input.get_base_ptr()),
              _stream_ptr(self.be.stream))
         return 0
