@@ -13,6 +13,7 @@ namespace
 {
 
 constexpr int SH_SMEM_MAX = 226 * 1024;
+constexpr int SH_FOREIGN = -2; // column of a block that a row does not add to
 
 // Chains of truncating accumulator updates longer than this go to two
 // accumulator sets.  The error of a chain of n updates is about n / 2 truncations
@@ -103,7 +104,13 @@ int align_up(int v, int a)
 
 std::vector<int> ShBuilder::row_code(const ShGeom& g, int phase, int i, int ew) const
 {
-    std::vector<int> code((size_t) TC_TMEM_COLS, -1);
+    std::vector<int> code((size_t) TC_TMEM_COLS, SH_FOREIGN);
+    for (int c = 0; c < (int) TC_TMEM_COLS; ++c)
+    {
+        const int in_row = c % g.rowst;
+        if (c >= g.set_off || in_row >= g.ns * g.blk)
+            code[(size_t) c] = -1; // nobody's
+    }
     for (int m = 0;; ++m)
     {
         const int ts = phase % g.st_s + m * g.st_s;
@@ -115,6 +122,8 @@ std::vector<int> ShBuilder::row_code(const ShGeom& g, int phase, int i, int ew) 
             const int tr = i - j * g.st_r;
             if (tr < 0 || tr >= g.fr)
                 continue;
+            for (int c = 0; c < g.blk; ++c)
+                code[(size_t) (ew * g.woff + j * g.rowst + slot * g.blk + c)] = -1; // open: may be covered with zeros
             for (int es = 0; es < g.e_s; ++es)
                 for (int er = 0; er < g.e_r; ++er)
                 {
@@ -132,17 +141,23 @@ std::vector<int> ShBuilder::row_code(const ShGeom& g, int phase, int i, int ew) 
 }
 
 // Column ranges (multiples of 16, at most 256 wide) that cover the used columns
-// at the least cost; columns nobody uses may be covered with zeros.
+// at the least cost.  Unused columns of open blocks may be covered with zeros,
+// blocks that the row does not add to may not.
 std::vector<std::pair<int, int>> ShBuilder::ranges(const std::vector<int>& code) const
 {
-    std::vector<int> u;
+    std::vector<int> u, foreign((size_t) code.size() / 16 + 1, 0); // used 16-column pieces; foreign ones before a piece
     for (int b = 0; b < (int) code.size() / 16; ++b)
+    {
+        bool used = false, other = false;
         for (int c = 0; c < 16; ++c)
-            if (code[(size_t) (b * 16 + c)] >= 0)
-            {
-                u.push_back(b);
-                break;
-            }
+        {
+            used = used || code[(size_t) (b * 16 + c)] >= 0;
+            other = other || code[(size_t) (b * 16 + c)] == SH_FOREIGN;
+        }
+        if (used)
+            u.push_back(b);
+        foreign[(size_t) b + 1] = foreign[(size_t) b] + (other ? 1 : 0);
+    }
     const int m = (int) u.size();
     std::vector<double> best((size_t) m + 1, 1e30);
     std::vector<int> from((size_t) m + 1, 0);
@@ -151,7 +166,7 @@ std::vector<std::pair<int, int>> ShBuilder::ranges(const std::vector<int>& code)
         for (int l = k - 1; l >= 0; --l)
         {
             const int n = 16 * (u[(size_t) k - 1] - u[(size_t) l] + 1);
-            if (n > 256)
+            if (n > 256 || foreign[(size_t) u[(size_t) k - 1] + 1] != foreign[(size_t) u[(size_t) l]])
                 break;
             const double c = best[(size_t) l] + sh_mma_cost(n);
             if (c < best[(size_t) k])
@@ -164,7 +179,7 @@ std::vector<std::pair<int, int>> ShBuilder::ranges(const std::vector<int>& code)
         r.push_back({a * 16, 16 * (u[(size_t) k - 1] - a + 1)});
     }
     std::reverse(r.begin(), r.end());
-    return r;
+    return best[(size_t) m] < 1e30 ? r : std::vector<std::pair<int, int>>();
 }
 
 // The k-steps of a staged row, per cell parity of the output row (ew) and per
@@ -301,6 +316,12 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     g.nph = g.ns * g.st_s;
     g.nsets = t.nsets;
     g.blk = g.nb * g.e_s * g.e_r;
+    // Instructions update whole multiples of 16 columns, also with zeros, and an
+    // update with zeros of a block that the epilogue is draining would bring its old
+    // values back.  Rows of blocks start on such multiples; the plane slots of a row
+    // have to as well, unless every staged plane adds to all of them.
+    if (m_flat || m_s.st > 1)
+        g.blk = align_up(g.blk, 16);
     g.rowst = align_up(g.ns * g.blk, 16);
     g.woff = g.th * g.rowst;
     g.set_off = g.e_w * g.woff;
@@ -388,7 +409,10 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
             for (int ew = 0; ew < g.e_w; ++ew)
             {
                 const std::vector<int> code = row_code(g, ph, i, ew);
-                for (const auto& r : ranges(code))
+                const auto rs = ranges(code);
+                if (rs.empty() && *std::max_element(code.begin(), code.end()) >= 0)
+                    return false; // a used piece that another block shares
+                for (const auto& r : rs)
                     all.push_back({ph, i, ew, r.first, r.second,
                                    std::vector<int>(code.begin() + r.first, code.begin() + r.first + r.second), -1, 0});
             }

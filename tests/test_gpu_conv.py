@@ -572,6 +572,9 @@ def test_backward_data_full_shard_16_channels_against_fp64():
     (1, 31, 31, (13, 131), (5, 5), 2),         # 2-D 5 x 5 stride 2
     (2, 1, 4, (40, 17), (3, 3), 1),            # one channel, 2-D
     (1, 6, 5, (4, 4, 4), (3, 3, 3), 2),        # smallest
+    (1, 1, 4, (900, 150), (3, 3), 1),          # few filters: blocks narrower than an instruction's 16 columns, many planes
+    (1, 8, 4, (40, 60, 132), (3, 3, 3), 2),    # the same where a plane adds to some of the live slots only
+    (1, 5, 24, (90, 84), (5, 5), 2),           # blocks of one and a half times 16 columns
 ])
 def test_shift_kernel_tile_and_table_edges(geom):
     N, C, K, sp, f, s = geom
