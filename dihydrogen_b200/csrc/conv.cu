@@ -137,9 +137,13 @@ int32_t dcb_conv_plan_create(const dcb_conv_desc* cd, const dcb_nd_desc* xd,
     }
     const size_t fbytes =
         (size_t) g.k * g.c * g.f[0] * g.f[1] * g.f[2] * sizeof(float);
-    p->workspace_bytes = simt_conv_bwd_filter_workspace(g);
-    bool ok = cudaMalloc(&p->workspace, p->workspace_bytes ? p->workspace_bytes : 16)
-              == cudaSuccess;
+    bool ok = true;
+    if (p->kind[2] == 0)
+    {
+        p->workspace_bytes = simt_conv_bwd_filter_workspace(g);
+        ok = cudaMalloc(&p->workspace, p->workspace_bytes ? p->workspace_bytes : 16)
+             == cudaSuccess;
+    }
     if (p->bwd_data_as_fwd && p->kind[1] == 0)
         ok = ok && cudaMalloc(&p->wflip, fbytes ? fbytes : 16) == cudaSuccess;
     if (p->kind[0] || p->kind[1] || p->kind[2])
@@ -282,14 +286,11 @@ int32_t dcb_conv_bwd_filter(dcb_conv_plan* p, double alpha, const void* x,
 {
     DCB_REQUIRE(p && x && dy && dw, "null argument");
     if (p->kind[2] == 1)
-    {
-        const int32_t st = tc_conv_bwd_filter(
-            p->tc, (float) alpha, static_cast<const float*>(x),
-            static_cast<const float*>(dy), (float) beta,
-            static_cast<float*>(dw), p->status, as_stream(stream));
-        if (st != DCB_UNSUPPORTED) // unaligned base pointers take the kernel below
-            return st;
-    }
+        return tc_conv_bwd_filter(p->tc, (float) alpha,
+                                  static_cast<const float*>(x),
+                                  static_cast<const float*>(dy), (float) beta,
+                                  static_cast<float*>(dw), p->status,
+                                  as_stream(stream));
     return simt_conv_bwd_filter(p->g, (float) alpha,
                                 static_cast<const float*>(x),
                                 static_cast<const float*>(dy), (float) beta,

@@ -1,9 +1,10 @@
 // tcgen05 sweep kernel (forward, few input channels) and backward filter, host
 // side: geometry, tensor maps, launches.
 #include "conv_tc.cuh"
+#include "conv_plan_cache.cuh"
 #include "conv_tc_encode.cuh"
 #include "conv_tc_sweep.cuh"
-#include "conv_tc_wgrad.cuh"
+#include "conv_tc_wgrad_api.cuh"
 
 #include <cstdlib>
 #include <vector>
@@ -149,76 +150,239 @@ bool sw_geom(const ConvGeom& cg, int math_mode, SwGeom* out)
     return true;
 }
 
-size_t wg_smem_need(const WgGeom& g)
+// clocks of one instruction of width n (measured, shared-memory operands)
+double wg_mma_cost(int n)
 {
-    const size_t unit = (size_t) (g.xbuf_bytes + g.dybuf_bytes + 127) / 128 * 128;
-    return 2 * unit + (size_t) WG_A_SLOTS * WG_B_FLOATS * 4 + (2 * WG_A_SLOTS + 8) * 8 + 64 + 1024;
+    const double a = n / 2.0, b = 32.0 + n / 4.0;
+    return a > b ? (a > 45.5 ? a : 45.5) : (b > 45.5 ? b : 45.5);
+}
+
+// One way to deal out the work; false when it does not fit.
+bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int kg, int B, int PW, double* cost)
+{
+    WgGeom& g = *out;
+    const int sh = cg.stride[1], fh = cg.f[1];
+    auto groups = [](int total, int per) { return (total + per - 1) / per; };
+    g.cg = cgp, g.kwg = kwg, g.kdg = kdg, g.kg = kg;
+    g.ncg = groups(cg.c, cgp), g.nkw = groups(cg.f[2], kwg), g.nkd = groups(cg.f[0], kdg), g.nkg = groups(cg.k, kg);
+    g.roles = g.ncg * g.nkd * g.nkg;
+    g.kgp = (kg + 7) / 8 * 8;
+    g.n8 = 2 * g.kgp;
+    g.r8 = (2 * cgp * kwg + 7) / 8 * 8;
+    if (g.r8 > 128 || g.n8 > 256 || g.roles > 4096)
+        return false;
+    g.B = B;
+    g.X = (B - 1) * sh + fh;
+    if (g.X > 255)
+        return false;
+    g.A = 128 / g.r8 < g.X ? 128 / g.r8 : g.X;
+    g.PW = PW;
+    g.Q = PW / 4;
+    // tiles and accumulator blocks of one kd plane
+    auto b_range = [&](int a0, int* lo, int* hi) {
+        const int num = a0 - (fh - 1);
+        *lo = num <= 0 ? 0 : (num + sh - 1) / sh;
+        *hi = (a0 + g.A - 1) / sh < B - 1 ? (a0 + g.A - 1) / sh : B - 1;
+    };
+    int dlo[2] = {1 << 20, 1 << 20}, dhi[2] = {-(1 << 20), -(1 << 20)};
+    for (int a0 = 0; a0 < g.X; a0 += g.A)
+    {
+        int lo, hi;
+        b_range(a0, &lo, &hi);
+        const int r = a0 % sh;
+        if (hi < lo)
+            continue;
+        dlo[r] = lo - a0 / sh < dlo[r] ? lo - a0 / sh : dlo[r];
+        dhi[r] = hi - a0 / sh > dhi[r] ? hi - a0 / sh : dhi[r];
+    }
+    g.nblocks = 0;
+    g.nclasses = sh;
+    for (int r = 0; r < sh; ++r)
+    {
+        g.class_lo[r] = dlo[r];
+        g.class_n[r] = dhi[r] >= dlo[r] ? dhi[r] - dlo[r] + 1 : 0;
+        g.class_col[r] = g.nblocks * g.n8;
+        g.nblocks += g.class_n[r];
+    }
+    g.kd_cols = g.nblocks * g.n8;
+    g.sum_col = kdg * g.kd_cols;
+    if (g.sum_col + kdg * g.nblocks * g.kgp > (int) TC_TMEM_COLS)
+        return false;
+    g.ntiles = 0;
+    int hits[512] = {0}, max_hits = 1; // updates of a block per k-step
+    double mma = 0;
+    for (int a0 = 0; a0 < g.X; a0 += g.A)
+    {
+        int lo, hi;
+        b_range(a0, &lo, &hi);
+        const int r = a0 % sh, most = 256 / g.n8;
+        for (int b = lo; b <= hi; b += most)
+        {
+            const int nb = hi - b + 1 < most ? hi - b + 1 : most;
+            if (g.ntiles == WG_MAX_TILES)
+                return false;
+            WgTile& t = g.tiles[g.ntiles++];
+            t.a16 = (uint32_t) (a0 * g.r8);
+            t.b16 = (uint32_t) (b * g.n8);
+            t.dcol = (uint32_t) (g.class_col[r] + (b - a0 / sh - g.class_lo[r]) * g.n8);
+            t.idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 4) << 24) | ((uint32_t) (nb * g.n8 >> 3) << 17);
+            mma += wg_mma_cost(nb * g.n8);
+            for (int i = 0; i < nb; ++i)
+            {
+                int& h = hits[t.dcol / g.n8 + i];
+                max_hits = ++h > max_hits ? h : max_hits;
+            }
+        }
+    }
+    g.flush_stages = WG_CHAIN / (max_hits * g.Q / 2);
+    if (g.flush_stages < 1)
+        g.flush_stages = 1;
+    g.kd_a16 = g.X * g.r8;
+    // offsets of a stage's items are 32 bits
+    if (4.0 * ((double) cgp * cg.xs_c + (double) kdg * cg.xs[0] + (double) g.X * cg.xs[1]) >= 4e9
+        || 4.0 * ((double) kg * cg.ys_c + (double) B * cg.ys[1]) >= 4e9)
+        return false;
+    // shared memory; 64 bytes behind every 128-byte multiple of cells keep the
+    // converters' stores (four rows x two cells at a time) on different banks
+    g.xrows = kdg * g.X * g.r8;
+    g.yrows = B * g.n8;
+    g.lbo_x = g.xrows * 16 + 64;
+    g.lbo_y = g.yrows * 16 + 64;
+    g.y_off = (g.Q * g.lbo_x + 127) / 128 * 128;
+    g.stage_bytes = g.y_off + (g.Q * g.lbo_y + 127) / 128 * 128;
+    g.cq = (cgp + 3) / 4;
+    g.kq = (kg + 3) / 4;
+    g.qg = (g.Q + 7) / 8;
+    g.items_x = kdg * g.X * g.cq * g.qg;
+    g.items_y = B * g.kq * g.qg;
+    const int tail = WG_MAX_TILES * (int) sizeof(WgTile) + (g.items_x + g.items_y) * 16 + 256 + 2048 + 128;
+    const int room = 226 * 1024 - tail, dump = g.kd_cols * 512;
+    g.nstages = room / g.stage_bytes < WG_MAX_STAGES ? room / g.stage_bytes : WG_MAX_STAGES;
+    if (g.nstages < 2 || dump > room || g.lbo_x >= 1 << 18 || g.lbo_y >= 1 << 18)
+        return false;
+    const int body = g.nstages * g.stage_bytes > dump ? g.nstages * g.stage_bytes : dump;
+    g.so_tiles = (body + 127) / 128 * 128;
+    g.so_items = g.so_tiles + WG_MAX_TILES * (int) sizeof(WgTile);
+    g.so_bars = g.so_items + (g.items_x + g.items_y) * 16;
+    // an instruction reads 128 rows from a tile's first one, used or not: the slack keeps that inside
+    g.smem = g.so_bars + 256 + 2048 + 128;
+    g.hblocks = (cg.out[1] + B - 1) / B;
+    g.wchunks = (cg.out[2] + PW - 1) / PW;
+    g.stages = (long long) cg.n * cg.out[0] * g.hblocks * g.wchunks;
+    if (g.stages >= (1ll << 31))
+        return false;
+    const int sms = num_sms();
+    g.parts = g.roles < sms ? sms / g.roles : 1;
+    if (g.parts > g.stages)
+        g.parts = (int) g.stages;
+    // clocks of a stage: the tensor pipe, the converters' instructions, their latency
+    const double pipe = kdg * mma * (g.Q / 2) * 1.1 + 200.0;
+    const int nv = 3 * cg.stride[2] + kwg;
+    const double ix = 60.0 + 6.0 * nv + 4.0 * kwg, iy = 70.0;
+    const double instr = (g.items_x * ix + g.items_y * iy) / 4.0 * 1.3;
+    // warps for x and dy, by the longer of their chains of item pairs
+    double lat = 1e30;
+    for (int wx = 1; wx < WG_CONV; ++wx)
+    {
+        const double px = (double) ((g.items_x + 2 * wx - 1) / (2 * wx)) * (200.0 + 4.0 * ix),
+                     py = (double) ((g.items_y + 2 * (WG_CONV - wx) - 1) / (2 * (WG_CONV - wx))) * (200.0 + 4.0 * iy);
+        const double m = px > py ? px : py;
+        if (m < lat)
+            lat = m, g.warps_x = wx;
+    }
+    double per = pipe > instr ? pipe : instr;
+    per = per > lat ? per : lat;
+    const double waves = (double) ((g.roles + sms - 1) / sms);
+    const double n = (double) ((g.stages + g.parts - 1) / g.parts);
+    const double harvest = (double) kdg * (g.nblocks * g.n8 * 4.0 + (double) kg * cgp * fh * kwg / WG_THREADS * 200.0);
+    const double flush = n / g.flush_stages * (300.0 + kdg * g.nblocks * g.kgp / 16.0 * 120.0);
+    const double fold = (double) g.parts / 8.0 * 100.0;
+    *cost = g.nkw * (waves * (n * per + flush + harvest) + 9000.0) + fold;
+    return true;
 }
 
 // Geometry of the tensor-core backward filter: x is the forward input window,
 // dy the forward output window.
 bool wg_geom(const ConvGeom& cg, int math_mode, WgGeom* out)
 {
-    WgGeom g;
-    std::memset(&g, 0, sizeof(g));
     if (math_mode == DCB_MATH_FP32_SIMT)
         return false;
     for (int i = 0; i < 3; ++i)
+        if (cg.stride[i] < 1 || cg.stride[i] > 2 || cg.dil[i] != 1 || cg.pad[i] > cg.f[i] - 1 || cg.f[i] > 16)
+            return false;
+    if ((long long) cg.n * cg.out[0] * cg.out[1] * cg.out[2] == 0 || cg.c == 0 || cg.k == 0
+        || cg.f[0] * cg.f[1] * cg.f[2] > 128)
+        return false;
+    WgGeom g, best;
+    std::memset(&g, 0, sizeof(g));
+    g.n = cg.n, g.c = cg.c, g.k = cg.k;
+    for (int i = 0; i < 3; ++i)
     {
-        if (cg.stride[i] < 1 || cg.stride[i] > 2 || cg.dil[i] != 1)
-            return false;
-        g.stride[i] = cg.stride[i];
-        g.in[i] = cg.in[i];
-        g.out[i] = cg.out[i];
-        g.f[i] = cg.f[i];
-        g.pad[i] = cg.pad[i];
-        if (g.pad[i] > g.f[i] - 1)
-            return false;
+        g.in[i] = cg.in[i], g.out[i] = cg.out[i], g.f[i] = cg.f[i], g.pad[i] = cg.pad[i], g.stride[i] = cg.stride[i];
+        g.xs[i] = cg.xs[i], g.ys[i] = cg.ys[i];
     }
-    g.n = cg.n;
-    g.c_total = cg.c;
-    g.k_total = cg.k;
-    const int taps = g.f[0] * g.f[1] * g.f[2];
-    g.c = 0;
-    for (int d = cg.c; d >= 1; --d)
-        if (cg.c % d == 0 && d * taps <= 128)
+    g.xs_n = cg.xs_n, g.xs_c = cg.xs_c, g.ys_n = cg.ys_n, g.ys_c = cg.ys_c;
+    double best_cost = -1;
+    for (int kwg : {1, 3, 5})
+    {
+        if (kwg > cg.f[2] && kwg > 1 && kwg - cg.f[2] > 1)
+            continue;
+        int last_c = 0;
+        for (int nc = 1; nc <= 64 && nc <= cg.c; ++nc)
         {
-            g.c = d;
-            break;
+            const int cgp = (cg.c + nc - 1) / nc;
+            if (cgp == last_c || 2 * cgp * kwg > 128)
+                continue;
+            last_c = cgp;
+            for (int kdg = cg.f[0]; kdg >= 1; kdg = kdg == 1 ? 0 : (kdg + 1) / 2)
+            {
+                int last_k = 0;
+                for (int nk = 1; nk <= 16 && nk <= cg.k; ++nk)
+                {
+                    const int kg = (cg.k + nk - 1) / nk;
+                    if (kg == last_k)
+                        continue;
+                    last_k = kg;
+                    for (int B : {1, 2, 3, 4, 6, 8, 12})
+                    {
+                        if (B > 1 && B > cg.out[1])
+                            break;
+                        for (int chunks = 1; chunks <= (cg.out[2] + 7) / 8; ++chunks)
+                        {
+                            const int pw = ((cg.out[2] + chunks - 1) / chunks + 7) / 8 * 8;
+                            if (pw > 64)
+                            {
+                                chunks = (cg.out[2] + 63) / 64 - 1;
+                                continue;
+                            }
+                            if (pw < 16 && chunks > 1)
+                                break;
+                            double cost;
+                            if (wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, &cost) && (best_cost < 0 || cost < best_cost))
+                                best_cost = cost, best = g;
+                            if (pw <= 16)
+                                break;
+                            // the next width that is a smaller multiple of 8
+                            const int next = pw - 8;
+                            chunks = (cg.out[2] + next - 1) / next - 1;
+                        }
+                    }
+                }
+            }
         }
-    if (g.c == 0 || cg.k == 0)
+    }
+    if (best_cost < 0)
         return false;
-    g.cgroups = cg.c / g.c;
-    g.k = cg.k < 16 ? cg.k : 16;
-    g.kgroups = (cg.k + 15) / 16;
-    if (g.cgroups * g.kgroups > 64)
-        return false; // every launch reads dy again: the CUDA-core kernel does better
-    g.mrows = g.c * taps;
-    if ((long long) cg.n * cg.out[0] * cg.out[1] * cg.out[2] == 0)
-        return false;
-    if (g.pad[2] > 4 || g.f[2] - 1 - g.pad[2] > 4 || g.f[1] > 16)
-        return false;
-    // bulk-copy compatible strides on both tensors (bases are checked per call)
-    if (!(cg.xs[1] % 4 == 0 && cg.xs[0] % 4 == 0 && cg.xs_c % 4 == 0 && cg.xs_n % 4 == 0))
-        return false;
-    if (!(cg.ys[1] % 4 == 0 && cg.ys[0] % 4 == 0 && cg.ys_c % 4 == 0 && cg.ys_n % 4 == 0))
-        return false;
-    g.xplane_bytes = g.c * g.f[1] * WG_XW * 4;
-    g.xhalf_floats = (g.xplane_bytes + 127) / 128 * 128 / 4;
-    g.xplane_floats = g.stride[2] * g.xhalf_floats;
-    g.xbuf_bytes = g.f[0] * g.xplane_floats * 4;
-    g.dybuf_bytes = 16 * WG_TW * 4;
-    if (wg_smem_need(g) > 200 * 1024)
-        return false;
-    g.tiles_w = (g.out[2] + WG_TW - 1) / WG_TW;
-    g.units = (long long) g.n * g.out[0] * g.out[1] * g.tiles_w;
-    if (g.units >= (1ll << 31))
-        return false;
-    *out = g;
+    *out = best;
     return true;
 }
 
 } // namespace
+
+static size_t wg_part_floats(const WgGeom& g)
+{
+    return (size_t) g.nkw * g.roles * g.parts * g.kg * g.cg * g.kdg * g.f[1] * g.kwg;
+}
 
 struct TcPlan
 {
@@ -228,8 +392,7 @@ struct TcPlan
     float* stat_part = nullptr; // per epilogue warp partial sums of the fused statistics
     bool has_wg = false;
     WgGeom wg;
-    ConvGeom wg_cg;             // strides of x and dy for the tensor maps
-    float* wg_part = nullptr;   // one 128 x 16 partial filter per CTA
+    float* wg_part = nullptr; // the CTAs' parts of the filter gradient
 };
 
 int32_t tc_plan_create(const ConvGeom& fwd, int math_mode, TcPlan** out)
@@ -237,8 +400,16 @@ int32_t tc_plan_create(const ConvGeom& fwd, int math_mode, TcPlan** out)
     *out = nullptr;
     auto* p = new TcPlan();
     p->has_sw = sw_geom(fwd, math_mode, &p->sw);
-    p->has_wg = wg_geom(fwd, math_mode, &p->wg);
-    p->wg_cg = fwd;
+    static PlanCache<std::pair<bool, WgGeom>> cache;
+    std::pair<bool, WgGeom> found;
+    cache.get(plan_key(fwd, 2, math_mode == DCB_MATH_FP32_SIMT), &found, [&]() {
+        std::pair<bool, WgGeom> r;
+        std::memset(&r.second, 0, sizeof(r.second));
+        r.first = wg_geom(fwd, math_mode, &r.second);
+        return r;
+    });
+    p->has_wg = found.first;
+    p->wg = found.second;
     if (!p->has_sw && !p->has_wg)
     {
         delete p;
@@ -249,7 +420,7 @@ int32_t tc_plan_create(const ConvGeom& fwd, int math_mode, TcPlan** out)
         ok = cudaMalloc(&p->sw_bimg, p->sw.b_bytes) == cudaSuccess
              && cudaMalloc(&p->stat_part, (size_t) num_sms() * SW_EPI * 32 * sizeof(float)) == cudaSuccess;
     if (ok && p->has_wg)
-        ok = cudaMalloc(&p->wg_part, (size_t) num_sms() * 128 * 16 * sizeof(float)) == cudaSuccess;
+        ok = cudaMalloc(&p->wg_part, wg_part_floats(p->wg) * sizeof(float)) == cudaSuccess;
     if (!ok)
     {
         (void) cudaGetLastError();
@@ -413,88 +584,59 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
     return DCB_OK;
 }
 
-// 5-D map (W, H, D, channels, N) of a strided window with the given box.
-// `skip` floats in front of the window are mapped with it (see x_skip): base - skip must be aligned.
-static bool wg_make_map(const float* base, const int ext[3], int channels, int n, const long long sp[3],
-                        long long s_c, long long s_n, int box_w, int box_h, int box_c, CUtensorMap* map,
-                        int skip = 0)
+// dw from the per-CTA parts: eight lanes per element, parts in order.
+static __global__ void __launch_bounds__(256) wg_fold_kernel(const __grid_constant__ WgGeom g, const float* __restrict__ part,
+                                                      float alpha, float beta, float* dw)
 {
-    EncodeTiledFn fn = encode_tiled_fn();
-    base -= skip;
-    if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) != 0)
-        return false;
-    const cuuint64_t dims[5] = {(cuuint64_t) (ext[2] + skip), (cuuint64_t) ext[1], (cuuint64_t) ext[0],
-                                (cuuint64_t) channels, (cuuint64_t) n};
-    const long long s1 = ext[1] > 1 ? sp[1] : ext[2];
-    const long long s0 = ext[0] > 1 ? sp[0] : s1 * ext[1];
-    const long long sc = channels > 1 ? s_c : s0 * ext[0];
-    const long long sn = n > 1 ? s_n : sc * channels;
-    const cuuint64_t strides[4] = {(cuuint64_t) s1 * 4, (cuuint64_t) s0 * 4, (cuuint64_t) sc * 4, (cuuint64_t) sn * 4};
-    for (int i = 0; i < 4; ++i)
-        if (strides[i] % 16 != 0 || strides[i] == 0)
-            return false;
-    const cuuint32_t box[5] = {(cuuint32_t) box_w, (cuuint32_t) box_h, 1, (cuuint32_t) box_c, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
-           == CUDA_SUCCESS;
+    const int taps = g.f[0] * g.f[1] * g.f[2];
+    const int e = (int) (blockIdx.x * 32 + threadIdx.x / 8), sub = threadIdx.x & 7;
+    const bool on = e < g.k * g.c * taps;
+    double s = 0.0;
+    if (on)
+    {
+        const int kw = e % g.f[2], kh = e / g.f[2] % g.f[1], kd = e / (g.f[2] * g.f[1]) % g.f[0];
+        const int c = e / taps % g.c, k = e / taps / g.c;
+        const int role = (k / g.kg * g.nkd + kd / g.kdg) * g.ncg + c / g.cg;
+        const int per = g.kg * g.cg * g.kdg * g.f[1] * g.kwg;
+        const float* p = part + ((long long) (kw / g.kwg) * g.parts * g.roles + role) * per
+                         + ((((long long) (k % g.kg) * g.cg + c % g.cg) * g.kdg + kd % g.kdg) * g.f[1] + kh) * g.kwg
+                         + kw % g.kwg;
+        const long long step = (long long) g.roles * per;
+#pragma unroll 4
+        for (int i = sub; i < g.parts; i += 8)
+            s += (double) p[i * step];
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+        s += __shfl_down_sync(0xffffffffu, s, o, 8);
+    if (on && sub == 0)
+        dw[e] = alpha * (float) s + (beta != 0.f ? beta * dw[e] : 0.f);
 }
 
-int32_t tc_conv_bwd_filter(TcPlan* p, float alpha, const float* x, const float* dy, float beta, float* dw,
-                           int* status, cudaStream_t stream)
+int32_t tc_conv_bwd_filter(TcPlan* p, float alpha, const float* x, const float* dy, float beta, float* dw, int* status,
+                           cudaStream_t stream)
 {
     if (!p || !p->has_wg)
         return DCB_UNSUPPORTED;
     WgGeom g = p->wg;
-    const ConvGeom& cg = p->wg_cg;
-    const int skip = x_skip(x);
-    // cells one bulk copy's outputs span: 128 at stride 1, 64 outputs at every second cell at stride 2
-    const int span = g.stride[2] == 2 ? 2 * (WG_TW / 2 - 1) + 1 : WG_TW;
-    if ((reinterpret_cast<uintptr_t>(x) & 3) != 0 || !skip_ok(skip, g.pad[2], g.f[2], span, WG_XW))
-        return DCB_UNSUPPORTED; // the caller falls back to the CUDA-core kernel
-    tc_row_window(g, skip);
-#if DCB_WG_KNOCKOUT
-    g.dbg = std::getenv("DCB_WG_DBG") ? std::atoi(std::getenv("DCB_WG_DBG")) : 0;
-#else
-    g.dbg = 0;
-#endif
-    size_t smem = wg_smem_need(g);
-    smem = smem < 120 * 1024 ? 120 * 1024 : smem; // one CTA per SM
-    long long grid = (long long) num_sms();
-    if (grid > g.units)
-        grid = g.units;
-    const int taps = g.f[0] * g.f[1] * g.f[2];
-    // all maps first: a pointer that cannot be mapped must refuse before anything ran
-    std::vector<CUtensorMap> xmaps((size_t) g.cgroups), dymaps((size_t) g.kgroups);
-    for (int cgp = 0; cgp < g.cgroups; ++cgp)
+    auto mult4 = [](long long a, long long b, long long c, long long d) { return ((a | b | c | d) & 3) == 0; };
+    g.skip_x = x_skip(x);
+    // (a piece that reaches past a row's last cell stays inside that cell's 16 bytes)
+    g.vec_x = mult4(g.n > 1 ? g.xs_n : 0, g.c > 1 ? g.xs_c : 0, g.in[0] > 1 ? g.xs[0] : 0, g.in[1] > 1 ? g.xs[1] : 0);
+    g.vec_y = mult4(g.n > 1 ? g.ys_n : 0, g.k > 1 ? g.ys_c : 0, g.out[0] > 1 ? g.ys[0] : 0, g.out[1] > 1 ? g.ys[1] : 0)
+              && (reinterpret_cast<uintptr_t>(dy) & 15) == 0;
+    const long long per_launch = (long long) wg_part_floats(g) / g.nkw;
+    for (int i = 0; i < g.nkw; ++i)
     {
-        std::memset(&xmaps[cgp], 0, sizeof(CUtensorMap));
-        if (!wg_make_map(x + (size_t) cgp * g.c * cg.xs_c, cg.in, g.c, cg.n, cg.xs, cg.xs_c, cg.xs_n, WG_XW, g.f[1],
-                         g.c, &xmaps[cgp], skip))
-            return DCB_UNSUPPORTED; // the caller falls back to the CUDA-core kernel
+        const int rkw = i * g.kwg, al = g.vec_x ? (rkw - g.pad[2] + g.skip_x) & 3 : -1;
+        const int32_t st = (g.stride[2] == 2 ? wg_launch_s2 : wg_launch_s1)(g, al, rkw, x, dy, p->wg_part + i * per_launch,
+                                                                            status, stream);
+        if (st != DCB_OK)
+            return st;
     }
-    for (int kg = 0; kg < g.kgroups; ++kg)
-    {
-        std::memset(&dymaps[kg], 0, sizeof(CUtensorMap));
-        const int kcur = g.k_total - kg * 16 < 16 ? g.k_total - kg * 16 : 16;
-        if (!wg_make_map(dy + (size_t) kg * 16 * cg.ys_c, cg.out, kcur, cg.n, cg.ys, cg.ys_c, cg.ys_n, WG_TW, 1, 16,
-                         &dymaps[kg]))
-            return DCB_UNSUPPORTED;
-    }
-    auto kernel = g.stride[2] == 2 ? wg_conv_kernel<2> : wg_conv_kernel<1>;
-    DCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (224 * 1024)));
-    for (int kg = 0; kg < g.kgroups; ++kg)
-        for (int cgp = 0; cgp < g.cgroups; ++cgp)
-        {
-            const int kcur = g.k_total - kg * 16 < 16 ? g.k_total - kg * 16 : 16;
-            kernel<<<(unsigned) grid, WG_THREADS, smem, stream>>>(g, p->wg_part, status, xmaps[cgp], dymaps[kg]);
-            DCB_LAUNCH_CHECK();
-            const int total = g.mrows * kcur;
-            wg_fold_kernel<<<(total + 255) / 256, 256, 0, stream>>>(p->wg_part, (int) grid, g.mrows, kcur, taps,
-                                                                    g.c_total, cgp * g.c, kg * 16, alpha, beta, dw);
-            DCB_LAUNCH_CHECK();
-        }
+    const int total = g.k * g.c * g.f[0] * g.f[1] * g.f[2];
+    wg_fold_kernel<<<(unsigned) ((total + 31) / 32), 256, 0, stream>>>(g, p->wg_part, alpha, beta, dw);
+    DCB_LAUNCH_CHECK();
     return DCB_OK;
 }
 

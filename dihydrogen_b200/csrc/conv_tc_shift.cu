@@ -1,6 +1,7 @@
 // Shift kernel, host side: tables, filter image, launches.
 #include "conv_tc_shift_api.cuh"
 
+#include "conv_plan_cache.cuh"
 #include "conv_tc_encode.cuh"
 #include "conv_tc_shift_plan.cuh"
 
@@ -721,9 +722,16 @@ bool sh_plan_create(const ConvGeom& g, bool transposed, int math_mode, ShPlan** 
 {
     *out = nullptr;
     *status = DCB_OK;
-    ShBuilder b(g, transposed, math_mode, num_sms());
+    static PlanCache<std::pair<bool, ShTables>> cache;
+    std::pair<bool, ShTables> found;
+    cache.get(plan_key(g, transposed ? 1 : 0, math_mode), &found, [&]() {
+        std::pair<bool, ShTables> r;
+        r.first = ShBuilder(g, transposed, math_mode, num_sms()).build(&r.second);
+        return r;
+    });
     auto* p = new ShPlan();
-    if (!b.build(&p->t))
+    p->t = std::move(found.second);
+    if (!found.first)
     {
         delete p;
         return false;

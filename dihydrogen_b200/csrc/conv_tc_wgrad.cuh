@@ -1,481 +1,581 @@
-// tcgen05 / TMEM backward filter (strides 1 or 2, dilation 1, c*fd*fh*fw <= 128
-// filter taps per output filter, K <= 16 per launch):
+// tcgen05 backward filter (strides 1 or 2 per dimension, dilation 1):
 //
 //   dw[k][c][kd][kh][kw] = sum over (n, od, oh, ow) dy[n][k][od][oh][ow] *
 //                          x[n][c][od*sd+kd-pd][oh*sh+kh-ph][ow*sw+kw-pw]
 //
-// (written below for unit strides; with stride 2 along W a unit's input rows
-// arrive as two half windows of the same shape, outputs 0..63 read the first
-// and 64..127 the second, at every second cell)
+// GEMM view: the reduction runs along W, eight positions per instruction, both
+// operands K-major in shared memory without swizzle (a cell is 16 bytes = four
+// positions of one row).
+//   A  rows (x row, part, kw, c): an input row once per tap kw, shifted by it, so
+//      that no address has to move by less than a cell
+//   B  rows (dy row, part, k)
+// `part` is the hi or the lo half of a two-way TF32 split.  One instruction
+// multiplies `A` consecutive input rows (up to 128 matrix rows) with `nb`
+// consecutive dy rows, all pairs at once; pair (a, b) is tap kh = a - b * sh, pairs
+// that are no tap are not read.  Rows of both operands are plentiful this way (4
+// channels x 3 taps x 2 parts x 5 input rows = 120 of 128, 3 dy rows x 16 filters x
+// 2 parts = 96 columns), where a plain im2col product of a layer with few channels
+// and filters would use a fraction of both.
 //
-// GEMM view: the reduction runs over the outputs, eight consecutive ow per
-// MMA (the K of a TF32 instruction).  M = the (c, kd, kh, kw) taps (up to 128
-// rows = TMEM lanes), N = the filters.  For one chunk of eight outputs
-//   A[m][kk] = x[c][od+kd-pd][oh+kh-ph][ow0 + kk + kw-pw]     (tensor memory)
-//   B[kk][k] = dy[k][od][oh][ow0 + kk]                        (shared memory)
-// and the accumulator D[m][k] stays in tensor memory: two buffers, swapped every
-// WG_FLUSH_UNITS units; four dump warps add the idle one into fp64 registers and
-// zero it.  When the CTA has walked all its units it writes its 128 x 16 partial
-// filter, and a second kernel folds the partials in CTA order (fp64) and applies
-// alpha / beta.
+// A stage is B dy rows and the X = (B - 1) * sh + fh input rows of each of its kd
+// planes, PW positions wide, in one of two to four shared-memory buffers.
+// Converter warps read x and dy straight from global memory, split them and write
+// the stage; one thread issues.  What does not fit tensor memory (512 columns,
+// accumulators and running sums) or the 128 matrix rows is dealt out in roles:
+// groups of channels, planes kd or filters, a CTA always working for one, and
+// launches for groups of taps kw.
 //
-// 3xTF32: D[:, 0:32] += A_hi x [B_hi | B_lo] (one instruction, N = 32) and
-// D[:, 0:16] += A_lo x B_hi (N = 16); the fold adds the two column halves.
-//
-// A unit is 128 outputs of one output row: 8 chunks of two k-steps.  Warp 15 copies the
-// fd * fh input rows (all channels, 4 cells of margin left and right, zeros
-// outside the tensor = the padding) and the dy row (all filters) of the next
-// unit into a two-deep shared-memory ring with bulk tensor copies.  Warps 0..11
-// are three converter groups: group g takes every third chunk, lane m of its
-// four warps writes row m of A (hi and lo parts) into the group's A slot and the
-// group writes the chunk's B tile; warps 12..14 issue, issuer g for group g.
-// All waits are bounded.
+// The tensor pipe adds into its fp32 accumulators by truncation: after
+// WG_CHAIN updates four warps add the hi columns into running sums beside them,
+// rounding to nearest, and zero them (the lo columns are 2^-11 of the result: their
+// chains may run to the end).
+// At the end every CTA reduces its accumulators to its part of the filter and
+// wg_fold_kernel adds the CTAs' parts in order, in fp64: the same result every run.
 #pragma once
 
-#include "conv_simt.cuh"
-#include "conv_tc_common.cuh"
+#include "conv_tc_wgrad_api.cuh"
 
 namespace dcb
 {
-namespace
+
+struct WgUnit
 {
-
-// A group's chunks go round its WG_SPG slots, and each slot has an issuer warp of its
-// own: issuing a tcgen05.mma (or a commit) occupies its thread for ~160 clocks whatever
-// the instruction's size, a chunk is four instructions and a commit, and with one issuer
-// per group that alone was over 1 ms of the kernel's 1.39 ms on the 256^3 shard.
-#ifndef DCB_WG_SPG
-#define DCB_WG_SPG 2
-#endif
-#ifndef DCB_WG_KS
-#define DCB_WG_KS 2
-#endif
-constexpr int WG_SPG = DCB_WG_SPG;         // slots, and issuers, per converter group
-constexpr int WG_ISSUER2_WARP = 20;        // issuers of the slots after a group's first: warps 20 ..
-constexpr int WG_THREADS = (20 + 3 * (WG_SPG - 1)) * 32; // 12 converters, 3 issuers, 1 copy, 4 dump warps, more issuers
-constexpr int WG_COPY_WARP = 15;
-constexpr int WG_DUMP_WARP = 16;
-constexpr int WG_TW = 128;                 // outputs per unit
-constexpr int WG_KS = DCB_WG_KS;           // k-steps (of eight outputs) per chunk: one hand-off per chunk
-constexpr int WG_CHUNKS = WG_TW / (8 * WG_KS); // chunks per unit
-constexpr int WG_XW = WG_TW + 12;          // staged input row: 4 cells of margin left, 8 right; the 140-float
-                                           // pitch keeps the taps of a warp's 32 lanes (about 11 rows x 3
-                                           // columns) on different banks, 136 would fold them three deep
-constexpr int WG_A_SLOTS = 3 * WG_SPG;     // slot s belongs to group s % 3
-constexpr int WG_A_COLS = 16 * WG_KS;      // an A slot: per k-step 8 hi + 8 lo columns
-constexpr uint32_t WG_TMEM_COLS = 64 + WG_A_SLOTS * 16 * 2 <= 256 ? 256 : 512; // two accumulator buffers of 32 columns + the A slots
-constexpr int WG_ACC_COLS = 64;            // the A ring starts here
-// The tensor pipe adds into an fp32 accumulator without rounding to nearest: over
-// a chain of n updates the error grows like n^1.5 * 2^-24 and does not average
-// out.  Measured on a 256^3 shard with one accumulator for the whole run: 4e-4
-// of the gradient's scale.  So a chain is cut after this many units (1024
-// outputs, 128 updates): the dump warps add the buffer into fp64 registers and
-// zero it while the issuers fill the other one (5e-6 by the same estimate).
-constexpr int WG_FLUSH_UNITS = 8;
-constexpr int WG_B_FLOATS = 256 * WG_KS;   // the B tiles of a chunk: per k-step 8 x 32 floats
-
-#ifndef DCB_WG_KNOCKOUT
-#define DCB_WG_KNOCKOUT 0
-#endif
-#if DCB_WG_KNOCKOUT
-#define WG_DBG(bit) ((g.dbg >> (bit)) & 1)
-#else
-#define WG_DBG(bit) 0
-#endif
-
-struct WgGeom
-{
-    int n, c, k;
-    int in[3], out[3], f[3], pad[3];
-    int lx, rx;             // as in TcGeom, for the staged input rows of a unit
-    int dbg;                // timing knock-outs (builds with DCB_WG_KNOCKOUT only): bit 0 no tap loads,
-                            // 1 no tensor-memory stores, 2 no B tile, 3 no MMAs, 4 no input copies
-    int mrows;              // c * fd * fh * fw
-    int tiles_w;
-    long long units;        // n * out_d * out_h * tiles_w
-    int stride[3];          // 1 or 2
-    int xhalf_floats;       // one bulk copy's box in a unit buffer: c * fh * WG_XW floats rounded up to
-                            // 128 bytes (a bulk copy's destination must be 128-byte aligned)
-    int xplane_floats;      // pitch of one filter plane of a unit: stride[2] boxes
-    int xplane_bytes;       // bytes one box brings: c * fh * WG_XW * 4
-    int xbuf_bytes;         // fd plane pitches
-    int dybuf_bytes;        // 16 x WG_TW floats
-    // One launch covers c input channels (c * taps <= 128) and at most 16
-    // filters; a larger filter tensor is cgroups x kgroups launches.
-    int c_total, k_total, cgroups, kgroups;
+    int n, od, h0, w0;
 };
 
-// dw[k_off + kk][c_off + c][tap] (of a [k_total][c_total][taps] filter tensor) from the
-// per-CTA partials of one launch; m = tap * c + c_index (c = channels of the launch).
-__global__ void wg_fold_kernel(const float* __restrict__ part, int nparts, int mrows, int k, int taps, int c_total,
-                               int c_off, int k_off, float alpha, float beta, float* dw)
+__device__ __forceinline__ WgUnit wg_unit(const WgGeom& g, long long s)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x; // (filter, tap row)
-    if (i >= mrows * k)
-        return;
-    const int kk = i / mrows, m = i % mrows;
-    double s = 0.0;
-    for (int p = 0; p < nparts; ++p)
-        s += (double) part[((size_t) p * 128 + m) * 16 + kk];
-    const int cl = mrows / taps; // channels of this launch
-    float* o = dw + ((size_t) (k_off + kk) * c_total + c_off + m % cl) * taps + m / cl;
-    const float prev = beta != 0.f ? *o : 0.f;
-    *o = alpha * (float) s + beta * prev;
+    WgUnit u;
+    uint32_t r = (uint32_t) s;
+    u.h0 = (int) (r % (uint32_t) g.hblocks) * g.B;
+    r /= (uint32_t) g.hblocks;
+    u.w0 = (int) (r % (uint32_t) g.wchunks) * g.PW;
+    r /= (uint32_t) g.wchunks;
+    u.od = (int) (r % (uint32_t) g.out[0]);
+    u.n = (int) (r / (uint32_t) g.out[0]);
+    return u;
 }
 
-template <int SW> // stride along W
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
+{
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void st_v4(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+struct WgConvArgs
+{
+    uint32_t base, full_s, empty_s;
+    const uint4* itab;
+    int items, warps, rc, rkw, rkd, rk, s0, s1, w, lane;
+    volatile int* abort_flag;
+};
+
+// Converters.  Some warps read x, the others dy; warp w of `warps` takes two items at
+// a time (w, w + warps; then the next two), loads one pair ahead.  A lane is four
+// positions of one channel or filter; the cells behind them are fetched as the aligned
+// 16-byte pieces they lie in, the first one AL cells below them (AL < 0: cell by cell).
+// Lanes outside the tensor store zeros (the padding).  A warp's own chain of dependent
+// instructions is what bounds a stage where channels are few: hence pairs of items
+// without branches between them, and stages that follow each other along H, so that
+// most of them only move a pointer.
+template <bool ISX, int SW, int KWG, int AL>
+__device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c, const float* __restrict__ src)
+{
+    constexpr int NV = ISX ? 3 * SW + KWG : 4;                  // cells behind four positions
+    constexpr int AO = AL < 0 ? 0 : AL, NB = (NV + AO + 3) / 4; // their offset in the pieces, pieces
+    constexpr uint32_t ALL = (1u << NV) - 1;
+    const int cl = c.lane & 3, ql = c.lane >> 2;
+    const uint32_t lane_dst = (uint32_t) (ql * (ISX ? g.lbo_x : g.lbo_y) + 16 * cl);
+    const uint32_t row16 = 16u * (uint32_t) (ISX ? g.cg : g.kgp);
+    const int rows_in = ISX ? g.in[1] : g.out[1], step_rows = ISX ? g.B * g.stride[1] : g.B;
+    const long long step = 4ll * step_rows * (ISX ? g.xs[1] : g.ys[1]);
+    float t[2][2][4 * NB];
+    uint32_t dst[2][2] = {{0, 0}, {0, 0}}, mask[2][2] = {{0, 0}, {0, 0}};
+    uint32_t wait[2] = {0, 0}, tell[2] = {0, 0};
+    bool has[2] = {false, false};
+    int item = c.w - 2 * c.warps, s = c.s0, buf = 0;
+    uint32_t lap = 0, st = c.base;
+    bool ok = true, more = c.s0 < c.s1, fresh = true;
+    const char* b0 = nullptr; // the stage's first cells, this lane's channel and positions
+    int h0 = 0, r0 = 0, id0 = 0;
+    uint32_t m8[2] = {0, 0}; // valid cells, per group of eight lanes along the row
+    auto locate = [&]() {
+        const WgUnit u = wg_unit(g, s);
+        h0 = u.h0;
+        const int w0 = ISX ? u.w0 * SW + c.rkw - g.pad[2] : u.w0, width = ISX ? g.in[2] : g.out[2];
+        if (ISX)
+        {
+            id0 = u.od * g.stride[0] + c.rkd - g.pad[0];
+            r0 = u.h0 * g.stride[1] - g.pad[1];
+            b0 = reinterpret_cast<const char*>(src + (long long) u.n * g.xs_n + (long long) (c.rc + cl) * g.xs_c
+                                               + (long long) id0 * g.xs[0] + (long long) r0 * g.xs[1] + w0 + 4 * ql * SW - AO);
+        }
+        else
+        {
+            r0 = u.h0;
+            b0 = reinterpret_cast<const char*>(src + (long long) u.n * g.ys_n + (long long) (c.rk + cl) * g.ys_c
+                                               + (long long) u.od * g.ys[0] + (long long) r0 * g.ys[1] + w0 + 4 * ql);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+        {
+            const int iw = w0 + (4 * ql + 32 * i) * (ISX ? SW : 1);
+            uint32_t m = ALL;
+            if (iw < 0)
+                m = iw <= -NV ? 0u : m << -iw & m;
+            if (iw + NV > width)
+                m = iw >= width ? 0u : m & ((1u << (width - iw)) - 1);
+            m8[i] = ql + 8 * i < g.Q ? m : 0u;
+        }
+    };
+    if (more)
+        locate();
+#pragma unroll 1
+    while (ok && (more || has[0]))
+    {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+        {
+            if (has[q])
+            {
+                if (wait[q] != 0)
+                    ok = ok && mbar_wait_s<20>(wait[q] & ~7u, wait[q] & 1u, c.abort_flag);
+                // tensor edges: cells that do not exist (and were not loaded) are zeros
+                if (__any_sync(0xffffffffu, mask[q][0] != ALL || mask[q][1] != ALL))
+                {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int e = 0; e < NV; ++e)
+                            t[q][i][AO + e] = mask[q][i] >> e & 1 ? t[q][i][AO + e] : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                {
+                    uint32_t hi[NV], lo[NV];
+#pragma unroll
+                    for (int e = 0; e < NV; ++e)
+                    {
+                        hi[e] = tf32_rna(t[q][i][AO + e]);
+                        // exact remainder below 2^-11 |x|; the pipe reads its upper 19 bits
+                        lo[e] = __float_as_uint(t[q][i][AO + e] - __uint_as_float(hi[e]));
+                    }
+                    if (dst[q][i] != 0 && ok)
+                    {
+                        uint32_t d = dst[q][i];
+                        if (ISX)
+                        {
+#pragma unroll
+                            for (int kw = 0; kw < KWG; ++kw, d += row16)
+                                st_v4(d, hi[kw], hi[kw + SW], hi[kw + 2 * SW], hi[kw + 3 * SW]);
+#pragma unroll
+                            for (int kw = 0; kw < KWG; ++kw, d += row16)
+                                st_v4(d, lo[kw], lo[kw + SW], lo[kw + 2 * SW], lo[kw + 3 * SW]);
+                        }
+                        else
+                        {
+                            st_v4(d, hi[0], hi[1], hi[2], hi[3]);
+                            st_v4(d + row16, lo[0], lo[1], lo[2], lo[3]);
+                        }
+                    }
+                }
+                if (tell[q] != 0)
+                {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (c.lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tell[q]) : "memory");
+                }
+                has[q] = false;
+            }
+            if (!more)
+                continue;
+            wait[q] = 0;
+            item += 2 * c.warps;
+            if (item >= c.items || fresh)
+            {
+                if (!fresh)
+                {
+                    item = c.w;
+                    if (++s == c.s1)
+                    {
+                        more = false;
+                        continue;
+                    }
+                    st += (uint32_t) g.stage_bytes;
+                    if (++buf == g.nstages)
+                    {
+                        buf = 0;
+                        st = c.base;
+                        ++lap;
+                    }
+                    h0 += g.B;
+                    if (h0 < g.out[1])
+                    {
+                        // the next rows of the same column
+                        r0 += step_rows;
+                        b0 += step;
+                    }
+                    else
+                        locate();
+                }
+                fresh = false;
+                if (lap > 0)
+                    wait[q] = (c.empty_s + 8u * (uint32_t) buf) | ((lap - 1) & 1u);
+            }
+            tell[q] = item + 2 * c.warps >= c.items ? c.full_s + 8u * (uint32_t) buf : 0u;
+            has[q] = true;
+            uint4 it[2];
+            it[0] = c.itab[item];
+            it[1] = item + c.warps < c.items ? c.itab[item + c.warps] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+            {
+                const int row = (int) (it[i].x >> 8 & 255u);
+                const bool second = (it[i].x >> 24) != 0; // group of lanes along the row
+                const bool stored = cl < (int) (it[i].x >> 16 & 15u) && (second ? ql + 8 : ql) < g.Q;
+                bool in = cl < (int) (it[i].x >> 20 & 15u) && (unsigned) (r0 + row) < (unsigned) rows_in;
+                if (ISX)
+                    in = in && (unsigned) (id0 + (int) (it[i].x >> 2 & 63u)) < (unsigned) g.in[0];
+                const uint32_t m = in ? (second ? m8[1] : m8[0]) : 0u;
+                dst[q][i] = stored ? st + it[i].y + lane_dst : 0u;
+                mask[q][i] = m;
+                const float* p = reinterpret_cast<const float*>(b0 + it[i].z);
+                if (AL >= 0)
+                {
+#pragma unroll
+                    for (int e = 0; e < NB; ++e)
+                    {
+                        // the valid cells among the piece's
+                        const int first = 4 * e - AO;
+                        const uint32_t bits = first >= 0 ? m >> (first >= 0 ? first : 0) & 15u
+                                                         : m & (15u >> (first < 0 ? -first : 0));
+                        if (bits != 0)
+                        {
+                            const float4 f = __ldg(reinterpret_cast<const float4*>(p) + e);
+                            t[q][i][4 * e] = f.x, t[q][i][4 * e + 1] = f.y, t[q][i][4 * e + 2] = f.z,
+                                           t[q][i][4 * e + 3] = f.w;
+                        }
+                    }
+                }
+                else
+                {
+#pragma unroll
+                    for (int e = 0; e < NV; ++e)
+                        if (m >> e & 1)
+                            t[q][i][e] = __ldg(p + e);
+                }
+            }
+        }
+    }
+    return ok;
+}
+
+// One launch per group of taps kw (rkw is the first): where a lane's cells start
+// inside a 16-byte piece is then the same for all, and the converters are compiled
+// for it.
+template <int SW, int KWG, int AL>
 __global__ void __launch_bounds__(WG_THREADS, 1)
-    wg_conv_kernel(WgGeom g, float* __restrict__ part, int* status, const __grid_constant__ CUtensorMap xmap,
-                   const __grid_constant__ CUtensorMap dymap)
+    wg_conv_kernel(const __grid_constant__ WgGeom g, const float* __restrict__ x, const float* __restrict__ dy,
+                   float* __restrict__ part, int* status, int rkw)
 {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int unit_bytes = (g.xbuf_bytes + g.dybuf_bytes + 127) / 128 * 128;
-    uint8_t* ubuf = smem;                                        // [2] unit buffers: x planes, then the dy row
-    float* bring = reinterpret_cast<float*>(smem + 2 * unit_bytes); // [WG_A_SLOTS] B tiles
-    uint64_t* bars = reinterpret_cast<uint64_t*>(bring + WG_A_SLOTS * WG_B_FLOATS);
-    uint64_t* a_full = bars;                 // [6]
-    uint64_t* a_empty = a_full + WG_A_SLOTS; // [6]
-    uint64_t* u_full = a_empty + WG_A_SLOTS; // [2]
-    uint64_t* u_empty = u_full + 2;          // [2]
-    uint64_t* d_full = u_empty + 2;          // [2] issuers -> dump warps: a batch of units is in the buffer
-    uint64_t* d_empty = d_full + 2;          // [2] dump warps -> issuers: the buffer is zero again
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 2);
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + g.so_bars); // [nstages] converters -> issuer
+    uint64_t* empty = full + WG_MAX_STAGES;                         // [nstages] issuer -> converters
+    uint64_t* chain_end = empty + WG_MAX_STAGES;                    // issuer -> running sums
+    uint64_t* cleared = chain_end + 1;                              // running sums -> issuer
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cleared + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int items = g.items_x + g.items_y;
+    const int role = (int) blockIdx.x % g.roles, slice = (int) blockIdx.x / g.roles;
+    const int rc = role % g.ncg * g.cg, rkd = role / g.ncg % g.nkd * g.kdg, rk = role / (g.ncg * g.nkd) * g.kg;
+    const int s0 = (int) (g.stages * slice / g.parts), s1 = (int) (g.stages * (slice + 1) / g.parts);
+
     if (tid == 0)
     {
-        for (int s = 0; s < WG_A_SLOTS; ++s)
+        for (int s = 0; s < WG_MAX_STAGES; ++s)
         {
-            mbar_init(&a_full[s], 4);
-            mbar_init(&a_empty[s], 1);
+            mbar_init(&full[s], (uint32_t) (min(g.items_x, g.warps_x) + min(g.items_y, WG_CONV - g.warps_x)));
+            mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b)
-        {
-            mbar_init(&u_full[b], 1);
-            mbar_init(&u_empty[b], 12);
-        }
-        for (int b = 0; b < 2; ++b)
-        {
-            mbar_init(&d_full[b], 3 * WG_SPG);
-            mbar_init(&d_empty[b], 4);
-        }
+        mbar_init(chain_end, 1);
+        mbar_init(cleared, WG_FLUSH);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == TC_MMA_WARP)
+    if (warp == 0)
     {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(WG_TMEM_COLS)
+                     "r"(TC_TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    WgTile* tiles = reinterpret_cast<WgTile*>(smem + g.so_tiles);
+    for (int i = tid; i < g.ntiles; i += WG_THREADS)
+        tiles[i] = g.tiles[i];
+    // warp items of a stage: what and how many channels or filters, where it goes, where it comes from
+    uint4* itab = reinterpret_cast<uint4*>(smem + g.so_items);
+    for (int i = tid; i < items; i += WG_THREADS)
+    {
+        const bool isx = i < g.items_x;
+        int r = isx ? i : i - g.items_x;
+        const int q0 = r % g.qg * 8;
+        r /= g.qg;
+        const int ch = r % (isx ? g.cq : g.kq) * 4;
+        r /= isx ? g.cq : g.kq; // kd * X + a, or b
+        const int kd = isx ? r / g.X : 0, row = isx ? r - kd * g.X : r;
+        // rows of the operand that exist (the others hold zeros), and of those the ones the tensor has
+        const int rows = min(4, (isx ? g.cg : g.kg) - ch);
+        const int real = max(0, min(rows, isx ? g.c - rc - ch : g.k - rk - ch));
+        const long long off = isx ? 4 * (ch * g.xs_c + kd * g.xs[0] + row * g.xs[1] + 4 * q0 * SW)
+                                  : 4 * (ch * g.ys_c + row * g.ys[1] + 4 * q0);
+        itab[i] = make_uint4((isx ? 1u : 2u) | (uint32_t) kd << 2 | (uint32_t) row << 8 | (uint32_t) rows << 16
+                                 | (uint32_t) real << 20 | (uint32_t) q0 << 24,
+                             (uint32_t) (isx ? q0 * g.lbo_x + 16 * (r * g.r8 + ch)
+                                             : g.y_off + q0 * g.lbo_y + 16 * (r * g.n8 + ch)),
+                             (uint32_t) off, 0u); // (below 4 GB: wg_layout)
+    }
+    // matrix rows that no item writes (filters up to a multiple of 8) stay zero
+    for (int i = tid; i < g.nstages * g.stage_bytes / 16; i += WG_THREADS)
+        reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-
-    const uint32_t nunits = (uint32_t) g.units;
+    const uint32_t tmem = *tmem_slot;
+    if (warp < 4)
+        for (uint32_t c = 0; c < TC_TMEM_COLS; c += 16)
+            tmem_st16_zero(tmem + ((uint32_t) (warp * 32) << 16) + c);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
     bool ok = true;
 
-    if (warp < 12)
+    if (warp < WG_FLUSH)
     {
-        // ------------------------------------------------------------------
-        // converters
-        // ------------------------------------------------------------------
-        const int gq = warp >> 2, quad = warp & 3;
-        const int m = quad * 32 + lane;
-        const uint32_t lane_addr = tmem_base + ((uint32_t) (quad * 32) << 16);
-        // where this lane's tap sits in a unit buffer (floats)
-        int src = -1;
-        if (m < g.mrows)
+        // running sums, pieces of eight hi columns
+        const uint32_t la = tmem + ((uint32_t) ((warp & 3) * 32) << 16);
+        const int pieces = g.kgp / 8, total = g.kdg * g.nblocks * pieces;
+        uint32_t par = 0;
+        for (int s = s0 + g.flush_stages; s < s1 && ok; s += g.flush_stages, par ^= 1)
         {
-            // row m of the partial filter is (tap, channel), channel fastest: with the
-            // channel slowest the lanes of a warp read three filter planes at the same
-            // bank offsets (a plane's rows start on a 128-byte boundary), three deep;
-            // this order is two deep at worst (4 channels x 3 x 3 x 3, 140-float rows)
-            const int c = m % g.c;
-            int r = m / g.c;
-            const int kw = r % g.f[2];
-            r /= g.f[2];
-            const int kh = r % g.f[1];
-            const int kd = r / g.f[1];
-            src = kd * g.xplane_floats + (c * g.f[1] + kh) * WG_XW + g.rx + kw;
-        }
-        // this lane's element of the B tile: filter quad*4 + lane/8, output lane%8
-        const int bk = quad * 4 + (lane >> 3), bkk = lane & 7;
-        const int b_off = (bkk >> 2) * 128 + (bk >> 3) * 32 + (bk & 7) * 4 + (bkk & 3); // + 64 for the lo half
-        int lap = 0;
-        uint32_t a_phase = 1, seq = 0;
-        bool a_first = true;
-        uint32_t ul = 0; // units done by this CTA
-        for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++ul)
-        {
-            const uint32_t b = ul & 1;
-            ok = mbar_wait(&u_full[b], (ul >> 1) & 1, abort_flag);
-            if (!ok)
-                break;
-            const float* xb = reinterpret_cast<const float*>(ubuf + (size_t) b * unit_bytes);
-            const float* dyb = reinterpret_cast<const float*>(ubuf + (size_t) b * unit_bytes + g.xbuf_bytes);
-            // chunks are dealt to the groups in sequence over the whole run
-            int q = (gq + 3 - (int) (seq % 3u)) % 3;
-            for (; q < WG_CHUNKS && ok; q += 3)
-            {
-                const int slot = gq + 3 * lap;
-                uint32_t hi[WG_KS][8], lo[WG_KS][8], dhi[WG_KS], dlo[WG_KS];
-#pragma unroll
-                for (int ks = 0; ks < WG_KS; ++ks)
-                {
-                    if (src >= 0 && !WG_DBG(0))
-                    {
-                        // output (q * WG_KS + ks) * 8 of the unit; with SW == 2 the second
-                        // 64 outputs read the second half window
-                        const int o = (q * WG_KS + ks) * 8;
-                        const uint32_t s0 = smem_u32(
-                            xb + src + (SW == 2 ? (o >= 64 ? g.xhalf_floats + (o - 64) * 2 : o * 2) : o));
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                        {
-                            const float xe = __uint_as_float(lds_u32(s0 + 4u * (uint32_t) (e * SW)));
-                            hi[ks][e] = tf32_rna(xe);
-                            // exact remainder, fed as it is: the pipe reads its upper 19 bits
-                            lo[ks][e] = __float_as_uint(xe - __uint_as_float(hi[ks][e]));
-                        }
-                    }
-                    else
-                    {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            hi[ks][e] = lo[ks][e] = 0u;
-                    }
-                    const float dv = WG_DBG(2) ? 0.f : dyb[bk * WG_TW + (q * WG_KS + ks) * 8 + bkk];
-                    dhi[ks] = tf32_rna(dv);
-                    dlo[ks] = tf32_rna(dv - __uint_as_float(dhi[ks]));
-                }
-                if (!a_first)
-                    ok = mbar_wait(&a_empty[slot], a_phase, abort_flag);
-                if (!ok)
-                    break;
-                tc_fence_after();
-                const uint32_t a_addr = lane_addr + (uint32_t) WG_ACC_COLS + (uint32_t) (slot * WG_A_COLS);
-                float* bt = bring + slot * WG_B_FLOATS;
-#pragma unroll
-                for (int ks = 0; ks < WG_KS; ++ks)
-                {
-                    if (!WG_DBG(1))
-                    {
-                        tmem_st8(a_addr + (uint32_t) (ks * 16), hi[ks]);
-                        tmem_st8(a_addr + (uint32_t) (ks * 16 + 8), lo[ks]);
-                    }
-                    if (!WG_DBG(2))
-                    {
-                        bt[ks * 256 + b_off] = __uint_as_float(dhi[ks]);
-                        bt[ks * 256 + b_off + 64] = __uint_as_float(dlo[ks]);
-                    }
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(&a_full[slot]);
-                if (++lap == WG_SPG)
-                {
-                    lap = 0;
-                    a_phase ^= 1;
-                    a_first = false;
-                }
-            }
-            seq += WG_CHUNKS;
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(&u_empty[b]);
-        }
-    }
-    else if (warp == WG_COPY_WARP)
-    {
-        // ------------------------------------------------------------------
-        // bulk tensor copies, one unit ahead
-        // ------------------------------------------------------------------
-        const uint32_t bytes = (uint32_t) ((WG_DBG(4) ? 0 : g.f[0] * SW * g.xplane_bytes) + g.dybuf_bytes);
-        uint32_t ul = 0;
-        for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++ul)
-        {
-            const uint32_t b = ul & 1;
-            if (ul >= 2)
-                ok = mbar_wait(&u_empty[b], ((ul >> 1) + 1) & 1, abort_flag);
-            if (!ok)
-                break;
-            if (lane == 0)
-            {
-                const uint32_t tw = u % (uint32_t) g.tiles_w;
-                uint32_t r = u / (uint32_t) g.tiles_w;
-                const int oh = (int) (r % (uint32_t) g.out[1]);
-                r /= (uint32_t) g.out[1];
-                const int od = (int) (r % (uint32_t) g.out[0]);
-                const int n = (int) (r / (uint32_t) g.out[0]);
-                const int ow0 = (int) tw * WG_TW;
-                uint8_t* dst = ubuf + (size_t) b * unit_bytes;
-                mbar_expect_tx(&u_full[b], bytes);
-                // the window starts at a multiple of 4 floats at or left of the first tap
-                for (int kd = 0; kd < g.f[0] && !WG_DBG(4); ++kd)
-#pragma unroll
-                    for (int h = 0; h < SW; ++h)
-                        tma_load_5d(dst + ((size_t) kd * g.xplane_floats + (size_t) h * g.xhalf_floats) * 4, &xmap,
-                                    ow0 * SW + g.lx + h * 128, oh * g.stride[1] - g.pad[1],
-                                    od * g.stride[0] - g.pad[0] + kd, 0, n, &u_full[b]);
-                tma_load_5d(dst + g.xbuf_bytes, &dymap, ow0, oh, od, 0, n, &u_full[b]);
-            }
-            __syncwarp();
-        }
-    }
-    else if ((warp >= TC_MMA_WARP && warp < TC_MMA_WARP + 3) || warp >= WG_ISSUER2_WARP)
-    {
-        // ------------------------------------------------------------------
-        // MMA issue: issuer (mq, mh) serves slot mq + 3 * mh, i.e. every
-        // WG_SPG-th chunk of group mq
-        // ------------------------------------------------------------------
-        const int mq = warp < WG_ISSUER2_WARP ? warp - TC_MMA_WARP : (warp - WG_ISSUER2_WARP) % 3;
-        const int mh = warp < WG_ISSUER2_WARP ? 0 : 1 + (warp - WG_ISSUER2_WARP) / 3;
-        // fp32 accumulate, tf32 x tf32, A K-major (tensor memory), B K-major, M = 128
-        const uint32_t idesc32 = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 4) << 24) | ((32u >> 3) << 17);
-        const uint32_t idesc16 = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 4) << 24) | ((16u >> 3) << 17);
-        int lap = 0;
-        uint32_t full_phase = 0, seq = 0, ul = 0;
-        bool open = false; // a batch this issuer has added into and not yet handed over
-        uint32_t batch = 0;
-        for (uint32_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++ul)
-        {
-            batch = ul / WG_FLUSH_UNITS;
-            const uint32_t db = batch & 1;
-            if (ul % WG_FLUSH_UNITS == 0)
-            {
-                // the buffer must have been drained and zeroed (initially: zeroed)
-                ok = mbar_wait_t<0>(&d_empty[db], (batch >> 1) & 1, abort_flag);
-                if (!ok)
-                    break;
-                open = true;
-            }
-            const uint32_t d_addr = tmem_base + db * 32u;
-            int q = (mq + 3 - (int) (seq % 3u)) % 3;
-            for (; q < WG_CHUNKS && ok; q += 3)
-            {
-                const int slot = mq + 3 * lap;
-                if (lap == mh)
-                    ok = mbar_wait_t<0>(&a_full[slot], full_phase, abort_flag);
-                if (!ok)
-                    break;
-                tc_fence_after();
-                if (lane == 0 && lap == mh)
-                {
-                    const uint32_t a_addr = tmem_base + (uint32_t) WG_ACC_COLS + (uint32_t) (slot * WG_A_COLS);
-                    // B tile of a k-step: [2 k-chunks][4 filter groups][8][4]: 512 bytes
-                    // between the k-chunks, 128 between the filter groups, 1 KiB per tile
-                    const uint64_t bd = make_desc(smem_u32(bring + slot * WG_B_FLOATS), 512u, 128u, 0u);
-#pragma unroll
-                    for (int ks = 0; ks < WG_KS && !WG_DBG(3); ++ks)
-                    {
-                        mma_tf32_ts(d_addr, a_addr + (uint32_t) (ks * 16), bd + (uint64_t) (ks * 64),
-                                    idesc32); // A_hi x [B_hi | B_lo]
-                        mma_tf32_ts(d_addr, a_addr + (uint32_t) (ks * 16 + 8), bd + (uint64_t) (ks * 64),
-                                    idesc16); // A_lo x B_hi
-                    }
-                    mma_commit(&a_empty[slot]);
-                    tc_fence_before();
-                }
-                __syncwarp();
-                if (++lap == WG_SPG)
-                {
-                    lap = 0;
-                    full_phase ^= 1;
-                }
-            }
-            seq += WG_CHUNKS;
-            if (ok && ul % WG_FLUSH_UNITS == WG_FLUSH_UNITS - 1)
-            {
-                // this issuer's share of the batch has completed when this arrives
-                if (lane == 0)
-                    mma_commit(&d_full[db]);
-                __syncwarp();
-                open = false;
-            }
-        }
-        if (ok && open)
-        {
-            if (lane == 0)
-                mma_commit(&d_full[batch & 1]);
-            __syncwarp();
-        }
-    }
-    else if (warp >= WG_DUMP_WARP)
-    {
-        // ------------------------------------------------------------------
-        // dump warps: zero both buffers, then per batch add the buffer into
-        // fp64 registers (D[:, 0:16] + D[:, 16:32]) and zero it again; at the
-        // end write the CTA's partial filter
-        // ------------------------------------------------------------------
-        const int quad = warp & 3;
-        const uint32_t la = tmem_base + ((uint32_t) (quad * 32) << 16);
-        for (int col = 0; col < WG_ACC_COLS; col += 16)
-            tmem_st16_zero(la + col);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0)
-        {
-            mbar_arrive(&d_empty[0]);
-            mbar_arrive(&d_empty[1]);
-        }
-        double acc[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k)
-            acc[k] = 0.0;
-        uint32_t my_units = 0;
-        for (uint32_t u = blockIdx.x; u < nunits; u += gridDim.x)
-            ++my_units;
-        const uint32_t nbatches = (my_units + WG_FLUSH_UNITS - 1) / WG_FLUSH_UNITS;
-        for (uint32_t bt = 0; bt < nbatches && ok; ++bt)
-        {
-            const uint32_t db = bt & 1;
-            ok = mbar_wait(&d_full[db], (bt >> 1) & 1, abort_flag);
+            ok = mbar_wait_t<500>(chain_end, par, abort_flag);
             if (!ok)
                 break;
             tc_fence_after();
-            uint32_t v0[16], v1[16];
-            tmem_ld16(la + db * 32u, v0);
-            tmem_ld16(la + db * 32u + 16u, v1);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            tmem_st16_zero(la + db * 32u);
-            tmem_st16_zero(la + db * 32u + 16u);
+#pragma unroll 1
+            for (int i = 0; i < total; ++i)
+            {
+                const int block = i / pieces, p8 = (i - block * pieces) * 8;
+                const uint32_t d = la + (uint32_t) (block / g.nblocks * g.kd_cols + block % g.nblocks * g.n8 + p8);
+                const uint32_t r = la + (uint32_t) (g.sum_col + block * g.kgp + p8);
+                float a[8], b[8];
+                tmem_ld8(d, a);
+                tmem_ld8(r, b);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                uint32_t v[8], z[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    v[j] = __float_as_uint(a[j] + b[j]), z[j] = 0u;
+                tmem_st8(r, v);
+                tmem_st8(d, z);
+            }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
-                mbar_arrive(&d_empty[db]);
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                acc[k] += (double) __uint_as_float(v0[k]) + (double) __uint_as_float(v1[k]);
+                mbar_arrive(cleared);
         }
-        if (ok)
+    }
+    else if (warp < WG_ISSUE_WARP)
+    {
+        const int w = warp - WG_FLUSH;
+        const bool isx = w < g.warps_x;
+        const WgConvArgs c = {smem_u32(smem), smem_u32(full), smem_u32(empty), isx ? itab : itab + g.items_x,
+                              isx ? g.items_x : g.items_y, isx ? g.warps_x : WG_CONV - g.warps_x, rc, rkw, rkd, rk, s0, s1,
+                              isx ? w : w - g.warps_x, lane, abort_flag};
+        if (c.w < c.items)
         {
-            float* o = part + ((size_t) blockIdx.x * 128 + quad * 32 + lane) * 16;
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                o[k] = (float) acc[k];
+            if (!isx)
+                ok = g.vec_y ? wg_convert<false, 1, 1, 0>(g, c, dy) : wg_convert<false, 1, 1, -1>(g, c, dy);
+            else
+                ok = wg_convert<true, SW, KWG, AL>(g, c, x);
+        }
+    }
+    else
+    {
+        // issuer
+        uint32_t elected;
+        asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+        const uint32_t base16 = smem_u32(smem) >> 4, dhi = 8u | (1u << 14); // SBO 128 bytes, descriptor version
+        const uint32_t lx = (uint32_t) g.lbo_x >> 4, ly = (uint32_t) g.lbo_y >> 4;
+        const int ksteps = g.Q / 2;
+        int buf = 0, left = g.flush_stages;
+        uint32_t par = 0, cpar = 0;
+#pragma unroll 1
+        for (int s = s0; s < s1 && ok; ++s)
+        {
+            if (left == 0)
+            {
+                if (elected)
+                    mma_commit(chain_end);
+                ok = mbar_wait_t<0>(cleared, cpar, abort_flag);
+                cpar ^= 1;
+                left = g.flush_stages;
+                if (!ok)
+                    break;
+            }
+            --left;
+            ok = mbar_wait_t<0>(&full[buf], par, abort_flag);
+            if (!ok)
+                break;
+            tc_fence_after();
+            const uint32_t a_st = base16 + (uint32_t) (buf * g.stage_bytes) / 16u, b_st = a_st + (uint32_t) g.y_off / 16u;
+            if (elected)
+            {
+#pragma unroll 1
+                for (int kd = 0; kd < g.kdg; ++kd)
+#pragma unroll 1
+                    for (int t = 0; t < g.ntiles; ++t)
+                    {
+                        const WgTile tl = tiles[t];
+                        uint32_t a = (a_st + tl.a16 + (uint32_t) (kd * g.kd_a16)) | lx << 16;
+                        uint32_t b = (b_st + tl.b16) | ly << 16;
+                        const uint32_t d = tmem + tl.dcol + (uint32_t) (kd * g.kd_cols);
+#pragma unroll 4
+                        for (int ks = 0; ks < ksteps; ++ks)
+                        {
+                            asm volatile("{\n\t.reg .pred t;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+                                         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, t;\n\t}" ::"r"(d),
+                                         "l"((uint64_t) dhi << 32 | a), "l"((uint64_t) dhi << 32 | b), "r"(tl.idesc));
+                            a += 2 * lx;
+                            b += 2 * ly;
+                        }
+                    }
+                mma_commit(&empty[buf]);
+                if (s + 1 == s1)
+                    mma_commit(chain_end);
+            }
+            __syncwarp();
+            if (++buf == g.nstages)
+            {
+                buf = 0;
+                par ^= 1;
+            }
         }
     }
 
+    // every role has left its loop (all waits are bounded and watch the abort
+    // flag); the last instructions' completion is one more phase of chain_end
+    __syncthreads();
+    if (ok && s1 > s0)
+        ok = mbar_wait(chain_end, (uint32_t) ((s1 - s0 - 1) / g.flush_stages) & 1, abort_flag);
+    tc_fence_after();
+    // reduction, one kd plane at a time: accumulators to shared memory (the
+    // stages' space) as [column][lane], then every output adds its pairs
+    float* dump = reinterpret_cast<float*>(smem);
+    const int fh = g.f[1], per_kd = g.kg * g.cg * fh * KWG;
+    float* out = part + (long long) blockIdx.x * g.kdg * per_kd;
+#pragma unroll 1
+    for (int kd = 0; kd < g.kdg; ++kd)
+    {
+        if (warp < WG_FLUSH)
+        {
+            const uint32_t la = tmem + ((uint32_t) ((warp & 3) * 32) << 16);
+            const int l = (warp & 3) * 32 + lane;
+#pragma unroll 1
+            for (int c8 = 0; c8 < g.nblocks * g.n8; c8 += 8)
+            {
+                float a[8], b[8];
+                tmem_ld8(la + (uint32_t) (kd * g.kd_cols + c8), a);
+                const int block = c8 / g.n8, in = c8 - block * g.n8;
+                if (in < g.kgp)
+                    tmem_ld8(la + (uint32_t) (g.sum_col + (kd * g.nblocks + block) * g.kgp + in), b);
+                else
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        b[j] = 0.f;
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    dump[(c8 + j) * 128 + l] = a[j] + b[j];
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int e = tid; e < per_kd; e += WG_THREADS)
+        {
+            // lanes of a warp walk (kw, c): neighbouring columns of shared memory
+            const int c = e % g.cg, kw = e / g.cg % KWG, kh = e / (g.cg * KWG) % fh, k = e / (g.cg * KWG * fh);
+            double sum = 0.0;
+#pragma unroll 1
+            for (int r = 0; r < g.nclasses; ++r)
+#pragma unroll 1
+                for (int al = 0; al < g.A; ++al)
+                {
+                    const int num = r + al - kh;
+                    int delta = num;
+                    if (g.stride[1] == 2)
+                    {
+                        if (num & 1)
+                            continue;
+                        delta = num >> 1;
+                    }
+                    const int i = delta - g.class_lo[r];
+                    if (i < 0 || i >= g.class_n[r])
+                        continue;
+                    const float* col = dump + (g.class_col[r] + i * g.n8 + k) * 128 + al * g.r8 + kw * g.cg + c;
+                    const int lo_k = g.kgp * 128, lo_x = KWG * g.cg;
+                    sum += (double) col[0] + ((double) col[lo_x] + (double) col[lo_k]) + (double) col[lo_k + lo_x];
+                }
+            out[(((long long) k * g.cg + c) * g.kdg + kd) * fh * KWG + kh * KWG + kw] = (float) sum;
+        }
+        __syncthreads();
+    }
     if (!ok && lane == 0)
         atomicExch(status, 1);
     tc_fence_before();
     __syncthreads();
-    if (warp == TC_MMA_WARP)
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
+}
+
+template <int SW, int KWG, int AL>
+int32_t wg_launch(const WgGeom& g, int rkw, const float* x, const float* dy, float* part, int* status, cudaStream_t stream)
+{
+    auto kernel = wg_conv_kernel<SW, KWG, AL>;
+    const size_t smem = g.smem < 120 * 1024 ? 120 * 1024 : (size_t) g.smem; // one CTA per SM: it owns all of tensor memory
+    DCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    kernel<<<(unsigned) (g.roles * g.parts), WG_THREADS, smem, stream>>>(g, x, dy, part, status, rkw);
+    DCB_LAUNCH_CHECK();
+    return DCB_OK;
+}
+
+template <int SW, int KWG>
+int32_t wg_launch_at(const WgGeom& g, int al, int rkw, const float* x, const float* dy, float* part, int* status,
+                     cudaStream_t stream)
+{
+    switch (al)
     {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(WG_TMEM_COLS)
-                     : "memory");
+    case 0: return wg_launch<SW, KWG, 0>(g, rkw, x, dy, part, status, stream);
+    case 1: return wg_launch<SW, KWG, 1>(g, rkw, x, dy, part, status, stream);
+    case 2: return wg_launch<SW, KWG, 2>(g, rkw, x, dy, part, status, stream);
+    case 3: return wg_launch<SW, KWG, 3>(g, rkw, x, dy, part, status, stream);
+    default: return wg_launch<SW, KWG, -1>(g, rkw, x, dy, part, status, stream);
     }
 }
 
-} // namespace
 } // namespace dcb

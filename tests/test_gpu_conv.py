@@ -591,3 +591,33 @@ def test_shift_kernel_tile_and_table_edges(geom):
     dx_ref = np.zeros_like(x)
     O.conv_bwd_data(w, dy, dx_ref, pads, strides)
     emu.assert_close(dx, 0.5 * dx_ref - dx0, TOL, "dx")
+
+
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, stride: edges of the backward filter's stages and roles
+    (1, 4, 16, (5, 7, 32), (3, 3, 3), 1),      # one stage wide, rows left over
+    (2, 3, 5, (3, 4, 33), (3, 3, 3), 1),       # rows no vector load can read, filters padded to 8
+    (1, 33, 9, (9, 40), (3, 3), 1),            # channels in roles
+    (1, 20, 40, (6, 6, 24), (3, 3, 3), 1),     # channels, planes kd and filters in roles
+    (1, 32, 32, (21, 70), (5, 5), 1),          # five taps along W
+    (1, 31, 7, (15, 67), (5, 5), 2),           # stride 2 with five taps
+    (2, 2, 3, (11, 18), (2, 2), 2),            # two taps
+    (1, 2, 3, (12, 36), (7, 7), 1),            # more taps than one launch takes
+    (4, 1, 4, (200, 130), (3, 3), 1),          # long sums: running sums used
+])
+def test_backward_filter_stage_and_role_edges(geom):
+    N, C, K, sp, f, s = geom
+    rng = np.random.default_rng(sum(sp) + K)
+    nsd, pads, strides = len(sp), [(e - 1) // 2 for e in f], [s] * len(sp)
+    x = rng.normal(0.2, 1, (N, C, *sp)).astype(np.float32)
+    w = np.zeros((K, C, *f), np.float32)
+    dy = rng.normal(0.1, 1, (N, K, *[O.conv_out_extent(i, ff, p, s, 1) for i, ff, p in zip(sp, f, pads)])).astype(np.float32)
+    xs, ws, dys = (torch.from_numpy(a).cuda() for a in (x, w, dy))
+    dw = torch.from_numpy(rng.normal(size=w.shape).astype(np.float32)).cuda()
+    dw0 = dw.cpu().numpy()
+    p = Plan(xs, ws, dys, pads, strides, [1] * nsd, _abi.MATH_FP32)
+    assert _abi.lib().dcb_conv_plan_kernel_kind(p.p, 2) == 1
+    p.bwd_filter(0.5, xs, dys, -2.0, dw)
+    torch.cuda.synchronize()
+    assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.OK
+    emu.assert_close(dw.cpu().numpy(), 0.5 * O.conv_bwd_filter(x, dy, f, pads, strides) - 2.0 * dw0, TOL, "dw")
