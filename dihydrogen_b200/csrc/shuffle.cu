@@ -30,10 +30,13 @@ namespace
 {
 
 constexpr int SHF_THREADS = 256;
+constexpr int SHF_UNROLL = 4;                           // accesses of a thread in flight
+constexpr int SHF_CHUNK = SHF_THREADS * SHF_UNROLL;     // accesses of a unit
 constexpr int SHF_MAX_RANKS = 64;
 constexpr size_t SHF_HEADER = 1024; // 64 flags, ticket, status
 
-// One box to move: `rows` runs of `len` contiguous cells.  Row r decodes into
+// One box to move: `rows` runs of `len` contiguous cells.  Dimensions that are
+// contiguous on both sides have been merged into the run.  Row r decodes into
 // (i1, i2, i3, i4) over ext[1..4]; its first cell sits at
 // a_off + sum i_k * a_stride[k] on the strided side and at
 // b_off + sum i_k * b_stride[k] on the dense side.
@@ -46,15 +49,20 @@ struct ShfJob
     float* peer;            // put: the destination's window (parity 0)
     long long parity_pitch; // put: floats between the two halves of that window
     uint32_t* flag;         // put: flag to publish there; wait: own flag to wait on
+    int vec;                // 16-byte accesses: offsets, strides and run allow them (if the bases do)
+    int split;              // long runs, in units of SHF_CHUNK accesses of one run; else units of that many accesses
+    long long units[2];     // per access width (4-byte, 16-byte)
+    long long per_run[2];   // accesses of a run
+    FastDiv by_run[2], by_ext[4];
 };
 
 struct ShfArgs
 {
     const ShfJob* jobs;
     int njobs;
-    long long total_rows;
     float* tensor;
     float* window; // wait_unpack: own window of this parity
+    int aligned;   // tensor starts on a 16-byte boundary (windows always do)
     int parity;    // put: which half of the destination windows
     uint32_t epoch;
     uint32_t* ticket;
@@ -62,22 +70,73 @@ struct ShfArgs
     long long budget_ns;
 };
 
-__device__ __forceinline__ void shf_locate(const ShfJob& j, long long r, long long* a, long long* b)
+template <class T>
+__device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, int wide, const float* from, float* to,
+                                         const long long* fs, const long long* ts, long long fo, long long to_off)
 {
-    long long ao = j.a_off, bo = j.b_off;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
+    constexpr int W = sizeof(T) / 4;
+    T v[SHF_UNROLL];
+    T* dst[SHF_UNROLL];
+    if (j.split)
     {
-        const long long i = r % j.ext[k];
-        r /= j.ext[k];
-        ao += i * j.a_stride[k];
-        bo += i * j.b_stride[k];
+        // SHF_CHUNK accesses of one long run
+        const long long cpr = (j.per_run[wide] + SHF_CHUNK - 1) / SHF_CHUNK;
+        long long r = u / cpr;
+        const long long e0 = (u - r * cpr) * SHF_CHUNK;
+        long long f = fo, t = to_off;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            const long long i = r % j.ext[k];
+            r /= j.ext[k];
+            f += i * fs[k];
+            t += i * ts[k];
+        }
+#pragma unroll
+        for (int k = 0; k < SHF_UNROLL; ++k)
+        {
+            const long long e = e0 + threadIdx.x + k * SHF_THREADS;
+            dst[k] = e < j.per_run[wide] ? reinterpret_cast<T*>(to + t) + e : nullptr;
+            if (dst[k] != nullptr)
+                v[k] = __ldcs(reinterpret_cast<const T*>(from + f) + e);
+        }
     }
-    *a = ao;
-    *b = bo;
+    else
+    {
+        const long long total = j.rows * j.per_run[wide];
+#pragma unroll
+        for (int k = 0; k < SHF_UNROLL; ++k)
+        {
+            const long long n = u * SHF_CHUNK + threadIdx.x + k * SHF_THREADS;
+            dst[k] = nullptr;
+            if (n < total)
+            {
+                uint32_t r = j.by_run[wide].div((uint32_t) n);
+                const uint32_t e = (uint32_t) n - r * j.by_run[wide].d;
+                long long f = fo + (long long) e * W, t = to_off + (long long) e * W;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                {
+                    const uint32_t d = j.by_ext[q].div(r), i = r - d * j.by_ext[q].d;
+                    r = d;
+                    f += (long long) i * fs[q];
+                    t += (long long) i * ts[q];
+                }
+                dst[k] = reinterpret_cast<T*>(to + t);
+                v[k] = __ldcs(reinterpret_cast<const T*>(from + f));
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < SHF_UNROLL; ++k)
+        if (dst[k] != nullptr)
+            *dst[k] = v[k];
 }
 
 // PUT: tensor (strided) -> peers' windows (dense).  !PUT: own window -> tensor.
+// A unit is SHF_CHUNK accesses, all loads of a thread before its stores.  A warp per
+// W run, decoded with eight run-time divisions and one access in flight per lane, took
+// 100 us for 134 MB.
 template <bool PUT>
 __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
 {
@@ -98,46 +157,39 @@ __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
             return;
         }
     }
-    // a warp per row: consecutive lanes move consecutive cells
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = SHF_THREADS / 32;
-    for (long long u = (long long) blockIdx.x * wpb + warp; u < a.total_rows; u += (long long) gridDim.x * wpb)
+    __shared__ ShfJob j;
+    long long u = blockIdx.x;
+    for (int q = 0; q < a.njobs; ++q)
     {
-        long long r = u;
-        int q = 0;
-        while (r >= a.jobs[q].rows)
+        __syncthreads();
+        for (int i = threadIdx.x; i < (int) (sizeof(ShfJob) / 4); i += SHF_THREADS)
+            reinterpret_cast<uint32_t*>(&j)[i] = reinterpret_cast<const uint32_t*>(&a.jobs[q])[i];
+        __syncthreads();
+        const int wide = j.vec && a.aligned ? 1 : 0;
+        float* w = PUT ? j.peer + a.parity * j.parity_pitch : a.window;
+        const float* from = PUT ? a.tensor : w;
+        float* to = PUT ? w : a.tensor;
+        const long long* fs = PUT ? j.a_stride : j.b_stride;
+        const long long* ts = PUT ? j.b_stride : j.a_stride;
+        const long long fo = PUT ? j.a_off : j.b_off, too = PUT ? j.b_off : j.a_off;
+        for (; u < j.units[wide]; u += gridDim.x)
         {
-            r -= a.jobs[q].rows;
-            ++q;
+            if (wide)
+                shf_unit<float4>(j, u, 1, from, to, fs, ts, fo, too);
+            else
+                shf_unit<float>(j, u, 0, from, to, fs, ts, fo, too);
         }
-        const ShfJob& j = a.jobs[q];
-        long long ao, bo;
-        shf_locate(j, r, &ao, &bo);
-        float* t = a.tensor + ao;
-        float* w = (PUT ? j.peer + a.parity * j.parity_pitch : a.window) + bo;
-        const float* from = PUT ? t : w;
-        float* to = PUT ? w : t;
-        if ((j.len & 3) == 0 && ((reinterpret_cast<uintptr_t>(from) | reinterpret_cast<uintptr_t>(to)) & 15) == 0)
-        {
-            // 16-byte accesses where the run allows them
-            const float4* f4 = reinterpret_cast<const float4*>(from);
-            float4* t4 = reinterpret_cast<float4*>(to);
-            for (long long e = lane; e < j.len / 4; e += 32)
-                t4[e] = f4[e];
-        }
-        else
-        {
-            for (long long e = lane; e < j.len; e += 32)
-                to[e] = from[e];
-        }
+        u -= j.units[wide];
     }
     if (PUT)
     {
-        // every thread makes its peer stores visible system-wide, then the last
-        // block to arrive release-stores the epoch at every destination
-        __threadfence_system();
+        // the block's peer stores become visible system-wide (the barrier orders them
+        // before the first thread's fence), then the last block to arrive
+        // release-stores the epoch at every destination
         __syncthreads();
         if (threadIdx.x == 0)
         {
+            __threadfence_system();
             const unsigned prev = atomicAdd(a.ticket, 1u);
             if (prev == gridDim.x - 1)
             {
@@ -147,6 +199,54 @@ __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
                     st_release_sys(a.jobs[q].flag, a.epoch);
             }
         }
+    }
+}
+
+// Merges what is contiguous on both sides into the run and derives how the job is
+// walked.
+void finish_job(ShfJob* j)
+{
+    int n = 0;
+    long long ext[4], as[4], bs[4];
+    bool run = true;
+    for (int k = 0; k < 4; ++k)
+    {
+        if (j->ext[k] == 1)
+            continue;
+        if (run && j->a_stride[k] == j->len && j->b_stride[k] == j->len)
+        {
+            j->len *= j->ext[k];
+            continue;
+        }
+        run = false;
+        if (n > 0 && j->a_stride[k] == as[n - 1] * ext[n - 1] && j->b_stride[k] == bs[n - 1] * ext[n - 1])
+        {
+            ext[n - 1] *= j->ext[k];
+            continue;
+        }
+        ext[n] = j->ext[k], as[n] = j->a_stride[k], bs[n] = j->b_stride[k];
+        ++n;
+    }
+    long long mix = j->len | j->a_off | j->b_off;
+    j->rows = 1;
+    for (int k = 0; k < 4; ++k)
+    {
+        j->ext[k] = k < n ? ext[k] : 1;
+        j->a_stride[k] = k < n ? as[k] : 0;
+        j->b_stride[k] = k < n ? bs[k] : 0;
+        j->rows *= j->ext[k];
+        mix |= j->a_stride[k] | j->b_stride[k];
+        j->by_ext[k] = FastDiv::of((uint32_t) j->ext[k]);
+    }
+    j->vec = (mix & 3) == 0;
+    // runs of at least two units, or too many accesses for 31-bit indices
+    j->split = j->len / (j->vec ? 4 : 1) >= 2 * SHF_CHUNK || j->rows * j->len >= 2000000000ll;
+    for (int w = 0; w < 2; ++w)
+    {
+        j->per_run[w] = j->len / (w ? 4 : 1);
+        j->by_run[w] = FastDiv::of(j->per_run[w] > 0 && j->per_run[w] < (1 << 30) ? (uint32_t) j->per_run[w] : 1u);
+        j->units[w] = j->split ? j->rows * ((j->per_run[w] + SHF_CHUNK - 1) / SHF_CHUNK)
+                               : (j->rows * j->per_run[w] + SHF_CHUNK - 1) / SHF_CHUNK;
     }
 }
 
@@ -213,7 +313,7 @@ struct dcb_shuffle_plan
     ShfJob* d_put = nullptr;
     ShfJob* d_wait = nullptr;
     int n_put = 0, n_wait = 0;
-    long long put_rows = 0, wait_rows = 0;
+    long long put_units = 0, wait_units = 0;
     uint32_t epoch = 0;
     bool connected = false;
 
@@ -337,7 +437,7 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
     const Box& my_src = p->src_boxes[p->rank];
     const Box& my_dst = p->dst_boxes[p->rank];
     std::vector<ShfJob> put, wait;
-    p->put_rows = p->wait_rows = 0;
+    p->put_units = p->wait_units = 0;
     for (int r = 0; r < nranks; ++r)
     {
         Box x;
@@ -383,8 +483,9 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
             j.peer = reinterpret_cast<float*>(base + SHF_HEADER);
             j.parity_pitch = (long long) b.parity_floats;
             j.flag = reinterpret_cast<uint32_t*>(base) + p->rank; // my slot among r's flags
+            finish_job(&j);
             put.push_back(j);
-            p->put_rows += j.rows;
+            p->put_units += j.units[j.vec];
         }
         // what rank r holds of my destination block
         if (my_dst.volume() > 0 && p->src_boxes[r].volume() > 0 && intersect(p->src_boxes[r], my_dst, &x))
@@ -411,8 +512,9 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
             }
             j.peer = nullptr;
             j.flag = p->flags() + r;
+            finish_job(&j);
             wait.push_back(j);
-            p->wait_rows += j.rows;
+            p->wait_units += j.units[j.vec];
         }
     }
     cudaFree(p->d_put);
@@ -434,11 +536,10 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
     return DCB_OK;
 }
 
-static unsigned shf_grid(long long rows)
+static unsigned shf_grid(long long units)
 {
-    const long long want = (rows + SHF_THREADS / 32 - 1) / (SHF_THREADS / 32);
     const long long cap = (long long) num_sms() * 8;
-    return (unsigned) (want < 1 ? 1 : (want > cap ? cap : want));
+    return (unsigned) (units < 1 ? 1 : (units > cap ? cap : units));
 }
 
 int32_t dcb_shuffle_put(dcb_shuffle_plan* p, const void* src, void* stream)
@@ -457,14 +558,14 @@ int32_t dcb_shuffle_put(dcb_shuffle_plan* p, const void* src, void* stream)
     std::memset(&a, 0, sizeof(a));
     a.jobs = p->d_put;
     a.njobs = p->n_put;
-    a.total_rows = p->put_rows;
+    a.aligned = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
     a.tensor = const_cast<float*>(static_cast<const float*>(src));
     a.parity = (int) (p->epoch & 1u);
     a.epoch = p->epoch;
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    shuffle_kernel<true><<<shf_grid(p->put_rows), SHF_THREADS, 0, as_stream(stream)>>>(a);
+    shuffle_kernel<true><<<shf_grid(p->put_units), SHF_THREADS, 0, as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;
 }
@@ -484,14 +585,14 @@ int32_t dcb_shuffle_wait_unpack(dcb_shuffle_plan* p, void* dst, void* stream)
     std::memset(&a, 0, sizeof(a));
     a.jobs = p->d_wait;
     a.njobs = p->n_wait;
-    a.total_rows = p->wait_rows;
+    a.aligned = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
     a.tensor = static_cast<float*>(dst);
     a.window = p->window() + (long long) (p->epoch & 1u) * p->parity_floats;
     a.epoch = p->epoch;
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    shuffle_kernel<false><<<shf_grid(p->wait_rows), SHF_THREADS, 0, as_stream(stream)>>>(a);
+    shuffle_kernel<false><<<shf_grid(p->wait_units), SHF_THREADS, 0, as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;
 }
