@@ -304,6 +304,19 @@ __global__ void __launch_bounds__(BN_THREADS)
     });
 }
 
+// Operation order of sums_to_statistics_functor (batchnorm.cu:297-312).
+__device__ __forceinline__ void sums_to_statistics(long long num_per_sum, float& sum, float& sqsum)
+{
+    const float nps = (float) num_per_sum;
+    const float m = sum / nps;
+    const float sq = sqsum / nps;
+    float v = sq - m * m;
+    v = v > 0.f ? v : 0.f;
+    v *= nps / (nps - 1.f);
+    sum = m;
+    sqsum = v;
+}
+
 __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
                                    float decay, float* mean, float* var,
                                    float* running_mean, float* running_var)
@@ -313,13 +326,8 @@ __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
         return;
     if (num_per_sum > 0)
     {
-        // Operation order of sums_to_statistics_functor (batchnorm.cu:297-312).
-        const float nps = (float) num_per_sum;
-        const float m = mean[c] / nps;
-        const float sq = var[c] / nps;
-        float v = sq - m * m;
-        v = v > 0.f ? v : 0.f;
-        v *= nps / (nps - 1.f);
+        float m = mean[c], v = var[c];
+        sums_to_statistics(num_per_sum, m, v);
         mean[c] = m;
         var[c] = v;
         running_mean[c] = decay * running_mean[c] + (1.f - decay) * m;
@@ -331,20 +339,60 @@ __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
     }
 }
 
+// What bn_finalize_kernel does, by the apply kernel itself: every block turns its
+// channel's sums into statistics, the last one of the channel to arrive (nobody reads
+// the sums any more then) writes them back.  One launch less between a small layer's
+// statistics and its output.
+struct FinalizeArgs
+{
+    long long num_per_sum;
+    float decay;
+    float *mean, *var, *running_mean, *running_var; // sums in, statistics out
+    unsigned* tickets;
+};
+
 // LEAKY: the leaky ReLU that follows the batch-norm in the same pass
 // (y > 0 ? y : slope * y), one trip through HBM instead of two.
-template <int V, bool LEAKY, bool PACKED>
+template <int V, bool LEAKY, bool PACKED, bool FINALIZE>
 __global__ void __launch_bounds__(BN_THREADS)
     bn_apply_kernel(const float* __restrict__ x, RunStrides xs,
                     float* __restrict__ y, RunStrides ys, UnitGeom ug,
-                    const float* __restrict__ mean,
-                    const float* __restrict__ var,
+                    const float* mean, const float* var,
                     const float* __restrict__ scale,
-                    const float* __restrict__ bias, float eps, float slope)
+                    const float* __restrict__ bias, float eps, float slope,
+                    FinalizeArgs fin)
 {
     const int c = blockIdx.y;
-    const float m = mean[c];
-    const float inv_stdev = rsqrtf(var[c] + eps);
+    float m, v0;
+    if (FINALIZE)
+    {
+        // one thread reads the sums, so that it knows when the block has them
+        __shared__ float stat[2];
+        if (threadIdx.x == 0)
+        {
+            float a = fin.mean[c], b = fin.var[c];
+            sums_to_statistics(fin.num_per_sum, a, b);
+            stat[0] = a;
+            stat[1] = b;
+        }
+        __syncthreads();
+        m = stat[0];
+        v0 = stat[1];
+        if (threadIdx.x == 0 && atomicAdd(&fin.tickets[c], 1u) == gridDim.x - 1)
+        {
+            fin.tickets[c] = 0;
+            fin.mean[c] = m;
+            fin.var[c] = v0;
+            fin.running_mean[c] = fin.decay * fin.running_mean[c] + (1.f - fin.decay) * m;
+            fin.running_var[c] = fin.decay * fin.running_var[c] + (1.f - fin.decay) * v0;
+        }
+    }
+    else
+    {
+        m = mean[c];
+        v0 = var[c];
+    }
+    const float inv_stdev = rsqrtf(v0 + eps);
     const float sc = scale[c], bi = bias[c];
     for (long long u = blockIdx.x; u < ug.upc; u += gridDim.x)
     {
@@ -719,7 +767,7 @@ int32_t dcb_bn_finalize(int32_t channels, int64_t num_per_sum, float decay,
 
 static int32_t bn_apply_impl(const dcb_nd_desc* xd, const void* x, const void* mean, const void* var,
                              const void* scale, const void* bias, float eps, bool leaky, float slope,
-                             const dcb_nd_desc* yd, void* y, void* stream)
+                             const dcb_nd_desc* yd, void* y, void* stream, const FinalizeArgs* fin = nullptr)
 {
     DCB_REQUIRE(x && y && mean && var && scale && bias, "null argument");
     const dcb_nd_desc* descs[2] = {xd, yd};
@@ -731,23 +779,36 @@ static int32_t bn_apply_impl(const dcb_nd_desc* xd, const void* x, const void* m
     if (mv.ug.upc == 0)
         return DCB_OK;
     const dim3 grid = bn_grid(mv.ug);
-#define CALL(VV, PP)                                                               \
-    if (leaky)                                                                 \
-        bn_apply_kernel<VV, true, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>( \
-            static_cast<const float*>(x), mv.s[0], static_cast<float*>(y),     \
-            mv.s[1], mv.ug, static_cast<const float*>(mean),                   \
-            static_cast<const float*>(var), static_cast<const float*>(scale),  \
-            static_cast<const float*>(bias), eps, slope);                      \
-    else                                                                       \
-        bn_apply_kernel<VV, false, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(\
-            static_cast<const float*>(x), mv.s[0], static_cast<float*>(y),     \
-            mv.s[1], mv.ug, static_cast<const float*>(mean),                   \
-            static_cast<const float*>(var), static_cast<const float*>(scale),  \
-            static_cast<const float*>(bias), eps, slope)
+    const FinalizeArgs f = fin ? *fin : FinalizeArgs();
+#define CALL(VV, PP)                                                                                               \
+    {                                                                                                              \
+        auto kernel = leaky ? (fin ? bn_apply_kernel<VV, true, PP, true> : bn_apply_kernel<VV, true, PP, false>)   \
+                            : (fin ? bn_apply_kernel<VV, false, PP, true> : bn_apply_kernel<VV, false, PP, false>); \
+        kernel<<<grid, BN_THREADS, 0, as_stream(stream)>>>(                                                        \
+            static_cast<const float*>(x), mv.s[0], static_cast<float*>(y), mv.s[1], mv.ug,                         \
+            static_cast<const float*>(mean), static_cast<const float*>(var), static_cast<const float*>(scale),     \
+            static_cast<const float*>(bias), eps, slope, f);                                                       \
+    }
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
     return DCB_OK;
+}
+
+int32_t dcb_bn_finalize_apply(dcb_bn_plan* plan, int64_t num_per_sum, float decay, void* mean, void* var,
+                              void* running_mean, void* running_var, const dcb_nd_desc* xd, const void* x,
+                              const void* scale, const void* bias, float eps, float slope, const dcb_nd_desc* yd, void* y,
+                              void* stream)
+{
+    DCB_REQUIRE(plan && running_mean && running_var && num_per_sum > 0, "null argument");
+    int32_t st = check_nd_desc(xd);
+    if (st != DCB_OK)
+        return st;
+    DCB_REQUIRE(xd->c == plan->xd.c && xd->n * xd->dims[0] * xd->dims[1] * xd->dims[2] > 0,
+                "the plan is for another channel count, or the shard is empty");
+    const FinalizeArgs f = {num_per_sum, decay, static_cast<float*>(mean), static_cast<float*>(var),
+                            static_cast<float*>(running_mean), static_cast<float*>(running_var), plan->tickets};
+    return bn_apply_impl(xd, x, mean, var, scale, bias, eps, slope != 1.f, slope, yd, y, stream, &f);
 }
 
 int32_t dcb_bn_apply(const dcb_nd_desc* xd, const void* x, const void* mean,

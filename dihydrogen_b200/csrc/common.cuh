@@ -64,6 +64,41 @@ inline cudaStream_t as_stream(void* s)
 }
 
 int num_sms();
+
+// Raises a kernel's limit of dynamic shared memory, once per kernel and device.
+int32_t allow_dynamic_smem(const void* kernel, int bytes);
+
+// Launches a kernel that may start while the kernel before it in the stream is still
+// running (once all of that one's blocks have called dependents_may_start or ended).
+// Whatever it does with that kernel's results, or over its operands, comes after
+// wait_for_previous_kernel.
+template <class... Params, class... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem,
+                                     cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+__device__ __forceinline__ void dependents_may_start()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+__device__ __forceinline__ void wait_for_previous_kernel()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 int64_t wait_budget_ns();
 
 // ---------------------------------------------------------------------------

@@ -564,7 +564,9 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
     if (!xiss)
         g.a_slots = g.groups;
     auto launch = [&](auto kernel, int xi) -> int32_t {
-        DCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (224 * 1024)));
+        const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 224 * 1024);
+        if (set != DCB_OK)
+            return set;
         kernel<<<(unsigned) grid, sw_threads(xi), smem, stream>>>(g, alpha, p->sw_bimg, y, status, map, ymap, use_ymap,
                                                                   p->stat_part);
         DCB_LAUNCH_CHECK();
@@ -592,6 +594,7 @@ static __global__ void __launch_bounds__(256) wg_fold_kernel(const __grid_consta
     const int e = (int) (blockIdx.x * 32 + threadIdx.x / 8), sub = threadIdx.x & 7;
     const bool on = e < g.k * g.c * taps;
     double s = 0.0;
+    wait_for_previous_kernel();
     if (on)
     {
         const int kw = e % g.f[2], kh = e / g.f[2] % g.f[1], kd = e / (g.f[2] * g.f[1]) % g.f[0];
@@ -635,8 +638,8 @@ int32_t tc_conv_bwd_filter(TcPlan* p, float alpha, const float* x, const float* 
             return st;
     }
     const int total = g.k * g.c * g.f[0] * g.f[1] * g.f[2];
-    wg_fold_kernel<<<(unsigned) ((total + 31) / 32), 256, 0, stream>>>(g, p->wg_part, alpha, beta, dw);
-    DCB_LAUNCH_CHECK();
+    DCB_CUDA_TRY(launch_overlapped(wg_fold_kernel, dim3((unsigned) ((total + 31) / 32)), 256, 0, stream, g, p->wg_part,
+                                   alpha, beta, dw));
     return DCB_OK;
 }
 

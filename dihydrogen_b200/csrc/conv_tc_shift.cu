@@ -28,6 +28,7 @@ __global__ void sh_pack_filter_kernel(const float* __restrict__ w, uint4* __rest
                                       int cpg, int cin, int kout, int kcols, long long w_ko, long long w_ci,
                                       uint32_t rnd_add, uint32_t rnd_mask, float alpha)
 {
+    dependents_may_start();
     const ShPack p = packs[blockIdx.y];
     const int kg = (int) blockIdx.z / cgroups, grp = (int) blockIdx.z % cgroups;
     uint4* o = out + (size_t) blockIdx.z * total16 + p.off16;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(SH_FOLD_WARPS * 32)
 {
     __shared__ double sm[SH_FOLD_WARPS][32];
     const int t = threadIdx.x & 31, w = threadIdx.x >> 5;
+    wait_for_previous_kernel();
     double acc = 0.0;
 #pragma unroll 4
     for (int i = w; i < nparts; i += SH_FOLD_WARPS)
@@ -833,10 +835,12 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
     const unsigned grid = std::min<unsigned>((unsigned) num_sms(), g.units);
     const size_t smem = std::max<size_t>(t.smem, 120 * 1024); // one CTA per SM: it owns all of tensor memory
     auto launch = [&](auto kernel) -> int32_t {
-        DCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        kernel<<<grid, SH_THREADS, smem, stream>>>(g, beta, x, p->image, p->tables, y, status, p->stat_part,
-                                                 ymap, use_ymap);
-        DCB_LAUNCH_CHECK();
+        const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 227 * 1024);
+        if (set != DCB_OK)
+            return set;
+        // starts beside the packing kernel: what it sets up does not depend on it
+        DCB_CUDA_TRY(launch_overlapped(kernel, dim3(grid), SH_THREADS, smem, stream, g, beta, x, p->image, p->tables, y,
+                                       status, p->stat_part, ymap, use_ymap));
         return DCB_OK;
     };
     int32_t st;
@@ -850,8 +854,8 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
         st = stats ? launch(sh_conv_kernel<1, 3, true>) : launch(sh_conv_kernel<1, 3, false>);
     if (st != DCB_OK || !stats)
         return st;
-    sh_stats_fold_kernel<<<1, SH_FOLD_WARPS * 32, 0, stream>>>(p->stat_part, (int) grid * SH_EPI, g.kout, sums, sqsums);
-    DCB_LAUNCH_CHECK();
+    DCB_CUDA_TRY(launch_overlapped(sh_stats_fold_kernel, dim3(1), SH_FOLD_WARPS * 32, 0, stream, p->stat_part,
+                                   (int) grid * SH_EPI, g.kout, sums, sqsums));
     return DCB_OK;
 }
 

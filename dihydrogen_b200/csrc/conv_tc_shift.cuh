@@ -467,6 +467,8 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // the filter image, the input and everything that is written
+    wait_for_previous_kernel();
     bool ok = true;
 
     if (warp < SH_EPI)

@@ -558,7 +558,9 @@ int32_t wg_launch(const WgGeom& g, int rkw, const float* x, const float* dy, flo
 {
     auto kernel = wg_conv_kernel<SW, KWG, AL>;
     const size_t smem = g.smem < 120 * 1024 ? 120 * 1024 : (size_t) g.smem; // one CTA per SM: it owns all of tensor memory
-    DCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 227 * 1024);
+    if (set != DCB_OK)
+        return set;
     kernel<<<(unsigned) (g.roles * g.parts), WG_THREADS, smem, stream>>>(g, x, dy, part, status, rkw);
     DCB_LAUNCH_CHECK();
     return DCB_OK;

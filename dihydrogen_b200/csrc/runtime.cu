@@ -1,6 +1,9 @@
 // Status strings, error record, device queries and the peer-mapped window.
 #include "common.cuh"
 
+#include <mutex>
+#include <utility>
+
 #include <unistd.h>
 
 #include <atomic>
@@ -19,6 +22,21 @@ void set_last_error(const std::string& msg)
 int64_t wait_budget_ns()
 {
     return g_wait_budget_ns.load();
+}
+
+int32_t allow_dynamic_smem(const void* kernel, int bytes)
+{
+    static std::mutex mutex;
+    static std::vector<std::pair<const void*, int>> done; // a few dozen at most
+    int device = 0;
+    DCB_CUDA_TRY(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lock(mutex);
+    for (const auto& d : done)
+        if (d.first == kernel && d.second == device)
+            return DCB_OK;
+    DCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.emplace_back(kernel, device);
+    return DCB_OK;
 }
 
 int num_sms()

@@ -635,6 +635,7 @@ class HaloExchange:
         self._plan = ctypes.c_void_p()
         d = tensor.desc()
         call("dcb_halo_plan_create", ctypes.byref(d), flat, tensor.locale.rank, ctypes.byref(self._plan))
+        self._idle = not any(tensor.dist.overlap)  # no halo anywhere: nothing to exchange or to clear
 
     def __del__(self):
         try:
@@ -692,8 +693,10 @@ class HaloExchange:
         dimension also zeroes that dimension's halo slabs that have no neighbour
         (what Tensor::clear_halo before the exchange leaves behind), saving one
         launch per partitioned dimension."""
-        call("dcb_halo_exchange", self._plan, _ptr(self.tensor.get_buffer()),
-             self._flags(is_reverse, skip_unpack, op, clear_boundary), _stream_ptr(stream))
+        flags = self._flags(is_reverse, skip_unpack, op, clear_boundary)
+        if self._idle:
+            return
+        call("dcb_halo_exchange", self._plan, _ptr(self.tensor.get_buffer()), flags, _stream_ptr(stream))
 
     def pack_put(self, dim, stream=None, is_reverse=False, op="ID", clear_boundary=False):
         call("dcb_halo_pack_put", self._plan, _ptr(self.tensor.get_buffer()), dim,
@@ -857,6 +860,7 @@ class Allreduce:
 
     def __init__(self, locale: Locale, kind="peer", max_count=4096, connect=True):
         self.locale, self.kind = locale, kind
+        self._alone = False
         self._comm = ctypes.c_void_p()
         if kind == "peer":
             call("dcb_comm_create_peer", locale.rank, locale.size, max_count, ctypes.byref(self._comm))
@@ -887,8 +891,11 @@ class Allreduce:
     def connect(self, blobs):
         joined = ctypes.create_string_buffer(b"".join(blobs), _abi.COMM_BLOB_BYTES * len(blobs))
         call("dcb_comm_connect", self._comm, joined, len(blobs))
+        self._alone = self.locale.size == 1 and self.kind == "peer"  # the sum over one rank is the vector itself
 
     def allreduce(self, ptr: int, count: int, stream=None):
+        if self._alone and self._comm and ptr:
+            return
         call("dcb_allreduce_sum", self._comm, _ptr(ptr), count, _stream_ptr(stream))
 
     def push(self, ptr: int, count: int, stream=None):
@@ -1120,7 +1127,7 @@ class Convolution:
         for n, (plan, xoff, yoff) in enumerate(regions):  # the interior comes first
             if n == 1 and halo_ready is not None:
                 stream.wait_event(halo_ready)  # the boundary slabs read the halo
-            call("dcb_conv_fwd", plan, float(alpha), _ptr(x0 + xoff), _ptr(filter.data_ptr()), float(beta),
+            call("dcb_conv_fwd", plan, float(alpha), _ptr(x0 + xoff), filter.data_ptr(), float(beta),
                  _ptr(y0 + yoff), _stream_ptr(stream))
 
     def _make_plan(self, xd: NdDesc, yd: NdDesc, pads):
@@ -1200,17 +1207,17 @@ class Convolution:
             self.halo_xch_input.exchange(s, clear_boundary=True)
             if prof:
                 torch.cuda.nvtx.range_pop()
-        if statistics is not None and float(beta) == 0.0 and input._geo().split_root:
-            st = _abi.lib().dcb_conv_fwd_stats(self._plan_fwd, float(alpha), _ptr(input.nd_ptr(self._x_lo)),
-                                               _ptr(filter.data_ptr()), _ptr(output.get_base_ptr()),
-                                               _ptr(statistics[0].data_ptr()), _ptr(statistics[1].data_ptr()),
+        if statistics is not None and self.nsd == 3 and float(beta) == 0.0 and input._geo().split_root:
+            st = _abi.lib().dcb_conv_fwd_stats(self._plan_fwd, float(alpha), input.nd_ptr(self._x_lo),
+                                               filter.data_ptr(), output.get_base_ptr(),
+                                               statistics[0].data_ptr(), statistics[1].data_ptr(),
                                                _stream_ptr(s))
             if st == _abi.OK:
                 return 1
             if st != _abi.UNSUPPORTED:
                 _abi.check(st, "dcb_conv_fwd_stats")
-        call("dcb_conv_fwd", self._plan_fwd, float(alpha), _ptr(input.nd_ptr(self._x_lo)), _ptr(filter.data_ptr()),
-             float(beta), _ptr(output.get_base_ptr()), _stream_ptr(s))
+        call("dcb_conv_fwd", self._plan_fwd, float(alpha), input.nd_ptr(self._x_lo), filter.data_ptr(),
+             float(beta), output.get_base_ptr(), _stream_ptr(s))
         return 0
 
     def backward_data(self, alpha, filter: torch.Tensor, d_output: Tensor, beta, d_input: Tensor,
@@ -1221,8 +1228,8 @@ class Convolution:
         s = self.be.stream
         if not skip_halo_exchange:
             self.backward_data_exchange_halo(d_output, s)
-        call("dcb_conv_bwd_data", self._plan_bwd, float(alpha), _ptr(filter.data_ptr()),
-             _ptr(d_output.get_buffer()), float(beta), _ptr(d_input.nd_ptr(self._dx_lo)), _stream_ptr(s))
+        call("dcb_conv_bwd_data", self._plan_bwd, float(alpha), filter.data_ptr(),
+             _ptr(d_output.get_buffer()), float(beta), d_input.nd_ptr(self._dx_lo), _stream_ptr(s))
         return 0
 
     def backward_filter(self, alpha, input: Tensor, d_output: Tensor, beta, d_filter: torch.Tensor, reduce=True,
@@ -1236,8 +1243,8 @@ class Convolution:
                 or not input._geo().split_root):
             _zero_on(s, d_filter)
         else:
-            call("dcb_conv_bwd_filter", self._plan_wgrad, float(alpha), _ptr(input.nd_ptr(self._x_lo)),
-                 _ptr(d_output.get_base_ptr()), float(beta), _ptr(d_filter.data_ptr()), _stream_ptr(s))
+            call("dcb_conv_bwd_filter", self._plan_wgrad, float(alpha), input.nd_ptr(self._x_lo),
+                 d_output.get_base_ptr(), float(beta), d_filter.data_ptr(), _stream_ptr(s))
         if reduce:
             self.allreduce_gradients(d_filter)
         return 0
@@ -1250,8 +1257,8 @@ class Convolution:
         if output.get_local_size() == 0:
             return 0
         yd = output._nd()
-        call("dcb_bias_fwd", float(alpha), _ptr(bias.data_ptr()), float(beta), yd,
-             _ptr(output.get_base_ptr()), _stream_ptr(self.be.stream))
+        call("dcb_bias_fwd", float(alpha), bias.data_ptr(), float(beta), yd,
+             output.get_base_ptr(), _stream_ptr(self.be.stream))
         return 0
 
     def backward_bias(self, alpha, d_output: Tensor, beta, bias_gradient: torch.Tensor, reduce=True):
@@ -1260,8 +1267,8 @@ class Convolution:
             _zero_on(self.be.stream, bias_gradient)
         else:
             yd = d_output._nd()
-            call("dcb_bias_bwd", float(alpha), yd, _ptr(d_output.get_base_ptr()), float(beta),
-                 _ptr(bias_gradient.data_ptr()), _stream_ptr(self.be.stream))
+            call("dcb_bias_bwd", float(alpha), yd, d_output.get_base_ptr(), float(beta),
+                 bias_gradient.data_ptr(), _stream_ptr(self.be.stream))
         if reduce:
             self.allreduce_gradients(bias_gradient)
         return 0
@@ -1320,8 +1327,8 @@ class BatchNormalization:
         if input.get_local_size() == 0 or not input._geo().split_root:
             _zero_on(s, mean, var)
             return 0
-        call("dcb_bn_stats", self._plan(input), _ptr(input.get_base_ptr()), _ptr(mean.data_ptr()),
-             _ptr(var.data_ptr()), _stream_ptr(s))
+        call("dcb_bn_stats", self._plan(input), input.get_base_ptr(), mean.data_ptr(),
+             var.data_ptr(), _stream_ptr(s))
         return 0
 
     def _allreduce_pair(self, a, b, fn):
@@ -1350,8 +1357,15 @@ class BatchNormalization:
         if is_training:
             stat_shape = input.shape if self.global_stats else input.local_shape
             nps = math.prod(stat_shape) // stat_shape[-2]
-            call("dcb_bn_finalize", C, nps, self.decay, _ptr(mean.data_ptr()), _ptr(var.data_ptr()),
-                 _ptr(running_mean.data_ptr()), _ptr(running_var.data_ptr()), _stream_ptr(s))
+            if input.get_local_size() != 0 and nps > 0:
+                call("dcb_bn_finalize_apply", self._plan(input), nps, self.decay, mean.data_ptr(), var.data_ptr(),
+                     running_mean.data_ptr(), running_var.data_ptr(), input._nd(), input.get_base_ptr(),
+                     scale.data_ptr(), bias.data_ptr(), self.epsilon,
+                     1.0 if leaky_relu_slope is None else float(leaky_relu_slope), output._nd(),
+                     output.get_base_ptr(), _stream_ptr(s))
+                return 0
+            call("dcb_bn_finalize", C, nps, self.decay, mean.data_ptr(), var.data_ptr(),
+                 running_mean.data_ptr(), running_var.data_ptr(), _stream_ptr(s))
             m, v = mean, var
         else:
             m, v = running_mean, running_var
@@ -1359,13 +1373,13 @@ class BatchNormalization:
             return 0
         xd, yd = input._nd(), output._nd()
         if leaky_relu_slope is not None:
-            call("dcb_bn_apply_leaky_relu", xd, _ptr(input.get_base_ptr()), _ptr(m.data_ptr()),
-                 _ptr(v.data_ptr()), _ptr(scale.data_ptr()), _ptr(bias.data_ptr()), self.epsilon,
-                 float(leaky_relu_slope), yd, _ptr(output.get_base_ptr()), _stream_ptr(s))
+            call("dcb_bn_apply_leaky_relu", xd, input.get_base_ptr(), m.data_ptr(),
+                 v.data_ptr(), scale.data_ptr(), bias.data_ptr(), self.epsilon,
+                 float(leaky_relu_slope), yd, output.get_base_ptr(), _stream_ptr(s))
             return 0
-        call("dcb_bn_apply", xd, _ptr(input.get_base_ptr()), _ptr(m.data_ptr()), _ptr(v.data_ptr()),
-             _ptr(scale.data_ptr()), _ptr(bias.data_ptr()), self.epsilon, yd,
-             _ptr(output.get_base_ptr()), _stream_ptr(s))
+        call("dcb_bn_apply", xd, input.get_base_ptr(), m.data_ptr(), v.data_ptr(),
+             scale.data_ptr(), bias.data_ptr(), self.epsilon, yd,
+             output.get_base_ptr(), _stream_ptr(s))
         return 0
 
     def forward(self, input, mean, var, running_mean, running_var, scale, bias, output, is_training=True,
@@ -1385,10 +1399,10 @@ class BatchNormalization:
         if input.get_local_size() == 0 or not input._geo().split_root:
             _zero_on(s, scale_gradient, bias_gradient, mean_gradient, var_gradient)
             return 0
-        call("dcb_bn_bwd_reduce", self._plan(input), _ptr(input.get_base_ptr()), d_output._nd(),
-             _ptr(d_output.get_base_ptr()), _ptr(mean.data_ptr()), _ptr(var.data_ptr()), _ptr(scale.data_ptr()),
-             self.epsilon, _ptr(scale_gradient.data_ptr()), _ptr(bias_gradient.data_ptr()),
-             _ptr(mean_gradient.data_ptr()), _ptr(var_gradient.data_ptr()), _stream_ptr(s))
+        call("dcb_bn_bwd_reduce", self._plan(input), input.get_base_ptr(), d_output._nd(),
+             d_output.get_base_ptr(), mean.data_ptr(), var.data_ptr(), scale.data_ptr(),
+             self.epsilon, scale_gradient.data_ptr(), bias_gradient.data_ptr(),
+             mean_gradient.data_ptr(), var_gradient.data_ptr(), _stream_ptr(s))
         return 0
 
     def backward_allreduce(self, scale_gradient, bias_gradient, mean_gradient, var_gradient,
@@ -1410,10 +1424,10 @@ class BatchNormalization:
         stat_shape = input.shape if self.global_stats else input.local_shape
         nps = math.prod(stat_shape) // stat_shape[-2]
         xd, dyd, dxd = input._nd(), d_output._nd(), d_input._nd()
-        call("dcb_bn_bwd_apply", xd, _ptr(input.get_base_ptr()), dyd,
-             _ptr(d_output.get_base_ptr()), _ptr(mean.data_ptr()), _ptr(var.data_ptr()), _ptr(scale.data_ptr()),
-             _ptr(mean_gradient.data_ptr()), _ptr(var_gradient.data_ptr()), self.epsilon, nps, dxd,
-             _ptr(d_input.get_base_ptr()), _stream_ptr(self.be.stream))
+        call("dcb_bn_bwd_apply", xd, input.get_base_ptr(), dyd,
+             d_output.get_base_ptr(), mean.data_ptr(), var.data_ptr(), scale.data_ptr(),
+             mean_gradient.data_ptr(), var_gradient.data_ptr(), self.epsilon, nps, dxd,
+             d_input.get_base_ptr(), _stream_ptr(self.be.stream))
         return 0
 
     def backward(self, input, d_output, mean, var, scale, scale_gradient, bias_gradient, mean_gradient,
@@ -1499,7 +1513,7 @@ class Pooling:
             return 0
         xd, yd = input._nd(self._lo, self._hi), output._nd()
         call("dcb_pool_fwd", ctypes.byref(self._pd), xd, yd, float(alpha),
-             _ptr(input.nd_ptr(self._lo)), float(beta), _ptr(output.get_base_ptr()), _stream_ptr(s))
+             input.nd_ptr(self._lo), float(beta), output.get_base_ptr(), _stream_ptr(s))
         return 0
 
     def backward(self, alpha, output: Tensor, d_output: Tensor, input: Tensor, beta, d_input: Tensor,
@@ -1521,8 +1535,8 @@ class Pooling:
                                                                yd)
                 self._ws = torch.empty(max(need, 0), dtype=torch.uint8, device=d_input.buffer.device)
             call("dcb_pool_bwd", ctypes.byref(self._pd), xd, yd, float(alpha),
-                 _ptr(output.get_base_ptr()), _ptr(d_output.get_base_ptr()), _ptr(input.nd_ptr(self._lo)),
-                 float(beta), _ptr(d_input.nd_ptr(self._lo)),
+                 output.get_base_ptr(), d_output.get_base_ptr(), input.nd_ptr(self._lo),
+                 float(beta), d_input.nd_ptr(self._lo),
                  _ptr(self._ws.data_ptr() if self._ws.numel() else 0), self._ws.numel(), _stream_ptr(s))
         if not skip_halo_exchange:
             self.halo_xch_d_input.exchange(s, is_reverse=True, op="SUM")
@@ -1542,15 +1556,15 @@ class LeakyReLU:
         if input.get_local_size() == 0:
             return 0
         xd, yd = input._nd(), output._nd()
-        call("dcb_leaky_relu_fwd", xd, _ptr(input.get_base_ptr()), float(negative_slope),
-             yd, _ptr(output.get_base_ptr()), _stream_ptr(self.be.stream))
+        call("dcb_leaky_relu_fwd", xd, input.get_base_ptr(), float(negative_slope),
+             yd, output.get_base_ptr(), _stream_ptr(self.be.stream))
         return 0
 
     def backward(self, input: Tensor, d_output: Tensor, negative_slope: float, d_input: Tensor):
         if input.get_local_size() == 0:
             return 0
         xd, dyd, dxd = input._nd(), d_output._nd(), d_input._nd()
-        call("dcb_leaky_relu_bwd", xd, _ptr(input.get_base_ptr()), dyd,
-             _ptr(d_output.get_base_ptr()), float(negative_slope), dxd, _ptr(d_input.get_base_ptr()),
+        call("dcb_leaky_relu_bwd", xd, input.get_base_ptr(), dyd,
+             d_output.get_base_ptr(), float(negative_slope), dxd, d_input.get_base_ptr(),
              _stream_ptr(self.be.stream))
         return 0

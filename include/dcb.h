@@ -298,6 +298,17 @@ int32_t dcb_bn_stats_noalloc(const dcb_nd_desc* xd, const void* x, void* sums,
 int32_t dcb_bn_finalize(int32_t channels, int64_t num_per_sum, float decay,
                         void* mean, void* var, void* running_mean,
                         void* running_var, void* stream);
+/* dcb_bn_finalize followed by dcb_bn_apply (slope 1) or dcb_bn_apply_leaky_relu in
+ * one launch, for a shard that is not empty.  mean / var hold the (all-reduced)
+ * sums and sums of squares on entry and the statistics afterwards.  `plan` is one
+ * of the same channel count (dcb_bn_plan_create); its calls must be ordered. */
+int32_t dcb_bn_finalize_apply(dcb_bn_plan* plan, int64_t num_per_sum,
+                              float decay, void* mean, void* var,
+                              void* running_mean, void* running_var,
+                              const dcb_nd_desc* xd, const void* x,
+                              const void* scale, const void* bias, float eps,
+                              float slope, const dcb_nd_desc* yd, void* y,
+                              void* stream);
 /* y = scale*(x-mean)*rsqrt(var+eps)+bias (batch_normalization,
  * batchnorm.cu:369-455).  yd may differ from xd in strides only. */
 int32_t dcb_bn_apply(const dcb_nd_desc* xd, const void* x, const void* mean,

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import dihydrogen_b200 as dc
+from dihydrogen_b200 import _abi
 from oracle import oracle as O
 
 import emu
@@ -85,6 +86,42 @@ def test_bn_forward_backward_local(shape, locale, overlap):
     bn.backward_stage2(x_t, dy_t, mean, var, scale, dmean, dvar, dx_t)
     dx_ref = O.bn_backprop2(x, dy, m_g, v_g, scale.cpu().numpy(), dmean.cpu().numpy(), dvar.cpu().numpy(), 1e-5, nps)
     emu.assert_close(dx_t.owned().cpu().numpy(), dx_ref, TOL, "dx")
+
+
+@pytest.mark.parametrize("shape,overlap", [
+    ([1, 1, 2, 1], [0, 0, 0, 0]),                  # one block per channel, two values
+    ([33, 7, 5, 3, 2], [0, 0, 0, 0, 0]),
+    ([128, 64, 64, 5, 1], [0, 0, 0, 0, 0]),        # several blocks per channel
+    ([512, 37, 3, 4, 1], [0, 0, 0, 0, 0]),
+])
+@pytest.mark.parametrize("slope", [None, 0.25])
+def test_finalize_inside_apply_equals_finalize_then_apply(shape, overlap, slope):
+    """One launch or two: the same operations in the same order, so bit for bit the same."""
+    rng = np.random.default_rng(11)
+    be = dc.BackendDNNLib(dc.Locale(0, 1))
+    x_t, y_t = (_rank0(shape, [1] * len(shape), overlap) for _ in range(2))
+    emu.upload(x_t, rng.normal(0.3, 1.5, x_t.np_real_shape()).astype(np.float32))
+    y_t.allocate()
+    C = shape[-2]
+    nps = int(np.prod(shape)) // C
+    scale = torch.from_numpy(rng.uniform(0.5, 1.5, C).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.normal(0, 1, C).astype(np.float32)).cuda()
+    bn = dc.BatchNormalization(be, len(shape), decay=0.9, epsilon=1e-5)
+    runs = []
+    for fused in (False, True, True):  # twice: the tickets are back at zero
+        mean, var, rm = (torch.zeros(C, device="cuda") for _ in range(3))
+        rv = torch.ones(C, device="cuda")
+        bn.forward_stage1(x_t, mean, var, True)
+        if fused:
+            bn.forward_stage2(x_t, mean, var, rm, rv, scale, bias, y_t, True, leaky_relu_slope=slope)
+        else:
+            _abi.call("dcb_bn_finalize", C, nps, 0.9, mean.data_ptr(), var.data_ptr(), rm.data_ptr(), rv.data_ptr(),
+                      be.stream.cuda_stream)
+            # statistics given: apply only, as in inference
+            bn.forward_stage2(x_t, mean, var, mean, var, scale, bias, y_t, False, leaky_relu_slope=slope)
+        torch.cuda.synchronize()
+        runs.append([t.cpu().numpy().tobytes() for t in (mean, var, rm, rv)] + [emu.download(y_t).tobytes()])
+    assert runs[1] == runs[0] and runs[2] == runs[0]
 
 
 def test_bn_stats_are_reproducible():
