@@ -491,6 +491,9 @@ __global__ void __launch_bounds__(BN_THREADS)
     });
 }
 
+// Goes through the tensors from their end: the reduction went through them forwards, so
+// what it read last is still in L2, and the backward filter finds the beginning there
+// (backward pass of 256^3 x 16 channels: 3190 us forwards, 3153 us like this).
 template <int V, bool PACKED>
 __global__ void __launch_bounds__(BN_THREADS)
     bn_bwd_apply_kernel(const float* x, RunStrides xs,
@@ -503,14 +506,14 @@ __global__ void __launch_bounds__(BN_THREADS)
                         const float* __restrict__ dvar, float eps,
                         long long num_per_sum)
 {
-    const int c = blockIdx.y;
+    const int c = gridDim.y - 1 - blockIdx.y; // the last one first, as the units below
     const float m = mean[c];
     const float sc = scale[c];
     const float inv_stdev = rsqrtf(var[c] + eps);
     // backprop2 (batchnorm.cu:1333-1335)
     const float dmean_term = dmean[c] / (float) num_per_sum;
     const float dvar_term = dvar[c] * 2 / (float) (num_per_sum - 1);
-    for (long long u = blockIdx.x; u < ug.upc; u += gridDim.x)
+    for (long long u = ug.upc - 1 - blockIdx.x; u >= 0; u -= gridDim.x)
     {
         const UnitPos p = decode_unit(ug, u);
         const float* xp = x + unit_offset(xs, ug.g, p, c);

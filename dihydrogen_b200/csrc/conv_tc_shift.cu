@@ -78,9 +78,18 @@ __global__ void __launch_bounds__(SH_FOLD_WARPS * 32)
     const int t = threadIdx.x & 31, w = threadIdx.x >> 5;
     wait_for_previous_kernel();
     double acc = 0.0;
-#pragma unroll 4
-    for (int i = w; i < nparts; i += SH_FOLD_WARPS)
-        acc += (double) part[(size_t) i * 32 + t];
+#pragma unroll 1
+    for (int i = w; i < nparts; i += SH_FOLD_WARPS * 16)
+    {
+        // 16 loads in flight: the kernel is three trips to memory and nothing else
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            v[k] = i + k * SH_FOLD_WARPS < nparts ? part[(size_t) (i + k * SH_FOLD_WARPS) * 32 + t] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            acc += (double) v[k];
+    }
     sm[w][t] = acc;
     __syncthreads();
     if (w != 0)

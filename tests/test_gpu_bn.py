@@ -106,7 +106,7 @@ def test_finalize_inside_apply_equals_finalize_then_apply(shape, overlap, slope)
     nps = int(np.prod(shape)) // C
     scale = torch.from_numpy(rng.uniform(0.5, 1.5, C).astype(np.float32)).cuda()
     bias = torch.from_numpy(rng.normal(0, 1, C).astype(np.float32)).cuda()
-    bn = dc.BatchNormalization(be, len(shape), decay=0.9, epsilon=1e-5)
+    bn = dc.BatchNormalization(be, len(shape), decay=0.9, epsilon=1e-5, global_stats=False)
     runs = []
     for fused in (False, True, True):  # twice: the tickets are back at zero
         mean, var, rm = (torch.zeros(C, device="cuda") for _ in range(3))
@@ -116,11 +116,11 @@ def test_finalize_inside_apply_equals_finalize_then_apply(shape, overlap, slope)
             bn.forward_stage2(x_t, mean, var, rm, rv, scale, bias, y_t, True, leaky_relu_slope=slope)
         else:
             _abi.call("dcb_bn_finalize", C, nps, 0.9, mean.data_ptr(), var.data_ptr(), rm.data_ptr(), rv.data_ptr(),
-                      be.stream.cuda_stream)
+                      torch.cuda.current_stream().cuda_stream)
             # statistics given: apply only, as in inference
             bn.forward_stage2(x_t, mean, var, mean, var, scale, bias, y_t, False, leaky_relu_slope=slope)
         torch.cuda.synchronize()
-        runs.append([t.cpu().numpy().tobytes() for t in (mean, var, rm, rv)] + [emu.download(y_t).tobytes()])
+        runs.append([t.cpu().numpy().tobytes() for t in (mean, var, rm, rv)] + [y_t.owned().cpu().numpy().tobytes()])
     assert runs[1] == runs[0] and runs[2] == runs[0]
 
 
