@@ -317,6 +317,12 @@ __device__ __forceinline__ void sums_to_statistics(long long num_per_sum, float&
     sqsum = v;
 }
 
+// (one rounding fewer than written, wherever it is inlined)
+__device__ __forceinline__ float running_update(float decay, float running, float value)
+{
+    return __fmaf_rn(decay, running, __fmul_rn(1.f - decay, value));
+}
+
 __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
                                    float decay, float* mean, float* var,
                                    float* running_mean, float* running_var)
@@ -330,8 +336,8 @@ __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
         sums_to_statistics(num_per_sum, m, v);
         mean[c] = m;
         var[c] = v;
-        running_mean[c] = decay * running_mean[c] + (1.f - decay) * m;
-        running_var[c] = decay * running_var[c] + (1.f - decay) * v;
+        running_mean[c] = running_update(decay, running_mean[c], m);
+        running_var[c] = running_update(decay, running_var[c], v);
     }
     else
     {
@@ -383,8 +389,8 @@ __global__ void __launch_bounds__(BN_THREADS)
             fin.tickets[c] = 0;
             fin.mean[c] = m;
             fin.var[c] = v0;
-            fin.running_mean[c] = fin.decay * fin.running_mean[c] + (1.f - fin.decay) * m;
-            fin.running_var[c] = fin.decay * fin.running_var[c] + (1.f - fin.decay) * v0;
+            fin.running_mean[c] = running_update(fin.decay, fin.running_mean[c], m);
+            fin.running_var[c] = running_update(fin.decay, fin.running_var[c], v0);
         }
     }
     else

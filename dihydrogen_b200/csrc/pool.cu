@@ -31,6 +31,7 @@
 #include "dcb.h"
 
 #include <cfloat>
+#include <type_traits>
 
 namespace dcb
 {
@@ -307,6 +308,229 @@ __global__ void __launch_bounds__(POOL_THREADS)
         float* yp =
             y + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (od * (int) g.ys[0] + oh * (int) g.ys[1] + ow);
         *yp = beta != 0.f ? alpha * r + beta * *yp : alpha * r;
+    }
+}
+
+// The same for windows of 3 with stride 2 along D too, the usual down-sampling of a
+// volume: a thread walks along D with its pair of outputs.  Window od covers planes
+// 2 od - pad .. + 2, so every second plane belongs to two windows: its maximum over the
+// thread's 3 x 5 cells (position, and first cell for the rule below) is carried over.  A
+// plane is then read and scanned once instead of 1.5 times; what is left is the overlap
+// of neighbouring output rows along H, which L1 has.
+// The scan's rule is "the window's first cell becomes the maximum, a later cell if it
+// is larger": a first cell that is not a number stays the maximum.  A plane's own
+// maximum is therefore taken over numbers only (start -inf), and the first cell is
+// looked at again where the plane opens a window.  Same results, bit for bit.
+// 16 x 256^3 floats, maximum: 312 -> 221 us forward, 312 -> 246 us for the indices of the
+// backward pass (184 and 170 us at the rate of a copy).  Bound by latency: four blocks an
+// SM (64 registers; with 80 and three blocks the index pass takes 264 us), six 16-byte
+// loads in flight per thread (three, with the range checks between them: 301 and 379 us).
+struct PoolPlane
+{
+    float m[2], f[2]; // maximum (or sum) and first cell, per output of the pair
+    int t[2];         // tap kh * 3 + kw of the maximum
+};
+
+template <bool MAXP, bool IDX>
+__global__ void __launch_bounds__(POOL_THREADS, 4)
+    pool_fwd_march_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ x, float* y,
+                          unsigned char* __restrict__ argmax, int tw_log2, long long rows, int seg)
+{
+    const int tq = (blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1)); // pair of outputs
+    const long long row = (long long) blockIdx.x * (POOL_THREADS >> tw_log2) + (threadIdx.x >> tw_log2);
+    if (row >= rows) // a warp never spans two rows: the whole warp leaves
+        return;
+    int s, oh;
+    pool_split_row(row, rows, g.out[1], &s, &oh);
+    const int c = blockIdx.z % g.c, n = blockIdx.z / g.c, lane = threadIdx.x & 31;
+    const bool live = 2 * tq < g.out[2], both = 2 * tq + 1 < g.out[2]; // dead lanes still take part in the shuffles
+    const int xs0 = (int) g.xs[0], xs1 = (int) g.xs[1];
+    const int h0 = oh * 2 - g.pad[1], w4 = 4 * tq; // cells w4 - 1 .. w4 + 3
+    const float* xp = x + (size_t) n * g.xs_n + (size_t) c * g.xs_c + (h0 * xs1 + w4);
+    const bool ledge = tq == 0, whole = w4 + 3 < g.in[2];
+    const float none = MAXP ? __int_as_float(0xff800000) : 0.f; // of a cell that does not exist
+    const bool any_row = max(h0, g.lo[1]) < min(h0 + 3, g.hi[1]);
+
+    // a plane's cells; FAST: all exist, no branches, so that all loads of a step are in flight together
+    auto load = [&](int id, float (&v)[3][5], auto fast) {
+#pragma unroll
+        for (int kh = 0; kh < 3; ++kh)
+        {
+            const float* rp = xp + (id * xs0 + kh * xs1);
+            if (fast.value)
+            {
+                const float4 q = __ldg(reinterpret_cast<const float4*>(rp));
+                v[kh][1] = q.x, v[kh][2] = q.y, v[kh][3] = q.z, v[kh][4] = q.w;
+                v[kh][0] = none;
+                if (lane == 0 && !ledge)
+                    v[kh][0] = __ldg(rp - 1);
+                continue;
+            }
+            v[kh][0] = v[kh][1] = v[kh][2] = v[kh][3] = v[kh][4] = none;
+            if (h0 + kh >= g.lo[1] && h0 + kh < g.hi[1]) // the same for the whole warp
+            {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (w4 + e < g.in[2])
+                        v[kh][1 + e] = __ldg(rp + e);
+                if (lane == 0 && live && !ledge)
+                    v[kh][0] = __ldg(rp - 1);
+            }
+        }
+    };
+    auto scan = [&](float (&v)[3][5], PoolPlane& p, auto fast) {
+        p.m[0] = p.m[1] = none;
+        p.f[0] = p.f[1] = none;
+        p.t[0] = p.t[1] = 0;
+        bool seen = false;
+#pragma unroll
+        for (int kh = 0; kh < 3; ++kh)
+        {
+            // cell w4 - 1 is the left neighbour's last one
+            const float left = __shfl_up_sync(0xffffffffu, v[kh][4], 1);
+            if (lane != 0)
+                v[kh][0] = left;
+            if (!fast.value && (h0 + kh < g.lo[1] || h0 + kh >= g.hi[1]))
+                continue;
+            if (MAXP && !seen)
+            {
+                seen = true;
+                p.f[0] = ledge ? v[kh][1] : v[kh][0];
+                p.f[1] = v[kh][2];
+                p.t[0] = kh * 3 + (ledge ? 1 : 0);
+                p.t[1] = kh * 3;
+            }
+#pragma unroll
+            for (int o = 0; o < 2; ++o)
+#pragma unroll
+                for (int kw = 0; kw < 3; ++kw)
+                {
+                    const float val = v[kh][2 * o + kw];
+                    if (!MAXP)
+                        p.m[o] += val;
+                    else if (val > p.m[o])
+                    {
+                        p.m[o] = val;
+                        if (IDX)
+                            p.t[o] = kh * 3 + kw;
+                    }
+                }
+        }
+    };
+
+    const int od0 = s * seg, od1 = min(od0 + seg, g.out[0]);
+    PoolPlane carry, mid, next;
+    int id = 2 * od0 - g.pad[0];
+    const std::false_type checked{};
+    auto scan_checked = [&](int plane, PoolPlane& p) {
+        float v[3][5];
+        if (plane >= g.lo[0] && plane < g.hi[0]) // the same for the whole warp
+            load(plane, v, checked), scan(v, p, checked);
+        else
+            p = {{none, none}, {none, none}, {0, 0}};
+    };
+    const bool inside = __all_sync(0xffffffffu, live && whole) && h0 >= g.lo[1] && h0 + 3 <= g.hi[1];
+    if (inside && id >= g.lo[0] && id < g.hi[0])
+    {
+        float v[3][5];
+        load(id, v, std::true_type{});
+        scan(v, carry, std::true_type{});
+    }
+    else
+        scan_checked(id, carry);
+    // every cell that the walk has yet to read exists
+    const bool fast = inside && id + 1 >= g.lo[0] && id + 2 * (od1 - od0) < g.hi[0];
+    for (int od = od0; od < od1; ++od, id += 2)
+    {
+        if (fast)
+        {
+            float v[3][5], w[3][5];
+            load(id + 1, v, std::true_type{});
+            load(id + 2, w, std::true_type{});
+            scan(v, mid, std::true_type{});
+            scan(w, next, std::true_type{});
+        }
+        else
+        {
+            scan_checked(id + 1, mid);
+            scan_checked(id + 2, next);
+        }
+        float r[2];
+        int b[2];
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+        {
+            if (!MAXP)
+            {
+                r[o] = (carry.m[o] + mid.m[o] + next.m[o]) / fmaxf(pool_count(g, od, oh, 2 * tq + o), 1.f);
+                continue;
+            }
+            bool open = false; // the window has had its first cell
+            r[o] = -FLT_MAX;
+            b[o] = -1;
+            const PoolPlane* const pl[3] = {&carry, &mid, &next};
+#pragma unroll
+            for (int kd = 0; kd < 3; ++kd)
+            {
+                if (!any_row || id + kd < g.lo[0] || id + kd >= g.hi[0])
+                    continue;
+                if (!open)
+                {
+                    const bool nan = !(pl[kd]->f[o] == pl[kd]->f[o]);
+                    r[o] = nan ? pl[kd]->f[o] : pl[kd]->m[o];
+                    // the first valid tap: without numbers above -inf t still says where that is
+                    b[o] = kd * 9 + pl[kd]->t[o];
+                    if (IDX && nan)
+                    {
+                        const int first = max(0, g.lo[1] - h0) * 3 + (o == 0 && ledge ? 1 : 0);
+                        b[o] = kd * 9 + first;
+                    }
+                    open = true;
+                }
+                else if (pl[kd]->m[o] > r[o])
+                {
+                    r[o] = pl[kd]->m[o];
+                    b[o] = kd * 9 + pl[kd]->t[o];
+                }
+            }
+        }
+        carry = next;
+        if (!live)
+            continue;
+        if (IDX)
+        {
+            unsigned char* ap = argmax + ((size_t) n * g.c + c) * ((size_t) g.out[0] * g.out[1] * g.out[2])
+                                + ((od * g.out[1] + oh) * g.out[2] + 2 * tq);
+            if (both && (reinterpret_cast<uintptr_t>(ap) & 1) == 0)
+                *reinterpret_cast<uchar2*>(ap) = make_uchar2((unsigned char) b[0], (unsigned char) b[1]);
+            else
+            {
+                ap[0] = (unsigned char) b[0];
+                if (both)
+                    ap[1] = (unsigned char) b[1];
+            }
+        }
+        if (!IDX || y)
+        {
+            float* yp = y + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (od * (int) g.ys[0] + oh * (int) g.ys[1] + 2 * tq);
+            if (both && (reinterpret_cast<uintptr_t>(yp) & 7) == 0)
+            {
+                float2 out = make_float2(alpha * r[0], alpha * r[1]);
+                if (beta != 0.f)
+                {
+                    const float2 old = *reinterpret_cast<const float2*>(yp);
+                    out.x += beta * old.x;
+                    out.y += beta * old.y;
+                }
+                *reinterpret_cast<float2*>(yp) = out;
+            }
+            else
+            {
+                yp[0] = beta != 0.f ? alpha * r[0] + beta * yp[0] : alpha * r[0];
+                if (both)
+                    yp[1] = beta != 0.f ? alpha * r[1] + beta * yp[1] : alpha * r[1];
+            }
+        }
     }
 }
 
@@ -602,12 +826,21 @@ __global__ void __launch_bounds__(POOL_THREADS)
 // rows q, q+1 only, at fixed taps (row 2q is tap 1 of window q; row 2q+1 tap 2 of
 // window q and tap 0 of window q+1), so the index bytes and gradients of the 2 x 2
 // window rows are loaded once for sixteen cells and every comparison is against a
-// constant.  Cells outside the global tensor never were a window's maximum, so they
-// need no mask.  Per cell the sums run in the same order (D, H, then W ascending).
+// constant.  For WD = 3 the thread walks along D: window plane p+1 is kept for the next
+// block, and the plane behind it is on its way while this one is compared (269 -> 258 us
+// for 16 x 256^3; 190 us at the rate of a copy).  Cells outside the global tensor never were a window's maximum, so they need no mask.  Per cell the
+// sums run in the same order (D, H, then W ascending).
+struct PoolWindows
+{
+    int a[3];   // index byte of windows 2t, 2t+1, 2t+2 (255: no window)
+    float d[3]; // their gradients
+};
+
 template <int WD>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_bwd_index_block_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ dy, float* dx,
-                                const unsigned char* __restrict__ argmax, int tw_log2, int blocks_h, long long rows)
+                                const unsigned char* __restrict__ argmax, int tw_log2, int blocks_h, long long rows,
+                                int seg, int blocks_d)
 {
     constexpr int JD = WD == 1 ? 1 : 2;
     const int t = (blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1));
@@ -615,112 +848,130 @@ __global__ void __launch_bounds__(POOL_THREADS)
     if (row >= rows) // a warp never spans two row blocks: the whole warp leaves
         return;
     const int iw0 = 4 * t, ow0 = 2 * t;
-    int p, q;
-    pool_split_row(row, rows, blocks_h, &p, &q);
+    int s, q;
+    pool_split_row(row, rows, blocks_h, &s, &q);
     const int c = blockIdx.z % g.c, n = blockIdx.z / g.c;
     const int lane = threadIdx.x & 31;
     // offsets inside one (sample, channel) volume fit 32 bits (checked at the launch)
     const int ys0 = (int) g.ys[0], ys1 = (int) g.ys[1], astep = g.out[1] * g.out[2];
     const unsigned char* abase =
-        argmax + ((size_t) n * g.c + c) * ((size_t) g.out[0] * astep) + ((p * g.out[1] + q) * g.out[2] + ow0);
-    const float* dbase = dy + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (p * ys0 + q * ys1 + ow0);
+        argmax + ((size_t) n * g.c + c) * ((size_t) g.out[0] * astep) + (q * g.out[2] + ow0);
+    const float* dbase = dy + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (q * ys1 + ow0);
     const bool two = ow0 + 1 < g.out[2], third = ow0 + 2 < g.out[2];
-    // window rows (p + jd, q + jh): which exist is the same for the whole warp
-    int a0[JD * 2], a1[JD * 2], a2[JD * 2];
-    float d0[JD * 2], d1[JD * 2], d2[JD * 2];
-#pragma unroll
-    for (int jd = 0; jd < JD; ++jd)
+    // rows q, q + 1 of window plane od: which exist is the same for the whole warp
+    auto fetch = [&](int od, PoolWindows (&w)[2]) {
 #pragma unroll
         for (int jh = 0; jh < 2; ++jh)
         {
-            const int k = jd * 2 + jh;
-            // 255 is the index pass's "empty window" and never a tap
-            a0[k] = a1[k] = 255;
-            d0[k] = d1[k] = 0.f;
-            if (p + jd < g.out[0] && q + jh < g.out[1] && two)
+            w[jh] = {{255, 255, 255}, {0.f, 0.f, 0.f}};
+            if (od < g.out[0] && q + jh < g.out[1] && two)
             {
-                const uchar2 a = __ldg(reinterpret_cast<const uchar2*>(abase + (jd * astep + jh * g.out[2])));
-                const float2 d = __ldg(reinterpret_cast<const float2*>(dbase + (jd * ys0 + jh * ys1)));
-                a0[k] = a.x;
-                a1[k] = a.y;
-                d0[k] = d.x;
-                d1[k] = d.y;
+                const unsigned char* ap = abase + (od * astep + jh * g.out[2]);
+                const float* dp = dbase + (od * ys0 + jh * ys1);
+                const uchar2 a = __ldg(reinterpret_cast<const uchar2*>(ap));
+                const float2 d = __ldg(reinterpret_cast<const float2*>(dp));
+                w[jh].a[0] = a.x, w[jh].a[1] = a.y;
+                w[jh].d[0] = d.x, w[jh].d[1] = d.y;
+                if (lane == 31 && third)
+                    w[jh].a[2] = __ldg(ap + 2), w[jh].d[2] = __ldg(dp + 2);
             }
         }
-#pragma unroll
-    for (int jd = 0; jd < JD; ++jd)
+    };
+    // window 2t+2 is the right-hand neighbour's first
+    auto share = [&](PoolWindows (&w)[2]) {
 #pragma unroll
         for (int jh = 0; jh < 2; ++jh)
         {
-            const int k = jd * 2 + jh;
-            a2[k] = __shfl_down_sync(0xffffffffu, a0[k], 1);
-            d2[k] = __shfl_down_sync(0xffffffffu, d0[k], 1);
-            if (lane == 31)
-            {
-                const bool in = third && p + jd < g.out[0] && q + jh < g.out[1];
-                a2[k] = in ? (int) __ldg(abase + (jd * astep + jh * g.out[2] + 2)) : 255;
-                d2[k] = in ? __ldg(dbase + (jd * ys0 + jh * ys1 + 2)) : 0.f;
-            }
+            const int a = __shfl_down_sync(0xffffffffu, w[jh].a[0], 1);
+            const float d = __shfl_down_sync(0xffffffffu, w[jh].d[0], 1);
+            if (lane != 31)
+                w[jh].a[2] = a, w[jh].d[2] = d;
         }
-    if (iw0 >= g.in[2])
-        return;
+    };
     float* xbase = dx + (size_t) n * g.xs_n + (size_t) c * g.xs_c;
     const int xs0 = (int) g.xs[0], xs1 = (int) g.xs[1];
-#pragma unroll
-    for (int pa = 0; pa < JD; ++pa)
-#pragma unroll
-        for (int rb = 0; rb < 2; ++rb)
+    const int p0 = s * seg, p1 = min(p0 + seg, blocks_d);
+    PoolWindows w[JD][2], ahead[2];
+    fetch(p0, w[0]);
+    if (JD == 2)
+        fetch(p0 + 1, ahead);
+    share(w[0]);
+#pragma unroll 1
+    for (int p = p0; p < p1; ++p)
+    {
+        if (JD == 2)
         {
-            const int id = JD == 2 ? 2 * p + pa : p, ih = 2 * q + rb;
-            if (id >= g.in[0] || ih >= g.in[1])
-                continue;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int jd = 0; jd < JD; ++jd)
-#pragma unroll
-                for (int jh = 0; jh < 2; ++jh)
-                {
-                    // tap of input (plane pa, row rb) in window (jd, jh): coordinate - (2 * window - 1)
-                    const int kd = JD == 2 ? pa - 2 * jd + 1 : 0, kh = rb - 2 * jh + 1;
-                    if (kd < 0 || kd > 2 || kh < 0 || kh > 2)
-                        continue;
-                    const int k = jd * 2 + jh;
-                    const int tb = (kd * 3 + kh) * 3; // tap at cell i of window ow: tb + i - (2 ow - 1)
-                    if (a0[k] == tb + 1)
-                        acc[0] += d0[k];
-                    if (a0[k] == tb + 2)
-                        acc[1] += d0[k];
-                    if (a1[k] == tb)
-                        acc[1] += d1[k];
-                    if (a1[k] == tb + 1)
-                        acc[2] += d1[k];
-                    if (a1[k] == tb + 2)
-                        acc[3] += d1[k];
-                    if (a2[k] == tb)
-                        acc[3] += d2[k];
-                }
-            float* xp = xbase + (id * xs0 + ih * xs1 + iw0);
-            if (iw0 + 4 <= g.in[2] && (reinterpret_cast<uintptr_t>(xp) & 15) == 0)
-            {
-                float4 o = make_float4(alpha * acc[0], alpha * acc[1], alpha * acc[2], alpha * acc[3]);
-                if (beta != 0.f)
-                {
-                    const float4 old = *reinterpret_cast<const float4*>(xp);
-                    o.x += beta * old.x;
-                    o.y += beta * old.y;
-                    o.z += beta * old.z;
-                    o.w += beta * old.w;
-                }
-                *reinterpret_cast<float4*>(xp) = o;
-            }
-            else
-            {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (iw0 + e < g.in[2])
-                        xp[e] = beta != 0.f ? alpha * acc[e] + beta * xp[e] : alpha * acc[e];
-            }
+            w[JD - 1][0] = ahead[0], w[JD - 1][1] = ahead[1];
+            if (p + 1 < p1)
+                fetch(p + 2, ahead);
+            share(w[JD - 1]);
         }
+#pragma unroll
+        for (int pa = 0; pa < JD; ++pa)
+#pragma unroll
+            for (int rb = 0; rb < 2; ++rb)
+            {
+                const int id = JD == 2 ? 2 * p + pa : p, ih = 2 * q + rb;
+                if (id >= g.in[0] || ih >= g.in[1] || iw0 >= g.in[2])
+                    continue;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int jd = 0; jd < JD; ++jd)
+#pragma unroll
+                    for (int jh = 0; jh < 2; ++jh)
+                    {
+                        // tap of input (plane pa, row rb) in window (jd, jh): coordinate - (2 * window - 1)
+                        const int kd = JD == 2 ? pa - 2 * jd + 1 : 0, kh = rb - 2 * jh + 1;
+                        if (kd < 0 || kd > 2 || kh < 0 || kh > 2)
+                            continue;
+                        const PoolWindows& v = w[jd][jh];
+                        const int tb = (kd * 3 + kh) * 3; // tap at cell i of window ow: tb + i - (2 ow - 1)
+                        if (v.a[0] == tb + 1)
+                            acc[0] += v.d[0];
+                        if (v.a[0] == tb + 2)
+                            acc[1] += v.d[0];
+                        if (v.a[1] == tb)
+                            acc[1] += v.d[1];
+                        if (v.a[1] == tb + 1)
+                            acc[2] += v.d[1];
+                        if (v.a[1] == tb + 2)
+                            acc[3] += v.d[1];
+                        if (v.a[2] == tb)
+                            acc[3] += v.d[2];
+                    }
+                float* xp = xbase + (id * xs0 + ih * xs1 + iw0);
+                if (iw0 + 4 <= g.in[2] && (reinterpret_cast<uintptr_t>(xp) & 15) == 0)
+                {
+                    float4 o = make_float4(alpha * acc[0], alpha * acc[1], alpha * acc[2], alpha * acc[3]);
+                    if (beta != 0.f)
+                    {
+                        const float4 old = *reinterpret_cast<const float4*>(xp);
+                        o.x += beta * old.x;
+                        o.y += beta * old.y;
+                        o.z += beta * old.z;
+                        o.w += beta * old.w;
+                    }
+                    *reinterpret_cast<float4*>(xp) = o;
+                }
+                else
+                {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (iw0 + e < g.in[2])
+                            xp[e] = beta != 0.f ? alpha * acc[e] + beta * xp[e] : alpha * acc[e];
+                }
+            }
+        if (JD == 2)
+            w[0][0] = w[JD - 1][0], w[0][1] = w[JD - 1][1];
+    }
+}
+
+// Outputs (or blocks) along D that one thread walks over: as many as leave the chip four
+// times the blocks it holds, 16 at most (a walk re-reads one plane of its 2 * seg + 1).
+int pool_walk(long long blocks_per_step, int steps)
+{
+    const long long seg = blocks_per_step * steps / ((long long) num_sms() * 8 * 4);
+    return seg < 1 ? 1 : seg > 16 ? 16 : (int) seg;
 }
 
 int32_t pool_geom(const dcb_pool_desc* pd, const dcb_nd_desc* xd, const dcb_nd_desc* yd, PoolGeom* g)
@@ -832,6 +1083,18 @@ int32_t launch_pool_fwd(const PoolGeom& g, float alpha, float beta, const float*
         return DCB_UNSUPPORTED;
     }
     const dim3 grid((unsigned) gx, (unsigned) tiles, (unsigned) planes);
+    if (pair && cube && g.lo[2] == 0 && g.hi[2] == g.in[2])
+    {
+        const int seg = pool_walk((g.out[1] + rpb - 1) / rpb * tiles * planes, g.out[0]);
+        const long long mrows = (long long) ((g.out[0] + seg - 1) / seg) * g.out[1];
+        const dim3 mgrid((unsigned) ((mrows + rpb - 1) / rpb), (unsigned) tiles, (unsigned) planes);
+        auto kernel = g.mode != DCB_POOL_MAX ? pool_fwd_march_kernel<false, false>
+                      : argmax               ? pool_fwd_march_kernel<true, true>
+                                             : pool_fwd_march_kernel<true, false>;
+        kernel<<<mgrid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, tw_log2, mrows, seg);
+        DCB_LAUNCH_CHECK();
+        return DCB_OK;
+    }
     if (pair)
     {
         if (cube)
@@ -933,17 +1196,19 @@ extern "C" int32_t dcb_pool_bwd(const dcb_pool_desc* pd, const dcb_nd_desc* xd, 
         if (block && tiles <= 65535)
         {
             const int blocks_h = (g.in[1] + 1) / 2;
-            const long long brows = (long long) (cube ? (g.in[0] + 1) / 2 : g.in[0]) * blocks_h;
+            const int blocks_d = cube ? (g.in[0] + 1) / 2 : g.in[0];
+            const int seg = cube ? pool_walk((blocks_h + rpb - 1) / rpb * tiles * grid.z, blocks_d) : 1;
+            const long long brows = (long long) ((blocks_d + seg - 1) / seg) * blocks_h;
             const long long bgx = (brows + rpb - 1) / rpb;
             const dim3 gridb((unsigned) bgx, (unsigned) tiles, grid.z);
             if (cube)
                 pool_bwd_index_block_kernel<3><<<gridb, POOL_THREADS, 0, as_stream(stream)>>>(
                     g, (float) alpha, (float) beta, static_cast<const float*>(dy), static_cast<float*>(dx), idx,
-                    tw_log2, blocks_h, brows);
+                    tw_log2, blocks_h, brows, seg, blocks_d);
             else
                 pool_bwd_index_block_kernel<1><<<gridb, POOL_THREADS, 0, as_stream(stream)>>>(
                     g, (float) alpha, (float) beta, static_cast<const float*>(dy), static_cast<float*>(dx), idx,
-                    tw_log2, blocks_h, brows);
+                    tw_log2, blocks_h, brows, seg, blocks_d);
             DCB_LAUNCH_CHECK();
             return DCB_OK;
         }

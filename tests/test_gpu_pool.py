@@ -88,6 +88,53 @@ def test_kernels_against_oracle(case, mode):
     emu.assert_close(dxb.cpu().numpy(), 0.5 * dx_ref - dx0, 4e-6, "dx blend")
 
 
+# window 3, stride 2: walks of several outputs along D (the last one shorter), one walk
+# per output, an odd row end, no padding along D
+@pytest.mark.parametrize("n,c,sp,pad_d", [(1, 512, (37, 31, 20), 1), (2, 512, (24, 9, 8), 0), (1, 2, (6, 5, 264), 1),
+                                          (1, 3, (1, 2, 8), 1)])
+def test_walk_along_depth(n, c, sp, pad_d):
+    rng = np.random.default_rng(9)
+    window, pads, strides = (3, 3, 3), (pad_d, 1, 1), (2, 2, 2)
+    x = rng.integers(-4, 5, size=(n, c, *sp)).astype(np.float32)
+    x[rng.random(x.shape) < 0.2] = np.nan  # a window's first cell that is no number stays its maximum
+    x[rng.random(x.shape) < 0.1] = -np.inf
+    o = [(e + 2 * p - 3) // 2 + 1 for e, p in zip(sp, pads)]
+    # the rule in words: cells in D, H, W order, the first becomes the maximum, a later one if it is larger
+    best, idx = np.full((n, c, *o), np.nan, np.float32), np.full((n, c, *o), -1)
+    total = np.zeros((n, c, *o))
+    at = np.meshgrid(*[np.arange(e) * 2 for e in o], indexing="ij")
+    for kd in range(3):
+        for kh in range(3):
+            for kw in range(3):
+                q = [a + k - p for a, k, p in zip(at, (kd, kh, kw), pads)]
+                ok = np.logical_and.reduce([(a >= 0) & (a < e) for a, e in zip(q, sp)])
+                v = x[:, :, *[np.clip(a, 0, e - 1) for a, e in zip(q, sp)]]
+                with np.errstate(invalid="ignore"):
+                    take = ok & ((idx < 0) | (v > best))
+                best, idx = np.where(take, v, best), np.where(take, np.ravel_multi_index(
+                    [np.clip(a, 0, e - 1) for a, e in zip(q, sp)], sp), idx)
+                total += np.where(ok & np.isfinite(v), v, 0)
+    dy = rng.integers(-8, 9, size=best.shape).astype(np.float32)  # whole numbers: sums are exact in any order
+    dx_ref = np.zeros((n * c, int(np.prod(sp))), np.float32)
+    np.add.at(dx_ref, (np.arange(n * c)[:, None], idx.reshape(n * c, -1)), dy.reshape(n * c, -1))
+    xs, dys = torch.from_numpy(x).cuda(), torch.from_numpy(dy).cuda()
+    y, dx = torch.zeros_like(dys), torch.zeros_like(xs)
+    P = lambda t: ctypes.c_void_p(t.data_ptr())
+    pd, xd, yd = _pd(window, pads, strides, "MAX"), _nd(xs), _nd(y)
+    _abi.call("dcb_pool_fwd", ctypes.byref(pd), ctypes.byref(xd), ctypes.byref(yd), 1.0, P(xs), 0.0, P(y), None)
+    ws = torch.empty(y.numel(), dtype=torch.uint8, device="cuda")
+    _abi.call("dcb_pool_bwd", ctypes.byref(pd), ctypes.byref(xd), ctypes.byref(yd), 1.0, P(y), P(dys), P(xs), 0.0,
+              P(dx), P(ws), ws.numel(), None)
+    torch.cuda.synchronize()
+    assert np.array_equal(y.cpu().numpy(), best, equal_nan=True)
+    assert np.array_equal(dx.cpu().numpy().reshape(dx_ref.shape), dx_ref)
+    # averages: whole numbers, so the sums are exact and one division rounds
+    pd, xf = _pd(window, pads, strides, "AVERAGE"), torch.from_numpy(np.where(np.isfinite(x), x, 0)).cuda()
+    _abi.call("dcb_pool_fwd", ctypes.byref(pd), ctypes.byref(xd), ctypes.byref(yd), 1.0, P(xf), 0.0, P(y), None)
+    torch.cuda.synchronize()
+    assert np.allclose(y.cpu().numpy(), total / 27, rtol=2.0 ** -23, atol=0)
+
+
 def test_rejects_mismatched_output_extent():
     x = torch.zeros(1, 1, 8, 8, device="cuda")
     y = torch.zeros(1, 1, 5, 4, device="cuda")
