@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(BN_THREADS)
                     double* partial, unsigned* tickets,
                     float* __restrict__ sums, float* __restrict__ sqsums)
 {
+    wait_for_previous_kernel(x);
     const int c = blockIdx.y;
     double acc[2] = {0.0, 0.0};
     for (long long u = blockIdx.x; u < ug.upc; u += gridDim.x)
@@ -327,6 +328,7 @@ __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
                                    float decay, float* mean, float* var,
                                    float* running_mean, float* running_var)
 {
+    wait_for_previous_kernel(mean, var, running_mean, running_var);
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= channels)
         return;
@@ -368,6 +370,7 @@ __global__ void __launch_bounds__(BN_THREADS)
                     const float* __restrict__ bias, float eps, float slope,
                     FinalizeArgs fin)
 {
+    wait_for_previous_kernel(x, mean, var, scale, bias);
     const int c = blockIdx.y;
     float m, v0;
     if (FINALIZE)
@@ -442,6 +445,7 @@ __global__ void __launch_bounds__(BN_THREADS)
                          float* __restrict__ dscale, float* __restrict__ dbias,
                          float* __restrict__ dmean, float* __restrict__ dvar)
 {
+    wait_for_previous_kernel(x, dy, mean, var, scale);
     const int c = blockIdx.y;
     const float m = mean[c];
     const float sc = scale[c];
@@ -512,6 +516,7 @@ __global__ void __launch_bounds__(BN_THREADS)
                         const float* __restrict__ dvar, float eps,
                         long long num_per_sum)
 {
+    wait_for_previous_kernel(x, dy, mean, var, scale, dmean, dvar);
     const int c = gridDim.y - 1 - blockIdx.y; // the last one first, as the units below
     const float m = mean[c];
     const float sc = scale[c];
@@ -563,6 +568,7 @@ __global__ void __launch_bounds__(BN_THREADS)
                       const float* __restrict__ dy, RunStrides ds, float* out,
                       RunStrides os, UnitGeom ug, float slope)
 {
+    wait_for_previous_kernel(x, dy);
     const int c = blockIdx.y;
     for (long long u = blockIdx.x; u < ug.upc; u += gridDim.x)
     {
@@ -751,9 +757,9 @@ int32_t dcb_bn_stats(dcb_bn_plan* plan, const void* x, void* sums,
     }
     const dim3 grid = bn_grid(mv.ug);
 #define CALL(VV, PP)                                                               \
-    bn_stats_kernel<VV, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(           \
+    DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),           \
         static_cast<const float*>(x), mv.s[0], mv.ug, plan->partial,           \
-        plan->tickets, static_cast<float*>(sums), static_cast<float*>(sqsums))
+        plan->tickets, static_cast<float*>(sums), static_cast<float*>(sqsums)))
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
@@ -766,10 +772,11 @@ int32_t dcb_bn_finalize(int32_t channels, int64_t num_per_sum, float decay,
 {
     DCB_REQUIRE(channels > 0, "channels must be positive");
     DCB_REQUIRE(mean && var && running_mean && running_var, "null argument");
-    bn_finalize_kernel<<<(channels + 127) / 128, 128, 0, as_stream(stream)>>>(
+    DCB_CUDA_TRY(launch_overlapped(bn_finalize_kernel, dim3((unsigned) ((channels + 127) / 128)), 128, 0,
+                                   as_stream(stream),
         channels, num_per_sum, decay, static_cast<float*>(mean),
         static_cast<float*>(var), static_cast<float*>(running_mean),
-        static_cast<float*>(running_var));
+        static_cast<float*>(running_var)));
     DCB_LAUNCH_CHECK();
     return DCB_OK;
 }
@@ -793,10 +800,10 @@ static int32_t bn_apply_impl(const dcb_nd_desc* xd, const void* x, const void* m
     {                                                                                                              \
         auto kernel = leaky ? (fin ? bn_apply_kernel<VV, true, PP, true> : bn_apply_kernel<VV, true, PP, false>)   \
                             : (fin ? bn_apply_kernel<VV, false, PP, true> : bn_apply_kernel<VV, false, PP, false>); \
-        kernel<<<grid, BN_THREADS, 0, as_stream(stream)>>>(                                                        \
+        DCB_CUDA_TRY(launch_overlapped(kernel, grid, BN_THREADS, 0, as_stream(stream),                                                        \
             static_cast<const float*>(x), mv.s[0], static_cast<float*>(y), mv.s[1], mv.ug,                         \
             static_cast<const float*>(mean), static_cast<const float*>(var), static_cast<const float*>(scale),     \
-            static_cast<const float*>(bias), eps, slope, f);                                                       \
+            static_cast<const float*>(bias), eps, slope, f));                                                       \
     }
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
@@ -860,13 +867,13 @@ int32_t dcb_bn_bwd_reduce(dcb_bn_plan* plan, const void* x,
     }
     const dim3 grid = bn_grid(mv.ug);
 #define CALL(VV, PP)                                                               \
-    bn_bwd_reduce_kernel<VV, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(      \
+    DCB_CUDA_TRY(launch_overlapped((bn_bwd_reduce_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),      \
         static_cast<const float*>(x), mv.s[0], static_cast<const float*>(dy),  \
         mv.s[1], mv.ug, static_cast<const float*>(mean),                       \
         static_cast<const float*>(var), static_cast<const float*>(scale), eps, \
         plan->partial, plan->tickets, static_cast<float*>(dscale),             \
         static_cast<float*>(dbias), static_cast<float*>(dmean),                \
-        static_cast<float*>(dvar))
+        static_cast<float*>(dvar)))
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
@@ -892,12 +899,12 @@ int32_t dcb_bn_bwd_apply(const dcb_nd_desc* xd, const void* x,
         return DCB_OK;
     const dim3 grid = bn_grid(mv.ug);
 #define CALL(VV, PP)                                                               \
-    bn_bwd_apply_kernel<VV, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(       \
+    DCB_CUDA_TRY(launch_overlapped((bn_bwd_apply_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),       \
         static_cast<const float*>(x), mv.s[0], static_cast<const float*>(dy),  \
         mv.s[1], static_cast<float*>(dx), mv.s[2], mv.ug,                      \
         static_cast<const float*>(mean), static_cast<const float*>(var),       \
         static_cast<const float*>(scale), static_cast<const float*>(dmean),    \
-        static_cast<const float*>(dvar), eps, (long long) num_per_sum)
+        static_cast<const float*>(dvar), eps, (long long) num_per_sum))
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
@@ -918,9 +925,9 @@ int32_t dcb_leaky_relu_fwd(const dcb_nd_desc* xd, const void* x, float slope,
         return DCB_OK;
     const dim3 grid = bn_grid(mv.ug);
 #define CALL(VV, PP)                                                               \
-    leaky_relu_kernel<VV, 0, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(      \
+    DCB_CUDA_TRY(launch_overlapped((leaky_relu_kernel<VV, 0, PP>), grid, BN_THREADS, 0, as_stream(stream),      \
         static_cast<const float*>(x), mv.s[0], nullptr, mv.s[0],               \
-        static_cast<float*>(y), mv.s[1], mv.ug, slope)
+        static_cast<float*>(y), mv.s[1], mv.ug, slope))
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
@@ -942,9 +949,9 @@ int32_t dcb_leaky_relu_bwd(const dcb_nd_desc* xd, const void* x,
         return DCB_OK;
     const dim3 grid = bn_grid(mv.ug);
 #define CALL(VV, PP)                                                               \
-    leaky_relu_kernel<VV, 1, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(      \
+    DCB_CUDA_TRY(launch_overlapped((leaky_relu_kernel<VV, 1, PP>), grid, BN_THREADS, 0, as_stream(stream),      \
         static_cast<const float*>(x), mv.s[0], static_cast<const float*>(dy),  \
-        mv.s[1], static_cast<float*>(dx), mv.s[2], mv.ug, slope)
+        mv.s[1], static_cast<float*>(dx), mv.s[2], mv.ug, slope))
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
@@ -1034,9 +1041,9 @@ extern "C" int32_t dcb_bn_stats_noalloc(const dcb_nd_desc* xd, const void* x, vo
     // the arrival tickets must start at zero.  Partials are overwritten.
     DCB_CUDA_TRY(cudaMemsetAsync(tickets, 0, xd->c * sizeof(unsigned), as_stream(stream)));
 #define CALL(VV, PP)                                                               \
-    bn_stats_kernel<VV, PP><<<grid, BN_THREADS, 0, as_stream(stream)>>>(           \
+    DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),           \
         static_cast<const float*>(x), mv.s[0], mv.ug, partial, tickets,        \
-        static_cast<float*>(sums), static_cast<float*>(sqsums))
+        static_cast<float*>(sums), static_cast<float*>(sqsums)))
     DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();

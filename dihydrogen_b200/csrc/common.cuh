@@ -68,10 +68,15 @@ int num_sms();
 // Raises a kernel's limit of dynamic shared memory, once per kernel and device.
 int32_t allow_dynamic_smem(const void* kernel, int bytes);
 
-// Launches a kernel that may start while the kernel before it in the stream is still
-// running (once all of that one's blocks have called dependents_may_start or ended).
-// Whatever it does with that kernel's results, or over its operands, comes after
-// wait_for_previous_kernel.
+// Launches a kernel that may start while the kernel before it in the stream is ending:
+// its launch, and what it sets up, are then off the path (a convolution beside the
+// packing of its filter, which calls dependents_may_start; 32^3 x 4 -> 16 forward and
+// backward, ten launches: 76 -> 73 us).  Whatever it does with that kernel's results, or
+// over its operands, comes after wait_for_previous_kernel, which waits for that kernel's
+// end; and so for everything before it, if all kernels launched like this wait.
+// The backward filter is launched plainly: its CTAs then start together and in order,
+// which its 1.4 ms on a 256^3 shard need more (2260 us with the pass before it, 2310 us
+// launched like this).
 template <class... Params, class... Args>
 inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem,
                                      cudaStream_t stream, Args&&... args)
@@ -95,9 +100,13 @@ __device__ __forceinline__ void dependents_may_start()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-__device__ __forceinline__ void wait_for_previous_kernel()
+// The pointers are what the kernel reads through: a read-only load could otherwise be
+// moved up across the wait.
+template <class... T>
+__device__ __forceinline__ void wait_for_previous_kernel(T&... through)
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    (([&] { asm volatile("" : "+l"(through)); }()), ...);
 }
 int64_t wait_budget_ns();
 

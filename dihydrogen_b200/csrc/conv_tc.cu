@@ -555,8 +555,8 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
     tc_row_window(g, x_skip(x));
     const int use_ymap = sw_make_y_map(g, y, &ymap) ? 1 : 0;
     const long long total = (long long) g.b_bytes / 4;
-    sw_pack_filter_kernel<<<(unsigned) ((total + 255) / 256), 256, 0, stream>>>(w, p->sw_bimg, g);
-    DCB_LAUNCH_CHECK();
+    DCB_CUDA_TRY(launch_overlapped(sw_pack_filter_kernel, dim3((unsigned) ((total + 255) / 256)), 256, 0, stream, w,
+                                   p->sw_bimg, g));
     size_t smem = sw_smem_need(g);
     smem = smem < 120 * 1024 ? 120 * 1024 : smem; // one CTA per SM: it owns all of tensor memory
     long long grid = (long long) num_sms();
@@ -572,9 +572,8 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
         const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 224 * 1024);
         if (set != DCB_OK)
             return set;
-        kernel<<<(unsigned) grid, sw_threads(xi), smem, stream>>>(g, alpha, p->sw_bimg, y, status, map, ymap, use_ymap,
-                                                                  p->stat_part);
-        DCB_LAUNCH_CHECK();
+        DCB_CUDA_TRY(launch_overlapped(kernel, dim3((unsigned) grid), sw_threads(xi), smem, stream, g, alpha, p->sw_bimg, y,
+                                       status, map, ymap, use_ymap, p->stat_part));
         return DCB_OK;
     };
     int32_t st;
@@ -586,8 +585,8 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
         st = c4f3 ? launch(sw_conv_kernel<true, false, 0>, 0) : launch(sw_conv_kernel<false, false, 0>, 0);
     if (st != DCB_OK || !stats)
         return st;
-    sw_stats_fold_kernel<<<1, SW_FOLD_WARPS * 32, 0, stream>>>(p->stat_part, (int) grid * SW_EPI, g.k, sums, sqsums);
-    DCB_LAUNCH_CHECK();
+    DCB_CUDA_TRY(launch_overlapped(sw_stats_fold_kernel, dim3(1), SW_FOLD_WARPS * 32, 0, stream, p->stat_part,
+                                   (int) grid * SW_EPI, g.k, sums, sqsums));
     return DCB_OK;
 }
 
@@ -599,7 +598,7 @@ static __global__ void __launch_bounds__(256) wg_fold_kernel(const __grid_consta
     const int e = (int) (blockIdx.x * 32 + threadIdx.x / 8), sub = threadIdx.x & 7;
     const bool on = e < g.k * g.c * taps;
     double s = 0.0;
-    wait_for_previous_kernel();
+    wait_for_previous_kernel(part);
     if (on)
     {
         const int kw = e % g.f[2], kh = e / g.f[2] % g.f[1], kd = e / (g.f[2] * g.f[1]) % g.f[0];

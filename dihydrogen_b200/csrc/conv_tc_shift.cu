@@ -29,6 +29,7 @@ __global__ void sh_pack_filter_kernel(const float* __restrict__ w, uint4* __rest
                                       uint32_t rnd_add, uint32_t rnd_mask, float alpha)
 {
     dependents_may_start();
+    wait_for_previous_kernel(w);
     const ShPack p = packs[blockIdx.y];
     const int kg = (int) blockIdx.z / cgroups, grp = (int) blockIdx.z % cgroups;
     uint4* o = out + (size_t) blockIdx.z * total16 + p.off16;
@@ -76,7 +77,8 @@ __global__ void __launch_bounds__(SH_FOLD_WARPS * 32)
 {
     __shared__ double sm[SH_FOLD_WARPS][32];
     const int t = threadIdx.x & 31, w = threadIdx.x >> 5;
-    wait_for_previous_kernel();
+    dependents_may_start();
+    wait_for_previous_kernel(part);
     double acc = 0.0;
 #pragma unroll 1
     for (int i = w; i < nparts; i += SH_FOLD_WARPS * 16)
@@ -832,12 +834,11 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
     const bool stats = sums != nullptr;
     if (stats && (beta != 0.f || !sh_has_stats(p)))
         return DCB_UNSUPPORTED;
-    sh_pack_filter_kernel<<<dim3((unsigned) ((p->max_image + 255) / 256), (unsigned) t.packs.size(),
-                                 (unsigned) (g.kgroups * g.cgroups)),
-                            256, 0, stream>>>(w, p->image, p->packs, p->chunks, p->codes, t.kind, t.parts, t.total16,
-                                              g.cgroups, g.cpg, g.cin, g.kout, g.kcols, t.w_ko, t.w_ci, g.rnd_add,
-                                              g.rnd_mask, alpha);
-    DCB_LAUNCH_CHECK();
+    DCB_CUDA_TRY(launch_overlapped(sh_pack_filter_kernel,
+                                   dim3((unsigned) ((p->max_image + 255) / 256), (unsigned) t.packs.size(),
+                                        (unsigned) (g.kgroups * g.cgroups)),
+                                   256, 0, stream, w, p->image, p->packs, p->chunks, p->codes, t.kind, t.parts, t.total16,
+                                   g.cgroups, g.cpg, g.cin, g.kout, g.kcols, t.w_ko, t.w_ci, g.rnd_add, g.rnd_mask, alpha));
     CUtensorMap ymap;
     std::memset(&ymap, 0, sizeof(ymap));
     const int use_ymap = beta == 0.f && sh_make_y_map(g, y, &ymap) ? 1 : 0;

@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     // the filter image, the input and everything that is written
-    wait_for_previous_kernel();
+    wait_for_previous_kernel(x);
     bool ok = true;
 
     if (warp < SH_EPI)

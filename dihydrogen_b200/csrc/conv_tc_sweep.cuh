@@ -133,6 +133,7 @@ __device__ __forceinline__ int sw_mod(int a, int m)
 // with kd = (r + pad - s) mod fd.
 __global__ void sw_pack_filter_kernel(const float* __restrict__ w, float* __restrict__ b, SwGeom g)
 {
+    wait_for_previous_kernel(w);
     const int fd = g.f[0], fh = g.f[1], fw = g.f[2];
     const int per_rot = g.kb * g.ntot;
     const long long total = (long long) fd * per_rot;
@@ -224,9 +225,20 @@ __global__ void __launch_bounds__(SW_FOLD_WARPS * 32)
 {
     __shared__ double sm[SW_FOLD_WARPS][32];
     const int t = threadIdx.x & 31, w = threadIdx.x >> 5;
+    wait_for_previous_kernel(part);
     double acc = 0.0;
-    for (int i = w; i < nparts; i += SW_FOLD_WARPS)
-        acc += (double) part[(size_t) i * 32 + t];
+#pragma unroll 1
+    for (int i = w; i < nparts; i += SW_FOLD_WARPS * 16)
+    {
+        // 16 loads in flight: the kernel is a few trips to memory and nothing else
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            v[k] = i + k * SW_FOLD_WARPS < nparts ? part[(size_t) (i + k * SW_FOLD_WARPS) * 32 + t] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            acc += (double) v[k];
+    }
     sm[w][t] = acc;
     __syncthreads();
     if (w != 0)
@@ -366,6 +378,8 @@ __global__ void __launch_bounds__(sw_threads(XISS), 1)
         const uint32_t sel = part < (g.split ? 2 : 1) ? (uint32_t) part : 2u;
         ktab[r] = sel == 2u ? ((2u << 16) | 4u) : (off | (sel << 16));
     }
+    // the filter image, the input and everything that is written
+    wait_for_previous_kernel(bimg);
     for (int i = tid; i < g.b_bytes / 16; i += sw_threads(XISS))
         reinterpret_cast<float4*>(b_smem)[i] = reinterpret_cast<const float4*>(bimg)[i];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

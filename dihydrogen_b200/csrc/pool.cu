@@ -828,8 +828,9 @@ __global__ void __launch_bounds__(POOL_THREADS)
 // window rows are loaded once for sixteen cells and every comparison is against a
 // constant.  For WD = 3 the thread walks along D: window plane p+1 is kept for the next
 // block, and the plane behind it is on its way while this one is compared (269 -> 258 us
-// for 16 x 256^3; 190 us at the rate of a copy).  Cells outside the global tensor never were a window's maximum, so they need no mask.  Per cell the
-// sums run in the same order (D, H, then W ascending).
+// for 16 x 256^3; 190 us at the rate of a copy).  Cells outside the global tensor never
+// were a window's maximum, so they need no mask.  Per cell the sums run in the same order
+// (D, H, then W ascending).
 struct PoolWindows
 {
     int a[3];   // index byte of windows 2t, 2t+1, 2t+2 (255: no window)
