@@ -29,44 +29,53 @@ __global__ void sh_pack_filter_kernel(const float* __restrict__ w, uint4* __rest
                                       uint32_t rnd_add, uint32_t rnd_mask, float alpha)
 {
     dependents_may_start();
-    wait_for_previous_kernel(w);
+    // the tables are the plan's: only the filter and the image have to wait
     const ShPack p = packs[blockIdx.y];
     const int kg = (int) blockIdx.z / cgroups, grp = (int) blockIdx.z % cgroups;
     uint4* o = out + (size_t) blockIdx.z * total16 + p.off16;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < p.n * p.nchunks; v += gridDim.x * blockDim.x)
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = v < p.n * p.nchunks;
+    const int c = v / p.n, col = v - c * p.n;
+    ShChunk ck = {};
+    int code = -1;
+    if (on)
+        ck = chunks[p.chunk0 + c], code = codes[p.code0 + col];
+    wait_for_previous_kernel(w);
+    if (!on)
+        return;
+    const int ko = kg * kcols + (code >> 16);
+    const int ch0 = grp * cpg + ck.ch;
+    const int CH = kind == 0 ? 4 : 8;
+    const bool any = ck.part >= 0 && code >= 0 && ko < kout;
+    const float* wp = w + ((long long) ko * w_ko + (long long) ch0 * w_ci + (code & 0xffff) + ck.kw);
+    float f[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        f[e] = any && e < CH && ch0 + e < cin && ck.ch + e < cpg ? alpha * wp[e * w_ci] : 0.f;
+    uint32_t r[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
     {
-        const int c = v / p.n, col = v - c * p.n;
-        const ShChunk ck = chunks[p.chunk0 + c];
-        const int code = codes[p.code0 + col];
-        const int ko = kg * kcols + (code >> 16);
-        const int ch0 = grp * cpg + ck.ch;
-        const int CH = kind == 0 ? 4 : 8;
-        uint32_t r[8];
-        for (int e = 0; e < 8; ++e)
-        {
-            float f = 0.f;
-            if (e < CH && ck.part >= 0 && code >= 0 && ko < kout && ch0 + e < cin && ck.ch + e < cpg)
-                f = alpha * w[(long long) ko * w_ko + (long long) (ch0 + e) * w_ci + (code & 0xffff) + ck.kw];
-            if (kind == 0)
-            {
-                const uint32_t hi = (__float_as_uint(f) + rnd_add) & rnd_mask;
-                r[e] = ck.part <= 0 ? hi : tf32_rna(f - __uint_as_float(hi));
-            }
-            else if (parts == 1)
-                r[e] = __float_as_uint(f) + rnd_add;
-            else
-            {
-                for (int s = 0; s < ck.part; ++s)
-                    f -= __uint_as_float(__float_as_uint(f) & 0xffff0000u);
-                r[e] = __float_as_uint(f);
-            }
-        }
         if (kind == 0)
-            o[v] = make_uint4(r[0], r[1], r[2], r[3]);
+        {
+            const uint32_t hi = (__float_as_uint(f[e]) + rnd_add) & rnd_mask;
+            r[e] = ck.part <= 0 ? hi : tf32_rna(f[e] - __uint_as_float(hi));
+        }
+        else if (parts == 1)
+            r[e] = __float_as_uint(f[e]) + rnd_add;
         else
-            o[v] = make_uint4(pack_hi16(r[0], r[1]), pack_hi16(r[2], r[3]), pack_hi16(r[4], r[5]),
-                              pack_hi16(r[6], r[7]));
+        {
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+                if (s < ck.part)
+                    f[e] -= __uint_as_float(__float_as_uint(f[e]) & 0xffff0000u);
+            r[e] = __float_as_uint(f[e]);
+        }
     }
+    if (kind == 0)
+        o[v] = make_uint4(r[0], r[1], r[2], r[3]);
+    else
+        o[v] = make_uint4(pack_hi16(r[0], r[1]), pack_hi16(r[2], r[3]), pack_hi16(r[4], r[5]), pack_hi16(r[6], r[7]));
 }
 
 // sums / sqsums[k] from the per epilogue warp partials of a launch, in order, in fp64.

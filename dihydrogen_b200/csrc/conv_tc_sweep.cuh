@@ -133,6 +133,7 @@ __device__ __forceinline__ int sw_mod(int a, int m)
 // with kd = (r + pad - s) mod fd.
 __global__ void sw_pack_filter_kernel(const float* __restrict__ w, float* __restrict__ b, SwGeom g)
 {
+    dependents_may_start();
     wait_for_previous_kernel(w);
     const int fd = g.f[0], fh = g.f[1], fw = g.f[2];
     const int per_rot = g.kb * g.ntot;
