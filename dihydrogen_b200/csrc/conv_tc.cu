@@ -158,7 +158,7 @@ double wg_mma_cost(int n)
 }
 
 // One way to deal out the work; false when it does not fit.
-bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int kg, int B, int PW, double* cost)
+bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int kg, int B, int PW, bool ring, double* cost)
 {
     WgGeom& g = *out;
     const int sh = cg.stride[1], fh = cg.f[1];
@@ -244,7 +244,9 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
         return false;
     // shared memory; 64 bytes behind every 128-byte multiple of cells keep the
     // converters' stores (four rows x two cells at a time) on different banks
-    g.xrows = kdg * g.X * g.r8;
+    const int planes = ring ? 1 : kdg; // of x that a stage brings
+    g.ring = ring;
+    g.xrows = planes * g.X * g.r8;
     g.yrows = B * g.n8;
     g.lbo_x = g.xrows * 16 + 64;
     g.lbo_y = g.yrows * 16 + 64;
@@ -253,12 +255,12 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
     g.cq = (cgp + 3) / 4;
     g.kq = (kg + 3) / 4;
     g.qg = (g.Q + 7) / 8;
-    g.items_x = kdg * g.X * g.cq * g.qg;
+    g.items_x = planes * g.X * g.cq * g.qg;
     g.items_y = B * g.kq * g.qg;
     const int tail = WG_MAX_TILES * (int) sizeof(WgTile) + (g.items_x + g.items_y) * 16 + 256 + 2048 + 128;
     const int room = 226 * 1024 - tail, dump = g.kd_cols * 512;
     g.nstages = room / g.stage_bytes < WG_MAX_STAGES ? room / g.stage_bytes : WG_MAX_STAGES;
-    if (g.nstages < 2 || dump > room || g.lbo_x >= 1 << 18 || g.lbo_y >= 1 << 18)
+    if (g.nstages < (ring ? kdg + 1 : 2) || dump > room || g.lbo_x >= 1 << 18 || g.lbo_y >= 1 << 18)
         return false;
     const int body = g.nstages * g.stage_bytes > dump ? g.nstages * g.stage_bytes : dump;
     g.so_tiles = (body + 127) / 128 * 128;
@@ -363,7 +365,13 @@ bool wg_geom(const ConvGeom& cg, int math_mode, WgGeom* out)
                             if (pw < 16 && chunks > 1)
                                 break;
                             double cost;
-                            if (wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, &cost) && (best_cost < 0 || cost < best_cost))
+                            // all planes kd in one role and unit stride along D: a walk along D converts a
+                            // plane of x once, not once per kd (and needs kdg - 1 steps to begin with)
+                            const bool ring = kdg > 1 && kdg == cg.f[0] && cg.stride[0] == 1 && cg.out[0] >= 4;
+                            bool found = ring && wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, true, &cost);
+                            if (!found || g.stages < 4ll * g.parts)
+                                found = wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, false, &cost);
+                            if (found && (best_cost < 0 || cost < best_cost))
                                 best_cost = cost, best = g;
                             if (pw <= 16)
                                 break;

@@ -43,16 +43,26 @@ struct WgUnit
     int n, od, h0, w0;
 };
 
+template <bool RING>
 __device__ __forceinline__ WgUnit wg_unit(const WgGeom& g, long long s)
 {
     WgUnit u;
     uint32_t r = (uint32_t) s;
+    if (RING)
+    {
+        u.od = (int) (r % (uint32_t) g.out[0]);
+        r /= (uint32_t) g.out[0];
+    }
     u.h0 = (int) (r % (uint32_t) g.hblocks) * g.B;
     r /= (uint32_t) g.hblocks;
     u.w0 = (int) (r % (uint32_t) g.wchunks) * g.PW;
     r /= (uint32_t) g.wchunks;
-    u.od = (int) (r % (uint32_t) g.out[0]);
-    u.n = (int) (r / (uint32_t) g.out[0]);
+    if (!RING)
+    {
+        u.od = (int) (r % (uint32_t) g.out[0]);
+        r /= (uint32_t) g.out[0];
+    }
+    u.n = (int) r;
     return u;
 }
 
@@ -88,7 +98,7 @@ struct WgConvArgs
 // instructions is what bounds a stage where channels are few: hence pairs of items
 // without branches between them, and stages that follow each other along H, so that
 // most of them only move a pointer.
-template <bool ISX, int SW, int KWG, int AL>
+template <bool ISX, int SW, int KWG, int AL, bool RING>
 __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c, const float* __restrict__ src)
 {
     constexpr int NV = ISX ? 3 * SW + KWG : 4;                  // cells behind four positions
@@ -98,7 +108,8 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
     const uint32_t lane_dst = (uint32_t) (ql * (ISX ? g.lbo_x : g.lbo_y) + 16 * cl);
     const uint32_t row16 = 16u * (uint32_t) (ISX ? g.cg : g.kgp);
     const int rows_in = ISX ? g.in[1] : g.out[1], step_rows = ISX ? g.B * g.stride[1] : g.B;
-    const long long step = 4ll * step_rows * (ISX ? g.xs[1] : g.ys[1]);
+    const long long step = RING ? 4ll * (ISX ? g.xs[0] : g.ys[0]) : 4ll * step_rows * (ISX ? g.xs[1] : g.ys[1]);
+    int seg = 0, seg_left = 0, odv = 0; // RING: stages and steps of a walk along D, dy plane of the step in it
     float t[2][2][4 * NB];
     uint32_t dst[2][2] = {{0, 0}, {0, 0}}, mask[2][2] = {{0, 0}, {0, 0}};
     uint32_t wait[2] = {0, 0}, tell[2] = {0, 0};
@@ -110,7 +121,15 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
     int h0 = 0, r0 = 0, id0 = 0;
     uint32_t m8[2] = {0, 0}; // valid cells, per group of eight lanes along the row
     auto locate = [&]() {
-        const WgUnit u = wg_unit(g, s);
+        WgUnit u = wg_unit<RING>(g, s);
+        if (RING)
+        {
+            seg = min(c.s1 - s, g.out[0] - u.od);
+            seg_left = seg + g.kdg - 1;
+            odv = 1 - g.kdg;
+            if (!ISX)
+                u.od += odv;
+        }
         h0 = u.h0;
         const int w0 = ISX ? u.w0 * SW + c.rkw - g.pad[2] : u.w0, width = ISX ? g.in[2] : g.out[2];
         if (ISX)
@@ -207,7 +226,11 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
                 if (!fresh)
                 {
                     item = c.w;
-                    if (++s == c.s1)
+                    if (RING)
+                        s += --seg_left == 0 ? seg : 0;
+                    else
+                        ++s;
+                    if (s == c.s1)
                     {
                         more = false;
                         continue;
@@ -220,7 +243,14 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
                         ++lap;
                     }
                     h0 += g.B;
-                    if (h0 < g.out[1])
+                    if (RING && seg_left != 0)
+                    {
+                        // the next plane
+                        ++id0;
+                        ++odv;
+                        b0 += step;
+                    }
+                    else if (!RING && h0 < g.out[1])
                     {
                         // the next rows of the same column
                         r0 += step_rows;
@@ -245,6 +275,8 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
                 const bool second = (it[i].x >> 24) != 0; // group of lanes along the row
                 const bool stored = cl < (int) (it[i].x >> 16 & 15u) && (second ? ql + 8 : ql) < g.Q;
                 bool in = cl < (int) (it[i].x >> 20 & 15u) && (unsigned) (r0 + row) < (unsigned) rows_in;
+                if (RING && !ISX)
+                    in = in && odv >= 0;
                 if (ISX)
                     in = in && (unsigned) (id0 + (int) (it[i].x >> 2 & 63u)) < (unsigned) g.in[0];
                 const uint32_t m = in ? (second ? m8[1] : m8[0]) : 0u;
@@ -409,10 +441,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                               isx ? w : w - g.warps_x, lane, abort_flag};
         if (c.w < c.items)
         {
-            if (!isx)
-                ok = g.vec_y ? wg_convert<false, 1, 1, 0>(g, c, dy) : wg_convert<false, 1, 1, -1>(g, c, dy);
+            if (g.ring)
+            {
+                if (!isx)
+                    ok = g.vec_y ? wg_convert<false, 1, 1, 0, true>(g, c, dy) : wg_convert<false, 1, 1, -1, true>(g, c, dy);
+                else
+                    ok = wg_convert<true, SW, KWG, AL, true>(g, c, x);
+            }
+            else if (!isx)
+                ok = g.vec_y ? wg_convert<false, 1, 1, 0, false>(g, c, dy) : wg_convert<false, 1, 1, -1, false>(g, c, dy);
             else
-                ok = wg_convert<true, SW, KWG, AL>(g, c, x);
+                ok = wg_convert<true, SW, KWG, AL, false>(g, c, x);
         }
     }
     else
@@ -425,10 +464,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         const int ksteps = g.Q / 2;
         int buf = 0, left = g.flush_stages;
         uint32_t par = 0, cpar = 0;
+        // ring: `lead` steps of a walk only bring planes of x; a step's buffer is free again when the
+        // last step that reads its plane is through
+        const int lead = g.ring ? g.kdg - 1 : 0;
+        int walk = lead, walk_end = 0, steps = 0; // position in the walk, its length
 #pragma unroll 1
-        for (int s = s0; s < s1 && ok; ++s)
+        for (int s = s0; s < s1 && ok;)
         {
-            if (left == 0)
+            if (g.ring && walk_end == 0)
+                walk = 0, walk_end = min(s1 - s, g.out[0] - s % g.out[0]) + lead;
+            const bool real = walk >= lead;
+            if (real && left == 0)
             {
                 if (elected)
                     mma_commit(chain_end);
@@ -438,21 +484,28 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                 if (!ok)
                     break;
             }
-            --left;
+            left -= real;
             ok = mbar_wait_t<0>(&full[buf], par, abort_flag);
             if (!ok)
                 break;
             tc_fence_after();
-            const uint32_t a_st = base16 + (uint32_t) (buf * g.stage_bytes) / 16u, b_st = a_st + (uint32_t) g.y_off / 16u;
+            const uint32_t b_st = base16 + (uint32_t) (buf * g.stage_bytes + g.y_off) / 16u;
+            const int oldest = buf - lead + (buf < lead ? g.nstages : 0);
             if (elected)
             {
+                int xb = oldest;
 #pragma unroll 1
-                for (int kd = 0; kd < g.kdg; ++kd)
+                for (int kd = 0; kd < g.kdg && real; ++kd)
+                {
+                    const uint32_t a_st =
+                        base16 + (uint32_t) (xb * g.stage_bytes) / 16u + (g.ring ? 0u : (uint32_t) (kd * g.kd_a16));
+                    if (g.ring && ++xb == g.nstages)
+                        xb = 0;
 #pragma unroll 1
                     for (int t = 0; t < g.ntiles; ++t)
                     {
                         const WgTile tl = tiles[t];
-                        uint32_t a = (a_st + tl.a16 + (uint32_t) (kd * g.kd_a16)) | lx << 16;
+                        uint32_t a = (a_st + tl.a16) | lx << 16;
                         uint32_t b = (b_st + tl.b16) | ly << 16;
                         const uint32_t d = tmem + tl.dcol + (uint32_t) (kd * g.kd_cols);
 #pragma unroll 4
@@ -465,11 +518,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                             b += 2 * ly;
                         }
                     }
-                mma_commit(&empty[buf]);
-                if (s + 1 == s1)
+                }
+                if (steps >= lead)
+                    mma_commit(&empty[oldest]);
+                if (real && s + 1 == s1)
                     mma_commit(chain_end);
             }
             __syncwarp();
+            ++steps;
+            s += real;
+            if (g.ring && ++walk == walk_end)
+                walk_end = 0;
             if (++buf == g.nstages)
             {
                 buf = 0;

@@ -12,7 +12,7 @@ constexpr int WG_FLUSH = 4;  // warps 0..3: running sums, one per lane quadrant
 constexpr int WG_CONV = 15;  // converter warps (20 warps in all leave 96 registers a thread)
 constexpr int WG_ISSUE_WARP = WG_FLUSH + WG_CONV;
 constexpr int WG_THREADS = (WG_FLUSH + WG_CONV + 1) * 32;
-constexpr int WG_MAX_STAGES = 4;
+constexpr int WG_MAX_STAGES = 8;
 constexpr int WG_MAX_TILES = 24;
 constexpr int WG_CHAIN = 128; // updates of an accumulator: 5e-6 of the result's scale on the longest sums
 
@@ -29,6 +29,7 @@ struct WgGeom
     long long xs_n, xs_c, xs[3], ys_n, ys_c, ys[3];
     int cg, ncg, kwg, nkw, kdg, nkd, kg, kgp, nkg; // channels, taps kw, planes kd, filters per role and their groups
     int roles, parts;
+    int ring;             // stages follow each other along D and keep the planes of x: see the kernel
     int A, X, B, PW, Q;   // input rows per tile, input and dy rows per stage, positions and cells of a row
     int r8, n8;           // matrix rows of an input row, of a dy row
     int xrows, yrows;     // matrix rows of a stage
