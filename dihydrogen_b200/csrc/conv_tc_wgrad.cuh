@@ -18,7 +18,11 @@
 // and filters would use a fraction of both.
 //
 // A stage is B dy rows and the X = (B - 1) * sh + fh input rows of each of its kd
-// planes, PW positions wide, in one of two to four shared-memory buffers.
+// planes, PW positions wide, in one of two to eight shared-memory buffers.
+// Few channels leave room for the accumulators of all kd in one role.  The stages then
+// walk along D (`ring`): a stage brings one plane of x and its dy rows, the kd planes are
+// those of the last kdg stages, and an input row is read, split and written once instead
+// of once per kd; the first kdg - 1 steps of a walk only bring x.
 // Converter warps read x and dy straight from global memory, split them and write
 // the stage; one thread issues.  What does not fit tensor memory (512 columns,
 // accumulators and running sums) or the 128 matrix rows is dealt out in roles:
@@ -110,10 +114,14 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
     const int rows_in = ISX ? g.in[1] : g.out[1], step_rows = ISX ? g.B * g.stride[1] : g.B;
     const long long step = RING ? 4ll * (ISX ? g.xs[0] : g.ys[0]) : 4ll * step_rows * (ISX ? g.xs[1] : g.ys[1]);
     int seg = 0, seg_left = 0, odv = 0; // RING: stages and steps of a walk along D, dy plane of the step in it
-    float t[2][2][4 * NB];
-    uint32_t dst[2][2] = {{0, 0}, {0, 0}}, mask[2][2] = {{0, 0}, {0, 0}};
-    uint32_t wait[2] = {0, 0}, tell[2] = {0, 0};
-    bool has[2] = {false, false};
+    // Pairs in flight.  dy of a walk along D comes from as many distant places as there are
+    // filters and takes few registers: four (256^3, 4 -> 16 channels: 1284 -> 1179 us); along
+    // H the next rows are near and more only costs (stride 2: 1084 -> 1108 us).
+    constexpr int AHEAD = !ISX && RING ? 4 : 2;
+    float t[AHEAD][2][4 * NB];
+    uint32_t dst[AHEAD][2] = {}, mask[AHEAD][2] = {};
+    uint32_t wait[AHEAD] = {}, tell[AHEAD] = {};
+    bool has[AHEAD] = {};
     int item = c.w - 2 * c.warps, s = c.s0, buf = 0;
     uint32_t lap = 0, st = c.base;
     bool ok = true, more = c.s0 < c.s1, fresh = true;
@@ -163,7 +171,7 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
     while (ok && (more || has[0]))
     {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < AHEAD; ++q)
         {
             if (has[q])
             {
