@@ -604,6 +604,9 @@ def test_shift_kernel_tile_and_table_edges(geom):
     (2, 2, 3, (11, 18), (2, 2), 2),            # two taps
     (1, 2, 3, (12, 36), (7, 7), 1),            # more taps than one launch takes
     (4, 1, 4, (200, 130), (3, 3), 1),          # long sums: running sums used
+    (1, 4, 16, (37, 29, 70), (3, 3, 3), 1),    # walks along D that begin and end inside a column
+    (2, 4, 16, (4, 101, 128), (3, 3, 3), 1),   # walks shorter than the ring of planes
+    (1, 5, 7, (66, 50, 41), (2, 3, 3), 1),     # two planes kd, rows no vector load can read
 ])
 def test_backward_filter_stage_and_role_edges(geom):
     N, C, K, sp, f, s = geom
