@@ -114,7 +114,7 @@ struct ShUnit
 };
 
 // Not inlined: several divisions, called at a handful of places once per unit.
-__device__ __noinline__ ShUnit sh_unit(const ShGeom& g, uint32_t u)
+static __device__ __noinline__ ShUnit sh_unit(const ShGeom& g, uint32_t u)
 {
     ShUnit t;
     const uint32_t tw = u % (uint32_t) g.tiles_w;
