@@ -687,8 +687,8 @@ def run_ours(args):
         k_fb = max(3, min(args.steps, 20))
         ms_fb = timed(fb_step, k_fb, 3)
         ms_b = timed(bwd_step, k_fb, 1)
-        names = {0: "fp32 CUDA-core", 1: "tcgen05 row", 2: "tcgen05 row (register-fed)", 3: "tcgen05 sweep or shift",
-                 4: "tcgen05 shift, two accumulator sets", 5: "tcgen05 backward filter"}
+        names = {0: "fp32 CUDA-core", 3: "tcgen05 sweep or shift, TF32", 4: "tcgen05 shift, three bf16 parts",
+                 5: "tcgen05 backward filter"}
         fwd_bwd = {"ms_per_pass": ms_fb, "backward_ms": ms_b, "steps": k_fb,
                    "kernels": {n: names.get(conv.kernel_variant(i), "?")
                                for i, n in enumerate(("conv_fwd", "conv_bwd_data", "conv_bwd_filter"))}}

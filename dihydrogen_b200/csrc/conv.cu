@@ -205,7 +205,7 @@ int32_t dcb_conv_plan_kernel_variant(const dcb_conv_plan* p, int32_t which)
         return -1;
     if (p->kind[which] != 1)
         return 0;
-    return which == 2 ? 5 : (sh_two_sets(p->sh[which]) ? 4 : 3);
+    return which == 2 ? 5 : (sh_bf16_split(p->sh[which]) ? 4 : 3);
 }
 
 int32_t dcb_conv_fwd(dcb_conv_plan* p, double alpha, const void* x,

@@ -189,9 +189,9 @@ bool sh_has_stats(const ShPlan* p)
     return g.kgroups == 1 && g.nb <= 16 && g.e_s * g.e_r * g.e_w == 1;
 }
 
-bool sh_two_sets(const ShPlan* p)
+bool sh_bf16_split(const ShPlan* p)
 {
-    return p->t.g.nsets > 1;
+    return p->t.parts == 3;
 }
 
 // The output as a 5-D tensor (W, R, S, filters, samples) whose box is what one

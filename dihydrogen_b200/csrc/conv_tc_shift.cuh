@@ -12,10 +12,11 @@
 // Precision of the products: one pass on TF32 or bf16 operands, or fp32 quality
 // as 3 products of a two-way TF32 split (few channels) or 6 products of an exact
 // three-way bf16 split (24 bits = 3 x 8; the dropped products are below 2^-24).
-// The tensor pipe adds into its fp32 accumulators by truncation, so long
-// reductions keep the leading products and the corrections in two accumulator
-// sets: the corrections are 2^-8 of the sum and their chain costs nothing, the
-// leading products are a third (TF32) or a sixth (bf16) of the updates.
+// The tensor pipe adds into its fp32 accumulators by truncation.  The corrections are
+// 2^-8 (bf16) or 2^-11 (TF32) of the sum and have an accumulator set of their own, where
+// their chain costs nothing; the leading products are a sixth or a third of the updates
+// and, where their chain would still be long, dealt out over several sets.  The epilogue
+// adds the sets, rounding to nearest.
 //
 // The output is swept along its slowest spatial dimension (S; D of a volume, H
 // of an image).  A column holds TH rows (R) of 128 outputs (W), with as many
@@ -323,33 +324,50 @@ __device__ __forceinline__ void sh_tmem_zero(uint32_t taddr, int n)
                          : "memory");
 }
 
+// The registers of a tensor-memory load may be read after this.
+__device__ __forceinline__ void sh_loaded(uint32_t (&v)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+                 :
+                 : "memory");
+}
+
 // Up to 16 accumulator columns of this warp's lanes: fetched (always 16, the
 // columns past n belong to other blocks and are ignored), summed over the sets,
-// zeroed in tensor memory.
+// zeroed in tensor memory.  A load takes some thousand clocks with products in
+// flight: those of the first two sets are on their way together.
 __device__ __forceinline__ void sh_drain(uint32_t taddr, int n, int nsets, int set_off, float (&v)[16])
 {
     uint32_t a[16];
     sh_tmem_ld16(taddr, a);
     if (in_loop(nsets) > 1)
     {
-        // the second set in halves: sixteen more live registers would spill
+        uint32_t b[16];
+        uint32_t set = taddr + (uint32_t) set_off;
+        sh_tmem_ld16(set, b);
+        sh_loaded(a);
+        sh_loaded(b);
 #pragma unroll
-        for (int h = 0; h < 16; h += 8)
+        for (int k = 0; k < 16; ++k)
+            v[k] = __uint_as_float(a[k]) + __uint_as_float(b[k]);
+        sh_tmem_zero(set, n);
+#pragma unroll 1
+        for (int s = 2; s < in_loop(nsets); ++s)
         {
-            uint32_t b[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                         : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7])
-                         : "r"(taddr + (uint32_t) (set_off + h)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            set += (uint32_t) set_off;
+            sh_tmem_ld16(set, b);
+            sh_loaded(b);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                v[h + k] = __uint_as_float(a[h + k]) + __uint_as_float(b[k]);
+            for (int k = 0; k < 16; ++k)
+                v[k] += __uint_as_float(b[k]);
+            sh_tmem_zero(set, n);
         }
-        sh_tmem_zero(taddr + (uint32_t) set_off, n);
     }
     else
     {
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        sh_loaded(a);
 #pragma unroll
         for (int k = 0; k < 16; ++k)
             v[k] = __uint_as_float(a[k]);

@@ -11,11 +11,13 @@ namespace
 constexpr int SH_SMEM_MAX = 226 * 1024;
 constexpr int SH_FOREIGN = -2; // column of a block that a row does not add to
 
-// Chains of truncating accumulator updates longer than this go to two
-// accumulator sets.  The error of a chain of n updates is about n / 2 truncations
-// of the running sum: 135 updates were measured to stay inside 1e-5 of the
-// result's scale on full shards, 180 to reach it.
+// The tensor pipe adds by truncation: a chain of n updates is off by about 2e-8 n of the
+// result, where the sums have a mean.  No chain of leading products is longer than this;
+// a layer that would need one takes the CUDA-core kernels.
 constexpr int SH_CHAIN_MAX = 96;
+// ... and most layers stay below this: 1e-6, as 3xTF32 products with one chain per
+// channel group.
+constexpr int SH_CHAIN_LOOSE = 60;
 
 int align_up(int v, int a)
 {
@@ -131,6 +133,7 @@ void ShBuilder::make_steps(ShTables* T, int J, std::vector<std::vector<std::vect
         for (int t = 0; t < m_w.taps; ++t)
             if (m_w.k(t, ew) >= 0)
                 taps.push_back({(t % m_w.st) * g.pt + t / m_w.st, m_w.k(t, ew)});
+        const int lead = g.nsets - (m_parts > 1 && g.nsets > 1 ? 1 : 0); // sets of the leading products
         std::vector<ShChunk>& ck = (*chunks)[(size_t) ew];
         auto a_of = [&](int p, int j, const Tap& t) { return (p * J + j) * m_w.st * g.pt + t.off; };
         struct Item
@@ -165,8 +168,10 @@ void ShBuilder::make_steps(ShTables* T, int J, std::vector<std::vector<std::vect
                     for (size_t t = 0; t < taps.size(); ++t)
                     {
                         int want = 0;
-                        if (g.nsets > 1)
-                            want = m_parts > 1 ? (pr.pa + pr.pb > 0) : (int) ((j * taps.size() + t) * 2 / (J * taps.size()));
+                        if (m_parts > 1 && pr.pa + pr.pb > 0)
+                            want = g.nsets - 1;
+                        else
+                            want = (int) ((j * taps.size() + t) * (size_t) lead / (J * taps.size()));
                         if (want == set)
                             list.push_back({a_of(pr.pa, j, taps[t]), pr.pa, j, (int) t,
                                             {pr.pb, taps[t].kw, j * m_ch}});
@@ -535,10 +540,43 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
 
 // Column height, filter groups, channel groups and segments together, by the
 // clocks of the busiest SM.
-bool ShBuilder::build(ShTables* out)
+bool ShBuilder::build(ShTables* out) const
 {
     if (!supported())
         return false;
+    // (one-pass products are off by far more than their sum)
+    double limit = m_parts == 1 ? SH_CHAIN_MAX : chain_limit();
+    for (; limit < SH_CHAIN_MAX; limit *= 1.5)
+        if (build_within(limit, out))
+            return true;
+    return build_within(SH_CHAIN_MAX, out);
+}
+
+// Longest chain of leading products to look for.  An fp32 FMA chain over T terms is off
+// by 1.45e-8 sqrt(T), which a chain of 0.85 sqrt(T) updates on activations (they have a
+// mean) and of sqrt(T) on gradients stays below.  Strided layers, and volumes with many
+// channels and filters, are held to that: 16 -> 32, stride 2, 256^3, forward 3.6e-7 with
+// FMAs, 6.0e-7 with 60 updates, 2.6e-7 like this (997 us against 1050); backward data 2.2e-7,
+// 1.7e-6 with the corrections in the same set, 1.9e-7 like this (850 us against 960).  The
+// others are not: 32 -> 32, 5 x 5, 2048 x 1024 x 2 would take 1420 us instead of 920 (1.0e-6),
+// 16 -> 4 on 256^3 1050 instead of 910 (4e-7).
+double ShBuilder::chain_limit() const
+{
+    const double terms = (double) m_cin * m_s.most() * m_r.most() * m_w.most();
+    const bool strided = m_cg.stride[0] > 1 || m_cg.stride[1] > 1 || m_cg.stride[2] > 1;
+    const bool as_fma = strided || (!m_flat && m_kout > 16 && m_cin >= 16);
+    return as_fma ? (m_tr ? 1.0 : 0.85) * std::sqrt(terms) : SH_CHAIN_LOOSE;
+}
+
+// The corrections (every product but the first) are small and have a set of their own.
+int ShBuilder::chain_of(int items, int lead, int cgroups) const
+{
+    const int steps = ((items + lead - 1) / lead + 1) / 2;
+    return steps * cgroups * m_s.most() * m_r.most();
+}
+
+bool ShBuilder::build_within(double limit, ShTables* out) const
+{
     std::vector<Try> tries;
     const int live = (m_s.taps + m_s.st - 1) / m_s.st; // planes live at once
     for (int kg = 1; kg <= 16 && kg <= m_kout; ++kg)
@@ -549,11 +587,15 @@ bool ShBuilder::build(ShTables* out)
                 Try t = {kg, th, live, cgroups, 1, 1, 0};
                 if (!layout(t, &T))
                     continue;
-                // updates of one output: taps x k-steps
                 const int J = T.g.cpg / m_ch;
-                const double ksteps = (double) J * m_w.taps / T.g.e_w * (m_parts == 1 ? 1 : (m_parts == 2 ? 3 : 6)) / 2;
-                const double chain = ksteps * cgroups * m_s.taps / T.g.e_s * m_r.taps / T.g.e_r;
-                t.nsets = chain > SH_CHAIN_MAX && J * m_w.taps > 1 ? 2 : 1;
+                // sets that the leading products of the cell with the most taps are dealt out to
+                const int items = J * m_w.most();
+                int lead = 1;
+                while (lead < items && chain_of(items, lead, cgroups) > limit)
+                    ++lead;
+                if (chain_of(items, lead, cgroups) > limit)
+                    continue;
+                t.nsets = lead + (m_parts > 1 ? 1 : 0);
                 if (m_flat)
                 {
                     // one row of blocks: spare plane slots decouple the issuer from the epilogue
@@ -587,7 +629,7 @@ bool ShBuilder::build(ShTables* out)
                         row_sum += std::max(c, T.g.ipr * J * (m_kind == 0 ? 30.0 : 45.0)) / m_s.st;
                     }
                 row_sum *= cgroups;
-                const double drain = T.g.th * (250.0 + 220.0 * ((T.g.nb + 15) / 16) * T.g.e_s * T.g.e_r * T.g.e_w) / 3;
+                const double drain = T.g.th * (250.0 + 220.0 * std::max(1, t.nsets - 1) * ((T.g.nb + 15) / 16) * T.g.e_s * T.g.e_r * T.g.e_w) / 3;
                 const double plane = std::max(row_sum, drain) + 40.0 * T.g.rows * cgroups;
                 double best = 0;
                 int best_ns = 0;
@@ -619,6 +661,7 @@ bool ShBuilder::build(ShTables* out)
         if (layout(t, &T) && finish(t, &T))
         {
             T.cost = t.cost;
+            T.chain = chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
             *out = T;
             return true;
         }

@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cmath>
 #include <map>
 #include <vector>
 
@@ -39,6 +40,14 @@ struct ShAxis // taps of one dimension in staged terms
     int in, q, o, st, e, taps, pad;
     // filter tap that staged tap t contributes to cell e, or -1
     int k(int t, int e_) const { return map[(size_t) e_ * taps + t]; }
+    // taps of the cell that has the most
+    int most() const
+    {
+        int m = 0;
+        for (int c = 0; c < e; ++c)
+            m = std::max(m, (int) std::count_if(map.begin() + c * taps, map.begin() + (c + 1) * taps, [](int v) { return v >= 0; }));
+        return m;
+    }
     std::vector<int> map;
 };
 
@@ -54,6 +63,7 @@ struct ShTables
     int c_of_cell;
     size_t smem;
     double cost;
+    int chain;                       // longest chain of leading products in one accumulator
     std::vector<uint8_t> blob;       // what the kernel copies to shared memory
     std::vector<ShPack> packs;       // filter images
     std::vector<ShChunk> chunks;
@@ -128,7 +138,7 @@ public:
                && m_w.taps <= 24;
     }
 
-    bool build(ShTables* out);
+    bool build(ShTables* out) const;
 
 private:
     ShAxis axis(int i) const
@@ -140,6 +150,9 @@ private:
         int kg, th, ns, cgroups, nsets, nseg;
         double cost;
     };
+    double chain_limit() const;
+    int chain_of(int items, int lead, int cgroups) const;
+    bool build_within(double limit, ShTables* out) const;
     bool layout(const Try& t, ShTables* T) const;
     void make_steps(ShTables* T, int J, std::vector<std::vector<std::vector<ShStep>>>* steps,
                     std::vector<std::vector<ShChunk>>* chunks) const;

@@ -1155,7 +1155,7 @@ class Convolution:
 
     def kernel_variant(self, which: int) -> int:
         """dcb_conv_plan_kernel_variant: 0 fp32 CUDA-core; tcgen05: 3 and 4 forward
-        and backward data (4: two accumulator sets), 5 backward filter."""
+        and backward data (4: operands as three bf16 parts), 5 backward filter."""
         return _abi.lib().dcb_conv_plan_kernel_variant(self._plan_of(which), which)
 
     # -- halo --

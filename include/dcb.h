@@ -253,8 +253,8 @@ int32_t dcb_conv_plan_status(dcb_conv_plan* plan, void* stream);
 int32_t dcb_conv_plan_kernel_kind(const dcb_conv_plan* plan, int32_t which);
 /* The kernel the plan prefers for that pass (cuDNN reports its choice as an
  * algorithm enum, util_cudnn.hpp:37-60): 0 fp32 CUDA-core; tcgen05 kernels:
- * 3 and 4 forward and backward data (4: leading products and corrections in
- * two accumulator sets), 5 backward filter (1 and 2 are not used any more). */
+ * 3 and 4 forward and backward data (4: fp32 operands as three bf16 parts; 3:
+ * TF32 or one-pass operands), 5 backward filter (1 and 2 are not used any more). */
 int32_t dcb_conv_plan_kernel_variant(const dcb_conv_plan* plan, int32_t which);
 /* y[n,k,...] = alpha*bias[k] + beta*y (cudnnAddTensor,
  * dnn_backend_cudnn.cpp.inc:386) and its gradient dbias[k] = alpha*sum dy +

@@ -1,0 +1,62 @@
+"""Decisions of the convolution planners, on the host: a small program prints them
+for the geometries below."""
+import math
+import os
+import shutil
+import subprocess
+
+import pytest
+
+import dihydrogen_b200.build as build
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+pytestmark = pytest.mark.skipif(not os.path.exists(build._nvcc()) and shutil.which(build._nvcc()) is None,
+                                reason="no nvcc")
+FP32, TF32 = 0, 1
+
+
+@pytest.fixture(scope="module")
+def planner(tmp_path_factory):
+    build.build()
+    exe = str(tmp_path_factory.mktemp("planner") / "conv_planner_check")
+    cmd = [build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1",
+           "-I", os.path.join(ROOT, "include"), "-I", build.CSRC, os.path.join(ROOT, "tests", "cpp", "conv_planner_check.cu"),
+           "-o", exe, "-L", build.PKG, "-ldistconv_b200", "-Xlinker", "-rpath=" + build.PKG]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def plan(*geometry):
+        r = subprocess.run([exe], input=" ".join(str(v) for v in geometry) + "\n", capture_output=True, text=True, timeout=60)
+        assert r.returncode == 0, r.stderr
+        return {l.split()[0]: [int(v) for v in l.split()[1:]] for l in r.stdout.splitlines()}
+
+    return plan
+
+
+@pytest.mark.parametrize("geometry", [
+    # n c k d h w f stride: the longest chain of leading products in an accumulator
+    (2, 128, 32, 16, 32, 32, 3, 1),   # 216 in one chain
+    (2, 256, 16, 16, 32, 32, 3, 1),   # 432
+    (8, 128, 32, 0, 56, 56, 5, 1),    # 200
+    (8, 256, 256, 0, 14, 14, 3, 1),
+    (8, 32, 32, 0, 64, 64, 11, 1),    # 242: the CUDA-core kernel may have it
+    (2, 16, 16, 32, 32, 32, 7, 1),
+])
+def test_chains_of_truncating_updates_are_bounded(planner, geometry):
+    for name, (ok, chain, nsets) in planner(*geometry, FP32).items():
+        assert not ok or (0 < chain <= 96 and nsets >= 2), (name, chain, nsets)
+
+
+@pytest.mark.parametrize("geometry", [
+    (1, 16, 32, 64, 64, 64, 3, 2), (8, 64, 128, 0, 56, 56, 3, 2), (1, 32, 32, 24, 40, 67, 3, 1), (2, 32, 32, 0, 96, 131, 5, 2),
+    (1, 8, 24, 24, 40, 64, 3, 2),
+])
+def test_strided_and_wide_layers_are_held_to_the_error_of_fp32_fma(planner, geometry):
+    n, c, k, d, h, w, f, s = geometry
+    taps = f ** (3 if d else 2)
+    most = ((f + s - 1) // s) ** (3 if d else 2)  # of an input cell, backward
+    plans = planner(*geometry, FP32)
+    assert plans["fwd"][0] == plans["bwd_data"][0] == 1
+    # (channels are padded to cells of 8; a chain has at least one update per tap row)
+    assert plans["fwd"][1] <= max(0.85 * math.sqrt(c * taps), taps // f), plans
+    assert plans["bwd_data"][1] <= max(math.sqrt(k * most), most ** 0.5), plans

@@ -1,6 +1,7 @@
 """Convolution kernels against the oracle and against outputs of the
 reference's own ref::Backend (golden fixtures).  fp32: 1e-5 relative."""
 import ctypes
+import math
 import os
 
 import numpy as np
@@ -624,3 +625,50 @@ def test_backward_filter_stage_and_role_edges(geom):
     torch.cuda.synchronize()
     assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.OK
     emu.assert_close(dw.cpu().numpy(), 0.5 * O.conv_bwd_filter(x, dy, f, pads, strides) - 2.0 * dw0, TOL, "dw")
+
+
+def _relative_errors(N, C, K, sp, f, s, mode):
+    """2-norm errors of y and dx against fp64; everything has a mean, so that the
+    tensor pipe's truncation cannot hide behind cancellation."""
+    import torch.nn.functional as F
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    pads, osp = [(e - 1) // 2 for e in f], [O.conv_out_extent(i, e, (e - 1) // 2, s, 1) for i, e in zip(sp, f)]
+    x = torch.randn(N, C, *sp, device="cuda", generator=gen) + 0.5
+    w = torch.randn(K, C, *f, device="cuda", generator=gen) * (2.0 / (C * math.prod(f))) ** 0.5 + 0.02
+    dy = torch.randn(N, K, *osp, device="cuda", generator=gen) + 0.3
+    y, dx = torch.empty_like(dy), torch.empty_like(x)
+    p = Plan(x, w, y, pads, [s] * len(sp), [1] * len(sp), mode)
+    p.fwd(1.0, x, w, 0.0, y)
+    p.bwd_data(1.0, w, dy, 0.0, dx)
+    torch.cuda.synchronize()
+    assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.OK
+    with torch.backends.cudnn.flags(enabled=False):
+        xr = x.double().requires_grad_()
+        yr = (F.conv3d if len(sp) == 3 else F.conv2d)(xr, w.double(), stride=s, padding=pads)
+        yr.backward(dy.double())
+    return [((a.double() - b).norm() / b.norm()).item() for a, b in ((y, yr.detach()), (dx, xr.grad))]
+
+
+@pytest.mark.parametrize("geom", [
+    (1, 128, 32, (8, 16, 32), (3, 3, 3)), (1, 256, 16, (8, 16, 32), (3, 3, 3)), (2, 128, 32, (28, 56), (5, 5)),
+    (2, 32, 32, (32, 64), (11, 11)), (1, 16, 16, (9, 16, 32), (7, 7, 7)),
+])
+def test_wide_layers_do_not_accumulate_in_one_chain(geom):
+    """A chain is at most 96 updates, each of which loses half a unit in the last
+    place of a sum that has reached half its value on average: 96 * 2^-25 of the
+    result, and as much again for the rounding of the sums."""
+    N, C, K, sp, f = geom
+    assert max(_relative_errors(N, C, K, sp, f, 1, _abi.MATH_FP32)) <= 96 * 2.0 ** -25
+
+
+@pytest.mark.parametrize("geom", [
+    (1, 16, 32, (24, 26, 70), (3, 3, 3), 2), (2, 64, 128, (28, 56), (3, 3), 2), (2, 3, 64, (56, 112), (7, 7), 2),
+    (1, 32, 32, (16, 20, 67), (3, 3, 3), 1), (2, 32, 32, (48, 131), (5, 5), 2), (1, 4, 16, (24, 40, 67), (3, 3, 3), 2),
+])
+def test_strided_and_wide_layers_are_as_exact_as_fp32_fma(geom):
+    """... whose error grows with the square root of the number of terms; 2^-22 for
+    what does not depend on it (the split, the sum of the accumulators)."""
+    got = _relative_errors(*geom, _abi.MATH_FP32)
+    fma = _relative_errors(*geom, _abi.MATH_FP32_SIMT)
+    assert all(a <= 1.25 * b + 2.0 ** -22 for a, b in zip(got, fma)), (got, fma)
