@@ -133,6 +133,8 @@ int32_t dcb_conv_plan_create(const dcb_conv_desc* cd, const dcb_nd_desc* xd,
             dcb_conv_plan_destroy(p);
             return st;
         }
+        // forward: either kernel will do
+        p->kind[0] = p->sh[0] || tc_has_sweep(p->tc) ? 1 : 0;
         p->kind[2] = tc_has_bwd_filter(p->tc) ? 1 : 0;
     }
     const size_t fbytes =
@@ -205,7 +207,7 @@ int32_t dcb_conv_plan_kernel_variant(const dcb_conv_plan* p, int32_t which)
         return -1;
     if (p->kind[which] != 1)
         return 0;
-    return which == 2 ? 5 : (sh_bf16_split(p->sh[which]) ? 4 : 3);
+    return which == 2 ? 5 : (p->sh[which] && sh_bf16_split(p->sh[which]) ? 4 : 3);
 }
 
 int32_t dcb_conv_fwd(dcb_conv_plan* p, double alpha, const void* x,
@@ -224,9 +226,10 @@ int32_t dcb_conv_fwd(dcb_conv_plan* p, double alpha, const void* x,
             if (st != DCB_UNSUPPORTED)
                 return st;
         }
-        return sh_conv(p->sh[0], (float) alpha, static_cast<const float*>(x),
-                       static_cast<const float*>(w), (float) beta,
-                       static_cast<float*>(y), p->status, as_stream(stream));
+        if (p->sh[0])
+            return sh_conv(p->sh[0], (float) alpha, static_cast<const float*>(x),
+                           static_cast<const float*>(w), (float) beta,
+                           static_cast<float*>(y), p->status, as_stream(stream));
     }
     return simt_conv_fwd(p->g, (float) alpha, static_cast<const float*>(x),
                          static_cast<const float*>(w), (float) beta,
@@ -245,7 +248,7 @@ int32_t dcb_conv_fwd_stats(dcb_conv_plan* p, double alpha, const void* x,
         static_cast<const float*>(w), static_cast<float*>(y), p->status,
         as_stream(stream), static_cast<float*>(sums),
         static_cast<float*>(sqsums));
-    if (st != DCB_UNSUPPORTED)
+    if (st != DCB_UNSUPPORTED || !p->sh[0])
         return st;
     return sh_conv(p->sh[0], (float) alpha, static_cast<const float*>(x),
                    static_cast<const float*>(w), 0.f, static_cast<float*>(y),

@@ -455,6 +455,11 @@ void tc_plan_destroy(TcPlan* p)
     delete p;
 }
 
+bool tc_has_sweep(const TcPlan* p)
+{
+    return p && p->has_sw;
+}
+
 bool tc_has_bwd_filter(const TcPlan* p)
 {
     return p && p->has_wg;

@@ -13,6 +13,7 @@ struct TcPlan;
 // stays null (and DCB_OK is returned) when neither kernel covers the geometry.
 int32_t tc_plan_create(const ConvGeom& fwd, int math_mode, TcPlan** out);
 void tc_plan_destroy(TcPlan* p);
+bool tc_has_sweep(const TcPlan* p);
 bool tc_has_bwd_filter(const TcPlan* p);
 // `status`: device word that a kernel sets when a bounded wait expires.
 // y = alpha * conv(x, w), optionally with the per-filter sums and sums of squares

@@ -5,7 +5,7 @@
 #include "conv_tc_encode.cuh"
 #include "conv_tc_shift_plan.cuh"
 
-#include <cstdlib>
+#include <type_traits>
 
 namespace dcb
 {
@@ -246,15 +246,17 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
                                        status, p->stat_part, ymap, use_ymap));
         return DCB_OK;
     };
-    int32_t st;
-    if (t.kind == 0 && t.parts == 1)
-        st = stats ? launch(sh_conv_kernel<0, 1, true>) : launch(sh_conv_kernel<0, 1, false>);
-    else if (t.kind == 0)
-        st = stats ? launch(sh_conv_kernel<0, 2, true>) : launch(sh_conv_kernel<0, 2, false>);
-    else if (t.parts == 1)
-        st = stats ? launch(sh_conv_kernel<1, 1, true>) : launch(sh_conv_kernel<1, 1, false>);
-    else
-        st = stats ? launch(sh_conv_kernel<1, 3, true>) : launch(sh_conv_kernel<1, 3, false>);
+    auto dispatch = [&](auto wide) -> int32_t {
+        constexpr bool W = decltype(wide)::value;
+        if (t.kind == 0 && t.parts == 1)
+            return stats ? launch(sh_conv_kernel<0, 1, true, W>) : launch(sh_conv_kernel<0, 1, false, W>);
+        if (t.kind == 0)
+            return stats ? launch(sh_conv_kernel<0, 2, true, W>) : launch(sh_conv_kernel<0, 2, false, W>);
+        if (t.parts == 1)
+            return stats ? launch(sh_conv_kernel<1, 1, true, W>) : launch(sh_conv_kernel<1, 1, false, W>);
+        return stats ? launch(sh_conv_kernel<1, 3, true, W>) : launch(sh_conv_kernel<1, 3, false, W>);
+    };
+    const int32_t st = t.wide ? dispatch(std::true_type()) : dispatch(std::false_type());
     if (st != DCB_OK || !stats)
         return st;
     DCB_CUDA_TRY(launch_overlapped(sh_stats_fold_kernel, dim3(1), SH_FOLD_WARPS * 32, 0, stream, p->stat_part,

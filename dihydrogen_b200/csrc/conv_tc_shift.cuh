@@ -406,7 +406,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 }
 
 
-template <int KIND, int PARTS, bool STATS>
+// WIDE: channels lie too far apart for 32-bit offsets.  (64-bit offsets throughout, or two
+// pointers per channel pair, make every other layer 1 to 2 % slower.)
+template <int KIND, int PARTS, bool STATS, bool WIDE>
 __global__ void __launch_bounds__(SH_THREADS, 1)
     sh_conv_kernel(const __grid_constant__ ShGeom g, float beta, const float* __restrict__ x,
                    const uint4* __restrict__ bimg, const uint8_t* __restrict__ tables, float* y, int* status,
@@ -686,13 +688,13 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         const int par = (int) (it & 255u), pos = (int) (it >> 8) + lane;
         const int lt = lanes[pos];
         const int sub = max(lt, 0) >> 16, xx = max(lt, 0) & 0xffff;
-        // staged cell of this lane relative to the row's first: in bytes, for
-        // the channels of a cell; planes and rows are added to the base pointers
+        // staged cell of this lane relative to the row's first: in bytes, for the channels
+        // of a cell (WIDE: for one channel); planes and rows are added to the base pointers
         uint32_t off[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
             off[e] = 4u * (uint32_t) (xx * g.st_w + par + sub * (g.pack_s * g.st_s * (int) g.xs_s + g.pack_r * g.st_r * (int) g.xs_r)
-                                      + e * (int) g.xs_c);
+                                      + (WIDE ? 0 : e * (int) g.xs_c));
         const uint32_t dpos = lt >= 0 ? smem_u32(smem + g.so_a) + 16u * (uint32_t) (par * g.pt + pos) : 0u;
         const uint32_t part_stride = (uint32_t) g.a_slot16 / PARTS * 16u;
         const uint32_t cell_stride = (uint32_t) (g.st_w * g.pt) * 16u;
@@ -710,7 +712,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         int left = 0, nch = 0, nch0 = 0, row = 0;
         const char* row_p = reinterpret_cast<const char*>(x); // the row's first cell, channel 0
         const char* p = row_p;
-        const long long row_step = 4ll * teams * g.xs_r, ch4_step = 16ll * g.xs_c;
+        const long long row_step = 4ll * teams * g.xs_r, ch_step = 4ll * g.xs_c, ch4_step = 4 * ch_step;
         const uint32_t slot_bytes = 16u * (uint32_t) g.a_slot16;
         uint32_t d = 0;
         bool in = false, plane_in = false;
@@ -784,14 +786,14 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                         {
 #pragma unroll
                             for (int e = 0; e < CH; ++e)
-                                v[q][e] = __ldg(reinterpret_cast<const float*>((e < 4 ? p : p + ch4_step) + off[e & 3]));
+                                v[q][e] = __ldg(reinterpret_cast<const float*>((e < 4 ? p : p + ch4_step) + (WIDE ? (e & 3) * ch_step : 0) + off[e & 3]));
                         }
                         else
                         {
 #pragma unroll
                             for (int e = 0; e < CH; ++e)
                                 if (e < nch)
-                                    v[q][e] = __ldg(reinterpret_cast<const float*>((e < 4 ? p : p + ch4_step) + off[e & 3]));
+                                    v[q][e] = __ldg(reinterpret_cast<const float*>((e < 4 ? p : p + ch4_step) + (WIDE ? (e & 3) * ch_step : 0) + off[e & 3]));
                         }
                     }
                     p += CH / 4 * ch4_step;

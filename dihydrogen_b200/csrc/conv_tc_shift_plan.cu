@@ -303,9 +303,13 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     g.units = (unsigned) units;
     g.rnd_add = m_bf16 ? 0x8000u : 0x1000u;
     g.rnd_mask = m_bf16 ? 0xffff0000u : 0xffffe000u;
-    // a lane's offsets from a row's base pointer are 32 bits: three channel strides and the sub-columns' distance
-    if (4 * (3 * (double) g.xs_c + (double) g.in_s * (double) g.xs_s) >= 4294967296.0)
+    // a lane's offsets from a row's base pointer are 32 bits, in bytes: the sub-columns' distance,
+    // the row and, unless they lie too far apart, three channel strides
+    const double subs = g.npack > 1 ? g.npack * ((double) g.pack_s * g.st_s * g.xs_s + (double) g.pack_r * g.st_r * g.xs_r) : 0.0,
+                 reach_bytes = 4.0 * (subs + 2.0 * g.in_w);
+    if (reach_bytes >= 2147483648.0)
         return false;
+    T->wide = reach_bytes + 12.0 * g.xs_c >= 2147483648.0;
     T->kind = m_kind, T->parts = m_parts, T->c_of_cell = m_ch;
     const int taps = cg.f[0] * cg.f[1] * cg.f[2];
     T->w_ko = m_tr ? taps : (long long) cg.c * taps;
@@ -568,6 +572,13 @@ double ShBuilder::chain_limit() const
     return as_fma ? (m_tr ? 1.0 : 0.85) * std::sqrt(terms) : SH_CHAIN_LOOSE;
 }
 
+// Few channels of a volume's dy: all three products in one chain of 45 updates (9.6e-7)
+// leave twice the rows a column that two sets do (16 -> 4 on 512^3: 4420 us against 5740).
+bool ShBuilder::one_set(int cgroups, int items) const
+{
+    return m_tr && !m_flat && m_parts == 2 && chain_limit() == SH_CHAIN_LOOSE && chain_of(3 * items, 1, cgroups) <= SH_CHAIN_LOOSE;
+}
+
 // The corrections (every product but the first) are small and have a set of their own.
 int ShBuilder::chain_of(int items, int lead, int cgroups) const
 {
@@ -596,6 +607,8 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
                 if (chain_of(items, lead, cgroups) > limit)
                     continue;
                 t.nsets = lead + (m_parts > 1 ? 1 : 0);
+                if (one_set(cgroups, items))
+                    t.nsets = 1;
                 if (m_flat)
                 {
                     // one row of blocks: spare plane slots decouple the issuer from the epilogue
@@ -661,7 +674,8 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
         if (layout(t, &T) && finish(t, &T))
         {
             T.cost = t.cost;
-            T.chain = chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
+            T.chain = T.g.nsets == 1 ? chain_of(m_parts * (m_parts + 1) / 2 * T.g.cpg / m_ch * m_w.most(), 1, T.g.cgroups)
+                                     : chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
             *out = T;
             return true;
         }

@@ -60,6 +60,7 @@ struct ShTables
 {
     ShGeom g;
     int kind, parts;
+    bool wide;                       // 64-bit channel offsets
     int c_of_cell;
     size_t smem;
     double cost;
@@ -151,6 +152,7 @@ private:
         double cost;
     };
     double chain_limit() const;
+    bool one_set(int cgroups, int items) const;
     int chain_of(int items, int lead, int cgroups) const;
     bool build_within(double limit, ShTables* out) const;
     bool layout(const Try& t, ShTables* T) const;

@@ -60,3 +60,10 @@ def test_strided_and_wide_layers_are_held_to_the_error_of_fp32_fma(planner, geom
     # (channels are padded to cells of 8; a chain has at least one update per tap row)
     assert plans["fwd"][1] <= max(0.85 * math.sqrt(c * taps), taps // f), plans
     assert plans["bwd_data"][1] <= max(math.sqrt(k * most), most ** 0.5), plans
+
+
+@pytest.mark.parametrize("extents", [(1024, 512, 512), (1000, 999, 997)])
+def test_large_volumes_are_not_refused(planner, extents):
+    """2^28 cells a channel and more (4 -> 16 channels hold 40 to 160 GB in a training step)."""
+    plans = planner(1, 4, 16, *extents, 3, 1, FP32)
+    assert plans["fwd"][0] == plans["bwd_data"][0] == 1, plans

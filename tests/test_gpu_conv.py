@@ -672,3 +672,40 @@ def test_strided_and_wide_layers_are_as_exact_as_fp32_fma(geom):
     got = _relative_errors(*geom, _abi.MATH_FP32)
     fma = _relative_errors(*geom, _abi.MATH_FP32_SIMT)
     assert all(a <= 1.25 * b + 2.0 ** -22 for a, b in zip(got, fma)), (got, fma)
+
+
+@pytest.mark.parametrize("sp", [(5, 7, 132), (5, 7, 45)])
+@pytest.mark.parametrize("channel_stride", [2 ** 28 + 64, 2 ** 30 + 64])
+def test_channels_far_apart(channel_stride, sp):
+    """Channels that lie further apart than 32-bit byte offsets reach, as in volumes of
+    2^28 cells and more; the shorter rows are not the sweep kernel's."""
+    N, C, K = 1, 4, 4
+    rng = np.random.default_rng(5)
+    x = rng.normal(size=(N, C, *sp)).astype(np.float32)
+    w = rng.normal(0, 0.2, (K, C, 3, 3, 3)).astype(np.float32)
+    dy = rng.normal(size=(N, K, *sp)).astype(np.float32)
+    store = torch.empty(3 * channel_stride + sp[0] * sp[1] * sp[2], device="cuda")
+
+    def far(a):
+        v = store.as_strided(a.shape, (4 * channel_stride, channel_stride, sp[1] * sp[2], sp[2], 1))
+        v.copy_(torch.from_numpy(a))
+        return v
+
+    wt, xf = torch.from_numpy(w).cuda(), far(x)
+    y = torch.zeros(dy.shape, device="cuda")
+    p = Plan(xf, wt, y, [1] * 3, [1] * 3, [1] * 3, _abi.MATH_FP32)
+    assert _abi.lib().dcb_conv_plan_kernel_kind(p.p, 0) == 1
+    p.fwd(1.0, xf, wt, 0.0, y)
+    emu.assert_close(y.cpu().numpy(), O.conv_fwd(x, w, [1] * 3, [1] * 3), TOL, "y")
+    dyn, dw = torch.from_numpy(dy).cuda(), torch.zeros_like(wt)
+    p.bwd_filter(1.0, xf, dyn, 0.0, dw)
+    emu.assert_close(dw.cpu().numpy(), O.conv_bwd_filter(x, dy, (3, 3, 3), [1] * 3, [1] * 3), TOL, "dw")
+    dyf = far(dy)
+    dx = torch.zeros(x.shape, device="cuda")
+    pb = Plan(dx, wt, dyf, [1] * 3, [1] * 3, [1] * 3, _abi.MATH_FP32)
+    assert _abi.lib().dcb_conv_plan_kernel_kind(pb.p, 1) == 1
+    pb.bwd_data(1.0, wt, dyf, 0.0, dx)
+    dx_ref = np.zeros_like(x)
+    O.conv_bwd_data(w, dy, dx_ref, [1] * 3, [1] * 3)
+    emu.assert_close(dx.cpu().numpy(), dx_ref, TOL, "dx")
+    assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.lib().dcb_conv_plan_status(pb.p, None) == _abi.OK
