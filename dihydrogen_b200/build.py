@@ -21,7 +21,7 @@ LIB = os.path.join(PKG, "libdistconv_b200.so")
 
 SOURCES = ["runtime.cu", "halo.cu", "bn.cu", "conv.cu", "conv_simt.cu", "conv_tc.cu",
            "conv_tc_wgrad_s1.cu", "conv_tc_wgrad_s2.cu", "conv_tc_shift.cu",
-           "conv_tc_shift_plan.cu", "comm.cu", "pool.cu", "shuffle.cu"]
+           "conv_tc_shift_plan.cu", "conv_tc_wgrad_plan.cu", "comm.cu", "pool.cu", "shuffle.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

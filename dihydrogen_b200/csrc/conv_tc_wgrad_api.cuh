@@ -50,6 +50,9 @@ struct WgGeom
     WgTile tiles[WG_MAX_TILES];
 };
 
+// The dealing out for a forward geometry on `sms` multiprocessors; false where the
+// kernel does not cover it.
+bool wg_geom(const ConvGeom& cg, int math_mode, int sms, WgGeom* out);
 // part[slice][role][filter gradient of the role] of the taps from rkw on; al: see
 // the kernel's template parameter.
 int32_t wg_launch_s1(const WgGeom& g, int al, int rkw, const float* x, const float* dy, float* part, int* status,
