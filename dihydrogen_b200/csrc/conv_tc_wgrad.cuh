@@ -290,7 +290,7 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
                 const uint32_t m = in ? (second ? m8[1] : m8[0]) : 0u;
                 dst[q][i] = stored ? st + it[i].y + lane_dst : 0u;
                 mask[q][i] = m;
-                const float* p = reinterpret_cast<const float*>(b0 + it[i].z);
+                const float* p = reinterpret_cast<const float*>(b0) + it[i].z;
                 if (AL >= 0)
                 {
 #pragma unroll
@@ -379,13 +379,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         // rows of the operand that exist (the others hold zeros), and of those the ones the tensor has
         const int rows = min(4, (isx ? g.cg : g.kg) - ch);
         const int real = max(0, min(rows, isx ? g.c - rc - ch : g.k - rk - ch));
-        const long long off = isx ? 4 * (ch * g.xs_c + kd * g.xs[0] + row * g.xs[1] + 4 * q0 * SW)
-                                  : 4 * (ch * g.ys_c + row * g.ys[1] + 4 * q0);
+        const long long off = isx ? ch * g.xs_c + kd * g.xs[0] + row * g.xs[1] + 4 * q0 * SW
+                                  : ch * g.ys_c + row * g.ys[1] + 4 * q0;
         itab[i] = make_uint4((isx ? 1u : 2u) | (uint32_t) kd << 2 | (uint32_t) row << 8 | (uint32_t) rows << 16
                                  | (uint32_t) real << 20 | (uint32_t) q0 << 24,
                              (uint32_t) (isx ? q0 * g.lbo_x + 16 * (r * g.r8 + ch)
                                              : g.y_off + q0 * g.lbo_y + 16 * (r * g.n8 + ch)),
-                             (uint32_t) off, 0u); // (below 4 GB: wg_layout)
+                             (uint32_t) off, 0u); // (elements, below 2^32: wg_layout)
     }
     // matrix rows that no item writes (filters up to a multiple of 8) stay zero
     for (int i = tid; i < g.nstages * g.stage_bytes / 16; i += WG_THREADS)

@@ -99,9 +99,10 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
     if (g.flush_stages < 1)
         g.flush_stages = 1;
     g.kd_a16 = g.X * g.r8;
-    // offsets of a stage's items are 32 bits
-    if (4.0 * ((double) cgp * cg.xs_c + (double) kdg * cg.xs[0] + (double) g.X * cg.xs[1]) >= 4e9
-        || 4.0 * ((double) kg * cg.ys_c + (double) B * cg.ys[1]) >= 4e9)
+    // offsets of a stage's items are 32 bits, in elements (a lane's own channel of four is added
+    // to the base pointer): 16 filters of 2^28 cells in one role
+    if ((cgp - 1) / 4 * 4 * (double) cg.xs_c + (kdg - 1) * (double) cg.xs[0] + g.X * (double) cg.xs[1] + 4.0 * PW >= 4294967296.0
+        || (kg - 1) / 4 * 4 * (double) cg.ys_c + B * (double) cg.ys[1] + 4.0 * PW >= 4294967296.0)
         return false;
     // shared memory; 64 bytes behind every 128-byte multiple of cells keep the
     // converters' stores (four rows x two cells at a time) on different banks

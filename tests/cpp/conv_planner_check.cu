@@ -2,6 +2,7 @@
 //   n c k d h w f stride math   (d = 0: 2-D; padding (f - 1) / 2, dense tensors)
 // Host code only; links against the library.
 #include "conv_tc_shift_plan.cuh"
+#include "conv_tc_wgrad_api.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -43,6 +44,9 @@ int main()
             const bool ok = ShBuilder(g, tr == 1, v[8], 148).build(&t);
             std::printf("%s %d %d %d\n", tr ? "bwd_data" : "fwd", ok ? 1 : 0, ok ? t.chain : 0, ok ? t.g.nsets : 0);
         }
+        WgGeom wg;
+        const bool ok = wg_geom(g, v[8], 148, &wg);
+        std::printf("bwd_filter %d %d\n", ok ? 1 : 0, ok ? wg.roles : 0);
     }
     return 0;
 }

@@ -43,7 +43,9 @@ def planner(tmp_path_factory):
     (2, 16, 16, 32, 32, 32, 7, 1),
 ])
 def test_chains_of_truncating_updates_are_bounded(planner, geometry):
-    for name, (ok, chain, nsets) in planner(*geometry, FP32).items():
+    plans = planner(*geometry, FP32)
+    for name in ("fwd", "bwd_data"):
+        ok, chain, nsets = plans[name]
         assert not ok or (0 < chain <= 96 and nsets >= 2), (name, chain, nsets)
 
 
@@ -67,3 +69,9 @@ def test_large_volumes_are_not_refused(planner, extents):
     """2^28 cells a channel and more (4 -> 16 channels hold 40 to 160 GB in a training step)."""
     plans = planner(1, 4, 16, *extents, 3, 1, FP32)
     assert plans["fwd"][0] == plans["bwd_data"][0] == 1, plans
+
+
+@pytest.mark.parametrize("extents", [(256, 256, 256), (400, 400, 400), (512, 512, 512), (1024, 512, 512)])
+def test_large_volumes_do_not_split_the_filters_of_the_backward_filter(planner, extents):
+    """Every role reads, splits and stores all of x again."""
+    assert planner(1, 4, 16, *extents, 3, 1, FP32)["bwd_filter"] == [1, 1]
