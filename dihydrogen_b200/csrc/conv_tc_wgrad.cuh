@@ -70,15 +70,21 @@ __device__ __forceinline__ WgUnit wg_unit(const WgGeom& g, long long s)
     return u;
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8])
 {
-    uint32_t r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        v[i] = __uint_as_float(r[i]);
+}
+
+// The registers of two tensor-memory loads may be read after this.
+__device__ __forceinline__ void tmem_loaded(uint32_t (&a)[8], uint32_t (&b)[8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7])
+                 :
+                 : "memory");
 }
 
 __device__ __forceinline__ void st_v4(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
@@ -416,22 +422,35 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             if (!ok)
                 break;
             tc_fence_after();
+            // two pieces at a time: a load takes some hundred clocks whatever it brings
 #pragma unroll 1
-            for (int i = 0; i < total; ++i)
+            for (int i = 0; i < total; i += 2)
             {
-                const int block = i / pieces, p8 = (i - block * pieces) * 8;
-                const uint32_t d = la + (uint32_t) (block / g.nblocks * g.kd_cols + block % g.nblocks * g.n8 + p8);
-                const uint32_t r = la + (uint32_t) (g.sum_col + block * g.kgp + p8);
-                float a[8], b[8];
-                tmem_ld8(d, a);
-                tmem_ld8(r, b);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                uint32_t v[8], z[8];
+                uint32_t d[2], r[2], a[2][8], b[2][8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    v[j] = __float_as_uint(a[j] + b[j]), z[j] = 0u;
-                tmem_st8(r, v);
-                tmem_st8(d, z);
+                for (int h = 0; h < 2; ++h)
+                {
+                    const int k = min(i + h, total - 1), block = k / pieces, p8 = (k - block * pieces) * 8;
+                    d[h] = la + (uint32_t) (block / g.nblocks * g.kd_cols + block % g.nblocks * g.n8 + p8);
+                    r[h] = la + (uint32_t) (g.sum_col + block * g.kgp + p8);
+                    tmem_ld8(d[h], a[h]);
+                    tmem_ld8(r[h], b[h]);
+                }
+                tmem_loaded(a[0], b[0]);
+                tmem_loaded(a[1], b[1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    uint32_t v[8], z[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        v[j] = __float_as_uint(__uint_as_float(a[h][j]) + __uint_as_float(b[h][j])), z[j] = 0u;
+                    if (i + h < total)
+                    {
+                        tmem_st8(r[h], v);
+                        tmem_st8(d[h], z);
+                    }
+                }
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
@@ -566,7 +585,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 #pragma unroll 1
             for (int c8 = 0; c8 < g.nblocks * g.n8; c8 += 8)
             {
-                float a[8], b[8];
+                uint32_t a[8], b[8];
                 tmem_ld8(la + (uint32_t) (kd * g.kd_cols + c8), a);
                 const int block = c8 / g.n8, in = c8 - block * g.n8;
                 if (in < g.kgp)
@@ -574,11 +593,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                 else
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        b[j] = 0.f;
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        b[j] = 0u;
+                tmem_loaded(a, b);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    dump[(c8 + j) * 128 + l] = a[j] + b[j];
+                    dump[(c8 + j) * 128 + l] = __uint_as_float(a[j]) + __uint_as_float(b[j]);
             }
         }
         __syncthreads();

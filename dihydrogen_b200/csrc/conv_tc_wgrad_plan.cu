@@ -3,6 +3,8 @@
 
 #include "dcb.h"
 
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace dcb
@@ -16,6 +18,22 @@ double wg_mma_cost(int n)
 {
     const double a = n / 2.0, b = 32.0 + n / 4.0;
     return a > b ? (a > 45.5 ? a : 45.5) : (b > 45.5 ? b : 45.5);
+}
+
+// Updates of an accumulator between flushes.  A chain of truncating updates is off by 1.7e-8
+// each (2.2e-6 with WG_CHAIN), fp32 FMAs over n positions, as the CUDA-core kernel deals them
+// out, by 1.4e-9 sqrt(n) and more where there are many sums.  Strided layers and rows that
+// cannot be read in aligned 16-byte pieces are held to that: 16 -> 16, 24 x 40 x 67, 1.9e-6
+// with WG_CHAIN, 7.4e-7 with FMAs.  The others are not: with chains of 64 4 -> 16 on 256^3
+// would take 1457 us instead of 1180.
+int wg_chain(const ConvGeom& cg)
+{
+    const bool aligned = ((cg.xs[0] | cg.xs[1] | cg.xs_c | cg.xs_n | cg.ys[0] | cg.ys[1] | cg.ys_c | cg.ys_n) & 3) == 0;
+    if (aligned && cg.stride[0] == 1 && cg.stride[1] == 1 && cg.stride[2] == 1)
+        return WG_CHAIN;
+    const double n = 0.1 * std::sqrt((double) cg.n * cg.out[0] * cg.out[1] * cg.out[2]),
+                 sums = aligned ? 1.0 : std::sqrt(std::max(1.0, cg.k * (double) cg.c / 64));
+    return (int) std::min((double) WG_CHAIN, std::max(16.0, n * sums));
 }
 
 // One way to deal out the work; false when it does not fit.
@@ -95,7 +113,7 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
             }
         }
     }
-    g.flush_stages = WG_CHAIN / (max_hits * g.Q / 2);
+    g.flush_stages = wg_chain(cg) / (max_hits * g.Q / 2);
     if (g.flush_stages < 1)
         g.flush_stages = 1;
     g.kd_a16 = g.X * g.r8;

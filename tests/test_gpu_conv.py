@@ -709,3 +709,33 @@ def test_channels_far_apart(channel_stride, sp):
     O.conv_bwd_data(w, dy, dx_ref, [1] * 3, [1] * 3)
     emu.assert_close(dx.cpu().numpy(), dx_ref, TOL, "dx")
     assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.lib().dcb_conv_plan_status(pb.p, None) == _abi.OK
+
+
+@pytest.mark.parametrize("geom", [
+    (1, 16, 16, (24, 40, 67), (3, 3, 3), 1), (2, 8, 24, (33, 41, 51), (3, 3, 3), 1), (2, 31, 17, (96, 131), (5, 5), 1),
+    (1, 16, 32, (24, 40, 64), (3, 3, 3), 2), (2, 32, 32, (95, 131), (5, 5), 2), (1, 8, 24, (24, 40, 150), (3, 3, 3), 2),
+])
+def test_backward_filter_of_strided_and_unaligned_layers_is_as_exact_as_fp32_fma(geom):
+    """... to half as much again, and 2^-21 for what does not depend on the number of
+    positions (shortest chain between flushes: 16 updates of 2^-25 of the sum, the parts)."""
+    import torch.nn.functional as F
+
+    N, C, K, sp, f, s = geom
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    pads, osp = [(e - 1) // 2 for e in f], [O.conv_out_extent(i, e, (e - 1) // 2, s, 1) for i, e in zip(sp, f)]
+    x = torch.randn(N, C, *sp, device="cuda", generator=gen)
+    x = torch.where(x < 0, 0.01 * x, x)
+    dy = 1e-2 * torch.randn(N, K, *osp, device="cuda", generator=gen)
+    w = torch.zeros(K, C, *f, device="cuda")
+    with torch.backends.cudnn.flags(enabled=False):
+        wr = w.double().requires_grad_()
+        (F.conv3d if len(sp) == 3 else F.conv2d)(x.double(), wr, stride=s, padding=pads).backward(dy.double())
+    errors = []
+    for mode in (_abi.MATH_FP32, _abi.MATH_FP32_SIMT):
+        p = Plan(x, w, dy, pads, [s] * len(sp), [1] * len(sp), mode)
+        assert _abi.lib().dcb_conv_plan_kernel_kind(p.p, 2) == (mode == _abi.MATH_FP32)
+        dw = torch.zeros_like(w)
+        p.bwd_filter(1.0, x, dy, 0.0, dw)
+        torch.cuda.synchronize()
+        errors.append(((dw.double() - wr.grad).norm() / wr.grad.norm()).item())
+    assert errors[0] <= 1.5 * errors[1] + 2.0 ** -21, errors
