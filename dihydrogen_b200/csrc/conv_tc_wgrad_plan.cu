@@ -163,7 +163,6 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
     const double instr = (g.items_x * ix + g.items_y * iy) / 4.0 * 1.3;
     // warps for x and dy: the longer of their chains of item pairs, and where several
     // splits have the same longest chain, the one whose warps are busy alike on average
-    // (x 8 -> 9 of 15 warps at 4 channels: 1391 -> 1364 us, 5 -> 7 at 16: 696 -> 662 us)
     double lat = 1e30, best = 1e30;
     for (int wx = 1; wx < WG_CONV; ++wx)
     {
@@ -176,14 +175,19 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
         if (score < best)
             best = score, lat = m, g.warps_x = wx;
     }
-    double per = pipe > instr ? pipe : instr;
-    per = per > lat ? per : lat;
+    // The terms' weights are a fit to the times of 1200 layouts of 33 layers (8 % rms; the layout
+    // that it picks of a layer is 1 % slower than the best of it, with all weights 1 it was 9 %):
+    // pipe and converters overlap in part, stages narrower than 32 positions fetch parts of lines,
+    // a walk's lead steps bring a plane each, a piece of eight columns costs a flush 280.
+    const double feed = std::max(instr, lat);
+    const double narrow = 1.0 + 0.285 * std::max(0, 32 - PW) / 32.0;
+    const double per = (1.2 * std::max(pipe, feed) + 0.64 * std::min(pipe, feed) + 530.0) * narrow;
     const double waves = (double) ((g.roles + sms - 1) / sms);
     const double n = (double) ((g.stages + g.parts - 1) / g.parts);
-    const double harvest = (double) kdg * (g.nblocks * g.n8 * 4.0 + (double) kg * cgp * fh * kwg / WG_THREADS * 200.0);
-    const double flush = n / g.flush_stages * (300.0 + kdg * g.nblocks * g.kgp / 16.0 * 120.0);
-    const double fold = (double) g.parts / 8.0 * 100.0;
-    *cost = g.nkw * (waves * (n * per + flush + harvest) + 9000.0) + fold;
+    const double lead = ring ? 0.7 * (kdg - 1) * (n / cg.out[0] + 1.0) : 0.0;
+    const double harvest = kdg * (g.nblocks * g.n8 * 35.0 + kg * cgp * kwg * 5.5);
+    const double flush = n / g.flush_stages * (kdg * g.nblocks * (g.kgp / 8)) * 280.0;
+    *cost = g.nkw * (waves * ((n + lead + 0.3) * per + flush + harvest) + 24000.0);
     return true;
 }
 
@@ -247,13 +251,13 @@ bool wg_geom(const ConvGeom& cg, int math_mode, int sms, WgGeom* out)
                                 break;
                             double cost;
                             // all planes kd in one role and unit stride along D: a walk along D converts a
-                            // plane of x once, not once per kd (and needs kdg - 1 steps to begin with)
-                            const bool ring = kdg > 1 && kdg == cg.f[0] && cg.stride[0] == 1 && cg.out[0] >= 4;
-                            bool found = ring && wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, true, sms, &cost);
-                            if (!found || g.stages < 4ll * g.parts)
-                                found = wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, false, sms, &cost);
-                            if (found && (best_cost < 0 || cost < best_cost))
-                                best_cost = cost, best = g;
+                            // plane of x once, not once per kd, and needs kdg - 1 steps to begin with
+                            // (256 x 256 x D: D = 8 72 us, 68 without a walk; D = 16 103 and 113)
+                            for (int walk = 0; walk < 2; ++walk)
+                                if ((walk == 0 || (kdg > 1 && kdg == cg.f[0] && cg.stride[0] == 1 && cg.out[0] >= 4))
+                                    && wg_layout(cg, &g, cgp, kwg, kdg, kg, B, pw, walk == 1, sms, &cost)
+                                    && (best_cost < 0 || cost < best_cost))
+                                    best_cost = cost, best = g;
                             if (pw <= 16)
                                 break;
                             // the next width that is a smaller multiple of 8
