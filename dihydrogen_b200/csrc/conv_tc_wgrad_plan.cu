@@ -24,16 +24,16 @@ double wg_mma_cost(int n)
 // each (2.2e-6 with WG_CHAIN), fp32 FMAs over n positions, as the CUDA-core kernel deals them
 // out, by 1.4e-9 sqrt(n) and more where there are many sums.  Strided layers and rows that
 // cannot be read in aligned 16-byte pieces are held to that: 16 -> 16, 24 x 40 x 67, 1.9e-6
-// with WG_CHAIN, 7.4e-7 with FMAs.  The others are not: with chains of 64 4 -> 16 on 256^3
-// would take 1457 us instead of 1180.
+// with WG_CHAIN, 7.4e-7 with FMAs.  The others are only where they are small: 64 updates (1e-6)
+// cost a few percent there, on 256^3 4 -> 16 would take 1457 us instead of 1180.
 int wg_chain(const ConvGeom& cg)
 {
     const bool aligned = ((cg.xs[0] | cg.xs[1] | cg.xs_c | cg.xs_n | cg.ys[0] | cg.ys[1] | cg.ys_c | cg.ys_n) & 3) == 0;
-    if (aligned && cg.stride[0] == 1 && cg.stride[1] == 1 && cg.stride[2] == 1)
-        return WG_CHAIN;
+    const bool strided = cg.stride[0] > 1 || cg.stride[1] > 1 || cg.stride[2] > 1;
     const double n = 0.1 * std::sqrt((double) cg.n * cg.out[0] * cg.out[1] * cg.out[2]),
-                 sums = aligned ? 1.0 : std::sqrt(std::max(1.0, cg.k * (double) cg.c / 64));
-    return (int) std::min((double) WG_CHAIN, std::max(16.0, n * sums));
+                 sums = aligned ? 1.0 : std::sqrt(std::max(1.0, cg.k * (double) cg.c / 64)),
+                 least = aligned && !strided ? 64.0 : 16.0;
+    return (int) std::min((double) WG_CHAIN, std::max(least, n * sums));
 }
 
 // One way to deal out the work; false when it does not fit.
