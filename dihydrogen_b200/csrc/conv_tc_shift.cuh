@@ -615,27 +615,64 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                         }
                         continue;
                     }
+                    if (in_loop(g.nb) < 16)
+                    {
+                        // Cells of the same parity along W lie side by side: a fetch of 16 columns
+                        // is four quarters, each of one cell (4 -> 16, stride 2, 64 x 128 x 128: 79 us
+                        // with a fetch per cell, 48 like this; of 16 filters 992 per cell, 1275).
 #pragma unroll 1
-                    for (int es = 0; es < in_loop(g.e_s); ++es)
+                        for (int ew = 0; ew < in_loop(g.e_w); ++ew)
+                        {
+                            const int ow = qw * g.e_w + ew, cols = g.e_s * g.e_r * g.nb;
+                            int es = 0, er = 0, k0 = 0; // of the next quarter
 #pragma unroll 1
-                        for (int er = 0; er < in_loop(g.e_r); ++er)
-#pragma unroll 1
-                            for (int ew = 0; ew < in_loop(g.e_w); ++ew)
+                            for (int c0 = 0; c0 < in_loop(cols); c0 += 16)
                             {
-                                const uint32_t cell = block + (uint32_t) (ew * g.woff + (es * g.e_r + er) * g.nb);
-                                const int os = q * g.e_s + es, orow = r * g.e_r + er, ow = qw * g.e_w + ew;
-                                const bool put = on && os < g.o_s && orow < g.o_r && ow < g.o_w;
-                                float* yc = yp + (long long) os * g.ys_s + (long long) orow * g.ys_r + ow;
-#pragma unroll 1
-                                for (int k0 = 0; k0 < in_loop(g.nb); k0 += 16)
+                                float v[16];
+                                sh_drain(block + (uint32_t) (ew * g.woff + c0), min(16, cols - c0), g.nsets, g.set_off, v);
+#pragma unroll
+                                for (int h = 0; h < 4; ++h)
                                 {
-                                    float v[16];
-                                    const int piece = min(16, g.nb - k0);
-                                    sh_drain(cell + (uint32_t) k0, piece, g.nsets, g.set_off, v);
-                                    if (in_loop(put))
-                                        sh_store(yc + (long long) k0 * g.ys_c, g.ys_c, min(piece, kn - k0), beta, v);
+                                    const int os = q * g.e_s + es, orow = r * g.e_r + er;
+                                    const bool put = on && es < g.e_s && os < g.o_s && orow < g.o_r && ow < g.o_w;
+                                    float* yc = yp + (long long) os * g.ys_s + (long long) orow * g.ys_r + ow + (long long) k0 * g.ys_c;
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k, yc += g.ys_c)
+                                        if (put && k0 + k < kn)
+                                            *yc = beta != 0.f ? fmaf(beta, *yc, v[4 * h + k]) : v[4 * h + k];
+                                    k0 += 4;
+                                    if (k0 >= g.nb)
+                                    {
+                                        k0 = 0;
+                                        if (++er == g.e_r)
+                                            er = 0, ++es;
+                                    }
                                 }
                             }
+                        }
+                    }
+                    else
+#pragma unroll 1
+                        for (int es = 0; es < in_loop(g.e_s); ++es)
+#pragma unroll 1
+                            for (int er = 0; er < in_loop(g.e_r); ++er)
+#pragma unroll 1
+                                for (int ew = 0; ew < in_loop(g.e_w); ++ew)
+                                {
+                                    const uint32_t cell = block + (uint32_t) (ew * g.woff + (es * g.e_r + er) * g.nb);
+                                    const int os = q * g.e_s + es, orow = r * g.e_r + er, ow = qw * g.e_w + ew;
+                                    const bool put = on && os < g.o_s && orow < g.o_r && ow < g.o_w;
+                                    float* yc = yp + (long long) os * g.ys_s + (long long) orow * g.ys_r + ow;
+#pragma unroll 1
+                                    for (int k0 = 0; k0 < in_loop(g.nb); k0 += 16)
+                                    {
+                                        float v[16];
+                                        const int piece = min(16, g.nb - k0);
+                                        sh_drain(cell + (uint32_t) k0, piece, g.nsets, g.set_off, v);
+                                        if (in_loop(put))
+                                            sh_store(yc + (long long) k0 * g.ys_c, g.ys_c, min(piece, kn - k0), beta, v);
+                                    }
+                                }
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();

@@ -149,9 +149,10 @@ private:
     struct Try
     {
         int kg, th, ns, cgroups, nsets, nseg;
-        double cost;
+        double cost, mma;
     };
     double chain_limit() const;
+    double clocks(const ShGeom& g, double mma, int teams) const;
     bool one_set(int cgroups, int items) const;
     int chain_of(int items, int lead, int cgroups) const;
     bool build_within(double limit, ShTables* out) const;
