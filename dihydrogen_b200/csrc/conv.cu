@@ -126,6 +126,12 @@ int32_t dcb_conv_plan_create(const dcb_conv_desc* cd, const dcb_nd_desc* xd,
                 dcb_conv_plan_destroy(p);
                 return st;
             }
+            if (p->sh[dir] && simt_is_faster(g, dir == 1, sh_estimate(p->sh[dir])))
+            {
+                sh_plan_destroy(p->sh[dir]);
+                p->sh[dir] = nullptr;
+                p->kind[dir] = 0;
+            }
         }
         st = tc_plan_create(g, cd->math_mode, &p->tc);
         if (st != DCB_OK)

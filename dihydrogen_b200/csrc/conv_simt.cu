@@ -674,4 +674,43 @@ int32_t simt_conv_bwd_filter(const ConvGeom& g, float alpha, const float* x,
     return DCB_OK;
 }
 
+// Estimates in microseconds: fits to layers of 1 to 32 channels and filters, 3 and 5 taps, on
+// 9 k to 1 M positions.  A launch is bound by its chain of taps where it is small and by FMAs
+// where it is large.  Forward, 512 x 512 x 2, us, these kernels / shift kernel: 1 -> 4, 3 x 3,
+// 8.5 / 36; 4 -> 8 27 / 36; 4 -> 16 41 / 36.  Stride 2, 64 x 128 x 128, forward: 1 -> 16 19 / 52,
+// 4 -> 16 51 / 52, 8 -> 16 97 / 57; backward data: 8 -> 4 55 / 81, 8 -> 16 97 / 82.
+// Volumes with stride 1 are left out: there the output's statistics come with the products.
+bool simt_is_faster(const ConvGeom& g, bool bwd_data, double tensor_us)
+{
+    const bool flat = g.f[0] == 1 && g.in[0] == 1, strided = g.stride[0] > 1 || g.stride[1] > 1 || g.stride[2] > 1;
+    for (int i = 0; i < 3; ++i)
+        if (g.dil[i] != 1 || g.stride[i] > 2)
+            return false;
+    if (!flat && !strided)
+        return false;
+    const double taps = (double) g.f[0] * g.f[1] * g.f[2];
+    const double in = 1e-6 * g.n * g.in[0] * g.in[1] * g.in[2], out = 1e-6 * g.n * g.out[0] * g.out[1] * g.out[2];
+    double us;
+    if (bwd_data && strided)
+    {
+        if (flat || g.c > 16)
+            return false;
+        us = 25.0 + 1.25 * g.k + in * (10.0 + g.k * (0.5 + 0.23 * g.c));
+    }
+    else
+    {
+        const double terms = taps * (bwd_data ? g.k : g.c);
+        const int filters = bwd_data ? g.c : g.k, few = filters < 16 ? filters : 16;
+        const double chain = 4.0 + 0.22 * terms;
+        const double fma = out / 0.524 * ((filters + 15) / 16)
+                           * ((few <= 4 ? 0.45 : few <= 8 ? 0.57 : 0.7) * terms + (few <= 4 ? 4.4 : few <= 8 ? 6.3 : 13.0));
+        us = strided ? chain + fma : (chain > fma ? chain : fma);
+        if (!flat) // the pass over the output that its statistics then take
+            us += 3.0 + 4.0 * out * g.k / 6.5;
+        if (bwd_data) // the filter is flipped first
+            us += 3.0;
+    }
+    return us < 0.8 * tensor_us; // (both are estimates)
+}
+
 } // namespace dcb

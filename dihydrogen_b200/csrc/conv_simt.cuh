@@ -35,5 +35,8 @@ int32_t simt_conv_bwd_filter(const ConvGeom& g, float alpha, const float* x,
 // a forward correlation of dy.
 int32_t flip_transpose_filter(const float* w, float* w2, int k, int c,
                               int taps, cudaStream_t stream);
+// Layers of few channels, taps and filters: do these kernels take clearly less than
+// `tensor_us`, what a tensor-core kernel would take?
+bool simt_is_faster(const ConvGeom& g, bool bwd_data, double tensor_us);
 
 } // namespace dcb

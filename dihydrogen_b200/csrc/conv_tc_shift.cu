@@ -189,6 +189,11 @@ bool sh_has_stats(const ShPlan* p)
     return g.kgroups == 1 && g.nb <= 16 && g.e_s * g.e_r * g.e_w == 1;
 }
 
+double sh_estimate(const ShPlan* p)
+{
+    return p->t.cost / 1900.0;
+}
+
 bool sh_bf16_split(const ShPlan* p)
 {
     return p->t.parts == 3;

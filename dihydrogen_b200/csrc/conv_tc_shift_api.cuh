@@ -15,6 +15,8 @@ bool sh_plan_create(const ConvGeom& g, bool transposed, int math_mode, ShPlan** 
 void sh_plan_destroy(ShPlan* p);
 // the epilogue can return per-filter sums and sums of squares of the output
 bool sh_has_stats(const ShPlan* p);
+// the planner's estimate of a launch, in microseconds (within a fifth or so)
+double sh_estimate(const ShPlan* p);
 // operands as three bf16 parts, six products
 bool sh_bf16_split(const ShPlan* p);
 // y = alpha * conv(x, w) + beta * y (transposed: x is dy, y is dx).  `status` is

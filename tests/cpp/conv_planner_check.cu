@@ -42,7 +42,8 @@ int main()
         {
             ShTables t;
             const bool ok = ShBuilder(g, tr == 1, v[8], 148).build(&t);
-            std::printf("%s %d %d %d\n", tr ? "bwd_data" : "fwd", ok ? 1 : 0, ok ? t.chain : 0, ok ? t.g.nsets : 0);
+            std::printf("%s %d %d %d %d\n", tr ? "bwd_data" : "fwd", ok ? 1 : 0, ok ? t.chain : 0, ok ? t.g.nsets : 0,
+                        ok && simt_is_faster(g, tr == 1, t.cost / 1900.0) ? 1 : 0);
         }
         WgGeom wg;
         const bool ok = wg_geom(g, v[8], 148, &wg);

@@ -45,7 +45,7 @@ def planner(tmp_path_factory):
 def test_chains_of_truncating_updates_are_bounded(planner, geometry):
     plans = planner(*geometry, FP32)
     for name in ("fwd", "bwd_data"):
-        ok, chain, nsets = plans[name]
+        ok, chain, nsets, _ = plans[name]
         assert not ok or (0 < chain <= 96 and nsets >= 2), (name, chain, nsets)
 
 
@@ -75,3 +75,15 @@ def test_large_volumes_are_not_refused(planner, extents):
 def test_large_volumes_do_not_split_the_filters_of_the_backward_filter(planner, extents):
     """Every role reads, splits and stores all of x again."""
     assert planner(1, 4, 16, *extents, 3, 1, FP32)["bwd_filter"] == [1, 1]
+
+
+@pytest.mark.parametrize("geometry,simt", [
+    # n c k d h w f stride; the CUDA-core kernels take forward, backward data
+    ((2, 1, 4, 0, 512, 512, 3, 1), (1, 1)), ((2, 1, 4, 0, 96, 128, 3, 2), (1, 0)), ((2, 4, 8, 0, 512, 512, 3, 1), (1, 0)),
+    ((1, 1, 16, 64, 128, 128, 3, 2), (1, 0)), ((1, 8, 4, 64, 128, 128, 3, 2), (0, 1)),
+    ((2, 32, 32, 0, 512, 512, 5, 1), (0, 0)), ((4, 16, 16, 0, 64, 64, 3, 1), (0, 0)), ((1, 16, 32, 256, 256, 256, 3, 2), (0, 0)),
+    ((1, 1, 4, 64, 128, 128, 3, 1), (0, 0)),
+])
+def test_layers_of_few_products_take_the_cuda_cores(planner, geometry, simt):
+    plans = planner(*geometry, FP32)
+    assert (plans["fwd"][3], plans["bwd_data"][3]) == simt, plans

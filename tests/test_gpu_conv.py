@@ -739,3 +739,25 @@ def test_backward_filter_of_strided_and_unaligned_layers_is_as_exact_as_fp32_fma
         torch.cuda.synchronize()
         errors.append(((dw.double() - wr.grad).norm() / wr.grad.norm()).item())
     assert errors[0] <= 1.5 * errors[1] + 2.0 ** -21, errors
+
+
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, stride, kernels of forward and backward data: either side of the rule
+    (2, 1, 4, (512, 512), (3, 3), 1, (0, 0)), (2, 4, 8, (512, 512), (3, 3), 1, (0, 1)), (2, 4, 16, (512, 512), (3, 3), 1, (1, 1)),
+    (2, 1, 4, (95, 131), (3, 3), 2, (0, 1)), (1, 8, 4, (64, 127, 128), (3, 3, 3), 2, (1, 0)), (1, 1, 16, (33, 64, 65), (3, 3, 3), 2, (0, 1)),
+])
+def test_layers_of_few_products_on_either_kernel(geom):
+    N, C, K, sp, f, s, kinds = geom
+    rng = np.random.default_rng(C + K)
+    pads, strides = [1] * len(sp), [s] * len(sp)
+    x = rng.normal(0, 1, (N, C, *sp)).astype(np.float32)
+    w = rng.normal(0, np.sqrt(2.0 / (C * np.prod(f))), (K, C, *f)).astype(np.float32)
+    dy = rng.normal(0, 1, (N, K, *[O.conv_out_extent(i, 3, 1, s, 1) for i in sp])).astype(np.float32)
+    xs = torch.from_numpy(x).cuda()
+    p = Plan(xs, torch.from_numpy(w).cuda(), torch.from_numpy(dy).cuda(), pads, strides, [1] * len(sp), _abi.MATH_FP32)
+    assert tuple(_abi.lib().dcb_conv_plan_kernel_kind(p.p, i) for i in (0, 1)) == kinds
+    y, dx, _ = run_all(x, w, dy, pads, strides, [1] * len(sp), _abi.MATH_FP32)
+    emu.assert_close(y, O.conv_fwd(x, w, pads, strides), TOL, "y")
+    dx_ref = np.zeros_like(x)
+    O.conv_bwd_data(w, dy, dx_ref, pads, strides)
+    emu.assert_close(dx, dx_ref, TOL, "dx")
