@@ -352,16 +352,16 @@ __global__ void bn_finalize_kernel(int channels, long long num_per_sum,
 }
 
 // What bn_finalize_kernel does, by the apply kernel itself: every block turns its
-// channel's sums into statistics, the last one of the channel to arrive (nobody reads
-// the sums any more then) writes them back.  One launch less between a small layer's
-// statistics and its output.
+// channel's sums into statistics, and when all blocks of the channel, a cluster, have read
+// the sums, the first one writes them back.  One launch less between a small layer's
+// statistics and its output, and nothing kept between calls.
 struct FinalizeArgs
 {
     long long num_per_sum;
     float decay;
     float *mean, *var, *running_mean, *running_var; // sums in, statistics out
-    unsigned* tickets;
 };
+constexpr unsigned BN_CLUSTER_MAX = 8; // blocks of a cluster that every device grants
 
 // LEAKY: the leaky ReLU that follows the batch-norm in the same pass
 // (y > 0 ? y : slope * y), one trip through HBM instead of two.
@@ -391,14 +391,7 @@ __global__ void __launch_bounds__(BN_THREADS)
         __syncthreads();
         m = stat[0];
         v0 = stat[1];
-        if (threadIdx.x == 0 && atomicAdd(&fin.tickets[c], 1u) == gridDim.x - 1)
-        {
-            fin.tickets[c] = 0;
-            fin.mean[c] = m;
-            fin.var[c] = v0;
-            fin.running_mean[c] = running_update(fin.decay, fin.running_mean[c], m);
-            fin.running_var[c] = running_update(fin.decay, fin.running_var[c], v0);
-        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     }
     else
     {
@@ -435,6 +428,17 @@ __global__ void __launch_bounds__(BN_THREADS)
                 }
                 v[k].store(yp + ep[k].template off<V>(ys));
             }
+    }
+    if (FINALIZE)
+    {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (threadIdx.x == 0 && blockIdx.x == 0)
+        {
+            fin.mean[c] = m;
+            fin.var[c] = v0;
+            fin.running_mean[c] = running_update(fin.decay, fin.running_mean[c], m);
+            fin.running_var[c] = running_update(fin.decay, fin.running_var[c], v0);
+        }
     }
 }
 
@@ -799,12 +803,21 @@ static int32_t bn_apply_impl(const dcb_nd_desc* xd, const void* x, const void* m
     if (mv.ug.upc == 0)
         return DCB_OK;
     const dim3 grid = bn_grid(mv.ug);
+    if (fin && grid.x > BN_CLUSTER_MAX)
+    {
+        // too many blocks for a cluster, and enough work to hide a launch
+        st = dcb_bn_finalize((int32_t) xd->c, fin->num_per_sum, fin->decay, fin->mean, fin->var, fin->running_mean,
+                             fin->running_var, stream);
+        if (st != DCB_OK)
+            return st;
+        fin = nullptr;
+    }
     const FinalizeArgs f = fin ? *fin : FinalizeArgs();
 #define CALL(VV, PP)                                                                                               \
     {                                                                                                              \
         auto kernel = leaky ? (fin ? bn_apply_kernel<VV, true, PP, true> : bn_apply_kernel<VV, true, PP, false>)   \
                             : (fin ? bn_apply_kernel<VV, false, PP, true> : bn_apply_kernel<VV, false, PP, false>); \
-        DCB_CUDA_TRY(launch_overlapped(kernel, grid, BN_THREADS, 0, as_stream(stream),                                                        \
+        DCB_CUDA_TRY(launch_overlapped_cluster(kernel, grid, fin ? grid.x : 1, BN_THREADS, 0, as_stream(stream),                               \
             static_cast<const float*>(x), mv.s[0], static_cast<float*>(y), mv.s[1], mv.ug,                         \
             static_cast<const float*>(mean), static_cast<const float*>(var), static_cast<const float*>(scale),     \
             static_cast<const float*>(bias), eps, slope, f));                                                       \
@@ -820,14 +833,14 @@ int32_t dcb_bn_finalize_apply(dcb_bn_plan* plan, int64_t num_per_sum, float deca
                               const void* scale, const void* bias, float eps, float slope, const dcb_nd_desc* yd, void* y,
                               void* stream)
 {
-    DCB_REQUIRE(plan && running_mean && running_var && num_per_sum > 0, "null argument");
+    DCB_REQUIRE(running_mean && running_var && num_per_sum > 0, "null argument");
     int32_t st = check_nd_desc(xd);
     if (st != DCB_OK)
         return st;
-    DCB_REQUIRE(xd->c == plan->xd.c && xd->n * xd->dims[0] * xd->dims[1] * xd->dims[2] > 0,
+    DCB_REQUIRE((!plan || xd->c == plan->xd.c) && xd->n * xd->dims[0] * xd->dims[1] * xd->dims[2] > 0,
                 "the plan is for another channel count, or the shard is empty");
     const FinalizeArgs f = {num_per_sum, decay, static_cast<float*>(mean), static_cast<float*>(var),
-                            static_cast<float*>(running_mean), static_cast<float*>(running_var), plan->tickets};
+                            static_cast<float*>(running_mean), static_cast<float*>(running_var)};
     return bn_apply_impl(xd, x, mean, var, scale, bias, eps, slope != 1.f, slope, yd, y, stream, &f);
 }
 

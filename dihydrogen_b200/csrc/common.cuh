@@ -78,21 +78,31 @@ int32_t allow_dynamic_smem(const void* kernel, int bytes);
 // which its 1.4 ms on a 256^3 shard need more (2260 us with the pass before it, 2310 us
 // launched like this).
 template <class... Params, class... Args>
-inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem,
-                                     cudaStream_t stream, Args&&... args)
+inline cudaError_t launch_overlapped_cluster(void (*kernel)(Params...), dim3 grid, unsigned cluster, unsigned threads,
+                                             size_t smem, cudaStream_t stream, Args&&... args)
 {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+template <class... Params, class... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem,
+                                     cudaStream_t stream, Args&&... args)
+{
+    return launch_overlapped_cluster(kernel, grid, 1, threads, smem, stream, std::forward<Args>(args)...);
 }
 
 __device__ __forceinline__ void dependents_may_start()

@@ -1358,7 +1358,7 @@ class BatchNormalization:
             stat_shape = input.shape if self.global_stats else input.local_shape
             nps = math.prod(stat_shape) // stat_shape[-2]
             if input.get_local_size() != 0 and nps > 0:
-                call("dcb_bn_finalize_apply", self._plan(input), nps, self.decay, mean.data_ptr(), var.data_ptr(),
+                call("dcb_bn_finalize_apply", None, nps, self.decay, mean.data_ptr(), var.data_ptr(),
                      running_mean.data_ptr(), running_var.data_ptr(), input._nd(), input.get_base_ptr(),
                      scale.data_ptr(), bias.data_ptr(), self.epsilon,
                      1.0 if leaky_relu_slope is None else float(leaky_relu_slope), output._nd(),

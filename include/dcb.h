@@ -298,10 +298,11 @@ int32_t dcb_bn_stats_noalloc(const dcb_nd_desc* xd, const void* x, void* sums,
 int32_t dcb_bn_finalize(int32_t channels, int64_t num_per_sum, float decay,
                         void* mean, void* var, void* running_mean,
                         void* running_var, void* stream);
-/* dcb_bn_finalize followed by dcb_bn_apply (slope 1) or dcb_bn_apply_leaky_relu in
- * one launch, for a shard that is not empty.  mean / var hold the (all-reduced)
- * sums and sums of squares on entry and the statistics afterwards.  `plan` is one
- * of the same channel count (dcb_bn_plan_create); its calls must be ordered. */
+/* dcb_bn_finalize followed by dcb_bn_apply (slope 1) or dcb_bn_apply_leaky_relu, in
+ * one launch where the shard is small; for a shard that is not empty.  mean / var hold
+ * the (all-reduced) sums and sums of squares on entry and the statistics afterwards.
+ * Nothing is allocated or kept: `plan` may be null, and is only checked for the channel
+ * count. */
 int32_t dcb_bn_finalize_apply(dcb_bn_plan* plan, int64_t num_per_sum,
                               float decay, void* mean, void* var,
                               void* running_mean, void* running_var,

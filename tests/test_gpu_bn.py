@@ -262,3 +262,64 @@ def test_empty_shard_zero_fills_run_on_the_backend_stream():
     torch.cuda.synchronize()
     for v in vals:
         assert float(v.abs().max()) == 0.0
+
+
+def _bn_problem(C=6, w=40):
+    """A layer whose statistics come with its convolution: sums in, normalised output out."""
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    be = dc.BackendDNNLib(dc.Locale(0, 1))
+    x, y = (dc.Tensor([w, 9, 7, C, 2], dc.Locale(0, 1), dc.Distribution.make_localized_distribution(5)) for _ in range(2))
+    for t in (x, y):
+        t.allocate()
+    x.buffer.copy_(torch.randn(x.buffer.shape, device="cuda", generator=gen) + 0.3)
+    sums = torch.cat([x.owned().double().sum((0, 2, 3, 4)), x.owned().double().square().sum((0, 2, 3, 4))]).float()
+    rest = [torch.zeros(C, device="cuda"), torch.ones(C, device="cuda"), torch.rand(C, device="cuda") + 0.5,
+            torch.randn(C, device="cuda")]
+    return be, x, y, sums, rest
+
+
+def test_forward_on_given_statistics_needs_no_call_before_a_capture():
+    """The first forward pass of a batch-norm whose sums are given may be a captured
+    one: it allocates nothing."""
+    be, x, y, sums, (rm, rv, scale, bias) = _bn_problem()
+    C = sums.numel() // 2
+    stats, bn = sums.clone(), dc.BatchNormalization(be, 5, 0.9, 1e-5, True)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        stats.copy_(sums)
+        bn.forward(x, stats[:C], stats[C:], rm, rv, scale, bias, y, True, statistics_ready=True)
+    rm.zero_(), rv.fill_(1.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    mean, var = x.owned().double().mean((0, 2, 3, 4)), x.owned().double().var((0, 2, 3, 4))
+    assert torch.allclose(stats[:C].double(), mean, atol=1e-6) and torch.allclose(stats[C:].double(), var, rtol=1e-5)
+    assert torch.allclose(rm.double(), 0.1 * mean, atol=1e-6)
+    sh = (1, C, 1, 1, 1)
+    ref = (x.owned().double() - mean.view(sh)) * (var.view(sh) + 1e-5).rsqrt() * scale.double().view(sh) + bias.double().view(sh)
+    assert torch.allclose(y.owned().double(), ref, atol=2e-5)
+
+
+def test_forward_passes_of_one_object_on_several_streams():
+    """forward_stage2 keeps nothing between calls: passes of one object over different
+    batches may run side by side, as separate finalize and apply calls may."""
+    be, x, _, sums, (_, _, scale, bias) = _bn_problem(C=16, w=64)
+    C, bn = 16, dc.BatchNormalization(be, 5, 0.9, 1e-5, True)
+    streams, outs = [torch.cuda.Stream() for _ in range(4)], []
+    for _ in range(8):
+        y = dc.Tensor(x.shape, x.locale, x.dist)
+        y.allocate()
+        outs.append((y, sums.clone(), torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")))
+    torch.cuda.synchronize()
+    for rep in range(20):
+        for i, (y, st, rm, rv) in enumerate(outs):
+            with torch.cuda.stream(streams[i % 4]):
+                st.copy_(sums), rm.zero_(), rv.fill_(1.0)
+                be.stream = streams[i % 4]
+                bn.forward_stage2(x, st[:C], st[C:], rm, rv, scale, bias, y, True)
+        torch.cuda.synchronize()
+        for y, st, rm, rv in outs[1:]:
+            assert torch.equal(st, outs[0][1]) and torch.equal(rm, outs[0][2]) and torch.equal(rv, outs[0][3])
+            assert torch.equal(y.buffer, outs[0][0].buffer)
+        assert not torch.equal(outs[0][1], sums)
