@@ -323,3 +323,21 @@ def test_forward_passes_of_one_object_on_several_streams():
             assert torch.equal(st, outs[0][1]) and torch.equal(rm, outs[0][2]) and torch.equal(rv, outs[0][3])
             assert torch.equal(y.buffer, outs[0][0].buffer)
         assert not torch.equal(outs[0][1], sums)
+
+
+def test_one_object_on_tensors_of_one_shape_and_several_pitches():
+    """The kernels read x through the plan's strides."""
+    be, x, y, sums, (rm, rv, scale, bias) = _bn_problem(C=4, w=33)
+    C, bn = 4, dc.BatchNormalization(be, 5, 0.9, 1e-5, True)
+    padded = dc.Tensor(x.shape, x.locale, x.dist, pitch_align=8)
+    padded.allocate()
+    padded.buffer.fill_(float("nan"))
+    padded.owned().copy_(x.owned())
+    assert padded.pitch != x.pitch and padded.get_local_shape() == x.get_local_shape()
+    for t in (x, padded, x):
+        st = torch.zeros(2 * C, device="cuda")
+        bn.forward_stage1(t, st[:C], st[C:], True)
+        assert torch.allclose(st, sums, rtol=1e-5, atol=1e-3)
+        grads = [torch.zeros(C, device="cuda") for _ in range(4)]
+        bn.backward_stage1(t, x, rm, rv, scale, *grads)
+        assert torch.allclose(grads[1], sums[:C], rtol=1e-5, atol=1e-3)  # dbias: the sum of dy
