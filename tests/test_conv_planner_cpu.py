@@ -15,15 +15,20 @@ pytestmark = pytest.mark.skipif(not os.path.exists(build._nvcc()) and shutil.whi
 FP32, TF32 = 0, 1
 
 
-@pytest.fixture(scope="module")
-def planner(tmp_path_factory):
+def compile_check(folder, name):
     build.build()
-    exe = str(tmp_path_factory.mktemp("planner") / "conv_planner_check")
+    exe = str(folder / name)
     cmd = [build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1",
-           "-I", os.path.join(ROOT, "include"), "-I", build.CSRC, os.path.join(ROOT, "tests", "cpp", "conv_planner_check.cu"),
+           "-I", os.path.join(ROOT, "include"), "-I", build.CSRC, os.path.join(ROOT, "tests", "cpp", name + ".cu"),
            "-o", exe, "-L", build.PKG, "-ldistconv_b200", "-Xlinker", "-rpath=" + build.PKG]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+    return exe
+
+
+@pytest.fixture(scope="module")
+def planner(tmp_path_factory):
+    exe = compile_check(tmp_path_factory.mktemp("planner"), "conv_planner_check")
 
     def plan(*geometry):
         r = subprocess.run([exe], input=" ".join(str(v) for v in geometry) + "\n", capture_output=True, text=True, timeout=60)
@@ -87,3 +92,9 @@ def test_large_volumes_do_not_split_the_filters_of_the_backward_filter(planner, 
 def test_layers_of_few_products_take_the_cuda_cores(planner, geometry, simt):
     plans = planner(*geometry, FP32)
     assert (plans["fwd"][3], plans["bwd_data"][3]) == simt, plans
+
+
+def test_threads_that_look_up_the_encoder_together_all_get_it(tmp_path):
+    """A thread that came second used to get none, and with it another kernel."""
+    r = subprocess.run([compile_check(tmp_path, "encode_fn_check")], capture_output=True, text=True, timeout=60)
+    assert (r.returncode, r.stdout.strip()) == (0, "0"), r.stdout + r.stderr
