@@ -32,6 +32,7 @@ namespace
 constexpr int SHF_THREADS = 256;
 constexpr int SHF_UNROLL = 4;                           // accesses of a thread in flight
 constexpr int SHF_CHUNK = SHF_THREADS * SHF_UNROLL;     // accesses of a unit
+constexpr long long SHF_MAX_CELLS = 2000000000ll;
 constexpr int SHF_MAX_RANKS = 64;
 constexpr size_t SHF_HEADER = 1024; // 64 flags, ticket, status
 
@@ -239,8 +240,8 @@ void finish_job(ShfJob* j)
         j->by_ext[k] = FastDiv::of((uint32_t) j->ext[k]);
     }
     j->vec = (mix & 3) == 0;
-    // runs of at least two units, or too many accesses for 31-bit indices
-    j->split = j->len / (j->vec ? 4 : 1) >= 2 * SHF_CHUNK || j->rows * j->len >= 2000000000ll;
+    // runs of at least two units, or (one run) too many accesses for 31-bit indices
+    j->split = j->len / (j->vec ? 4 : 1) >= 2 * SHF_CHUNK || j->rows * j->len >= SHF_MAX_CELLS;
     for (int w = 0; w < 2; ++w)
     {
         j->per_run[w] = j->len / (w ? 4 : 1);
@@ -248,6 +249,35 @@ void finish_job(ShfJob* j)
         j->units[w] = j->split ? j->rows * ((j->per_run[w] + SHF_CHUNK - 1) / SHF_CHUNK)
                                : (j->rows * j->per_run[w] + SHF_CHUNK - 1) / SHF_CHUNK;
     }
+}
+
+// Adds a job, in pieces of fewer than SHF_MAX_CELLS cells: inside one, indices and extents have
+// 31 bits.  (A job of 2.9e9 cells in runs of 500 otherwise took a block per run.)
+void add_jobs(ShfJob j, std::vector<ShfJob>* out, long long* units)
+{
+    long long cells = j.len;
+    int outer = 0;
+    for (int k = 0; k < 4; ++k)
+    {
+        cells *= j.ext[k];
+        if (j.ext[k] > 1)
+            outer = k;
+    }
+    if (cells >= SHF_MAX_CELLS && j.ext[outer] > 1)
+    {
+        ShfJob rest = j;
+        j.ext[outer] /= 2;
+        rest.ext[outer] -= j.ext[outer];
+        j.rows = rest.rows = 0; // (finish_job counts them)
+        rest.a_off += j.ext[outer] * j.a_stride[outer];
+        rest.b_off += j.ext[outer] * j.b_stride[outer];
+        add_jobs(j, out, units);
+        add_jobs(rest, out, units);
+        return;
+    }
+    finish_job(&j);
+    out->push_back(j);
+    *units += j.units[j.vec];
 }
 
 struct ShfBlob
@@ -483,9 +513,7 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
             j.peer = reinterpret_cast<float*>(base + SHF_HEADER);
             j.parity_pitch = (long long) b.parity_floats;
             j.flag = reinterpret_cast<uint32_t*>(base) + p->rank; // my slot among r's flags
-            finish_job(&j);
-            put.push_back(j);
-            p->put_units += j.units[j.vec];
+            add_jobs(j, &put, &p->put_units);
         }
         // what rank r holds of my destination block
         if (my_dst.volume() > 0 && p->src_boxes[r].volume() > 0 && intersect(p->src_boxes[r], my_dst, &x))
@@ -512,9 +540,7 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
             }
             j.peer = nullptr;
             j.flag = p->flags() + r;
-            finish_job(&j);
-            wait.push_back(j);
-            p->wait_units += j.units[j.vec];
+            add_jobs(j, &wait, &p->wait_units);
         }
     }
     cudaFree(p->d_put);

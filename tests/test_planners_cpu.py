@@ -1,5 +1,4 @@
-"""Decisions of the convolution planners, on the host: a small program prints them
-for the geometries below."""
+"""Host code of the kernels' planners: small programs print their decisions."""
 import math
 import os
 import shutil
@@ -98,3 +97,16 @@ def test_threads_that_look_up_the_encoder_together_all_get_it(tmp_path):
     """A thread that came second used to get none, and with it another kernel."""
     r = subprocess.run([compile_check(tmp_path, "encode_fn_check")], capture_output=True, text=True, timeout=60)
     assert (r.returncode, r.stdout.strip()) == (0, "0"), r.stdout + r.stderr
+
+
+def test_large_redistributions_are_dealt_out_in_pieces(tmp_path):
+    """Above 2e9 cells short runs took a block each, and an extent of 2^32 divided by zero."""
+    exe = compile_check(tmp_path, "shuffle_jobs_check")
+    jobs = "500 1200 1200 4 1\n64 4294967296 1 1 1\n300 700 100 3 2\n1048576 4096 1 1 1\n"
+    r = subprocess.run([exe], input=jobs, capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    lines = [[int(v) for v in l.split()] for l in r.stdout.splitlines()]
+    assert len(lines) == 4
+    for pieces, most, covered, per_unit in lines:
+        assert covered and most < 2000000000 and per_unit >= 1000
+    assert lines[2][0] == 1
