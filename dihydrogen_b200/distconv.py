@@ -693,10 +693,10 @@ class HaloExchange:
         dimension also zeroes that dimension's halo slabs that have no neighbour
         (what Tensor::clear_halo before the exchange leaves behind), saving one
         launch per partitioned dimension."""
-        flags = self._flags(is_reverse, skip_unpack, op, clear_boundary)
+        flags, buffer = self._flags(is_reverse, skip_unpack, op, clear_boundary), self.tensor.get_buffer()
         if self._idle:
             return
-        call("dcb_halo_exchange", self._plan, _ptr(self.tensor.get_buffer()), flags, _stream_ptr(stream))
+        call("dcb_halo_exchange", self._plan, _ptr(buffer), flags, _stream_ptr(stream))
 
     def pack_put(self, dim, stream=None, is_reverse=False, op="ID", clear_boundary=False):
         call("dcb_halo_pack_put", self._plan, _ptr(self.tensor.get_buffer()), dim,

@@ -266,3 +266,15 @@ def test_peer_allreduce_takes_vectors_longer_than_its_slots():
         assert np.array_equal(t.cpu().numpy(), np.arange(count, dtype=np.float32) * (rep + 1))
     with pytest.raises(_abi.DcbError):  # the emulation halves keep the limit
         be.allreducer.push(t.data_ptr(), count)
+
+
+def test_exchange_of_a_tensor_without_memory_or_with_an_unknown_operation_is_refused():
+    """... also where there is no halo and so nothing to do."""
+    for overlap in ([0] * 5, [0, 0, 1, 0, 0]):
+        t = dc.Tensor([8, 8, 8, 2, 1], dc.Locale(0, 2), dc.Distribution.make_overlapped_distribution([1, 1, 2, 1, 1], overlap))
+        ex = dc.HaloExchange(t)
+        with pytest.raises(Exception):
+            ex.exchange()
+        t.allocate()
+        with pytest.raises(KeyError):
+            ex.exchange(op="MEAN")
