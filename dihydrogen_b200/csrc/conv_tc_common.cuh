@@ -33,6 +33,22 @@ __device__ __forceinline__ uint32_t tf32_rna(float x)
     return (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
 }
 
+// An operand's bits rounded to TF32 (0x1000, 0xffffe000) or bf16 (0x8000, 0xffff0000), ties
+// away from zero.  What is not a number stays that: the NaN that CUDA's arithmetic returns
+// has all mantissa bits set and would be carried over into a zero.
+__device__ __forceinline__ uint32_t round_operand(float x, uint32_t add, uint32_t mask)
+{
+    return x == x ? (__float_as_uint(x) + add) & mask : 0x7fc00000u;
+}
+
+// The same for converters, one instruction instead of two behind the addition (a comparison
+// per value made the sweep kernel take 106 us instead of 70 at 128^3): the sum's upper bits,
+// and of the NaNs only the one that arithmetic returns, 0x7fffffff, is looked after.
+__device__ __forceinline__ uint32_t round_fast(float x, uint32_t add)
+{
+    return (uint32_t) min(__float_as_int(x), 0x7fff7fff) + add;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -194,9 +210,11 @@ __device__ __forceinline__ uint32_t lds_u32(uint32_t saddr)
 }
 
 // ktab8 / raw are shared-window addresses; the loads are explicit ld.shared so
-// that they are issued back to back (generic loads were serialised).
-__device__ __forceinline__ void convert_chunk(uint32_t ktab8, uint32_t raw_lane, uint32_t (&v)[8],
-                                              uint32_t rnd_add = 0x1000u, uint32_t rnd_mask = 0xffffe000u)
+// that they are issued back to back (generic loads were serialised).  SPLIT: hi and lo
+// parts, else one operand rounded as given.
+template <bool SPLIT>
+__device__ __forceinline__ void convert_chunk(uint32_t ktab8, uint32_t raw_lane, uint32_t (&v)[8], uint32_t rnd_add,
+                                              uint32_t rnd_mask)
 {
     // All loads first and unconditional (a padding row reads cell 4 and is
     // zeroed afterwards), so the eight chains run in parallel without branches.
@@ -211,9 +229,15 @@ __device__ __forceinline__ void convert_chunk(uint32_t ktab8, uint32_t raw_lane,
     for (int e = 0; e < 8; ++e)
     {
         const uint32_t part = tb[e] >> 16;
-        const float xe = part < 2 ? __uint_as_float(xv[e]) : 0.f;
-        const uint32_t hi = (__float_as_uint(xe) + rnd_add) & rnd_mask;
-        const uint32_t lo = tf32_rna(xe - __uint_as_float(hi));
+        const uint32_t xe = part < 2 ? xv[e] : 0u;
+        if (!SPLIT)
+        {
+            v[e] = round_fast(__uint_as_float(xe), rnd_add) & rnd_mask;
+            continue;
+        }
+        const uint32_t hi = (xe + 0x1000u) & 0xffffe000u;
+        const int rest = __float_as_int(__uint_as_float(xe) - __uint_as_float(hi));
+        const uint32_t lo = (uint32_t) min(rest, 0x7fffefff) + 0x1000u; // the pipe reads the upper 19 bits
         v[e] = part == 0 ? hi : lo;
     }
 }

@@ -49,11 +49,11 @@ __global__ void sh_pack_filter_kernel(const float* __restrict__ w, uint4* __rest
     {
         if (kind == 0)
         {
-            const uint32_t hi = (__float_as_uint(f[e]) + rnd_add) & rnd_mask;
+            const uint32_t hi = round_operand(f[e], rnd_add, rnd_mask);
             r[e] = ck.part <= 0 ? hi : tf32_rna(f[e] - __uint_as_float(hi));
         }
         else if (parts == 1)
-            r[e] = __float_as_uint(f[e]) + rnd_add;
+            r[e] = round_operand(f[e], rnd_add, 0xffffffffu);
         else
         {
 #pragma unroll

@@ -190,9 +190,9 @@ __device__ __forceinline__ void sh_convert_store(const float (&v)[KIND == 0 ? 4 
 #pragma unroll
         for (int c = 0; c < CH; ++c)
         {
-            const uint32_t hi = (__float_as_uint(v[c]) + rnd_add) & rnd_mask;
+            const uint32_t hi = (PARTS == 1 ? round_fast(v[c], rnd_add) : __float_as_uint(v[c]) + rnd_add) & rnd_mask;
             w[0][c & 3] = hi;
-            if (PARTS > 1) // exact remainder below 2^-11 |x|; the pipe reads its upper 19 bits
+            if (PARTS > 1) // exact remainder below 2^-11 |x| (or not a number); the pipe reads its upper 19 bits
                 w[PARTS - 1][c & 3] = __float_as_uint(v[c] - __uint_as_float(hi));
         }
     }
@@ -200,7 +200,7 @@ __device__ __forceinline__ void sh_convert_store(const float (&v)[KIND == 0 ? 4 
     {
 #pragma unroll
         for (int c = 0; c < CH; c += 2)
-            w[0][c / 2] = pack_hi16(__float_as_uint(v[c]) + rnd_add, __float_as_uint(v[c + 1 < CH ? c + 1 : c]) + rnd_add);
+            w[0][c / 2] = pack_hi16(round_fast(v[c], rnd_add), round_fast(v[c + 1 < CH ? c + 1 : c], rnd_add));
     }
     else
     {

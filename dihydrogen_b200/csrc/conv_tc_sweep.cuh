@@ -177,7 +177,7 @@ __global__ void sw_pack_filter_kernel(const float* __restrict__ w, float* __rest
         if (ko < g.k && part < 3)
         {
             const float wv = w[((((size_t) ko * g.c + c) * fd + kd) * fh + kh) * fw + kw];
-            const float hi = __uint_as_float((__float_as_uint(wv) + g.rnd_add) & g.rnd_mask);
+            const float hi = __uint_as_float(round_operand(wv, g.rnd_add, g.rnd_mask));
             val = part < 2 ? hi : __uint_as_float(tf32_rna(wv - hi));
         }
         b[i] = val;
@@ -457,7 +457,10 @@ __global__ void __launch_bounds__(sw_threads(XISS), 1)
                             for (int r0 = 0; r0 < g.kr; r0 += 8)
                             {
                                 uint32_t v[8];
-                                convert_chunk(ktab_s + 4u * r0, raw_s, v, g.rnd_add, g.rnd_mask);
+                                if (g.split)
+                                    convert_chunk<true>(ktab_s + 4u * r0, raw_s, v, g.rnd_add, g.rnd_mask);
+                                else
+                                    convert_chunk<false>(ktab_s + 4u * r0, raw_s, v, g.rnd_add, g.rnd_mask);
                                 tmem_st8(a_addr + (uint32_t) r0, v);
                             }
                         }

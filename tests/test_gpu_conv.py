@@ -761,3 +761,40 @@ def test_layers_of_few_products_on_either_kernel(geom):
     dx_ref = np.zeros_like(x)
     O.conv_bwd_data(w, dy, dx_ref, pads, strides)
     emu.assert_close(dx, dx_ref, TOL, "dx")
+
+
+NAN_ALL_ONES = np.uint32(0x7FFFFFFF).view(np.float32)  # what CUDA's arithmetic returns
+NON_FINITE_GEOMS = [
+    (1, 4, 16, (6, 9, 140), (3, 3, 3), 1),   # sweep kernel
+    (1, 2, 8, (6, 9, 132), (3, 3, 3), 1),    # ... without its special case of 4 channels
+    (1, 4, 16, (6, 9, 33), (3, 3, 3), 1),    # shift kernel, TF32 cells
+    (1, 16, 16, (12, 37), (3, 3), 1),        # ... bf16 cells
+    (2, 8, 16, (7, 9, 20), (3, 3, 3), 2),
+    (1, 12, 20, (17, 30), (5, 5), 2),
+]
+
+
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_TF32, _abi.MATH_BF16])
+@pytest.mark.parametrize("geom", NON_FINITE_GEOMS)
+def test_what_is_not_a_number_stays_that(geom, mode):
+    """In every mode, in the input, the filter and the gradient."""
+    N, C, K, sp, f, s = geom
+    rng = np.random.default_rng(8)
+    pads, strides, dil = [(e - 1) // 2 for e in f], [s] * len(sp), [1] * len(sp)
+    x = rng.normal(size=(N, C, *sp)).astype(np.float32)
+    w = rng.normal(size=(K, C, *f)).astype(np.float32)
+    dy = rng.normal(size=(N, K, *[O.conv_out_extent(i, e, (e - 1) // 2, s, 1) for i, e in zip(sp, f)])).astype(np.float32)
+    xn, wn, dyn = x.copy(), w.copy(), dy.copy()
+    xn[(0, C - 1) + tuple(e // 2 for e in sp)] = dyn[(0, K - 1) + tuple(e // 2 for e in dy.shape[2:])] = NAN_ALL_ONES
+    wn[(K - 1, 0) + tuple(e // 2 for e in f)] = NAN_ALL_ONES
+    seen_y = O.conv_fwd(np.isnan(xn).astype(np.float32), np.ones_like(w), pads, strides) > 0
+    seen_dx = np.zeros_like(x)
+    O.conv_bwd_data(np.ones_like(w), np.isnan(dyn).astype(np.float32), seen_dx, pads, strides)
+    y, dx, dw = run_all(xn, w, dyn, pads, strides, dil, mode)
+    assert np.isnan(y[seen_y]).all() and np.isnan(dx[seen_dx > 0]).all()
+    # (the gradient's NaN reaches all of its filter, the input's every tap that sees it)
+    assert np.isnan(dw[K - 1]).all() and np.isnan(dw[:, C - 1]).any(axis=tuple(range(1, 1 + len(f)))).all()
+    assert not np.isnan(dw[:K - 1, :C - 1]).any()
+    y, dx, _ = run_all(x, wn, dy, pads, strides, dil, mode)
+    assert np.isnan(y[:, K - 1]).any() and not np.isnan(y[:, :K - 1]).any()
+    assert np.isnan(dx[:, 0]).any() and not np.isnan(dx[:, 1:]).any()
