@@ -363,15 +363,52 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
     return DCB_OK;
 }
 
+// One element of the filter gradient by FMAs over all positions, by a warp.  For sums that are
+// no numbers: an infinity has no second part (inf - inf), and rows outside dy are multiplied as
+// zeros, so that the parts may hold a NaN where there is a number or an infinity.
+static __device__ __noinline__ float wg_exact(const WgGeom& g, const float* __restrict__ x, const float* __restrict__ dy, int e)
+{
+    const int taps = g.f[0] * g.f[1] * g.f[2], lane = threadIdx.x & 31;
+    const int kw = e % g.f[2], kh = e / g.f[2] % g.f[1], kd = e / (g.f[2] * g.f[1]) % g.f[0], c = e / taps % g.c, k = e / taps / g.c;
+    float acc = 0.f;
+    for (int n = 0; n < g.n; ++n)
+        for (int od = 0; od < g.out[0]; ++od)
+        {
+            const int id = od * g.stride[0] + kd - g.pad[0];
+            if (id < 0 || id >= g.in[0])
+                continue;
+            for (int oh = 0; oh < g.out[1]; ++oh)
+            {
+                const int ih = oh * g.stride[1] + kh - g.pad[1];
+                if (ih < 0 || ih >= g.in[1])
+                    continue;
+                const float* xp = x + (long long) n * g.xs_n + (long long) c * g.xs_c + (long long) id * g.xs[0] + (long long) ih * g.xs[1];
+                const float* dp = dy + (long long) n * g.ys_n + (long long) k * g.ys_c + (long long) od * g.ys[0] + (long long) oh * g.ys[1];
+                for (int ow = lane; ow < g.out[2]; ow += 32)
+                {
+                    const int iw = ow * g.stride[2] + kw - g.pad[2];
+                    if (iw >= 0 && iw < g.in[2])
+                        acc = fmaf(xp[iw], dp[ow], acc);
+                }
+            }
+            if (__any_sync(0xffffffffu, acc != acc))
+                return __int_as_float(0x7fc00000); // and stays that
+        }
+    for (int o = 16; o > 0; o >>= 1)
+        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
+
 // dw from the per-CTA parts: eight lanes per element, parts in order.
 static __global__ void __launch_bounds__(256) wg_fold_kernel(const __grid_constant__ WgGeom g, const float* __restrict__ part,
-                                                      float alpha, float beta, float* dw)
+                                                      const float* __restrict__ x, const float* __restrict__ dy, float alpha,
+                                                      float beta, float* dw)
 {
     const int taps = g.f[0] * g.f[1] * g.f[2];
     const int e = (int) (blockIdx.x * 32 + threadIdx.x / 8), sub = threadIdx.x & 7;
     const bool on = e < g.k * g.c * taps;
     double s = 0.0;
-    wait_for_previous_kernel(part);
+    wait_for_previous_kernel(part, x, dy);
     if (on)
     {
         const int kw = e % g.f[2], kh = e / g.f[2] % g.f[1], kd = e / (g.f[2] * g.f[1]) % g.f[0];
@@ -388,9 +425,19 @@ static __global__ void __launch_bounds__(256) wg_fold_kernel(const __grid_consta
     }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1)
-        s += __shfl_down_sync(0xffffffffu, s, o, 8);
+        s += __shfl_xor_sync(0xffffffffu, s, o, 8);
+    float sum = (float) s;
+    const unsigned bad = __ballot_sync(0xffffffffu, on && sub == 0 && !(fabsf(sum) <= 3.402823466e+38f));
+    if (bad != 0)
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q)
+            if (bad >> (8 * q) & 1)
+            {
+                const float v = wg_exact(g, x, dy, __shfl_sync(0xffffffffu, e, 8 * q));
+                sum = (threadIdx.x & 31) / 8 == q ? v : sum;
+            }
     if (on && sub == 0)
-        dw[e] = alpha * (float) s + (beta != 0.f ? beta * dw[e] : 0.f);
+        dw[e] = alpha * sum + (beta != 0.f ? beta * dw[e] : 0.f);
 }
 
 int32_t tc_conv_bwd_filter(TcPlan* p, float alpha, const float* x, const float* dy, float beta, float* dw, int* status,
@@ -416,7 +463,7 @@ int32_t tc_conv_bwd_filter(TcPlan* p, float alpha, const float* x, const float* 
     }
     const int total = g.k * g.c * g.f[0] * g.f[1] * g.f[2];
     DCB_CUDA_TRY(launch_overlapped(wg_fold_kernel, dim3((unsigned) ((total + 31) / 32)), 256, 0, stream, g, p->wg_part,
-                                   alpha, beta, dw));
+                                   x, dy, alpha, beta, dw));
     return DCB_OK;
 }
 

@@ -41,12 +41,12 @@ __device__ __forceinline__ uint32_t round_operand(float x, uint32_t add, uint32_
     return x == x ? (__float_as_uint(x) + add) & mask : 0x7fc00000u;
 }
 
-// The same for converters, one instruction instead of two behind the addition (a comparison
-// per value made the sweep kernel take 106 us instead of 70 at 128^3): the sum's upper bits,
-// and of the NaNs only the one that arithmetic returns, 0x7fffffff, is looked after.
+// The same for converters (a comparison per value made the sweep kernel take 106 us instead of
+// 70 at 128^3): the sum's upper bits.
 __device__ __forceinline__ uint32_t round_fast(float x, uint32_t add)
 {
-    return (uint32_t) min(__float_as_int(x), 0x7fff7fff) + add;
+    // the addition of zero makes every NaN that of arithmetic, which is positive
+    return (uint32_t) min(__float_as_int(x + 0.f), 0x7fff7fff) + add;
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)

@@ -17,7 +17,7 @@ __global__ void sh_pack_filter_kernel(const float* __restrict__ w, uint4* __rest
                                       const ShPack* __restrict__ packs, const ShChunk* __restrict__ chunks,
                                       const int* __restrict__ codes, int kind, int parts, int total16, int cgroups,
                                       int cpg, int cin, int kout, int kcols, long long w_ko, long long w_ci,
-                                      uint32_t rnd_add, uint32_t rnd_mask, float alpha)
+                                      uint32_t rnd_add, uint32_t rnd_mask, float alpha, uint32_t* w_flag, uint32_t call)
 {
     dependents_may_start();
     // the tables are the plan's: only the filter and the image have to wait
@@ -43,6 +43,12 @@ __global__ void sh_pack_filter_kernel(const float* __restrict__ w, uint4* __rest
 #pragma unroll
     for (int e = 0; e < 8; ++e)
         f[e] = any && e < CH && ch0 + e < cin && ck.ch + e < cpg ? alpha * wp[e * w_ci] : 0.f;
+    float most = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        most = fmaxf(most, fabsf(f[e]) <= 3.402823466e+38f ? 0.f : 1.f);
+    if (most != 0.f)
+        *w_flag = call;
     uint32_t r[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e)
@@ -121,6 +127,8 @@ struct ShPlan
     ShChunk* chunks = nullptr;
     int* codes = nullptr;
     float* stat_part = nullptr;
+    uint32_t* w_flag = nullptr; // two: numbers of the last call whose filter, whose output had an element that is no number
+    uint32_t call = 0;
     int max_image = 0;
 };
 
@@ -153,7 +161,8 @@ bool sh_plan_create(const ConvGeom& g, bool transposed, int math_mode, ShPlan** 
     std::memcpy(host.data() + tab, t.packs.data(), t.packs.size() * sizeof(ShPack));
     std::memcpy(host.data() + tab + pk, t.chunks.data(), t.chunks.size() * sizeof(ShChunk));
     std::memcpy(host.data() + tab + pk + ck, t.codes.data(), t.codes.size() * sizeof(int));
-    if (cudaMalloc(&p->dev, img + host.size() + sp) != cudaSuccess
+    if (cudaMalloc(&p->dev, img + host.size() + sp + 2 * sizeof(uint32_t)) != cudaSuccess
+        || cudaMemset(p->dev + img + host.size() + sp, 0, 2 * sizeof(uint32_t)) != cudaSuccess
         || cudaMemcpy(p->dev + img, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     {
         (void) cudaGetLastError();
@@ -169,6 +178,7 @@ bool sh_plan_create(const ConvGeom& g, bool transposed, int math_mode, ShPlan** 
     p->chunks = reinterpret_cast<ShChunk*>(p->tables + tab + pk);
     p->codes = reinterpret_cast<int*>(p->tables + tab + pk + ck);
     p->stat_part = reinterpret_cast<float*>(p->tables + tab + pk + ck + cd);
+    p->w_flag = reinterpret_cast<uint32_t*>(p->dev + img + host.size() + sp);
     for (const ShPack& k : t.packs)
         p->max_image = std::max(p->max_image, k.n * k.nchunks);
     *out = p;
@@ -236,18 +246,25 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
                                    dim3((unsigned) ((p->max_image + 255) / 256), (unsigned) t.packs.size(),
                                         (unsigned) (g.kgroups * g.cgroups)),
                                    256, 0, stream, w, p->image, p->packs, p->chunks, p->codes, t.kind, t.parts, t.total16,
-                                   g.cgroups, g.cpg, g.cin, g.kout, g.kcols, t.w_ko, t.w_ci, g.rnd_add, g.rnd_mask, alpha));
+                                   g.cgroups, g.cpg, g.cin, g.kout, g.kcols, t.w_ko, t.w_ci, g.rnd_add, g.rnd_mask, alpha, p->w_flag, ++p->call));
     CUtensorMap ymap;
     std::memset(&ymap, 0, sizeof(ymap));
     const int use_ymap = beta == 0.f && sh_make_y_map(g, y, &ymap) ? 1 : 0;
     const unsigned grid = std::min<unsigned>((unsigned) num_sms(), g.units);
     const size_t smem = std::max<size_t>(t.smem, 120 * 1024); // one CTA per SM: it owns all of tensor memory
+    ShExact exact = t.exact;
+    exact.w_flag = p->w_flag;
+    exact.out_flag = p->w_flag + 1;
+    exact.call = p->call;
+    exact.x = x;
+    exact.w = w;
+    exact.alpha = alpha;
     auto launch = [&](auto kernel) -> int32_t {
         const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 227 * 1024);
         if (set != DCB_OK)
             return set;
         // starts beside the packing kernel: what it sets up does not depend on it
-        DCB_CUDA_TRY(launch_overlapped(kernel, dim3(grid), SH_THREADS, smem, stream, g, beta, x, p->image, p->tables, y,
+        DCB_CUDA_TRY(launch_overlapped(kernel, dim3(grid), SH_THREADS, smem, stream, g, exact, beta, x, p->image, p->tables, y,
                                        status, p->stat_part, ymap, use_ymap));
         return DCB_OK;
     };
@@ -262,6 +279,9 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
         return stats ? launch(sh_conv_kernel<1, 3, true, W>) : launch(sh_conv_kernel<1, 3, false, W>);
     };
     const int32_t st = t.wide ? dispatch(std::true_type()) : dispatch(std::false_type());
+    if (st == DCB_OK && t.parts == 1 && beta == 0.f && g.st_s * g.st_r * g.st_w * g.e_s * g.e_r * g.e_w > 1)
+        DCB_CUDA_TRY(launch_overlapped(stats ? sh_repair_kernel<true> : sh_repair_kernel<false>, dim3(grid), SH_THREADS, 0,
+                                       stream, g, exact, y, p->stat_part));
     if (st != DCB_OK || !stats)
         return st;
     DCB_CUDA_TRY(launch_overlapped(sh_stats_fold_kernel, dim3(1), SH_FOLD_WARPS * 32, 0, stream, p->stat_part,

@@ -291,6 +291,141 @@ struct ShCursor
     }
 };
 
+// What a product is of, for the outputs whose accumulators are no numbers.  Spatial triples are
+// in sweep terms, as in ShGeom.
+struct ShExact
+{
+    const float *x, *w; // (the kernel's own x occupies registers, here it is a constant)
+    float alpha;
+    const uint32_t* w_flag; // holds `call` if the filter of this call has an element that is no number
+    uint32_t* out_flag;     // ... if an output may be none
+    uint32_t call;
+    int transposed, one_pass;
+    int f[3], stride[3], pad[3];
+    long long w_ko, w_ci;
+};
+
+// An infinity has no second part (inf - inf), and an instruction also multiplies it with the
+// zeros that stand for taps an output does not have: either leaves a NaN where there may be a
+// number or an infinity.  So one output by FMAs over its taps, as the CUDA-core kernels do it.
+__device__ __noinline__ static float sh_exact(const ShGeom& g, const ShExact& e, int n, int ko, int os, int orow, int ow)
+{
+    float acc = 0.f;
+    auto staged = [&](int d, int o, int k, int extent) { // staged index of tap k, or -1
+        int i = e.transposed ? o + e.pad[d] - k : o * e.stride[d] + k - e.pad[d];
+        if (e.transposed)
+            i = i >= 0 && i % e.stride[d] == 0 ? i / e.stride[d] : -1;
+        return i < extent ? i : -1;
+    };
+    for (int ks = 0; ks < e.f[0]; ++ks)
+    {
+        const int is = staged(0, os, ks, g.in_s);
+        if (is < 0)
+            continue;
+        for (int kr = 0; kr < e.f[1]; ++kr)
+        {
+            const int ir = staged(1, orow, kr, g.in_r);
+            if (ir < 0)
+                continue;
+            for (int kw = 0; kw < e.f[2]; ++kw)
+            {
+                const int iw = staged(2, ow, kw, g.in_w);
+                if (iw < 0)
+                    continue;
+                const float* xp = e.x + (long long) n * g.xs_n + (long long) is * g.xs_s + (long long) ir * g.xs_r + iw;
+                const float* wp = e.w + (long long) ko * e.w_ko + (ks * e.f[1] + kr) * e.f[2] + kw;
+                for (int c = 0; c < g.cin; ++c)
+                {
+                    float a = xp[(long long) c * g.xs_c], b = wp[(long long) c * e.w_ci];
+                    if (e.one_pass)
+                    {
+                        a = __uint_as_float(round_operand(a, g.rnd_add, g.rnd_mask));
+                        b = __uint_as_float(round_operand(e.alpha * b, g.rnd_add, g.rnd_mask));
+                    }
+                    acc = fmaf(a, b, acc);
+                    if (acc != acc)
+                        return acc; // and stays that
+                }
+            }
+        }
+    }
+    return e.one_pass ? acc : e.alpha * acc;
+}
+
+__device__ __forceinline__ bool sh_number(float v)
+{
+    return fabsf(v) <= 3.402823466e+38f;
+}
+
+// Goes through the outputs of this CTA's units once more and computes those that are no numbers
+// by themselves; then the statistics, if there are any, from what stands there.  After the
+// kernel's last barrier, by all threads; not for beta != 0, where the old output is gone.
+template <bool STATS>
+__device__ __noinline__ static void sh_repair(const ShGeom& g, const ShExact& ex, float* y, float* stat_part)
+{
+    const int cells = g.e_s * g.e_r * g.e_w, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int subs_s = g.pack_s > 0 ? g.npack : 1, subs_r = g.pack_r > 0 ? g.npack : 1;
+    float st1 = 0.f, st2 = 0.f; // of filter `warp`
+    asm volatile("fence.proxy.async;" ::: "memory"); // bulk stores before plain loads
+    for (int pass = 0; pass < (STATS ? 2 : 1); ++pass)
+    {
+#pragma unroll 1
+        for (uint32_t unit = blockIdx.x; unit < g.units; unit += gridDim.x)
+        {
+            const ShUnit u = sh_unit(g, unit);
+            const int kbase = u.kg * g.kcols, kn = min(g.kcols, g.kout - kbase), planes = u.q1 - u.q0;
+            const long long rows = (long long) planes * subs_s * g.th * subs_r;
+#pragma unroll 1
+            for (long long row = pass == 0 ? warp : 0; row < rows; row += pass == 0 ? SH_THREADS / 32 : 1)
+            {
+                // (sub-column, plane, sub-column, row)
+                const int r = u.row0 + (int) (row % g.th) + (int) (row / g.th % subs_r) * g.pack_r;
+                const int q = u.q0 + (int) (row / g.th / subs_r % planes) + (int) (row / g.th / subs_r / planes) * g.pack_s;
+                if (r >= g.q_r || q >= g.q_s)
+                    continue;
+#pragma unroll 1
+                for (int i = lane; i < g.tile_w * cells; i += 32)
+                {
+                    const int qw = u.ow0 + i / cells, cell = i % cells;
+                    const int os = q * g.e_s + cell / (g.e_r * g.e_w), orow = r * g.e_r + cell / g.e_w % g.e_r, ow = qw * g.e_w + cell % g.e_w;
+                    if (qw >= g.q_w || os >= g.o_s || orow >= g.o_r || ow >= g.o_w)
+                        continue;
+                    float* yp = y + (long long) u.n * g.ys_n + (long long) kbase * g.ys_c + (long long) os * g.ys_s
+                                + (long long) orow * g.ys_r + ow;
+                    if (pass == 0)
+                    {
+#pragma unroll 1
+                        for (int k = 0; k < kn; ++k)
+                            if (!sh_number(yp[k * g.ys_c]))
+                                yp[k * g.ys_c] = sh_exact(g, ex, u.n, kbase + k, os, orow, ow);
+                    }
+                    else if (warp < kn)
+                    {
+                        const float v = yp[warp * g.ys_c];
+                        st1 += v;
+                        st2 = fmaf(v, v, st2);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (STATS && warp < 16)
+    {
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            st1 += __shfl_xor_sync(0xffffffffu, st1, o);
+            st2 += __shfl_xor_sync(0xffffffffu, st2, o);
+        }
+        for (int w = lane; w < SH_EPI; w += 32) // the epilogue warps' partials
+        {
+            float* part = stat_part + ((size_t) blockIdx.x * SH_EPI + w) * 32;
+            part[warp] = w == 0 ? st1 : 0.f;
+            part[16 + warp] = w == 0 ? st2 : 0.f;
+        }
+    }
+}
+
 // Keeps a uniform condition inside its loop: hoisted out, every such condition
 // doubles the loop, and the roles of this kernel share one instruction cache
 // (95 KB of code ran four times slower than 30 KB).
@@ -410,7 +545,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 // pointers per channel pair, make every other layer 1 to 2 % slower.)
 template <int KIND, int PARTS, bool STATS, bool WIDE>
 __global__ void __launch_bounds__(SH_THREADS, 1)
-    sh_conv_kernel(const __grid_constant__ ShGeom g, float beta, const float* __restrict__ x,
+    sh_conv_kernel(const __grid_constant__ ShGeom g, const __grid_constant__ ShExact ex, float beta, const float* __restrict__ x,
                    const uint4* __restrict__ bimg, const uint8_t* __restrict__ tables, float* y, int* status,
                    float* __restrict__ stat_part, const __grid_constant__ CUtensorMap ymap, int use_ymap)
 {
@@ -458,6 +593,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
             mbar_init(&ev_empty[b], 4);
         }
         *abort_flag = 0;
+        abort_flag[1] = 0; // an output that is no number
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0)
@@ -512,6 +648,9 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         for (int k = 0; k < (STATS ? 16 : 1); ++k)
             st1[k] = st2[k] = 0.f;
         uint32_t slot = 0, lap = 0; // plane slot of the block, uses of it before
+        // An element of x that is no number makes one of every filter's sum (times zero too): the
+        // first filter of a fetch shows it.  Elements of w are looked at when they are packed.
+        bool numbers = true;
         const uint32_t stage_s = smem_u32(smem + g.so_stage) + (uint32_t) (warp * g.stage);
         const uint32_t stage_lane = stage_s + 4u * lane;
         const bool store_w = quad * 32 < g.tile_w;
@@ -553,6 +692,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                             mbar_arrive(&ev_empty[b]);
                         if (!live || r >= g.q_r || !store_w)
                             continue;
+                        numbers = numbers && sh_number(v[0]);
                         if (STATS && lane_w)
                         {
 #pragma unroll
@@ -600,6 +740,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                                 if (lane == 0)
                                     mbar_arrive(&ev_empty[b]);
                             }
+                            numbers = numbers && sh_number(v[0]);
                             if (STATS && in_loop(on))
                             {
                                 // (columns past the filters hold zeros or are not folded)
@@ -630,6 +771,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                             {
                                 float v[16];
                                 sh_drain(block + (uint32_t) (ew * g.woff + c0), min(16, cols - c0), g.nsets, g.set_off, v);
+                                numbers = numbers && sh_number(v[0]) && sh_number(v[4]) && sh_number(v[8]) && sh_number(v[12]);
 #pragma unroll
                                 for (int h = 0; h < 4; ++h)
                                 {
@@ -669,6 +811,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                                         float v[16];
                                         const int piece = min(16, g.nb - k0);
                                         sh_drain(cell + (uint32_t) k0, piece, g.nsets, g.set_off, v);
+                                        numbers = numbers && sh_number(v[0]);
                                         if (in_loop(put))
                                             sh_store(yc + (long long) k0 * g.ys_c, g.ys_c, min(piece, kn - k0), beta, v);
                                     }
@@ -687,6 +830,8 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                 }
             }
         }
+        if (!numbers)
+            abort_flag[1] = 1;
         if (use_ymap && lane == 0)
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         if (STATS)
@@ -1112,6 +1257,24 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TC_TMEM_COLS)
                      : "memory");
+    // (in the one-pass variants the call would cost the converters registers: a kernel of its own)
+    if (PARTS == 1)
+    {
+        if (abort_flag[1] != 0 && tid == 0)
+            *ex.out_flag = ex.call;
+    }
+    else if ((abort_flag[1] != 0 || *ex.w_flag == ex.call) && beta == 0.f)
+        sh_repair<STATS>(g, ex, y, stat_part);
+}
+
+// sh_repair behind a one-pass kernel, with that kernel's grid.
+template <bool STATS>
+__global__ void __launch_bounds__(SH_THREADS)
+    sh_repair_kernel(const __grid_constant__ ShGeom g, const __grid_constant__ ShExact ex, float* y, float* stat_part)
+{
+    wait_for_previous_kernel(y);
+    if (*ex.out_flag == ex.call || *ex.w_flag == ex.call)
+        sh_repair<STATS>(g, ex, y, stat_part);
 }
 
 } // namespace dcb

@@ -314,6 +314,15 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     const int taps = cg.f[0] * cg.f[1] * cg.f[2];
     T->w_ko = m_tr ? taps : (long long) cg.c * taps;
     T->w_ci = m_tr ? (long long) cg.c * taps : taps;
+    ShExact& e = T->exact;
+    std::memset(&e, 0, sizeof(e));
+    e.transposed = m_tr, e.one_pass = m_parts == 1;
+    e.w_ko = T->w_ko, e.w_ci = T->w_ci;
+    for (int d = 0; d < 3; ++d)
+    {
+        const int i = m_flat && d < 2 ? 1 - d : d; // an image is swept along H
+        e.f[d] = cg.f[i], e.stride[d] = cg.stride[i], e.pad[d] = cg.pad[i];
+    }
     return true;
 }
 

@@ -70,6 +70,7 @@ struct ShTables
     std::vector<ShChunk> chunks;
     std::vector<int> codes;
     int total16;                     // 16-byte units of one (filter group, channel group)
+    ShExact exact;                   // without the tensors and alpha
     long long w_ko, w_ci;            // strides of the filter tensor
 };
 

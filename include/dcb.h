@@ -223,7 +223,12 @@ typedef struct dcb_conv_plan dcb_conv_plan;
 int32_t dcb_conv_plan_create(const dcb_conv_desc* cd, const dcb_nd_desc* xd,
                              const dcb_nd_desc* yd, dcb_conv_plan** plan);
 int32_t dcb_conv_plan_destroy(dcb_conv_plan* plan);
-/* w is dense [K][C][fd][fh][fw]. */
+/* w is dense [K][C][fd][fh][fw].
+ * Values that are not finite: a NaN reaches every result that it is a term of, in every
+ * mode.  Infinities and their signs come out as fp32 FMAs give them.  Where a zero of the
+ * padding or of a filter stands beside them they may give a NaN instead: forward of 3-D
+ * stride-1 layers of few channels in fp32 mode (the sweep kernel), stride-1 layers in the
+ * one-pass modes, and beta != 0. */
 int32_t dcb_conv_fwd(dcb_conv_plan* plan, double alpha, const void* x,
                      const void* w, double beta, void* y, void* stream);
 /* y = alpha * conv(x, w), and from the same pass sums[k] = sum of y over filter

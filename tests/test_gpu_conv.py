@@ -798,3 +798,57 @@ def test_what_is_not_a_number_stays_that(geom, mode):
     y, dx, _ = run_all(x, wn, dy, pads, strides, dil, mode)
     assert np.isnan(y[:, K - 1]).any() and not np.isnan(y[:, :K - 1]).any()
     assert np.isnan(dx[:, 0]).any() and not np.isnan(dx[:, 1:]).any()
+
+
+@pytest.mark.parametrize("value", [np.float32(np.inf), NAN_ALL_ONES])
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_TF32, _abi.MATH_BF16])
+@pytest.mark.parametrize("geom", NON_FINITE_GEOMS[2:] + [
+    (1, 4, 4, (8, 9, 64), (3, 3, 3), 2),     # backward data: cells of four columns drained together
+    (1, 8, 16, (20, 64), (3, 3), 1),         # bulk stores
+    (1, 16, 24, (5, 6, 40), (3, 3, 3), 1),
+    (1, 4, 8, (9, 33), (1, 1), 2),           # one tap: its k-step's other half is the neighbour's cell
+])
+def test_infinities_and_nans_come_out_as_from_fp32_fma(geom, mode, value):
+    """... and only where they are a term: the cells around keep their values (strides 2:
+    an instruction also multiplies a cell with the zeros of taps that an output does not have)."""
+    N, C, K, sp, f, s = geom
+    if mode != _abi.MATH_FP32 and s == 1 and np.isinf(value):
+        pytest.skip("one pass, stride 1: an infinity beside a zero may give a NaN")
+    rng = np.random.default_rng(9)
+    pads, strides, dil = [(e - 1) // 2 for e in f], [s] * len(sp), [1] * len(sp)
+    x = rng.normal(size=(N, C, *sp)).astype(np.float32)
+    w = rng.normal(size=(K, C, *f)).astype(np.float32)
+    w[0] = 1.0  # exactly representable: no second part to meet an infinity
+    dy = rng.normal(size=(N, K, *[O.conv_out_extent(i, e, (e - 1) // 2, s, 1) for i, e in zip(sp, f)])).astype(np.float32)
+    for at in (tuple(e // 2 for e in sp), (0,) * len(sp), tuple(e - 1 for e in sp)):
+        x[(0, C - 1) + at] = value
+        dy[(0, K - 1) + tuple(min(a // s, e - 1) for a, e in zip(at, dy.shape[2:]))] = -value
+    got = run_all(x, w, dy, pads, strides, dil, mode)
+    with np.errstate(all="ignore"):
+        ref = [O.conv_fwd(x, w, pads, strides), np.zeros_like(x), O.conv_bwd_filter(x, dy, f, pads, strides)]
+        O.conv_bwd_data(w, dy, ref[1], pads, strides)
+    for name, a, b in zip(("y", "dx", "dw"), got, ref):
+        assert np.array_equal(np.isnan(a), np.isnan(b)), name
+        assert np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b)), name
+        assert np.isfinite(b).any()
+        scale = np.sqrt(np.mean(np.square(b[np.isfinite(b)])))
+        bound = 2e-5 if mode == _abi.MATH_FP32 or name == "dw" else 4e-2
+        assert np.abs(a - b)[np.isfinite(b)].max() <= bound * (scale + np.abs(b[np.isfinite(b)]).max()), name
+
+
+def test_statistics_of_an_output_with_an_infinity():
+    """The statistics' epilogue sees the repaired values."""
+    rng = np.random.default_rng(10)
+    N, C, K, sp = 1, 4, 16, (6, 9, 33)
+    x = torch.from_numpy(rng.normal(size=(N, C, *sp)).astype(np.float32)).cuda()
+    w = torch.ones(K, C, 3, 3, 3, device="cuda")
+    w[1:] = torch.from_numpy(rng.normal(size=(K - 1, C, 3, 3, 3)).astype(np.float32)).cuda()
+    w[3, 1] = 0.0  # inf * 0
+    x[0, 1, 3, 4, 5] = float("inf")
+    y, sums = torch.empty(N, K, *sp, device="cuda"), torch.zeros(2, K, device="cuda")
+    p = Plan(x, w, y, [1] * 3, [1] * 3, [1] * 3, _abi.MATH_FP32)
+    assert _abi.lib().dcb_conv_fwd_stats(p.p, 1.0, x.data_ptr(), w.data_ptr(), y.data_ptr(), sums[0].data_ptr(),
+                                         sums[1].data_ptr(), None) == _abi.OK
+    torch.cuda.synchronize()
+    assert torch.equal(torch.isnan(sums[0]), torch.isnan(y.sum((0, 2, 3, 4)))) and bool(torch.isnan(sums[0][3]))
+    assert float(sums[0][0]) == float("inf") and float(sums[1][0]) == float("inf")
