@@ -281,8 +281,8 @@ __device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitc
 
 // ---------------------------------------------------------------------------
 // Warps: 0..11 converters (three groups of four), 12..14 MMA issuers (issuer q
-// serves group q), 15 bulk copies, 16..23 epilogue (two per TMEM quadrant,
-// even / odd output rows).  TMEM columns: [accumulators th * fd * 16][A ring].
+// serves group q), 15 bulk copies, 16..27 epilogue (three per TMEM quadrant,
+// every third output row).  TMEM columns: [accumulators th * fd * 16][A ring].
 // ---------------------------------------------------------------------------
 // STATS: the epilogue also adds up, per filter, the outputs it stores and their
 // squares (what a batch-norm statistics pass over y would read again): each
@@ -301,10 +301,9 @@ __device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitc
 // and issuer (q, 1) those in the second.  Free-running, the three issuers of the
 // plain kernel need as long as its busiest epilogue warps (0.35 ms on the 256^3
 // shard, ~140 clocks per tcgen05.mma or commit, seven per staged row); with six the
-// kernel takes 0.378 ms instead of 0.433.  The variants whose epilogue does more
-// (statistics, blend) are held by their epilogue warps and by registers (the extra
-// warps lower the cap to 66 per thread, their epilogues then spill): they keep
-// three issuers and one slot per group.
+// kernel takes 0.378 ms instead of 0.433.  The variant with statistics is
+// held by its epilogue warps and by registers (the extra warps lower the cap to 66
+// per thread, its epilogue then spills): it keeps three issuers and one slot per group.
 constexpr int SW_EPI = 12;
 __host__ __device__ constexpr int sw_threads(int xiss)
 {

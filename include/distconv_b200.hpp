@@ -1874,7 +1874,8 @@ public:
     {
         return dcb_conv_plan_kernel_kind(which == 0 ? m_plan_fwd : (which == 1 ? m_plan_bwd : m_plan_wgrad), which);
     }
-    // 0 fp32 CUDA-core, 1 / 2 tcgen05 row kernel, 3 sweep, 4 multi-group sweep, 5 tcgen05 backward filter
+    // 0 fp32 CUDA-core; tcgen05: 3 sweep, or shift on TF32 or one-pass operands, 4 shift on three bf16
+    // parts, 5 backward filter
     int kernel_variant(int which) const
     {
         return dcb_conv_plan_kernel_variant(which == 0 ? m_plan_fwd : (which == 1 ? m_plan_bwd : m_plan_wgrad),
