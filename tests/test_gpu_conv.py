@@ -112,16 +112,16 @@ GEOMS = [
     (3, 5, 7, (9, 21), (3, 3), (1, 1), (2, 2), (1, 1)),                       # 2-D stride 2, odd extents
     (1, 4, 8, (6, 9, 36), (3, 2, 3), (1, 0, 1), (1, 1, 1), (1, 1, 1)),        # two filter rows: two converter groups
     (2, 3, 5, (5, 6, 40), (2, 1, 3), (1, 0, 1), (1, 1, 1), (1, 1, 1)),        # one filter row: one converter group
-    (2, 3, 12, (7, 10, 132), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),     # backward data: 3 channel groups -> 3 filters
+    (2, 3, 12, (7, 10, 132), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),     # backward data: 12 channels -> 3 filters
     (1, 4, 16, (9, 30, 64), (3, 3, 3), (0, 1, 1), (1, 1, 1), (1, 1, 1)),      # backward data: tall columns, no padding in D
-    (2, 32, 32, (12, 140), (5, 5), (2, 2), (1, 1), (1, 1)),                   # cfg4 channels: 4 channel x 2 filter group launches
+    (2, 32, 32, (12, 140), (5, 5), (2, 2), (1, 1), (1, 1)),                   # cfg4 channels
     (1, 24, 40, (10, 70), (3, 3), (1, 1), (1, 1), (1, 1)),                    # ragged last filter group
-    (1, 16, 32, (6, 8, 36), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),      # 3-D, 32 filters: row kernel, grouped backward filter
-    (1, 16, 16, (5, 7, 40), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),      # 3-D, 4 channel groups in the sweep kernels
+    (1, 16, 32, (6, 8, 36), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),      # 3-D, 32 filters
+    (1, 16, 16, (5, 7, 40), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),      # 3-D, 16 channels
     (1, 8, 20, (7, 12, 280), (3, 3, 3), (1, 1, 1), (2, 2, 2), (1, 1, 1)),     # stride 2, two W tiles (ragged), grouped backward filter
     (2, 4, 16, (9, 300), (3, 3), (1, 1), (1, 2), (1, 1)),                     # stride 2 along W only
     (1, 3, 5, (10, 264), (5, 5), (2, 2), (2, 2), (1, 1)),                     # 5x5 stride 2
-    (1, 4, 32, (6, 9, 40), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),       # backward data with 8 channel groups: group launches, not one accumulator chain
+    (1, 4, 32, (6, 9, 40), (3, 3, 3), (1, 1, 1), (1, 1, 1), (1, 1, 1)),       # backward data over 32 channels: leading products apart from the corrections
 ]
 
 
@@ -399,8 +399,8 @@ def _round_bf16(a):
 
 @pytest.mark.parametrize("mode", [_abi.MATH_BF16, _abi.MATH_TF32])
 @pytest.mark.parametrize("shape", [
-    (1, 4, 16, (20, 23, 140), (3, 3, 3)),     # the bench layer's family: sweep kernel, multi-group backward data
-    (2, 16, 8, (40, 70), (3, 3)),             # 2-D: row kernel
+    (1, 4, 16, (20, 23, 140), (3, 3, 3)),     # the bench layer's family: sweep kernel, shift kernel backward
+    (2, 16, 8, (40, 70), (3, 3)),             # 2-D
     (1, 12, 16, (9, 17, 33), (3, 3, 3)),      # channel groups
 ])
 def test_reduced_precision_modes_equal_the_rounded_operands_product(shape, mode):
@@ -529,9 +529,8 @@ def test_stride_2_backward_filter_on_a_window_above_a_16_byte_boundary(lead):
 
 def test_backward_data_full_shard_16_channels_against_fp64():
     """Backward data of the benchmark layer on its 256^3 shard: dy has 16
-    channels, which the multi-group sweep kernel walks as four groups inside one
-    launch, two per accumulator set (a single truncating chain of 180 updates
-    sat on the 1e-5 bound).  dy carries a mean so that a truncation bias cannot
+    channels, six products of three bf16 parts; the leading ones have an accumulator
+    set of their own (a single truncating chain of 180 updates sat on the 1e-5 bound).  dy carries a mean so that a truncation bias cannot
     hide behind cancellation; sampled blocks of dx (a corner, an edge, the
     interior) are recomputed in fp64."""
     import torch.nn.functional as F
@@ -542,7 +541,7 @@ def test_backward_data_full_shard_16_channels_against_fp64():
     w = torch.randn(16, 4, 3, 3, 3, device="cuda", generator=gen) * 0.14 + 0.02
     dx = torch.full((1, 4, D, 256, 256), float("nan"), device="cuda")
     p = Plan(dx, w, dy, [1] * 3, [1] * 3, [1] * 3, _abi.MATH_FP32)
-    assert _abi.lib().dcb_conv_plan_kernel_variant(p.p, 1) == 4, "expected the multi-group sweep kernel"
+    assert _abi.lib().dcb_conv_plan_kernel_variant(p.p, 1) == 4, "expected the shift kernel on bf16 parts"
     for rep in range(3):  # the order in which the issuers' instructions land varies from run to run
         p.bwd_data(1.0, w, dy, 0.0, dx)
         torch.cuda.synchronize()
@@ -576,9 +575,12 @@ def test_backward_data_full_shard_16_channels_against_fp64():
     (1, 1, 4, (900, 150), (3, 3), 1),          # few filters: blocks narrower than an instruction's 16 columns, many planes
     (1, 8, 4, (40, 60, 132), (3, 3, 3), 2),    # the same where a plane adds to some of the live slots only
     (1, 5, 24, (90, 84), (5, 5), 2),           # blocks of one and a half times 16 columns
+    (2, 4, 4, (40, 17), (3, 3), 1),            # the layers of one channel above with products enough for this kernel
+    (1, 16, 4, (900, 150), (3, 3), 1, [1, 0]),  # 4 filters: forward here, backward data on CUDA cores
+    (1, 4, 16, (900, 150), (3, 3), 1, [0, 1]),  # the other way round
 ])
 def test_shift_kernel_tile_and_table_edges(geom):
-    N, C, K, sp, f, s = geom
+    N, C, K, sp, f, s = geom[:6]
     rng = np.random.default_rng(sum(sp) + C)
     nsd, pads, strides = len(sp), [(e - 1) // 2 for e in f], [s] * len(sp)
     x = rng.normal(0, 1, (N, C, *sp)).astype(np.float32)
@@ -586,6 +588,10 @@ def test_shift_kernel_tile_and_table_edges(geom):
     dy = rng.normal(0, 1, (N, K, *[O.conv_out_extent(i, ff, p, s, 1) for i, ff, p in zip(sp, f, pads)])).astype(np.float32)
     y0 = rng.normal(size=dy.shape).astype(np.float32)
     dx0 = rng.normal(size=x.shape).astype(np.float32)
+    p = Plan(*(torch.from_numpy(a).cuda() for a in (x, w, dy)), pads, strides, [1] * nsd, _abi.MATH_FP32)
+    kinds = [_abi.lib().dcb_conv_plan_kernel_kind(p.p, i) for i in (0, 1)]
+    want = geom[6] if len(geom) > 6 else [1, 1]
+    assert kinds == want or (C == 1 and nsd == 2), "one channel may take the CUDA cores, the others are here for the shift kernel"
     y, dx, _ = run_all(x, w, dy, pads, strides, [1] * nsd, _abi.MATH_FP32, alpha=0.5, beta=-1.0, y0=y0, dx0=dx0,
                        dw0=np.zeros_like(w))
     emu.assert_close(y, 0.5 * O.conv_fwd(x, w, pads, strides) - y0, TOL, "y")
@@ -852,3 +858,36 @@ def test_statistics_of_an_output_with_an_infinity():
     torch.cuda.synchronize()
     assert torch.equal(torch.isnan(sums[0]), torch.isnan(y.sum((0, 2, 3, 4)))) and bool(torch.isnan(sums[0][3]))
     assert float(sums[0][0]) == float("inf") and float(sums[1][0]) == float("inf")
+
+
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_BF16])
+@pytest.mark.parametrize("geom", [
+    (1, 4, 16, (6, 9, 9), (3, 3, 3), 1),      # sub-columns side by side
+    (2, 8, 7, (5, 11, 31), (3, 3, 3), 1),     # two samples, filters padded
+    (1, 16, 16, (7, 9, 101), (3, 3, 3), 1),   # ragged rows: plain stores
+    (1, 16, 4, (8, 9, 132), (3, 3, 3), 2),    # stride 2
+    (1, 32, 16, (64, 64, 64), (3, 3, 3), 1),  # channel groups, bulk stores
+])
+def test_statistics_from_the_shift_kernel(geom, mode):
+    """Sums and sums of squares of the output that it wrote, to fp32 rounding of partial sums:
+    2^-24 per addition of a lane's chain, some hundred of them."""
+    N, C, K, sp, f, s = geom
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(N, C, *sp, device="cuda", generator=gen) + 0.5
+    w = torch.randn(K, C, *f, device="cuda", generator=gen) * 0.1
+    y = torch.full((N, K, *[O.conv_out_extent(i, 3, 1, s, 1) for i in sp]), float("nan"), device="cuda")
+    sums = torch.full((2, K), float("nan"), device="cuda")
+    p = Plan(x, w, y, [1] * 3, [s] * 3, [1] * 3, mode)
+    assert _abi.lib().dcb_conv_plan_kernel_kind(p.p, 0) == 1
+    assert _abi.lib().dcb_conv_fwd_stats(p.p, 1.0, x.data_ptr(), w.data_ptr(), y.data_ptr(), sums[0].data_ptr(),
+                                         sums[1].data_ptr(), None) == _abi.OK
+    torch.cuda.synchronize()
+    assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.OK
+    # not against dcb_conv_fwd's bits: the pipe truncates and the issuers' instructions land in an
+    # order that varies from run to run, so that two plain forward passes differ in their last bits too
+    xr, wr = (x, w) if mode == _abi.MATH_FP32 else (torch.from_numpy(_round_bf16(a.cpu().numpy())).cuda() for a in (x, w))
+    ref = torch.nn.functional.conv3d(xr.double(), wr.double(), None, s, 1)
+    emu.assert_close(y.cpu().numpy(), ref.cpu().numpy(), TOL, "y")
+    d, over = y.double(), (0, 2, 3, 4)
+    for got, ref, size in ((sums[0], d.sum(over), d.abs().sum(over)), (sums[1], d.square().sum(over), d.square().sum(over))):
+        assert ((got.double() - ref).abs() <= 1e-5 * size).all()
