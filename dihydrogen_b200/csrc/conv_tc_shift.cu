@@ -259,26 +259,33 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
     exact.x = x;
     exact.w = w;
     exact.alpha = alpha;
-    auto launch = [&](auto kernel) -> int32_t {
+    auto launch = [&](auto kernel, auto size) -> int32_t {
         const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 227 * 1024);
         if (set != DCB_OK)
             return set;
+        ShConst<decltype(size)::value> ct;
+        std::memcpy(&ct, t.issue.data(), t.issue.size());
         // starts beside the packing kernel: what it sets up does not depend on it
-        DCB_CUDA_TRY(launch_overlapped(kernel, dim3(grid), SH_THREADS, smem, stream, g, exact, beta, x, p->image, p->tables, y,
+        DCB_CUDA_TRY(launch_overlapped(kernel, dim3(grid), SH_THREADS, smem, stream, g, exact, beta, ct, x, p->image, p->tables, y,
                                        status, p->stat_part, ymap, use_ymap));
         return DCB_OK;
     };
-    auto dispatch = [&](auto wide) -> int32_t {
+    auto dispatch = [&](auto wide, auto size) -> int32_t {
         constexpr bool W = decltype(wide)::value;
+        constexpr int C = decltype(size)::value;
         if (t.kind == 0 && t.parts == 1)
-            return stats ? launch(sh_conv_kernel<0, 1, true, W>) : launch(sh_conv_kernel<0, 1, false, W>);
+            return stats ? launch(sh_conv_kernel<0, 1, true, W, C>, size) : launch(sh_conv_kernel<0, 1, false, W, C>, size);
         if (t.kind == 0)
-            return stats ? launch(sh_conv_kernel<0, 2, true, W>) : launch(sh_conv_kernel<0, 2, false, W>);
+            return stats ? launch(sh_conv_kernel<0, 2, true, W, C>, size) : launch(sh_conv_kernel<0, 2, false, W, C>, size);
         if (t.parts == 1)
-            return stats ? launch(sh_conv_kernel<1, 1, true, W>) : launch(sh_conv_kernel<1, 1, false, W>);
-        return stats ? launch(sh_conv_kernel<1, 3, true, W>) : launch(sh_conv_kernel<1, 3, false, W>);
+            return stats ? launch(sh_conv_kernel<1, 1, true, W, C>, size) : launch(sh_conv_kernel<1, 1, false, W, C>, size);
+        return stats ? launch(sh_conv_kernel<1, 3, true, W, C>, size) : launch(sh_conv_kernel<1, 3, false, W, C>, size);
     };
-    const int32_t st = t.wide ? dispatch(std::true_type()) : dispatch(std::false_type());
+    using Large = std::integral_constant<int, SH_CONST>;
+    using Small = std::integral_constant<int, SH_CONST_SMALL>;
+    const int32_t st = t.wide ? dispatch(std::true_type(), Large())
+                              : (t.issue.size() > SH_CONST_SMALL ? dispatch(std::false_type(), Large())
+                                                                 : dispatch(std::false_type(), Small()));
     if (st == DCB_OK && t.parts == 1 && beta == 0.f && g.st_s * g.st_r * g.st_w * g.e_s * g.e_r * g.e_w > 1)
         DCB_CUDA_TRY(launch_overlapped(stats ? sh_repair_kernel<true> : sh_repair_kernel<false>, dim3(grid), SH_THREADS, 0,
                                        stream, g, exact, y, p->stat_part));

@@ -55,7 +55,6 @@ constexpr int SH_EPI = 8;
 constexpr int SH_CONV = 12;
 constexpr int SH_ISS = 3;
 constexpr int SH_THREADS = (SH_EPI + SH_CONV + SH_ISS + 1) * 32;
-constexpr int SH_REG_STEPS = 6; // k-steps that fit an issuer's registers
 constexpr int SH_MAX_ITEMS = SH_CONV; // warp-sized pieces of a staged row: never more than the warps of a team
 constexpr int SH_MAX_SLOTS = 9;   // A slots: a multiple of SH_ISS
 constexpr int SH_MAX_BLOCKS = 64; // (row, plane slot) accumulator blocks of a column
@@ -66,6 +65,20 @@ struct ShGroup // one accumulator range of a staged row
     uint16_t step0, nst; // its k-steps
     uint32_t b16;        // filter image, 16-byte units from the start of its set
     uint32_t pad_;
+};
+
+// The issuers' tables (steps, groups, rows: offsets in ShGeom), in the constant bank.  What an
+// instruction needs is then in uniform registers, where it has to be: alone on its SM, a warp
+// issues an instruction every 45 clocks (N = 48), every 69 with the tables in shared memory, and
+// beside the converters' traffic the difference grows.  16 -> 32, stride 2, 256^3 1048 -> 910 us,
+// 16 -> 4 channels (backward data) 905 -> 868, 32 -> 32, 5 x 5 943 -> 901.  They are an argument of
+// their own size class: 8 KB with every launch made passes of 30 us, which wait for the host, 3 %
+// slower; the tables of most small layers fit 1 KB.
+constexpr int SH_CONST = 8192, SH_CONST_SMALL = 1024;
+template <int BYTES>
+struct ShConst
+{
+    uint4 v[BYTES / 16];
 };
 
 // Spatial triples are in sweep terms: S (slowest), R, W.  "Super" output
@@ -89,7 +102,6 @@ struct ShGeom
     int cpg, cgroups;        // channels per group (a multiple of the cell's)
     int pt;                  // positions per plane of the A slot
     int ipr;                 // items (32 positions, all cells of the channel group) of a staged row
-    int reg_steps;           // > 0: every range has these k-steps, in one table
     int a_slot16, a_slots;
     int teams;               // converter teams; a_slots is a multiple of it and of SH_ISS
     int npack, pack_s, pack_r; // sub-columns side by side in the 128 lanes, their distance in super units
@@ -102,7 +114,8 @@ struct ShGeom
     uint32_t rnd_add, rnd_mask;
     // byte offsets in shared memory
     int stage;               // bytes per epilogue warp for bulk stores, 0: none
-    int so_stage, so_a, so_steps, so_groups, so_rows, so_sets, so_items, so_lanes, so_bars;
+    int so_stage, so_a, so_sets, so_items, so_lanes, so_bars;
+    int co_groups, co_rows; // in the constant tables, 16-byte and 4-byte units (the steps stand first)
     // byte offsets in the table buffer (same order), total to copy
     int tab_bytes;
 };
@@ -426,6 +439,18 @@ __device__ __noinline__ static void sh_repair(const ShGeom& g, const ShExact& ex
     }
 }
 
+// A value that all lanes of a converged warp have, where the compiler does not know it.
+__device__ __forceinline__ uint32_t uniform(uint32_t v)
+{
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// A wait may end for one lane as it runs out for another: the warp stays together.
+__device__ __forceinline__ bool all_lanes(bool ok)
+{
+    return __all_sync(0xffffffffu, ok) != 0;
+}
+
 // Keeps a uniform condition inside its loop: hoisted out, every such condition
 // doubles the loop, and the roles of this kernel share one instruction cache
 // (95 KB of code ran four times slower than 30 KB).
@@ -543,18 +568,15 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 
 // WIDE: channels lie too far apart for 32-bit offsets.  (64-bit offsets throughout, or two
 // pointers per channel pair, make every other layer 1 to 2 % slower.)
-template <int KIND, int PARTS, bool STATS, bool WIDE>
+template <int KIND, int PARTS, bool STATS, bool WIDE, int CONST>
 __global__ void __launch_bounds__(SH_THREADS, 1)
-    sh_conv_kernel(const __grid_constant__ ShGeom g, const __grid_constant__ ShExact ex, float beta, const float* __restrict__ x,
-                   const uint4* __restrict__ bimg, const uint8_t* __restrict__ tables, float* y, int* status,
+    sh_conv_kernel(const __grid_constant__ ShGeom g, const __grid_constant__ ShExact ex, float beta, const __grid_constant__ ShConst<CONST> ct,
+                   const float* __restrict__ x, const uint4* __restrict__ bimg, const uint8_t* __restrict__ tables, float* y, int* status,
                    float* __restrict__ stat_part, const __grid_constant__ CUtensorMap ymap, int use_ymap)
 {
     constexpr int CH = KIND == 0 ? 4 : 8;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-    const uint2* steps = reinterpret_cast<const uint2*>(smem + g.so_steps);
-    const ShGroup* groups = reinterpret_cast<const ShGroup*>(smem + g.so_groups);
-    const uint32_t* rowtab = reinterpret_cast<const uint32_t*>(smem + g.so_rows);
     const uint2* sets = reinterpret_cast<const uint2*>(smem + g.so_sets);
     const uint32_t* items = reinterpret_cast<const uint32_t*>(smem + g.so_items);
     const int* lanes = reinterpret_cast<const int*>(smem + g.so_lanes);
@@ -605,7 +627,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
     }
 #pragma unroll 1
     for (int i = tid; i < g.tab_bytes / 16; i += SH_THREADS)
-        reinterpret_cast<uint4*>(smem + g.so_steps)[i] = reinterpret_cast<const uint4*>(tables)[i];
+        reinterpret_cast<uint4*>(smem + g.so_sets)[i] = reinterpret_cast<const uint4*>(tables)[i];
     // positions that no item writes are read by the MMAs of lanes nobody stores: keep them finite
 #pragma unroll 1
     for (int i = tid; i < g.a_slots * g.a_slot16; i += SH_THREADS)
@@ -1001,10 +1023,10 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         const uint32_t hi = 8u | (1u << 14); // SBO 128 bytes, descriptor version, no swizzle
         const uint32_t fmt = KIND == 0 ? 2u : 1u;
         const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t) (TC_M >> 4) << 24);
-        uint2 rs[SH_REG_STEPS];
-#pragma unroll
-        for (int s = 0; s < SH_REG_STEPS; ++s)
-            rs[s] = s < g.reg_steps ? steps[s] : make_uint2(0, 0);
+        const uint2* steps = reinterpret_cast<const uint2*>(ct.v);
+        const uint4* groups = ct.v + g.co_groups;
+        const uint32_t* rowtab = reinterpret_cast<const uint32_t*>(ct.v) + g.co_rows;
+        const uint32_t tmem_u = uniform(tmem_base);
         uint32_t slot = (uint32_t) iss_w, a_par = 0; // A ring: this issuer's next slot
         int skip = (int) slot;                                      // staged rows until its next one
         uint32_t stage = 0, b_par = 0;          // filter image stages
@@ -1019,7 +1041,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
             if (!g.stream && u.kg != kg_have && u.z_hi > u.z_lo)
             {
                 kg_have = u.kg;
-                ok = mbar_wait_t<0>(&b_full[0], b_par, abort_flag);
+                ok = all_lanes(mbar_wait_t<0>(&b_full[0], b_par, abort_flag));
                 b_par ^= 1;
             }
             const int nq = (u.nz - g.fs) / g.st_s + 1; // planes opened and closed
@@ -1036,7 +1058,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                     uint32_t bset = b16;
                     if (g.stream && real)
                     {
-                        ok = mbar_wait_t<0>(&b_full[stage], b_par, abort_flag);
+                        ok = all_lanes(mbar_wait_t<0>(&b_full[stage], b_par, abort_flag));
                         bset += stage * (uint32_t) g.b_stage16;
                     }
                     else if (!g.stream)
@@ -1054,57 +1076,31 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                     for (; i < i_hi && ok; i += SH_ISS)
                     {
                         // what the row does, before waiting for what it needs
-                        const uint32_t rt = rowtab[phase * (uint32_t) g.rows + (uint32_t) i];
-                        uint32_t gi = rt & 0xffffu;
-                        const uint32_t g1 = gi + (rt >> 16);
-                        uint4 gr = *reinterpret_cast<const uint4*>(&groups[gi]);
+                        const uint32_t rt = rowtab[uniform(phase * (uint32_t) g.rows + (uint32_t) i)];
+                        const uint32_t g0 = rt & 0xffffu, g1 = g0 + (rt >> 16);
 #pragma unroll 1
                         for (; j_open * g.st_r <= i && j_open < g.th && ok; ++j_open)
                             ok = mbar_wait_t<0>(&ev_empty[j_open * g.ns + (int) first_slot], (first_lap - 1) & 1,
                                                 abort_flag);
-                        ok = ok && mbar_wait_t<0>(&a_full[slot], a_par, abort_flag);
+                        ok = all_lanes(ok && mbar_wait_t<0>(&a_full[slot], a_par, abort_flag));
                         if (!ok)
                             break;
                         tc_fence_after();
-                        const uint32_t aslot = a16 + slot * (uint32_t) g.a_slot16;
+                        const uint32_t aslot = uniform(a16 + slot * (uint32_t) g.a_slot16), bs = uniform(bset);
 #pragma unroll 1
-                        while (gi < g1)
+                        for (uint32_t gi = g0; gi < g1; ++gi)
                         {
-                            const uint32_t d = tmem_base + (gr.x & 0xffffu);
+                            const uint4 gr = groups[gi];
+                            const uint32_t d = tmem_u + (gr.x & 0xffffu);
                             const uint32_t idesc = idesc0 | (gr.x >> 16 >> 3 << 17);
-                            const uint32_t bb = bset + gr.z;
-                            const uint2* sp = steps + (gr.y & 0xffffu);
-                            const int n = (int) (gr.y >> 16);
-                            gr = *reinterpret_cast<const uint4*>(&groups[++gi]);
-                            if (g.reg_steps > 0)
+                            const uint32_t bb = bs + gr.z;
+                            const uint32_t s0 = gr.y & 0xffffu, s1 = s0 + (gr.y >> 16);
+#pragma unroll 3
+                            for (uint32_t s = s0; s < s1; ++s)
                             {
-#pragma unroll
-                                for (int s = 0; s < SH_REG_STEPS; ++s)
-                                    if (s < n)
-                                        sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + rs[s].x),
-                                                     (uint64_t) hi << 32 | (bb + rs[s].y), idesc, elected);
-                                continue;
-                            }
-                            int s = 0;
-#pragma unroll 1
-                            for (; s + 4 <= n; s += 4)
-                            {
-                                const uint2 s0 = sp[s], s1 = sp[s + 1], s2 = sp[s + 2], s3 = sp[s + 3];
-                                sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + s0.x),
-                                             (uint64_t) hi << 32 | (bb + s0.y), idesc, elected);
-                                sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + s1.x),
-                                             (uint64_t) hi << 32 | (bb + s1.y), idesc, elected);
-                                sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + s2.x),
-                                             (uint64_t) hi << 32 | (bb + s2.y), idesc, elected);
-                                sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + s3.x),
-                                             (uint64_t) hi << 32 | (bb + s3.y), idesc, elected);
-                            }
-#pragma unroll 1
-                            for (; s < n; ++s)
-                            {
-                                const uint2 s0 = sp[s];
-                                sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + s0.x),
-                                             (uint64_t) hi << 32 | (bb + s0.y), idesc, elected);
+                                const uint2 st = steps[s];
+                                sh_mma<KIND>(d, (uint64_t) hi << 32 | (aslot + st.x), (uint64_t) hi << 32 | (bb + st.y), idesc,
+                                             elected);
                             }
                         }
                         if (elected)
@@ -1124,6 +1120,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
 #pragma unroll 1
                     for (; grp == 0 && j_open < g.th && ok; ++j_open)
                         ok = mbar_wait_t<0>(&ev_empty[j_open * g.ns + (int) first_slot], (first_lap - 1) & 1, abort_flag);
+                    ok = all_lanes(ok);
 #pragma unroll 1
                     for (; j_close < g.th && ok; ++j_close)
                         if (elected)

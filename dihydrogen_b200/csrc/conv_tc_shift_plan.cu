@@ -488,9 +488,14 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
             return (int) at;
         };
         T->blob.clear();
-        const int o_steps = put(st.data(), st.size() * sizeof(uint2));
-        const int o_groups = put(groups.data(), groups.size() * sizeof(ShGroup));
-        const int o_rows = put(rowtab.data(), rowtab.size() * 4);
+        put(st.data(), st.size() * sizeof(uint2));
+        g.co_groups = put(groups.data(), groups.size() * sizeof(ShGroup)) / 16;
+        g.co_rows = put(rowtab.data(), rowtab.size() * 4) / 4;
+        T->too_long = T->blob.size() > SH_CONST;
+        if (T->too_long)
+            return false;
+        T->issue.swap(T->blob);
+        T->blob.clear();
         const int o_sets = put(sets.data(), sets.size() * sizeof(uint2));
         const int o_items = put(items.data(), items.size() * 4);
         const int o_lanes = put(lanes.data(), lanes.size() * 4);
@@ -520,15 +525,11 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
         }
         if (slots == 0)
             continue;
-        g.reg_steps = tab.size() == 1 && (int) st.size() <= SH_REG_STEPS ? (int) st.size() : 0;
         g.a_slots = slots;
-        g.so_steps = g.so_a + 16 * g.a_slot16 * slots;
-        g.so_groups = g.so_steps + o_groups - o_steps;
-        g.so_rows = g.so_steps + o_rows;
-        g.so_sets = g.so_steps + o_sets;
-        g.so_items = g.so_steps + o_items;
-        g.so_lanes = g.so_steps + o_lanes;
-        g.so_bars = g.so_steps + g.tab_bytes;
+        g.so_sets = g.so_a + 16 * g.a_slot16 * slots;
+        g.so_items = g.so_sets + o_items - o_sets;
+        g.so_lanes = g.so_sets + o_lanes - o_sets;
+        g.so_bars = g.so_sets + g.tab_bytes;
         T->smem = (size_t) g.so_bars + bars + 128;
         g.nsteps = (int) st.size();
         g.ngroups = (int) groups.size();
@@ -686,10 +687,12 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
     int left = 24, found = 0;
     for (const Try& t : tries)
     {
-        if (left-- == 0 || found == 4 || (found > 0 && t.cost >= out->cost))
+        if (left == 0 || found == 4 || (found > 0 && t.cost >= out->cost))
             break;
         ShTables T;
-        if (layout(t, &T) && finish(t, &T))
+        const bool fits = layout(t, &T) && finish(t, &T);
+        left -= !T.too_long; // (lower columns have shorter tables)
+        if (fits)
         {
             T.cost = clocks(T.g, t.mma, T.g.teams);
             T.chain = T.g.nsets == 1 ? chain_of(m_parts * (m_parts + 1) / 2 * T.g.cpg / m_ch * m_w.most(), 1, T.g.cgroups)

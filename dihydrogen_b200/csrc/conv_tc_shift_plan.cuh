@@ -65,7 +65,9 @@ struct ShTables
     size_t smem;
     double cost;
     int chain;                       // longest chain of leading products in one accumulator
-    std::vector<uint8_t> blob;       // what the kernel copies to shared memory
+    std::vector<uint8_t> issue;      // issuers' tables
+    bool too_long = false;           // they would not fit
+    std::vector<uint8_t> blob;       // the other roles' tables, which the kernel copies to shared memory
     std::vector<ShPack> packs;       // filter images
     std::vector<ShChunk> chunks;
     std::vector<int> codes;
