@@ -100,7 +100,7 @@ struct ShGeom
     int nb, kcols, kgroups;  // columns per cell block, filters per group
     int blk, rowst, woff, nsets, set_off; // columns: block, row of blocks, cell parity along W, set
     int cpg, cgroups;        // channels per group (a multiple of the cell's)
-    int pt;                  // positions per plane of the A slot
+    int pt, used;            // positions per plane of the A slot, those that items write
     int ipr;                 // items (32 positions, all cells of the channel group) of a staged row
     int a_slot16, a_slots;
     int teams;               // converter teams; a_slots is a multiple of it and of SH_ISS
@@ -595,27 +595,31 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
     const bool is_conv = warp >= SH_EPI && (warp & 3) != 3;
     const int conv_w = turn_w * 3 + (warp & 3), iss_w = turn_w;
 
-    if (tid == 0)
+    // A small layer is one pass through this set-up: a thread per barrier (64 blocks at most)
+    static_assert(SH_MAX_SLOTS <= 32 && SH_MAX_BLOCKS <= 64, "a warp's lanes");
+    if (warp == 1)
     {
-#pragma unroll 1
-        for (int s = 0; s < g.a_slots; ++s)
+        if (lane < g.a_slots)
         {
-            mbar_init(&a_full[s], (uint32_t) g.ipr);
-            mbar_init(&a_empty[s], 1);
+            mbar_init(&a_full[lane], (uint32_t) g.ipr);
+            mbar_init(&a_empty[lane], 1);
         }
-        for (int s = 0; s < 2; ++s)
+        if (lane < 2)
         {
-            mbar_init(&b_full[s], 1);
-            mbar_init(&b_empty[s], SH_ISS);
+            mbar_init(&b_full[lane], 1);
+            mbar_init(&b_empty[lane], SH_ISS);
         }
 #pragma unroll 1
-        for (int b = 0; b < g.th * g.ns; ++b)
+        for (int b = lane; b < g.th * g.ns; b += 32)
         {
             mbar_init(&ev_full[b], SH_ISS);
             mbar_init(&ev_empty[b], 4);
         }
-        *abort_flag = 0;
-        abort_flag[1] = 0; // an output that is no number
+        if (lane == 0)
+        {
+            *abort_flag = 0;
+            abort_flag[1] = 0; // an output that is no number
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0)
@@ -630,17 +634,19 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         reinterpret_cast<uint4*>(smem + g.so_sets)[i] = reinterpret_cast<const uint4*>(tables)[i];
     // positions that no item writes are read by the MMAs of lanes nobody stores: keep them finite
 #pragma unroll 1
-    for (int i = tid; i < g.a_slots * g.a_slot16; i += SH_THREADS)
-        reinterpret_cast<uint4*>(smem + g.so_a)[i] = make_uint4(0, 0, 0, 0);
+    for (int plane = warp; plane < g.a_slots * g.a_slot16 / g.pt; plane += SH_THREADS / 32)
+#pragma unroll 1
+        for (int i = g.used + lane; i < g.pt; i += 32)
+            reinterpret_cast<uint4*>(smem + g.so_a)[plane * g.pt + i] = make_uint4(0, 0, 0, 0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (warp < 4)
+    if (warp < SH_EPI)
 #pragma unroll 1
-        for (uint32_t c = 0; c < TC_TMEM_COLS; c += 16)
-            sh_tmem_zero(tmem_base + ((uint32_t) (warp * 32) << 16) + c, 16);
+        for (int c = (warp >> 2) * 16; c < g.set_off * g.nsets; c += 32)
+            sh_tmem_zero(tmem_base + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) c, 16);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     tc_fence_before();
     __syncthreads();
