@@ -273,21 +273,10 @@ __global__ void __launch_bounds__(HALO_THREADS) halo_kernel(HaloArgs a)
 
     if (MODE == MODE_PACK && j.flag != nullptr)
     {
-        // Publish: the block's peer stores become visible system-wide (the barrier
-        // orders them before the first thread's fence), then the last block to
-        // arrive release-stores the epoch.
+        // Publish: the last block to arrive release-stores the epoch.
         __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            __threadfence_system();
-            const unsigned prev = atomicAdd(j.ticket, 1u);
-            if (prev == gridDim.x - 1)
-            {
-                __threadfence_system();
-                *j.ticket = 0;
-                st_release_sys(j.flag, j.epoch);
-            }
-        }
+        if (threadIdx.x == 0 && last_block(j.ticket, gridDim.x))
+            st_release_sys(j.flag, j.epoch);
     }
 }
 

@@ -184,22 +184,11 @@ __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
     }
     if (PUT)
     {
-        // the block's peer stores become visible system-wide (the barrier orders them
-        // before the first thread's fence), then the last block to arrive
-        // release-stores the epoch at every destination
+        // the last block to arrive release-stores the epoch at every destination
         __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            __threadfence_system();
-            const unsigned prev = atomicAdd(a.ticket, 1u);
-            if (prev == gridDim.x - 1)
-            {
-                __threadfence_system();
-                *a.ticket = 0;
-                for (int q = 0; q < a.njobs; ++q)
-                    st_release_sys(a.jobs[q].flag, a.epoch);
-            }
-        }
+        if (threadIdx.x == 0 && last_block(a.ticket, gridDim.x))
+            for (int q = 0; q < a.njobs; ++q)
+                st_release_sys(a.jobs[q].flag, a.epoch);
     }
 }
 
