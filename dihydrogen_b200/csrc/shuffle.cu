@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "dcb.h"
 
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -30,11 +31,34 @@ namespace
 {
 
 constexpr int SHF_THREADS = 256;
-constexpr int SHF_UNROLL = 4;                           // accesses of a thread in flight
-constexpr int SHF_CHUNK = SHF_THREADS * SHF_UNROLL;     // accesses of a unit
+// Accesses of a thread in flight: 4, and 2 pieces, which are up to four loads each (us there and
+// back, 2 ranks, with 4 and with 2: aligned rows 2 x 16 x 128^3 392 and 441, 2 x 16 x 206 x 32 x 120
+// 175 and 204; in pieces 2 x 16 x 56 x 189 x 38 166 and 141, 2 x 16 x 77 x 91 x 45 203 and 153).
+template <int WAY>
+constexpr int shf_unroll = WAY == 2 ? 2 : 4;
 constexpr long long SHF_MAX_CELLS = 2000000000ll;
 constexpr int SHF_MAX_RANKS = 64;
 constexpr size_t SHF_HEADER = 1024; // 64 flags, ticket, status
+
+// How a job's cells are moved: one by one, by four where everything is a multiple of 16 bytes,
+// or in the pieces that lie on 16-byte boundaries of the destination: loads as wide as
+// the source allows, one 16-byte store, a place decoded once for four cells (two ranks, there and
+// back, one by one / in pieces: 2 x 16 x 56 x 189 x 38 split along H 260 / 141 us, 2 x 4 x 232 x 69
+// x 60 along W 189 / 128).
+enum ShfAccess : int
+{
+    SHF_CELL = 0,
+    SHF_VEC = 1,
+    SHF_PIECE = 2
+};
+// Runs of fewer cells go one by one: a piece is a slot of a thread, and a run of L cells has
+// up to (L + 6) / 4 of them.
+constexpr long long SHF_PIECE_MIN = 6;
+
+__host__ __device__ __forceinline__ int shf_way(int vec, long long len, int aligned)
+{
+    return vec && aligned ? SHF_VEC : (len >= SHF_PIECE_MIN ? SHF_PIECE : SHF_CELL);
+}
 
 // One box to move: `rows` runs of `len` contiguous cells.  Dimensions that are
 // contiguous on both sides have been merged into the run.  Row r decodes into
@@ -51,10 +75,10 @@ struct ShfJob
     long long parity_pitch; // put: floats between the two halves of that window
     uint32_t* flag;         // put: flag to publish there; wait: own flag to wait on
     int vec;                // 16-byte accesses: offsets, strides and run allow them (if the bases do)
-    int split;              // long runs, in units of SHF_CHUNK accesses of one run; else units of that many accesses
-    long long units[2];     // per access width (4-byte, 16-byte)
-    long long per_run[2];   // accesses of a run
-    FastDiv by_run[2], by_ext[4];
+    int split;              // long runs, a unit's accesses of one run; else of the job
+    long long units[3];     // per way of access (ShfAccess)
+    long long per_run[3];   // accesses of a run
+    FastDiv by_run[3], by_ext[4];
 };
 
 struct ShfArgs
@@ -71,74 +95,148 @@ struct ShfArgs
     long long budget_ns;
 };
 
-template <class T>
-__device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, int wide, const float* from, float* to,
-                                         const long long* fs, const long long* ts, long long fo, long long to_off)
+// Where access n of a job is (or, split, access e0 of run r onwards): its run's first cells.
+struct ShfRun
 {
-    constexpr int W = sizeof(T) / 4;
-    T v[SHF_UNROLL];
-    T* dst[SHF_UNROLL];
-    if (j.split)
-    {
-        // SHF_CHUNK accesses of one long run
-        const long long cpr = (j.per_run[wide] + SHF_CHUNK - 1) / SHF_CHUNK;
-        long long r = u / cpr;
-        const long long e0 = (u - r * cpr) * SHF_CHUNK;
-        long long f = fo, t = to_off;
+    const float* from;
+    float* to;
+};
+
+__device__ __forceinline__ ShfRun shf_run(const ShfJob& j, uint32_t r, const float* from, float* to, const long long* fs,
+                                          const long long* ts)
+{
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+    for (int q = 0; q < 4; ++q)
+    {
+        const uint32_t d = j.by_ext[q].div(r), i = r - d * j.by_ext[q].d;
+        r = d;
+        from += (long long) i * fs[q];
+        to += (long long) i * ts[q];
+    }
+    return {from, to};
+}
+
+// Piece q of a run: up to four cells, from the 16-byte boundary of the destination that is q
+// pieces above the one at or below the run's first cell.  Loads, then (put) the stores.
+struct ShfPiece
+{
+    float v[4];
+    float* to;
+    int lo, hi; // cells lo .. hi - 1 of the piece exist
+
+    __device__ __forceinline__ void get(const ShfRun& run, long long q, long long len)
+    {
+        const int head = (int) (reinterpret_cast<uintptr_t>(run.to) >> 2 & 3);
+        const long long e = 4 * q - head;
+        const float* from = run.from + e;
+        to = run.to + e;
+        lo = e < 0 ? head : 0;
+        hi = len - e < 4 ? (int) (len - e > 0 ? len - e : 0) : 4;
+        if (lo == 0 && hi == 4)
         {
-            const long long i = r % j.ext[k];
-            r /= j.ext[k];
-            f += i * fs[k];
-            t += i * ts[k];
+            const int at = (int) (reinterpret_cast<uintptr_t>(from) >> 2 & 3);
+            if (at == 0)
+            {
+                const float4 f = __ldcs(reinterpret_cast<const float4*>(from));
+                v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+                return;
+            }
+            if (at == 2)
+            {
+                const float2 f = __ldcs(reinterpret_cast<const float2*>(from)), h = __ldcs(reinterpret_cast<const float2*>(from) + 1);
+                v[0] = f.x, v[1] = f.y, v[2] = h.x, v[3] = h.y;
+                return;
+            }
+        }
+        // (cached: the lanes' cells of one load share sectors with those of the next)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i >= lo && i < hi)
+                v[i] = from[i];
+    }
+    __device__ __forceinline__ void none() { lo = hi = 0; }
+    __device__ __forceinline__ void put() const
+    {
+        if (lo == 0 && hi == 4)
+        {
+            *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+            return;
         }
 #pragma unroll
-        for (int k = 0; k < SHF_UNROLL; ++k)
+        for (int i = 0; i < 4; ++i)
+            if (i >= lo && i < hi)
+                to[i] = v[i];
+    }
+};
+
+template <class T>
+struct ShfCell
+{
+    T v;
+    T* to;
+    __device__ __forceinline__ void get(const ShfRun& run, long long e, long long)
+    {
+        to = reinterpret_cast<T*>(run.to) + e;
+        v = __ldcs(reinterpret_cast<const T*>(run.from) + e);
+    }
+    __device__ __forceinline__ void none() { to = nullptr; }
+    __device__ __forceinline__ void put() const
+    {
+        if (to != nullptr)
+            *to = v;
+    }
+};
+
+template <int WAY, class T>
+__device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, const float* from, float* to, const long long* fs,
+                                         const long long* ts)
+{
+    T a[shf_unroll<WAY>];
+    constexpr int CHUNK = SHF_THREADS * shf_unroll<WAY>; // accesses of a unit
+    if (j.split)
+    {
+        // CHUNK accesses of one long run
+        const long long cpr = (j.per_run[WAY] + CHUNK - 1) / CHUNK;
+        const long long r = u / cpr, e0 = (u - r * cpr) * CHUNK;
+        const ShfRun run = shf_run(j, (uint32_t) r, from, to, fs, ts);
+#pragma unroll
+        for (int k = 0; k < shf_unroll<WAY>; ++k)
         {
             const long long e = e0 + threadIdx.x + k * SHF_THREADS;
-            dst[k] = e < j.per_run[wide] ? reinterpret_cast<T*>(to + t) + e : nullptr;
-            if (dst[k] != nullptr)
-                v[k] = __ldcs(reinterpret_cast<const T*>(from + f) + e);
+            if (e < j.per_run[WAY])
+                a[k].get(run, e, j.len);
+            else
+                a[k].none();
         }
     }
     else
     {
-        const long long total = j.rows * j.per_run[wide];
+        const long long total = j.rows * j.per_run[WAY];
 #pragma unroll
-        for (int k = 0; k < SHF_UNROLL; ++k)
+        for (int k = 0; k < shf_unroll<WAY>; ++k)
         {
-            const long long n = u * SHF_CHUNK + threadIdx.x + k * SHF_THREADS;
-            dst[k] = nullptr;
+            const long long n = u * CHUNK + threadIdx.x + k * SHF_THREADS;
             if (n < total)
             {
-                uint32_t r = j.by_run[wide].div((uint32_t) n);
-                const uint32_t e = (uint32_t) n - r * j.by_run[wide].d;
-                long long f = fo + (long long) e * W, t = to_off + (long long) e * W;
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                {
-                    const uint32_t d = j.by_ext[q].div(r), i = r - d * j.by_ext[q].d;
-                    r = d;
-                    f += (long long) i * fs[q];
-                    t += (long long) i * ts[q];
-                }
-                dst[k] = reinterpret_cast<T*>(to + t);
-                v[k] = __ldcs(reinterpret_cast<const T*>(from + f));
+                const uint32_t r = j.by_run[WAY].div((uint32_t) n);
+                a[k].get(shf_run(j, r, from, to, fs, ts), (uint32_t) n - r * j.by_run[WAY].d, j.len);
             }
+            else
+                a[k].none();
         }
     }
 #pragma unroll
-    for (int k = 0; k < SHF_UNROLL; ++k)
-        if (dst[k] != nullptr)
-            *dst[k] = v[k];
+    for (int k = 0; k < shf_unroll<WAY>; ++k)
+        a[k].put();
 }
 
 // PUT: tensor (strided) -> peers' windows (dense).  !PUT: own window -> tensor.
-// A unit is SHF_CHUNK accesses, all loads of a thread before its stores.  A warp per
+// A unit is SHF_THREADS x shf_unroll accesses, all loads of a thread before its stores.  A warp per
 // W run, decoded with eight run-time divisions and one access in flight per lane, took
 // 100 us for 134 MB.
-template <bool PUT>
+// PIECES: some job of the call takes them (a kernel of its own: with their registers the others took
+// 5 us more of 50).
+template <bool PUT, bool PIECES>
 __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
 {
     if (!PUT)
@@ -166,21 +264,22 @@ __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
         for (int i = threadIdx.x; i < (int) (sizeof(ShfJob) / 4); i += SHF_THREADS)
             reinterpret_cast<uint32_t*>(&j)[i] = reinterpret_cast<const uint32_t*>(&a.jobs[q])[i];
         __syncthreads();
-        const int wide = j.vec && a.aligned ? 1 : 0;
+        const int way = shf_way(j.vec, j.len, a.aligned);
         float* w = PUT ? j.peer + a.parity * j.parity_pitch : a.window;
-        const float* from = PUT ? a.tensor : w;
-        float* to = PUT ? w : a.tensor;
         const long long* fs = PUT ? j.a_stride : j.b_stride;
         const long long* ts = PUT ? j.b_stride : j.a_stride;
-        const long long fo = PUT ? j.a_off : j.b_off, too = PUT ? j.b_off : j.a_off;
-        for (; u < j.units[wide]; u += gridDim.x)
+        const float* from = (PUT ? a.tensor : w) + (PUT ? j.a_off : j.b_off);
+        float* to = (PUT ? w : a.tensor) + (PUT ? j.b_off : j.a_off);
+        for (; u < j.units[way]; u += gridDim.x)
         {
-            if (wide)
-                shf_unit<float4>(j, u, 1, from, to, fs, ts, fo, too);
+            if (way == SHF_VEC)
+                shf_unit<SHF_VEC, ShfCell<float4>>(j, u, from, to, fs, ts);
+            else if (PIECES && way == SHF_PIECE)
+                shf_unit<SHF_PIECE, ShfPiece>(j, u, from, to, fs, ts);
             else
-                shf_unit<float>(j, u, 0, from, to, fs, ts, fo, too);
+                shf_unit<SHF_CELL, ShfCell<float>>(j, u, from, to, fs, ts);
         }
-        u -= j.units[wide];
+        u -= j.units[way];
     }
     if (PUT)
     {
@@ -230,13 +329,13 @@ void finish_job(ShfJob* j)
     }
     j->vec = (mix & 3) == 0;
     // runs of at least two units, or (one run) too many accesses for 31-bit indices
-    j->split = j->len / (j->vec ? 4 : 1) >= 2 * SHF_CHUNK || j->rows * j->len >= SHF_MAX_CELLS;
-    for (int w = 0; w < 2; ++w)
+    j->split = j->len / (j->vec ? 4 : 1) >= 2 * SHF_THREADS * shf_unroll<SHF_VEC> || j->rows * j->len >= SHF_MAX_CELLS;
+    for (int w = 0; w < 3; ++w)
     {
-        j->per_run[w] = j->len / (w ? 4 : 1);
+        j->per_run[w] = w == SHF_PIECE ? (j->len + 6) / 4 : j->len / (w == SHF_VEC ? 4 : 1);
         j->by_run[w] = FastDiv::of(j->per_run[w] > 0 && j->per_run[w] < (1 << 30) ? (uint32_t) j->per_run[w] : 1u);
-        j->units[w] = j->split ? j->rows * ((j->per_run[w] + SHF_CHUNK - 1) / SHF_CHUNK)
-                               : (j->rows * j->per_run[w] + SHF_CHUNK - 1) / SHF_CHUNK;
+        const long long chunk = SHF_THREADS * (w == SHF_PIECE ? shf_unroll<SHF_PIECE> : shf_unroll<SHF_VEC>);
+        j->units[w] = j->split ? j->rows * ((j->per_run[w] + chunk - 1) / chunk) : (j->rows * j->per_run[w] + chunk - 1) / chunk;
     }
 }
 
@@ -266,7 +365,7 @@ void add_jobs(ShfJob j, std::vector<ShfJob>* out, long long* units)
     }
     finish_job(&j);
     out->push_back(j);
-    *units += j.units[j.vec];
+    *units += j.units[shf_way(j.vec, j.len, 1)];
 }
 
 struct ShfBlob
@@ -333,6 +432,7 @@ struct dcb_shuffle_plan
     ShfJob* d_wait = nullptr;
     int n_put = 0, n_wait = 0;
     long long put_units = 0, wait_units = 0;
+    bool put_pieces[2] = {}, wait_pieces[2] = {}; // whether a job takes pieces; by whether the tensor is 16-byte aligned
     uint32_t epoch = 0;
     bool connected = false;
 
@@ -535,6 +635,12 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
     cudaFree(p->d_put);
     cudaFree(p->d_wait);
     p->d_put = p->d_wait = nullptr;
+    for (int aligned = 0; aligned < 2; ++aligned)
+    {
+        auto pieces = [&](const ShfJob& j) { return shf_way(j.vec, j.len, aligned) == SHF_PIECE; };
+        p->put_pieces[aligned] = std::any_of(put.begin(), put.end(), pieces);
+        p->wait_pieces[aligned] = std::any_of(wait.begin(), wait.end(), pieces);
+    }
     p->n_put = (int) put.size();
     p->n_wait = (int) wait.size();
     if (p->n_put)
@@ -580,7 +686,8 @@ int32_t dcb_shuffle_put(dcb_shuffle_plan* p, const void* src, void* stream)
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    shuffle_kernel<true><<<shf_grid(p->put_units), SHF_THREADS, 0, as_stream(stream)>>>(a);
+    (p->put_pieces[a.aligned] ? shuffle_kernel<true, true> : shuffle_kernel<true, false>)<<<shf_grid(p->put_units), SHF_THREADS, 0,
+                                                                                        as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;
 }
@@ -607,7 +714,8 @@ int32_t dcb_shuffle_wait_unpack(dcb_shuffle_plan* p, void* dst, void* stream)
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    shuffle_kernel<false><<<shf_grid(p->wait_units), SHF_THREADS, 0, as_stream(stream)>>>(a);
+    (p->wait_pieces[a.aligned] ? shuffle_kernel<false, true> : shuffle_kernel<false, false>)<<<shf_grid(p->wait_units),
+                                                                                           SHF_THREADS, 0, as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;
 }

@@ -67,6 +67,23 @@ def test_forward_and_backward(shape, sgrid, dgrid, dov):
     assert all(sh.status("fwd") == _abi.OK and sh.status("bwd") == _abi.OK for sh in shufflers)
 
 
+@pytest.mark.parametrize("shape,sgrid,dgrid,dov", [
+    # runs of 5 and 6 cells: cell by cell and, from 6 on, in pieces
+    ([11, 5, 4, 3, 2], [1, 1, 1, 1, 2], [2, 1, 1, 1, 1], [0, 0, 0, 0, 0]),
+    # ... with a halo along W, where rows start 1 to 3 cells off a boundary
+    ([13, 6, 4, 2, 2], [1, 1, 1, 1, 2], [2, 1, 1, 1, 1], [1, 0, 0, 0, 0]),
+    ([14, 6, 4, 2, 2], [1, 1, 1, 1, 2], [2, 1, 1, 1, 1], [2, 1, 0, 0, 0]),
+    # merged rows of odd length, split in H
+    ([13, 11, 9, 3, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 0, 0, 0, 0]),
+    ([10, 9, 5, 3, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 1, 0, 0, 0]),
+    # whole odd planes: runs of several units, in pieces
+    ([97, 91, 3, 2, 2], [1, 1, 1, 1, 2], [1, 1, 2, 1, 1], [0, 0, 0, 0, 0]),
+    ([98, 91, 3, 1, 2], [1, 1, 1, 1, 2], [1, 1, 2, 1, 1], [0, 0, 1, 0, 0]),
+])
+def test_runs_off_16_byte_boundaries(shape, sgrid, dgrid, dov):
+    test_forward_and_backward(shape, sgrid, dgrid, dov)
+
+
 def test_wait_expires_with_status_when_a_sender_never_comes():
     """A rank whose peer never puts gets DCB_PEER_TIMEOUT from the bounded wait,
     not a hang, and the destination stays as it was."""
