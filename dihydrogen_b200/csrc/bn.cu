@@ -186,6 +186,23 @@ struct Vec<4>
     }
 };
 
+// Long runs whose starts are not 16-byte aligned (planes of odd size): the reductions read them
+// in the aligned pieces of four that they lie in, all tensors of a call alike (pieces_fit).  Piece
+// q of a run that starts `head` floats above a boundary is its elements 4 q - head onwards; those
+// at the run's ends have fewer than four.
+struct Piece
+{
+    long long e;
+    int lo, hi; // of the piece's elements, those of the run
+    __device__ __forceinline__ Piece(long long q, int head, long long len)
+    {
+        e = 4 * q - head;
+        lo = e < 0 ? head : 0;
+        hi = len - e < 4 ? (int) (len - e > 0 ? len - e : 0) : 4;
+    }
+    __device__ __forceinline__ bool whole() const { return lo == 0 && hi == 4; }
+};
+
 // Sum NV doubles across the block; result valid in thread 0.
 template <int NV>
 __device__ __forceinline__ void block_reduce(double (&val)[NV])
@@ -265,7 +282,7 @@ __device__ __forceinline__ void finish_channel(double (&val)[NV],
     }
 }
 
-template <int V, bool PACKED>
+template <int V, bool PACKED, bool PIECES = false>
 __global__ void __launch_bounds__(BN_THREADS)
     bn_stats_kernel(const float* __restrict__ x, RunStrides xs, UnitGeom ug,
                     double* partial, unsigned* tickets,
@@ -281,17 +298,35 @@ __global__ void __launch_bounds__(BN_THREADS)
         const int nv = p.count / V;
         Vec<V> v[bn_unroll_red<V>];
         bool on[bn_unroll_red<V>];
+        float s = 0.f, q = 0.f;
+        const float* run = xp - p.e0;
+        const int head = (int) (reinterpret_cast<uintptr_t>(run) >> 2 & 3);
 #pragma unroll
         for (int k = 0; k < bn_unroll_red<V>; ++k)
         {
+            if (PIECES)
+            {
+                const Piece pc(p.e0 / 4 + threadIdx.x + k * BN_THREADS, head, ug.g.len);
+                on[k] = pc.whole();
+                if (on[k])
+                    v[k].load(run + pc.e);
+                else
+                    for (int i = pc.lo; i < pc.hi; ++i)
+                    {
+                        const float f = run[pc.e + i];
+                        s += f;
+                        q = fmaf(f, f, q);
+                    }
+                continue;
+            }
             const ElemPos ep = elem_pos<PACKED>(ug, p, threadIdx.x + k * BN_THREADS, nv);
             on[k] = ep.on;
             if (on[k])
                 v[k].load(xp + ep.template off<V>(xs));
         }
-        float s = 0.f, q = 0.f;
 #pragma unroll
         for (int k = 0; k < bn_unroll_red<V>; ++k)
+        {
             if (on[k])
 #pragma unroll
                 for (int i = 0; i < V; ++i)
@@ -299,6 +334,14 @@ __global__ void __launch_bounds__(BN_THREADS)
                     s += v[k].v[i];
                     q = fmaf(v[k].v[i], v[k].v[i], q);
                 }
+            if (PIECES && k == bn_unroll_red<V> / 2 - 1)
+            {
+                // (sums of sixteen in fp32, as element by element)
+                acc[0] += (double) s;
+                acc[1] += (double) q;
+                s = q = 0.f;
+            }
+        }
         acc[0] += (double) s;
         acc[1] += (double) q;
     }
@@ -442,7 +485,7 @@ __global__ void __launch_bounds__(BN_THREADS)
     }
 }
 
-template <int V, bool PACKED>
+template <int V, bool PACKED, bool PIECES = false>
 __global__ void __launch_bounds__(BN_THREADS)
     bn_bwd_reduce_kernel(const float* __restrict__ x, RunStrides xs,
                          const float* __restrict__ dy, RunStrides ds,
@@ -468,9 +511,35 @@ __global__ void __launch_bounds__(BN_THREADS)
         const int nv = p.count / V;
         Vec<V> vx[bn_unroll_red<V>], vd[bn_unroll_red<V>];
         bool on[bn_unroll_red<V>];
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+        auto add = [&](float xv, float g) {
+            // backprop1 (batchnorm.cu:940-952)
+            const float xhat = (xv - m) * inv_stdev;
+            a0 += g * xhat;
+            a1 += g;
+            const float dxhat = g * sc;
+            a2 += -dxhat * inv_stdev;
+            a3 += -dxhat * (xv - m) * dvar_factor;
+        };
+        const float *xrun = xp - p.e0, *drun = dp - p.e0;
+        const int head = (int) (reinterpret_cast<uintptr_t>(xrun) >> 2 & 3);
 #pragma unroll
         for (int k = 0; k < bn_unroll_red<V>; ++k)
         {
+            if (PIECES)
+            {
+                const Piece pc(p.e0 / 4 + threadIdx.x + k * BN_THREADS, head, ug.g.len);
+                on[k] = pc.whole();
+                if (on[k])
+                {
+                    vx[k].load(xrun + pc.e);
+                    vd[k].load(drun + pc.e);
+                }
+                else
+                    for (int i = pc.lo; i < pc.hi; ++i)
+                        add(xrun[pc.e + i], drun[pc.e + i]);
+                continue;
+            }
             const ElemPos ep = elem_pos<PACKED>(ug, p, threadIdx.x + k * BN_THREADS, nv);
             on[k] = ep.on;
             if (on[k])
@@ -479,22 +548,22 @@ __global__ void __launch_bounds__(BN_THREADS)
                 vd[k].load(dp + ep.template off<V>(ds));
             }
         }
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll
         for (int k = 0; k < bn_unroll_red<V>; ++k)
+        {
             if (on[k])
 #pragma unroll
                 for (int i = 0; i < V; ++i)
-                {
-                    // backprop1 (batchnorm.cu:940-952)
-                    const float xv = vx[k].v[i], g = vd[k].v[i];
-                    const float xhat = (xv - m) * inv_stdev;
-                    a0 += g * xhat;
-                    a1 += g;
-                    const float dxhat = g * sc;
-                    a2 += -dxhat * inv_stdev;
-                    a3 += -dxhat * (xv - m) * dvar_factor;
-                }
+                    add(vx[k].v[i], vd[k].v[i]);
+            if (PIECES && k == bn_unroll_red<V> / 2 - 1)
+            {
+                acc[0] += (double) a0;
+                acc[1] += (double) a1;
+                acc[2] += (double) a2;
+                acc[3] += (double) a3;
+                a0 = a1 = a2 = a3 = 0.f;
+            }
+        }
         acc[0] += (double) a0;
         acc[1] += (double) a1;
         acc[2] += (double) a2;
@@ -624,10 +693,26 @@ struct MultiView
     UnitGeom ug;
     RunStrides s[3];
     int vec;
+    bool pieces; // reductions: aligned pieces of four (see Piece), in units of 16-byte vectors
 };
 
+// Whether all tensors' runs start equally far above a 16-byte boundary.
+static bool pieces_fit(const MultiView& mv, const void* const* ptrs, int count)
+{
+    const RunStrides& a = mv.s[0];
+    for (int i = 1; i < count; ++i)
+    {
+        const RunStrides& b = mv.s[i];
+        const long long differ = (a.sn - b.sn) | (a.sc - b.sc) | (a.s_inner - b.s_inner) | (a.s_outer - b.s_outer);
+        if ((differ & 3) != 0 || ((reinterpret_cast<uintptr_t>(ptrs[0]) ^ reinterpret_cast<uintptr_t>(ptrs[i])) & 15) != 0)
+            return false;
+    }
+    return true;
+}
+
 static int32_t make_multi(const dcb_nd_desc* const* descs,
-                          const void* const* ptrs, int count, MultiView* mv, int unroll, int unroll1)
+                          const void* const* ptrs, int count, MultiView* mv, int unroll, int unroll1,
+                          bool reduction = false)
 {
     int level = 2;
     for (int i = 0; i < count; ++i)
@@ -655,6 +740,15 @@ static int32_t make_multi(const dcb_nd_desc* const* descs,
     }
     mv->ug = make_units(g, vec, vec == 1 ? unroll1 : unroll);
     mv->vec = vec;
+    // Shorter runs are mostly their partial ends.  2 x 24 x 67 x 83 x 101, element by element / in
+    // pieces: statistics 31.4 / 22.2 us, backward sums 53.6 / 51.0.
+    mv->pieces = reduction && vec == 1 && mv->ug.vpr == 0 && g.len >= 1024 && pieces_fit(*mv, ptrs, count);
+    if (mv->pieces)
+    {
+        mv->ug.unit = BN_THREADS * unroll * 4;
+        mv->ug.upr = ((g.len + 6) / 4 + BN_THREADS * unroll - 1) / (BN_THREADS * unroll);
+        mv->ug.upc = g.n * g.rows * mv->ug.upr;
+    }
     DCB_REQUIRE(g.c <= 65535, "too many channels");
     return DCB_OK;
 }
@@ -752,7 +846,7 @@ int32_t dcb_bn_stats(dcb_bn_plan* plan, const void* x, void* sums,
     const dcb_nd_desc* descs[1] = {&plan->xd};
     const void* ptrs[1] = {x};
     MultiView mv;
-    int32_t st = make_multi(descs, ptrs, 1, &mv, BN_UNROLL_RED, bn_unroll_red<1>);
+    int32_t st = make_multi(descs, ptrs, 1, &mv, BN_UNROLL_RED, bn_unroll_red<1>, true);
     if (st != DCB_OK)
         return st;
     if (mv.ug.upc == 0)
@@ -764,11 +858,16 @@ int32_t dcb_bn_stats(dcb_bn_plan* plan, const void* x, void* sums,
         return DCB_OK;
     }
     const dim3 grid = bn_grid(mv.ug);
-#define CALL(VV, PP)                                                               \
-    DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),           \
+#define CALL(VV, ...)                                                               \
+    DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, __VA_ARGS__>), grid, BN_THREADS, 0, as_stream(stream),           \
         static_cast<const float*>(x), mv.s[0], mv.ug, plan->partial,           \
         plan->tickets, static_cast<float*>(sums), static_cast<float*>(sqsums)))
-    DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
+    if (mv.pieces)
+    {
+        CALL(4, false, true);
+    }
+    else
+        DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
     return DCB_OK;
@@ -872,7 +971,7 @@ int32_t dcb_bn_bwd_reduce(dcb_bn_plan* plan, const void* x,
     const dcb_nd_desc* descs[2] = {&plan->xd, dyd};
     const void* ptrs[2] = {x, dy};
     MultiView mv;
-    int32_t st = make_multi(descs, ptrs, 2, &mv, BN_UNROLL_RED, bn_unroll_red<1>);
+    int32_t st = make_multi(descs, ptrs, 2, &mv, BN_UNROLL_RED, bn_unroll_red<1>, true);
     if (st != DCB_OK)
         return st;
     if (mv.ug.upc == 0)
@@ -883,15 +982,20 @@ int32_t dcb_bn_bwd_reduce(dcb_bn_plan* plan, const void* x,
         return DCB_OK;
     }
     const dim3 grid = bn_grid(mv.ug);
-#define CALL(VV, PP)                                                               \
-    DCB_CUDA_TRY(launch_overlapped((bn_bwd_reduce_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),      \
+#define CALL(VV, ...)                                                               \
+    DCB_CUDA_TRY(launch_overlapped((bn_bwd_reduce_kernel<VV, __VA_ARGS__>), grid, BN_THREADS, 0, as_stream(stream),      \
         static_cast<const float*>(x), mv.s[0], static_cast<const float*>(dy),  \
         mv.s[1], mv.ug, static_cast<const float*>(mean),                       \
         static_cast<const float*>(var), static_cast<const float*>(scale), eps, \
         plan->partial, plan->tickets, static_cast<float*>(dscale),             \
         static_cast<float*>(dbias), static_cast<float*>(dmean),                \
         static_cast<float*>(dvar)))
-    DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
+    if (mv.pieces)
+    {
+        CALL(4, false, true);
+    }
+    else
+        DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
     return DCB_OK;
@@ -1014,7 +1118,7 @@ extern "C" int32_t dcb_bn_stats_noalloc(const dcb_nd_desc* xd, const void* x, vo
     const dcb_nd_desc* descs[1] = {xd};
     const void* ptrs[1] = {x};
     MultiView mv;
-    int32_t st = make_multi(descs, ptrs, 1, &mv, BN_UNROLL_RED, bn_unroll_red<1>);
+    int32_t st = make_multi(descs, ptrs, 1, &mv, BN_UNROLL_RED, bn_unroll_red<1>, true);
     if (st != DCB_OK)
         return st;
     if (xd->c < 1 || xd->c > NOALLOC_MAX_CHANNELS)
@@ -1057,11 +1161,16 @@ extern "C" int32_t dcb_bn_stats_noalloc(const dcb_nd_desc* xd, const void* x, vo
     // The array keeps whatever the previous call (or an interrupted one) left:
     // the arrival tickets must start at zero.  Partials are overwritten.
     DCB_CUDA_TRY(cudaMemsetAsync(tickets, 0, xd->c * sizeof(unsigned), as_stream(stream)));
-#define CALL(VV, PP)                                                               \
-    DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, PP>), grid, BN_THREADS, 0, as_stream(stream),           \
+#define CALL(VV, ...)                                                               \
+    DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, __VA_ARGS__>), grid, BN_THREADS, 0, as_stream(stream),           \
         static_cast<const float*>(x), mv.s[0], mv.ug, partial, tickets,        \
         static_cast<float*>(sums), static_cast<float*>(sqsums)))
-    DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
+    if (mv.pieces)
+    {
+        CALL(4, false, true);
+    }
+    else
+        DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
 #undef CALL
     DCB_LAUNCH_CHECK();
     return DCB_OK;

@@ -88,6 +88,16 @@ def test_bn_forward_backward_local(shape, locale, overlap):
     emu.assert_close(dx_t.owned().cpu().numpy(), dx_ref, TOL, "dx")
 
 
+@pytest.mark.parametrize("shape", [
+    [41, 25, 1, 3, 2],   # 1025 elements a plane: just long enough for pieces of four, every start
+    [91, 89, 1, 5, 1],   # 8099: the pieces of one unit and its last, partial one
+    [91, 91, 1, 4, 2],   # 8281: a second unit of 22 pieces
+    [67, 83, 3, 2, 2],
+])
+def test_planes_of_odd_size(shape):
+    test_bn_forward_backward_local(shape, [1] * 5, [0] * 5)
+
+
 @pytest.mark.parametrize("shape,overlap", [
     ([1, 1, 2, 1], [0, 0, 0, 0]),                  # one block per channel, two values
     ([33, 7, 5, 3, 2], [0, 0, 0, 0, 0]),
