@@ -59,6 +59,7 @@ class _Geometry:
         self.strides = t.get_strides()
         self.base = 4 * t.get_local_offset([0] * t.nd)
         self.split_root = t.is_split_root()
+        self.owned = tuple(slice(o, o + l) for o, l in reversed(list(zip(self.overlap, self.local))))
         self.descs = {}    # widths -> NdDesc
         self.offsets = {}  # widths -> byte offset of the window
 
@@ -411,8 +412,7 @@ class Tensor:
         return self.buffer.data_ptr() + self._geo().base
 
     def owned(self) -> torch.Tensor:
-        sl = tuple(slice(o, o + l) for o, l in reversed(list(zip(self.dist.overlap, self.local_shape))))
-        return self.buffer[sl]
+        return self.buffer[self._geo().owned]
 
     def zero(self, stream=None):
         _zero_on(stream, self._storage)
