@@ -116,6 +116,20 @@ __device__ __forceinline__ ShfRun shf_run(const ShfJob& j, uint32_t r, const flo
     return {from, to};
 }
 
+// The cells e + lo .. e + hi - 1 of a run that are its piece q, where the run starts `head` cells
+// above a boundary.
+struct ShfRange
+{
+    long long e;
+    int lo, hi;
+};
+
+__host__ __device__ __forceinline__ ShfRange shf_range(int head, long long q, long long len)
+{
+    const long long e = 4 * q - head;
+    return {e, e < 0 ? head : 0, len - e < 4 ? (int) (len - e > 0 ? len - e : 0) : 4};
+}
+
 // Piece q of a run: up to four cells, from the 16-byte boundary of the destination that is q
 // pieces above the one at or below the run's first cell.  Loads, then (put) the stores.
 struct ShfPiece
@@ -126,12 +140,11 @@ struct ShfPiece
 
     __device__ __forceinline__ void get(const ShfRun& run, long long q, long long len)
     {
-        const int head = (int) (reinterpret_cast<uintptr_t>(run.to) >> 2 & 3);
-        const long long e = 4 * q - head;
-        const float* from = run.from + e;
-        to = run.to + e;
-        lo = e < 0 ? head : 0;
-        hi = len - e < 4 ? (int) (len - e > 0 ? len - e : 0) : 4;
+        const ShfRange r = shf_range((int) (reinterpret_cast<uintptr_t>(run.to) >> 2 & 3), q, len);
+        const float* from = run.from + r.e;
+        to = run.to + r.e;
+        lo = r.lo;
+        hi = r.hi;
         if (lo == 0 && hi == 4)
         {
             const int at = (int) (reinterpret_cast<uintptr_t>(from) >> 2 & 3);

@@ -110,3 +110,11 @@ def test_large_redistributions_are_dealt_out_in_pieces(tmp_path):
     for pieces, most, covered, per_unit in lines:
         assert covered and most < 2000000000 and per_unit >= 1000
     assert lines[2][0] == 1
+
+
+def test_pieces_of_unaligned_runs_cover_them_once(tmp_path):
+    exe = compile_check(tmp_path, "shuffle_pieces_check")
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    good, pairs = map(int, r.stdout.split())
+    assert good == pairs > 500
