@@ -88,15 +88,11 @@ __device__ __forceinline__ void pool_split_row(long long row, long long rows, in
 // first maximum (dense [n][c][od][oh][ow]); y may then be null.
 constexpr int POOL_TW = POOL_THREADS;
 
-template <int WD, int W, int S>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_fwd_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ x, float* y,
                     unsigned char* __restrict__ argmax, int tw_log2, long long rows)
 {
-    // window / stride as compile-time constants where the launch found a match
-    // (unrolled loops, shifts for the divisions); 0 = read them from the geometry
-    const int w0_ = WD ? WD : g.win[0], w1_ = W ? W : g.win[1], w2_ = W ? W : g.win[2];
-    const int s0_ = S ? (WD == 1 ? 1 : S) : g.stride[0], s1_ = S ? S : g.stride[1], s2_ = S ? S : g.stride[2];
+    const int w0_ = g.win[0], w1_ = g.win[1], w2_ = g.win[2], s0_ = g.stride[0], s1_ = g.stride[1], s2_ = g.stride[2];
     // a block is 256 >> tw_log2 output rows of (1 << tw_log2) cells: short rows (128
     // outputs of a 256-cell input row) would otherwise leave half the block idle
     const int ow = (blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1));
@@ -110,13 +106,11 @@ __global__ void __launch_bounds__(POOL_THREADS)
     const int kw_lo = max(0, g.lo[2] - w0), kw_hi = min(w2_, g.hi[2] - w0);
     float m = -FLT_MAX, s = 0.f;
     int best = -1;
-#pragma unroll
     for (int kd = 0; kd < w0_; ++kd)
     {
         const int id = d0 + kd;
         if (id < g.lo[0] || id >= g.hi[0])
             continue;
-#pragma unroll
         for (int kh = 0; kh < w1_; ++kh)
         {
             const int ih = h0 + kh;
@@ -124,7 +118,6 @@ __global__ void __launch_bounds__(POOL_THREADS)
                 continue;
             const float* row = xp + (size_t) id * g.xs[0] + (size_t) ih * g.xs[1] + w0;
             const int tap0 = (kd * w1_ + kh) * w2_;
-#pragma unroll
             for (int kw = 0; kw < w2_; ++kw)
             {
                 if (kw < kw_lo || kw >= kw_hi)
@@ -148,6 +141,92 @@ __global__ void __launch_bounds__(POOL_THREADS)
     const float r = g.mode == DCB_POOL_MAX ? m : s / fmaxf(pool_count(g, od, oh, ow), 1.f);
     float* yp = y + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1] + ow;
     *yp = beta != 0.f ? alpha * r + beta * *yp : alpha * r;
+}
+
+// The same for the common windows, four neighbouring outputs a thread: a window row's cells are
+// loaded once for all four and the addresses worked out once.  Same scan order, same bits (us, an
+// output a thread before: 8 x 128^3, 3 / 1, averages 309 -> 140; 16 x 64 x 100 x 90, 2 / 2, maxima
+// 19.6 -> 13.8, 3 / 1 182 -> 174).
+template <int WD, int W, int S, bool MAXP>
+__global__ void __launch_bounds__(POOL_THREADS)
+    pool_fwd_cells_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ x, float* y,
+                          unsigned char* __restrict__ argmax, int tw_log2, long long rows)
+{
+    constexpr int SD = WD == 1 ? 1 : S, NC = 3 * S + W; // cells behind four outputs
+    const int ow0 = ((blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1))) * 4;
+    const long long row = (long long) blockIdx.x * (POOL_THREADS >> tw_log2) + (threadIdx.x >> tw_log2);
+    if (ow0 >= g.out[2] || row >= rows)
+        return;
+    int od, oh;
+    pool_split_row(row, rows, g.out[1], &od, &oh);
+    const int c = blockIdx.z % g.c, n = blockIdx.z / g.c;
+    const int d0 = od * SD - g.pad[0], h0 = oh * S - g.pad[1], w0 = ow0 * S - g.pad[2];
+    const float* xp = x + (size_t) n * g.xs_n + (size_t) c * g.xs_c + (long long) d0 * g.xs[0] + (long long) h0 * g.xs[1] + w0;
+    const bool all = w0 >= g.lo[2] && w0 + NC <= g.hi[2]; // every cell exists
+    float r[4];
+    int best[4];
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+        r[o] = MAXP ? -FLT_MAX : 0.f, best[o] = -1;
+#pragma unroll
+    for (int kd = 0; kd < WD; ++kd)
+    {
+        if (d0 + kd < g.lo[0] || d0 + kd >= g.hi[0])
+            continue;
+#pragma unroll
+        for (int kh = 0; kh < W; ++kh)
+        {
+            if (h0 + kh < g.lo[1] || h0 + kh >= g.hi[1])
+                continue;
+            const float* rp = xp + kd * g.xs[0] + kh * g.xs[1];
+            float v[NC];
+            if (all)
+            {
+#pragma unroll
+                for (int i = 0; i < NC; ++i)
+                    v[i] = __ldg(rp + i);
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < NC; ++i)
+                    v[i] = w0 + i >= g.lo[2] && w0 + i < g.hi[2] ? __ldg(rp + i) : 0.f;
+            }
+#pragma unroll
+            for (int o = 0; o < 4; ++o)
+#pragma unroll
+                for (int kw = 0; kw < W; ++kw)
+                {
+                    const int i = o * S + kw;
+                    if (!MAXP)
+                        r[o] += v[i]; // (cells that do not exist are zeros)
+                    else if ((all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) && (best[o] < 0 || v[i] > r[o]))
+                    {
+                        r[o] = v[i];
+                        best[o] = (kd * W + kh) * W + kw;
+                    }
+                }
+        }
+    }
+    const int left = min(4, g.out[2] - ow0);
+    if (argmax)
+    {
+        unsigned char* ap = argmax + ((((size_t) n * g.c + c) * g.out[0] + od) * g.out[1] + oh) * g.out[2] + ow0;
+#pragma unroll
+        for (int o = 0; o < 4; ++o)
+            if (o < left)
+                ap[o] = (unsigned char) best[o];
+        if (!y)
+            return;
+    }
+    float* yp = y + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1] + ow0;
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+        if (o < left)
+        {
+            const float q = MAXP ? r[o] : r[o] / fmaxf(pool_count(g, od, oh, ow0 + o), 1.f);
+            yp[o] = beta != 0.f ? alpha * q + beta * yp[o] : alpha * q;
+        }
 }
 
 // Forward for windows of 3 with stride 2 and pad 1 along W (and H; WD = 3 with stride 2
@@ -559,10 +638,12 @@ __device__ __forceinline__ void pool_cover(int i, int stride, int pad, int win, 
     *hi = min(hq, nout - 1);
 }
 
+// Maximum, backward, without a workspace: a thread per input cell looks at the windows that hold it
+// and scans those whose maximum it equals.
 template <int WD, int W, int S>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_bwd_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ y, const float* __restrict__ dy,
-                    const float* __restrict__ x, float* dx, const unsigned char* __restrict__ argmax)
+                    const float* __restrict__ x, float* dx)
 {
     // window / stride as compile-time constants where the launch found a match
     // (unrolled loops, shifts for the divisions); 0 = read them from the geometry
@@ -580,39 +661,17 @@ __global__ void __launch_bounds__(POOL_THREADS)
     pool_cover(id, s0_, g.pad[0], w0_, g.out[0], &dlo, &dhi);
     pool_cover(ih, s1_, g.pad[1], w1_, g.out[1], &hlo, &hhi);
     pool_cover(iw, s2_, g.pad[2], w2_, g.out[2], &wlo, &whi);
-    const float xv = g.mode == DCB_POOL_MAX && !argmax ? __ldg(x + me) : 0.f;
+    const float xv = __ldg(x + me);
     float acc = 0.f;
     // a cell outside the global tensor is padding: no window gives it anything
     const bool real = id >= g.lo[0] && id < g.hi[0] && ih >= g.lo[1] && ih < g.hi[1] && iw >= g.lo[2] && iw < g.hi[2];
     if (!real)
         dhi = dlo - 1;
-    if (argmax)
-    {
-        // the index pass recorded every window's first maximum: one byte to compare
-        const size_t plane = ((size_t) n * g.c + c) * g.out[0];
-        for (int od = dlo; od <= dhi; ++od)
-            for (int oh = hlo; oh <= hhi; ++oh)
-            {
-                const size_t drow = ((plane + od) * g.out[1] + oh) * g.out[2];
-                const float* dyrow = dy + yoff + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1];
-                const int tap0 = ((id - (od * s0_ - g.pad[0])) * w1_ + (ih - (oh * s1_ - g.pad[1])))
-                                 * w2_;
-                for (int ow = wlo; ow <= whi; ++ow)
-                    if ((int) __ldg(argmax + drow + ow) == tap0 + iw - (ow * s2_ - g.pad[2]))
-                        acc += __ldg(dyrow + ow);
-            }
-        dlo = dhi + 1;
-    }
     for (int od = dlo; od <= dhi; ++od)
         for (int oh = hlo; oh <= hhi; ++oh)
             for (int ow = wlo; ow <= whi; ++ow)
             {
                 const size_t o = yoff + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1] + ow;
-                if (g.mode != DCB_POOL_MAX)
-                {
-                    acc += __ldg(dy + o) / fmaxf(pool_count(g, od, oh, ow), 1.f);
-                    continue;
-                }
                 if (__ldg(y + o) != xv)
                     continue;
                 // the maximum goes to the first cell that holds it: is one before me?
@@ -639,21 +698,25 @@ __global__ void __launch_bounds__(POOL_THREADS)
     dx[me] = beta != 0.f ? alpha * acc + beta * dx[me] : alpha * acc;
 }
 
-// MAX backward with the index workspace: a thread owns four consecutive cells of
-// an input row, walks the (od, oh) pairs whose windows hold the row once for all
-// four, and compares one byte per (cell, window).  Every instruction here is
-// paid 268 M times on the bench shard: the per-cell version spent 430 per cell.
-template <int WD, int W, int S>
+// Backward for any window: averages, and maxima by the index workspace.  A thread owns four
+// consecutive cells of an input row and walks the windows that hold the row, each gradient (and
+// index byte, or quotient) once for all four cells.  Short rows share a block.  Bound by
+// instruction issue: what a thread does per window is what counts (us, a cell a thread for averages
+// and one row a block before: 2 x 16 x 100 x 96 x 128, 3 / 2, averages 644 -> 234; 8 x 128^3, 3 / 1,
+// averages 940 -> 492; 16 x 64 x 100 x 90, 2 / 2, maxima 68 -> 54; 4 x 30 x 30 x 31, 3 / 1, 28.5 -> 9).
+template <int WD, int W, int S, bool MAXP>
 __global__ void __launch_bounds__(POOL_THREADS)
-    pool_bwd_index_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ dy, float* dx,
-                          const unsigned char* __restrict__ argmax)
+    pool_bwd_cells_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ dy, float* dx,
+                          const unsigned char* __restrict__ argmax, int tw_log2, long long rows)
 {
     const int w0_ = WD ? WD : g.win[0], w1_ = W ? W : g.win[1], w2_ = W ? W : g.win[2];
     const int s0_ = S ? (WD == 1 ? 1 : S) : g.stride[0], s1_ = S ? S : g.stride[1], s2_ = S ? S : g.stride[2];
-    const int iw0 = (blockIdx.y * POOL_THREADS + threadIdx.x) * 4;
-    if (iw0 >= g.in[2])
+    const int iw0 = ((blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1))) * 4;
+    const long long row = (long long) blockIdx.x * (POOL_THREADS >> tw_log2) + (threadIdx.x >> tw_log2);
+    if (iw0 >= g.in[2] || row >= rows)
         return;
-    const int ih = blockIdx.x % g.in[1], id = blockIdx.x / g.in[1];
+    int id, ih;
+    pool_split_row(row, rows, g.in[1], &id, &ih);
     const int c = blockIdx.z % g.c, n = blockIdx.z / g.c;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     int dlo, dhi, hlo, hhi;
@@ -661,13 +724,15 @@ __global__ void __launch_bounds__(POOL_THREADS)
     pool_cover(ih, s1_, g.pad[1], w1_, g.out[1], &hlo, &hhi);
     if (id < g.lo[0] || id >= g.hi[0] || ih < g.lo[1] || ih >= g.hi[1])
         dhi = dlo - 1; // a row outside the global tensor is padding
-    int wlo[4], whi[4];
+    int wlo[4], whi[4], first = g.out[2], last = -1; // windows of each cell, of all
 #pragma unroll
     for (int e = 0; e < 4; ++e)
     {
         pool_cover(iw0 + e, s2_, g.pad[2], w2_, g.out[2], &wlo[e], &whi[e]);
         if (iw0 + e < g.lo[2] || iw0 + e >= g.hi[2] || iw0 + e >= g.in[2])
             whi[e] = wlo[e] - 1;
+        if (whi[e] >= wlo[e])
+            first = min(first, wlo[e]), last = max(last, whi[e]);
     }
     const size_t plane = ((size_t) n * g.c + c) * g.out[0];
     const float* dyp = dy + (size_t) n * g.ys_n + (size_t) c * g.ys_c;
@@ -677,11 +742,15 @@ __global__ void __launch_bounds__(POOL_THREADS)
             const unsigned char* arow = argmax + ((plane + od) * g.out[1] + oh) * g.out[2];
             const float* dyrow = dyp + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1];
             const int tap0 = ((id - (od * s0_ - g.pad[0])) * w1_ + (ih - (oh * s1_ - g.pad[1]))) * w2_ + g.pad[2] + iw0;
+            for (int ow = first; ow <= last; ++ow)
+            {
+                const float d = MAXP ? __ldg(dyrow + ow) : __ldg(dyrow + ow) / fmaxf(pool_count(g, od, oh, ow), 1.f);
+                const int tap = MAXP ? (int) __ldg(arow + ow) - (tap0 - ow * s2_) : 0; // the cell it is, of the four
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                for (int ow = wlo[e]; ow <= whi[e]; ++ow)
-                    if ((int) __ldg(arow + ow) == tap0 + e - ow * s2_)
-                        acc[e] += __ldg(dyrow + ow);
+                for (int e = 0; e < 4; ++e)
+                    if (ow >= wlo[e] && ow <= whi[e] && (!MAXP || tap == e))
+                        acc[e] += d;
+            }
         }
     float* xp = dx + (size_t) n * g.xs_n + (size_t) c * g.xs_c + (size_t) id * g.xs[0] + (size_t) ih * g.xs[1] + iw0;
     if (iw0 + 4 <= g.in[2] && (reinterpret_cast<uintptr_t>(xp) & 15) == 0)
@@ -1057,6 +1126,17 @@ bool pool_grid(int w, long long rows, long long planes, dim3* grid)
             DCB_POOL_CALL(0, 0, 0);                                                                                   \
     } while (0)
 
+template <int WD, int W, int S>
+void launch_pool_cells(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax, dim3 qgrid,
+                       int qw_log2, dim3 grid, int tw_log2, long long rows, cudaStream_t stream)
+{
+    if constexpr (WD == 0)
+        pool_fwd_kernel<<<grid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, tw_log2, rows);
+    else
+        (g.mode == DCB_POOL_MAX ? pool_fwd_cells_kernel<WD, W, S, true> : pool_fwd_cells_kernel<WD, W, S, false>)
+            <<<qgrid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, qw_log2, rows);
+}
+
 int32_t launch_pool_fwd(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax,
                         cudaStream_t stream)
 {
@@ -1105,8 +1185,13 @@ int32_t launch_pool_fwd(const PoolGeom& g, float alpha, float beta, const float*
         DCB_LAUNCH_CHECK();
         return DCB_OK;
     }
-#define DCB_POOL_CALL(WD, W, S)                                                                                        \
-    pool_fwd_kernel<WD, W, S><<<grid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, tw_log2, rows)
+    const int quads = (g.out[2] + 3) / 4;
+    int qw_log2 = 8;
+    while (qw_log2 > 2 && (1 << (qw_log2 - 1)) >= quads)
+        --qw_log2;
+    const long long qpb = POOL_THREADS >> qw_log2;
+    const dim3 qgrid((unsigned) ((rows + qpb - 1) / qpb), (unsigned) ((quads + (1 << qw_log2) - 1) >> qw_log2), (unsigned) planes);
+#define DCB_POOL_CALL(WD, W, S) launch_pool_cells<WD, W, S>(g, alpha, beta, x, y, argmax, qgrid, qw_log2, grid, tw_log2, rows, stream)
     DCB_POOL_DISPATCH(g);
 #undef DCB_POOL_CALL
     DCB_LAUNCH_CHECK();
@@ -1230,12 +1315,19 @@ extern "C" int32_t dcb_pool_bwd(const dcb_pool_desc* pd, const dcb_nd_desc* xd, 
             return DCB_OK;
         }
     }
-    if (idx)
+    if (idx || g.mode != DCB_POOL_MAX)
     {
-        const dim3 grid4(grid.x, (unsigned) ((g.in[2] + 4 * POOL_THREADS - 1) / (4 * POOL_THREADS)), grid.z);
+        const int wcells = (g.in[2] + 3) / 4; // threads a row needs
+        int tw_log2 = 8;
+        while (tw_log2 > 2 && (1 << (tw_log2 - 1)) >= wcells)
+            --tw_log2;
+        const long long rows = (long long) g.in[0] * g.in[1], rpb = POOL_THREADS >> tw_log2;
+        // (as many blocks in x and y as pool_grid has allowed, or fewer)
+        const dim3 grid4((unsigned) ((rows + rpb - 1) / rpb), (unsigned) ((wcells + (1 << tw_log2) - 1) >> tw_log2), grid.z);
 #define DCB_POOL_CALL(WD, W, S)                                                                                       \
-    pool_bwd_index_kernel<WD, W, S><<<grid4, POOL_THREADS, 0, as_stream(stream)>>>(                                  \
-        g, (float) alpha, (float) beta, static_cast<const float*>(dy), static_cast<float*>(dx), idx)
+    (idx ? pool_bwd_cells_kernel<WD, W, S, true> : pool_bwd_cells_kernel<WD, W, S, false>)                            \
+        <<<grid4, POOL_THREADS, 0, as_stream(stream)>>>(g, (float) alpha, (float) beta, static_cast<const float*>(dy), \
+                                                       static_cast<float*>(dx), idx, tw_log2, rows)
         DCB_POOL_DISPATCH(g);
 #undef DCB_POOL_CALL
         DCB_LAUNCH_CHECK();
@@ -1244,7 +1336,7 @@ extern "C" int32_t dcb_pool_bwd(const dcb_pool_desc* pd, const dcb_nd_desc* xd, 
 #define DCB_POOL_CALL(WD, W, S)                                                                                       \
     pool_bwd_kernel<WD, W, S><<<grid, POOL_THREADS, 0, as_stream(stream)>>>(                                         \
         g, (float) alpha, (float) beta, static_cast<const float*>(y), static_cast<const float*>(dy),                  \
-        static_cast<const float*>(x), static_cast<float*>(dx), idx)
+        static_cast<const float*>(x), static_cast<float*>(dx))
     DCB_POOL_DISPATCH(g);
 #undef DCB_POOL_CALL
     DCB_LAUNCH_CHECK();

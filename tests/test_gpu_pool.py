@@ -88,6 +88,23 @@ def test_kernels_against_oracle(case, mode):
     emu.assert_close(dxb.cpu().numpy(), 0.5 * dx_ref - dx0, 4e-6, "dx blend")
 
 
+# four cells a thread: rows around multiples of four and of a block's shares of rows, padding on
+# either side, gaps between windows, a window of each compiled kind and a general one
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("window,pad,stride,widths", [
+    (2, 0, 2, (2, 3, 8, 9, 10, 17, 66)),
+    (3, 1, 1, (1, 2, 4, 5, 7, 16, 33, 1025)),
+    (3, 1, 2, (1, 5, 6, 7, 9, 33, 35)),
+    (2, 0, 3, (5, 8, 13)),
+    (4, 2, 2, (3, 8, 21)),
+])
+def test_rows_of_all_lengths(window, pad, stride, widths, mode):
+    for w in widths:
+        for sp in ((5, 4, w), (6, w)):
+            if min(sp) + 2 * pad >= window:
+                test_kernels_against_oracle((1, 2, sp, *([v] * len(sp) for v in (window, pad, stride))), mode)
+
+
 # window 3, stride 2: walks of several outputs along D (the last one shorter), one walk
 # per output, an odd row end, no padding along D
 @pytest.mark.parametrize("n,c,sp,pad_d", [(1, 512, (37, 31, 20), 1), (2, 512, (24, 9, 8), 0), (1, 2, (6, 5, 264), 1),
