@@ -100,7 +100,7 @@ struct ShGeom
     int nb, kcols, kgroups;  // columns per cell block, filters per group
     int blk, rowst, woff, nsets, set_off; // columns: block, row of blocks, cell parity along W, set
     int cpg, cgroups;        // channels per group (a multiple of the cell's)
-    int pt, used;            // positions per plane of the A slot, those that items write
+    int pt;                  // positions per plane of the A slot
     int ipr;                 // items (32 positions, all cells of the channel group) of a staged row
     int a_slot16, a_slots;
     int teams;               // converter teams; a_slots is a multiple of it and of SH_ISS
@@ -634,10 +634,8 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         reinterpret_cast<uint4*>(smem + g.so_sets)[i] = reinterpret_cast<const uint4*>(tables)[i];
     // positions that no item writes are read by the MMAs of lanes nobody stores: keep them finite
 #pragma unroll 1
-    for (int plane = warp; plane < g.a_slots * g.a_slot16 / g.pt; plane += SH_THREADS / 32)
-#pragma unroll 1
-        for (int i = g.used + lane; i < g.pt; i += 32)
-            reinterpret_cast<uint4*>(smem + g.so_a)[plane * g.pt + i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < g.a_slots * g.a_slot16; i += SH_THREADS)
+        reinterpret_cast<uint4*>(smem + g.so_a)[i] = make_uint4(0, 0, 0, 0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();

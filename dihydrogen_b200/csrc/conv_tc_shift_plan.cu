@@ -279,7 +279,6 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     }
     const int used = g.npack * (g.tile_w + reach);
     g.pt = std::max(TC_M + reach, used) + 1;
-    g.used = used;
     const int npb = (used + 31) / 32;
     g.ipr = g.st_w * npb;
     if (g.ipr > SH_MAX_ITEMS)
