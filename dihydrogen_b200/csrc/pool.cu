@@ -50,20 +50,18 @@ struct PoolGeom
 
 constexpr int POOL_THREADS = 256;
 
-__device__ __forceinline__ float pool_count(const PoolGeom& g, int od, int oh, int ow)
+// Cells along axis i that output o's average is over.
+__device__ __forceinline__ int pool_extent(const PoolGeom& g, int i, int o)
 {
     if (g.mode == DCB_POOL_AVERAGE)
-        return (float) (g.win[0] * g.win[1] * g.win[2]);
-    int cnt = 1;
-    const int o[3] = {od, oh, ow};
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-    {
-        const int lo = max(g.lo[i], o[i] * g.stride[i] - g.pad[i]);
-        const int hi = min(g.hi[i], o[i] * g.stride[i] - g.pad[i] + g.win[i]);
-        cnt *= max(0, hi - lo);
-    }
-    return (float) cnt;
+        return g.win[i];
+    const int lo = max(g.lo[i], o * g.stride[i] - g.pad[i]), hi = min(g.hi[i], o * g.stride[i] - g.pad[i] + g.win[i]);
+    return max(0, hi - lo);
+}
+
+__device__ __forceinline__ float pool_count(const PoolGeom& g, int od, int oh, int ow)
+{
+    return (float) (pool_extent(g, 0, od) * pool_extent(g, 1, oh) * pool_extent(g, 2, ow));
 }
 
 // row = plane * extent + line, with the 32-bit division when the row count allows it
@@ -703,7 +701,7 @@ __global__ void __launch_bounds__(POOL_THREADS)
 // index byte, or quotient) once for all four cells.  Short rows share a block.  Bound by
 // instruction issue: what a thread does per window is what counts (us, a cell a thread for averages
 // and one row a block before: 2 x 16 x 100 x 96 x 128, 3 / 2, averages 644 -> 234; 8 x 128^3, 3 / 1,
-// averages 940 -> 492; 16 x 64 x 100 x 90, 2 / 2, maxima 68 -> 54; 4 x 30 x 30 x 31, 3 / 1, 28.5 -> 9).
+// averages 940 -> 411; 16 x 64 x 100 x 90, 2 / 2, maxima 68 -> 54; 4 x 30 x 30 x 31, 3 / 1, 28.5 -> 9).
 template <int WD, int W, int S, bool MAXP>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_bwd_cells_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ dy, float* dx,
@@ -734,6 +732,10 @@ __global__ void __launch_bounds__(POOL_THREADS)
         if (whi[e] >= wlo[e])
             first = min(first, wlo[e]), last = max(last, whi[e]);
     }
+    // stride 1: the loads of all windows along W go out together (maxima of 16 x 64 x 100 x 90
+    // 365 -> 325 us, averages of 8 x 128^3 488 -> 411; with stride 2 there are two or three, and
+    // a fixed number of them costs more: averages of 2 x 16 x 100 x 96 x 128 231 -> 320)
+    constexpr int M = S == 1 ? W + 3 : 1;
     const size_t plane = ((size_t) n * g.c + c) * g.out[0];
     const float* dyp = dy + (size_t) n * g.ys_n + (size_t) c * g.ys_c;
     for (int od = dlo; od <= dhi; ++od)
@@ -742,14 +744,30 @@ __global__ void __launch_bounds__(POOL_THREADS)
             const unsigned char* arow = argmax + ((plane + od) * g.out[1] + oh) * g.out[2];
             const float* dyrow = dyp + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1];
             const int tap0 = ((id - (od * s0_ - g.pad[0])) * w1_ + (ih - (oh * s1_ - g.pad[1]))) * w2_ + g.pad[2] + iw0;
-            for (int ow = first; ow <= last; ++ow)
+            // (windows of 2 with stride 2: one window a cell, nothing to share; 68 us like that, 60 so)
+            const int cells = MAXP || W == 2 ? 0 : pool_extent(g, 0, od) * pool_extent(g, 1, oh);
+            for (int ow0 = first; ow0 <= last; ow0 += M)
             {
-                const float d = MAXP ? __ldg(dyrow + ow) : __ldg(dyrow + ow) / fmaxf(pool_count(g, od, oh, ow), 1.f);
-                const int tap = MAXP ? (int) __ldg(arow + ow) - (tap0 - ow * s2_) : 0; // the cell it is, of the four
+                float d[M];
+                int tap[M]; // the cell that the maximum is, of the four
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (ow >= wlo[e] && ow <= whi[e] && (!MAXP || tap == e))
-                        acc[e] += d;
+                for (int k = 0; k < M; ++k)
+                {
+                    const int ow = ow0 + k;
+                    d[k] = ow <= last ? __ldg(dyrow + ow) : 0.f;
+                    tap[k] = MAXP && ow <= last ? (int) __ldg(arow + ow) - (tap0 - ow * s2_) : -1;
+                }
+#pragma unroll
+                for (int k = 0; k < M; ++k)
+                {
+                    const int ow = ow0 + k;
+                    if (!MAXP)
+                        d[k] /= fmaxf(W == 2 ? pool_count(g, od, oh, ow) : (float) (cells * pool_extent(g, 2, ow)), 1.f);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (ow >= wlo[e] && ow <= whi[e] && (!MAXP || tap[k] == e))
+                            acc[e] += d[k];
+                }
             }
         }
     float* xp = dx + (size_t) n * g.xs_n + (size_t) c * g.xs_c + (size_t) id * g.xs[0] + (size_t) ih * g.xs[1] + iw0;
