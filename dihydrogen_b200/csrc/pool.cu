@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(POOL_THREADS)
 
 // The same for the common windows, four neighbouring outputs a thread: a window row's cells are
 // loaded once for all four and the addresses worked out once.  Same scan order, same bits (us, an
-// output a thread before: 8 x 128^3, 3 / 1, averages 309 -> 140; 16 x 64 x 100 x 90, 2 / 2, maxima
-// 19.6 -> 13.8, 3 / 1 182 -> 174).
+// output a thread before: 8 x 128^3, 3 / 1, averages 309 -> 124; 16 x 64 x 100 x 90, 2 / 2, maxima
+// 19.6 -> 12.8, 3 / 1 182 -> 155).
 template <int WD, int W, int S, bool MAXP>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_fwd_cells_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ x, float* y,
@@ -171,25 +171,23 @@ __global__ void __launch_bounds__(POOL_THREADS)
     {
         if (d0 + kd < g.lo[0] || d0 + kd >= g.hi[0])
             continue;
+        // a plane's rows before the first is looked at: their loads are in flight together
+        // (3 / 1, maxima 172 -> 155 us)
+        float v[W][NC];
+#pragma unroll
+        for (int kh = 0; kh < W; ++kh)
+        {
+            const float* rp = xp + kd * g.xs[0] + kh * g.xs[1];
+            const bool row_in = h0 + kh >= g.lo[1] && h0 + kh < g.hi[1];
+#pragma unroll
+            for (int i = 0; i < NC; ++i)
+                v[kh][i] = row_in && (all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) ? __ldg(rp + i) : 0.f;
+        }
 #pragma unroll
         for (int kh = 0; kh < W; ++kh)
         {
             if (h0 + kh < g.lo[1] || h0 + kh >= g.hi[1])
                 continue;
-            const float* rp = xp + kd * g.xs[0] + kh * g.xs[1];
-            float v[NC];
-            if (all)
-            {
-#pragma unroll
-                for (int i = 0; i < NC; ++i)
-                    v[i] = __ldg(rp + i);
-            }
-            else
-            {
-#pragma unroll
-                for (int i = 0; i < NC; ++i)
-                    v[i] = w0 + i >= g.lo[2] && w0 + i < g.hi[2] ? __ldg(rp + i) : 0.f;
-            }
 #pragma unroll
             for (int o = 0; o < 4; ++o)
 #pragma unroll
@@ -197,10 +195,10 @@ __global__ void __launch_bounds__(POOL_THREADS)
                 {
                     const int i = o * S + kw;
                     if (!MAXP)
-                        r[o] += v[i]; // (cells that do not exist are zeros)
-                    else if ((all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) && (best[o] < 0 || v[i] > r[o]))
+                        r[o] += v[kh][i]; // (cells that do not exist are zeros)
+                    else if ((all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) && (best[o] < 0 || v[kh][i] > r[o]))
                     {
-                        r[o] = v[i];
+                        r[o] = v[kh][i];
                         best[o] = (kd * W + kh) * W + kw;
                     }
                 }
@@ -700,7 +698,7 @@ __global__ void __launch_bounds__(POOL_THREADS)
 // consecutive cells of an input row and walks the windows that hold the row, each gradient (and
 // index byte, or quotient) once for all four cells.  Short rows share a block.  Bound by
 // instruction issue: what a thread does per window is what counts (us, a cell a thread for averages
-// and one row a block before: 2 x 16 x 100 x 96 x 128, 3 / 2, averages 644 -> 234; 8 x 128^3, 3 / 1,
+// and one row a block before: 2 x 16 x 100 x 96 x 128, 3 / 2, averages 644 -> 217; 8 x 128^3, 3 / 1,
 // averages 940 -> 411; 16 x 64 x 100 x 90, 2 / 2, maxima 68 -> 54; 4 x 30 x 30 x 31, 3 / 1, 28.5 -> 9).
 template <int WD, int W, int S, bool MAXP>
 __global__ void __launch_bounds__(POOL_THREADS)
