@@ -600,6 +600,16 @@ def test_shift_kernel_tile_and_table_edges(geom):
     emu.assert_close(dx, 0.5 * dx_ref - dx0, TOL, "dx")
 
 
+# the issuers' tables as an argument of 1 KB and of 8 KB
+@pytest.mark.parametrize("geom", [
+    (1, 4, 4, (9, 12, 40), (3, 3, 3), 1),
+    (1, 16, 16, (12, 14, 40), (5, 5, 5), 1),
+    (1, 4, 4, (16, 16, 16), (7, 7, 7), 1),
+])
+def test_shift_kernel_short_and_long_tables(geom):
+    test_shift_kernel_tile_and_table_edges(geom)
+
+
 @pytest.mark.parametrize("geom", [
     # N, C, K, spatial, filter, stride: edges of the backward filter's stages and roles
     (1, 4, 16, (5, 7, 32), (3, 3, 3), 1),      # one stage wide, rows left over
