@@ -365,6 +365,16 @@ __device__ __noinline__ static float sh_exact(const ShGeom& g, const ShExact& e,
     return e.one_pass ? acc : e.alpha * acc;
 }
 
+// Columns of tensor memory that the epilogue may fetch: 16 at a time, also where fewer are left of
+// the last block.  What it fetches it may look at, so all of them are zeroed first.  (With only the
+// accumulators' columns zeroed, backward data of 4 channels on 64 x 128 x 128, stride 2 along D and
+// W, took what an earlier kernel had left beyond them for outputs that are no numbers and went to
+// look for those: 112 us behind a kernel of NaNs, 77 behind others; 79 and 77 like this.)
+__host__ __device__ __forceinline__ int sh_columns(const ShGeom& g)
+{
+    return g.set_off * g.nsets + (g.nb % 16 ? 16 - g.nb % 16 : 0);
+}
+
 __device__ __forceinline__ bool sh_number(float v)
 {
     return fabsf(v) <= 3.402823466e+38f;
@@ -643,7 +653,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
     const uint32_t tmem_base = *tmem_slot;
     if (warp < SH_EPI)
 #pragma unroll 1
-        for (int c = (warp >> 2) * 16; c < g.set_off * g.nsets; c += 32)
+        for (int c = (warp >> 2) * 16; c < sh_columns(g); c += 32)
             sh_tmem_zero(tmem_base + ((uint32_t) ((warp & 3) * 32) << 16) + (uint32_t) c, 16);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     tc_fence_before();

@@ -252,8 +252,7 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     g.rowst = align_up(g.ns * g.blk, 16);
     g.woff = g.th * g.rowst;
     g.set_off = g.e_w * g.woff;
-    // (the epilogue reads 16 columns at a time, also where fewer are left)
-    if (g.set_off * g.nsets + (g.nb % 16 ? 16 - g.nb % 16 : 0) > (int) TC_TMEM_COLS || g.th * g.ns > SH_MAX_BLOCKS)
+    if (sh_columns(g) > (int) TC_TMEM_COLS || g.th * g.ns > SH_MAX_BLOCKS)
         return false;
     const int cells = (m_cin + m_ch - 1) / m_ch;
     const int J = (cells + t.cgroups - 1) / t.cgroups;

@@ -600,6 +600,31 @@ def test_shift_kernel_tile_and_table_edges(geom):
     emu.assert_close(dx, 0.5 * dx_ref - dx0, TOL, "dx")
 
 
+# strides that differ: an epilogue that fetches beyond its accumulators, after a kernel that left NaNs there
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_BF16])
+@pytest.mark.parametrize("channels,f,strides", [
+    (4, 3, (2, 1, 1)), (4, 3, (1, 1, 2)), (3, 3, (2, 1, 2)), (4, 3, (1, 2, 1)), (8, 2, (1, 1, 2)), (4, 2, (1, 2, 2)),
+    (5, 3, (2, 2, 1)),
+])
+def test_shift_kernel_strides_that_differ(channels, f, strides, mode):
+    rng = np.random.default_rng(channels + f)
+    sp, pads = (9, 18, 70), [(f - 1) // 2] * 3
+    x = rng.normal(0, 1, (2, channels, *sp)).astype(np.float32)
+    w = rng.normal(0, np.sqrt(2.0 / (channels * f ** 3)), (16, channels, f, f, f)).astype(np.float32)
+    dy = rng.normal(0, 1, (2, 16, *[O.conv_out_extent(i, f, p, s, 1) for i, p, s in zip(sp, pads, strides)])).astype(np.float32)
+    if mode == _abi.MATH_BF16:
+        w, dy = _round_bf16(w), _round_bf16(dy)
+    g = [torch.from_numpy(a).cuda() for a in (x, w, dy)]
+    p = Plan(*g, pads, list(strides), [1] * 3, mode)
+    assert _abi.lib().dcb_conv_plan_kernel_kind(p.p, 1) == 1, "expected the shift kernel"
+    p.bwd_filter(1.0, g[0], torch.full_like(g[2], float("nan")), 0.0, torch.zeros_like(g[1]))
+    dx = torch.full_like(g[0], float("nan"))
+    p.bwd_data(1.0, g[1], g[2], 0.0, dx)
+    dx_ref = np.zeros_like(x)
+    O.conv_bwd_data(w, dy, dx_ref, pads, list(strides))
+    emu.assert_close(dx.cpu().numpy(), dx_ref, TOL, "dx")
+
+
 # the issuers' tables as an argument of 1 KB and of 8 KB
 @pytest.mark.parametrize("geom", [
     (1, 4, 4, (9, 12, 40), (3, 3, 3), 1),

@@ -118,3 +118,11 @@ def test_pieces_of_unaligned_runs_cover_them_once(tmp_path):
     assert r.returncode == 0, r.stderr
     good, pairs = map(int, r.stdout.split())
     assert good == pairs > 500
+
+
+def test_shift_kernel_fetches_zeroed_columns_only(tmp_path):
+    """Columns that were fetched with the last block but not zeroed held what an earlier kernel left."""
+    r = subprocess.run([compile_check(tmp_path, "shift_columns_check")], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    passes, beyond, bad = map(int, r.stdout.split())
+    assert passes > 1000 and beyond > 100 and bad == 0, r.stdout
