@@ -75,8 +75,9 @@ struct ShfJob
     long long parity_pitch; // put: floats between the two halves of that window
     uint32_t* flag;         // put: flag to publish there; wait: own flag to wait on
     int vec;                // 16-byte accesses: offsets, strides and run allow them (if the bases do)
-    int split;              // long runs, a unit's accesses of one run; else of the job
-    long long units[3];     // per way of access (ShfAccess)
+    // per way of access (ShfAccess)
+    int split[3];           // long runs: a unit's accesses are of one run; else of the job
+    long long units[3];
     long long per_run[3];   // accesses of a run
     FastDiv by_run[3], by_ext[4];
 };
@@ -206,7 +207,7 @@ __device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, const flo
 {
     T a[shf_unroll<WAY>];
     constexpr int CHUNK = SHF_THREADS * shf_unroll<WAY>; // accesses of a unit
-    if (j.split)
+    if (j.split[WAY])
     {
         // CHUNK accesses of one long run
         const long long cpr = (j.per_run[WAY] + CHUNK - 1) / CHUNK;
@@ -341,14 +342,17 @@ void finish_job(ShfJob* j)
         j->by_ext[k] = FastDiv::of((uint32_t) j->ext[k]);
     }
     j->vec = (mix & 3) == 0;
-    // runs of at least two units, or (one run) too many accesses for 31-bit indices
-    j->split = j->len / (j->vec ? 4 : 1) >= 2 * SHF_THREADS * shf_unroll<SHF_VEC> || j->rows * j->len >= SHF_MAX_CELLS;
     for (int w = 0; w < 3; ++w)
     {
         j->per_run[w] = w == SHF_PIECE ? (j->len + 6) / 4 : j->len / (w == SHF_VEC ? 4 : 1);
         j->by_run[w] = FastDiv::of(j->per_run[w] > 0 && j->per_run[w] < (1 << 30) ? (uint32_t) j->per_run[w] : 1u);
         const long long chunk = SHF_THREADS * (w == SHF_PIECE ? shf_unroll<SHF_PIECE> : shf_unroll<SHF_VEC>);
-        j->units[w] = j->split ? j->rows * ((j->per_run[w] + chunk - 1) / chunk) : (j->rows * j->per_run[w] + chunk - 1) / chunk;
+        // Runs of at least two units, so that at most a third of a run's threads are idle in its last
+        // one, or (one run) too many accesses for 31-bit indices.  By this way's own accesses: with
+        // the cells of a run in pieces counted instead, 2 x 16 x 96 x 90 x 47 along H (runs of 2115)
+        // took 204 us there and back, like this 160; runs of 3355 234 and 216, from 3969 on the same.
+        j->split[w] = j->per_run[w] >= 2 * chunk || j->rows * j->len >= SHF_MAX_CELLS;
+        j->units[w] = j->split[w] ? j->rows * ((j->per_run[w] + chunk - 1) / chunk) : (j->rows * j->per_run[w] + chunk - 1) / chunk;
     }
 }
 

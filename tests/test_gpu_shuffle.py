@@ -76,6 +76,10 @@ def test_forward_and_backward(shape, sgrid, dgrid, dov):
     # merged rows of odd length, split in H
     ([13, 11, 9, 3, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 0, 0, 0, 0]),
     ([10, 9, 5, 3, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 1, 0, 0, 0]),
+    # runs of 2070 and 4092 cells, below and at the 1024 pieces from which a run has its own units
+    ([45, 92, 3, 3, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 0, 0, 0, 0]),
+    ([62, 132, 3, 2, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 1, 0, 0, 0]),
+    ([45, 182, 3, 2, 2], [1, 1, 1, 1, 2], [1, 2, 1, 1, 1], [0, 0, 0, 0, 0]),
     # whole odd planes: runs of several units, in pieces
     ([97, 91, 3, 2, 2], [1, 1, 1, 1, 2], [1, 1, 2, 1, 1], [0, 0, 0, 0, 0]),
     ([98, 91, 3, 1, 2], [1, 1, 1, 1, 2], [1, 1, 2, 1, 1], [0, 0, 1, 0, 0]),

@@ -126,3 +126,14 @@ def test_shift_kernel_fetches_zeroed_columns_only(tmp_path):
     assert r.returncode == 0, r.stderr
     passes, beyond, bad = map(int, r.stdout.split())
     assert passes > 1000 and beyond > 100 and bad == 0, r.stdout
+
+
+def test_units_of_a_redistribution_are_not_mostly_empty(tmp_path):
+    """A run in pieces used to be split by the count of its cells: 2049 of them left half of its units' threads idle."""
+    exe = compile_check(tmp_path, "shuffle_units_check")
+    r = subprocess.run([exe], input="\n".join(str(n) for n in range(1, 20000, 7)), capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    lines = [[int(v) for v in l.split()] for l in r.stdout.splitlines()]
+    assert {way for _, way, _ in lines} == {0, 1, 2}
+    # from two units on a run has its own, of which the last may have one access
+    assert min(full for _, _, full in lines) >= 66, min((full, way, n) for n, way, full in lines)
