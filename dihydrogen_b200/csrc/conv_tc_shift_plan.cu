@@ -490,9 +490,9 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
         put(st.data(), st.size() * sizeof(uint2));
         g.co_groups = put(groups.data(), groups.size() * sizeof(ShGroup)) / 16;
         g.co_rows = put(rowtab.data(), rowtab.size() * 4) / 4;
-        T->too_long = T->blob.size() > SH_CONST;
+        T->too_long = T->blob.size() > (size_t) m_issue_bytes;
         if (T->too_long)
-            return false;
+            return false; // (streamed, every image stands again and maybe others beside it: the steps are no fewer)
         T->issue.swap(T->blob);
         T->blob.clear();
         const int o_sets = put(sets.data(), sets.size() * sizeof(uint2));

@@ -113,8 +113,9 @@ inline double sh_mma_cost(int n)
 class ShBuilder
 {
 public:
-    ShBuilder(const ConvGeom& cg, bool transposed, int math_mode, int sms)
-        : m_cg(cg), m_tr(transposed), m_sms(sms)
+    // issue_bytes: what the issuers' tables may take, SH_CONST at most
+    ShBuilder(const ConvGeom& cg, bool transposed, int math_mode, int sms, int issue_bytes = SH_CONST)
+        : m_cg(cg), m_tr(transposed), m_sms(sms), m_issue_bytes(std::min(issue_bytes, (int) SH_CONST))
     {
         m_flat = cg.in[0] == 1 && cg.out[0] == 1 && cg.f[0] == 1 && cg.pad[0] == 0 && cg.stride[0] == 1;
         const int s = m_flat ? 1 : 0;
@@ -168,7 +169,7 @@ private:
 
     ConvGeom m_cg;
     bool m_tr, m_flat, m_fp32, m_bf16;
-    int m_sms, m_cin, m_kout, m_kind, m_parts, m_ch;
+    int m_sms, m_issue_bytes, m_cin, m_kout, m_kind, m_parts, m_ch;
     ShAxis m_s, m_r, m_w;
 };
 

@@ -137,3 +137,28 @@ def test_units_of_a_redistribution_are_not_mostly_empty(tmp_path):
     assert {way for _, way, _ in lines} == {0, 1, 2}
     # from two units on a run has its own, of which the last may have one access
     assert min(full for _, _, full in lines) >= 66, min((full, way, n) for n, way, full in lines)
+
+
+def test_tables_that_do_not_fit_leave_a_lower_column(tmp_path):
+    """Layouts whose issuers' tables are longer than their argument are passed over; no layer of the other
+    tests comes near its 8 KB, so that the limit is lowered here."""
+    geometries = [((1, 4, 16, 256, 256, 256, 3, 1), (2048, 1536, 1024, 768, 512)), ((2, 8, 24, 67, 83, 101, 3, 1), (2048, 1024, 768, 512)),
+                  ((1, 16, 32, 256, 256, 256, 3, 2), (2048, 1536, 1024, 768)), ((2, 64, 64, 32, 32, 32, 3, 1), (2048, 1536, 1024))]
+    exe = compile_check(tmp_path, "shift_tables_check")
+    lines = [g + (limit,) for g, limits in geometries for limit in (8192,) + limits]
+    r = subprocess.run([exe], input="\n".join(" ".join(map(str, l)) for l in lines), capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    got = [[int(v) for v in l.split()] for l in r.stdout.splitlines()]
+    assert len(got) == 2 * len(lines)
+    lower = 0
+    for i, line in enumerate(lines):
+        for tr in range(2):
+            ok, size, _, rows, chain, _ = got[2 * i + tr]
+            assert ok and size <= line[-1] and 0 < chain <= 96, (line, tr, got[2 * i + tr])
+            if line[-1] == 8192:
+                full = got[2 * i:2 * i + 2]
+            elif full[tr][1] <= line[-1]:
+                assert got[2 * i + tr] == full[tr], (line, tr)  # a limit that does not bind changes nothing
+            else:
+                lower += rows < full[tr][3]
+    assert lower >= 8
