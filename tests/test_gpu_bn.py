@@ -91,11 +91,31 @@ def test_bn_forward_backward_local(shape, locale, overlap):
 @pytest.mark.parametrize("shape", [
     [41, 25, 1, 3, 2],   # 1025 elements a plane: just long enough for pieces of four, every start
     [91, 89, 1, 5, 1],   # 8099: the pieces of one unit and its last, partial one
-    [91, 91, 1, 4, 2],   # 8281: a second unit of 22 pieces
+    [91, 91, 1, 4, 2],   # 8281: a second unit of 23 pieces
     [67, 83, 3, 2, 2],
 ])
 def test_planes_of_odd_size(shape):
     test_bn_forward_backward_local(shape, [1] * 5, [0] * 5)
+
+
+def test_ends_of_unaligned_runs_are_summed_with_their_half():
+    """A plane of 1300 pieces of four and three elements: the thread that has those three, in the second half
+    of its unit, has whole pieces of large values that cancel in the first."""
+    H, W = 43, 121  # 5203
+    be = dc.BackendDNNLib(dc.Locale(0, 1))
+    x_t, dy_t = (_rank0([W, H, 1, 1], [1] * 4, [0] * 4) for _ in range(2))
+    big = np.zeros(H * W, np.float32)
+    big[:4096:2], big[1:4096:2] = 2.0 ** 26, -(2.0 ** 26)
+    big[5200:] = 1.0
+    for t in (x_t, dy_t):
+        emu.upload(t, big.reshape(1, 1, H, W))
+    bn = dc.BatchNormalization(be, 4, decay=0.9, epsilon=1e-5, global_stats=False)
+    sums = torch.zeros(2, device="cuda")
+    bn.forward_stage1(x_t, sums[:1], sums[1:], True)
+    mean, var, scale = torch.zeros(1, device="cuda"), torch.ones(1, device="cuda"), torch.ones(1, device="cuda")
+    grads = [torch.zeros(1, device="cuda") for _ in range(4)]
+    bn.backward_stage1(x_t, dy_t, mean, var, scale, *grads)
+    assert sums[0].item() == 3.0 and grads[1].item() == 3.0  # exact: powers of two and small whole numbers
 
 
 @pytest.mark.parametrize("shape,overlap", [
