@@ -52,6 +52,14 @@ def upload(t: dc.Tensor, arr: np.ndarray):
     t.buffer.copy_(torch.from_numpy(np.ascontiguousarray(arr)))
 
 
+def allocate_off_boundary(t: dc.Tensor, floats: int):
+    """Memory for t that starts so many floats above a 16-byte boundary."""
+    shape = tuple(reversed(t.get_local_pitched_shape()))
+    n = int(np.prod(shape))
+    t.set_view(torch.zeros(n + floats, device="cuda")[floats:].view(shape))
+    assert t.buffer.data_ptr() % 16 == (4 * (floats + t.lead)) % 16
+
+
 def scatter_owned(t: dc.Tensor, g: np.ndarray):
     """Allocate t and fill its owned cells from the global array g."""
     t.allocate()

@@ -98,6 +98,36 @@ def test_planes_of_odd_size(shape):
     test_bn_forward_backward_local(shape, [1] * 5, [0] * 5)
 
 
+def test_several_long_runs_a_plane_that_start_anywhere():
+    """A halo in H of odd rows: a run of 5561 elements per (n, c, d), each with a start of its own."""
+    test_bn_forward_backward_local([67, 166, 3, 2, 2], [1, 2, 1, 1, 1], [0, 1, 0, 0, 0])
+
+
+@pytest.mark.parametrize("x_off,dy_off", [(0, 0), (1, 1), (3, 3), (0, 2), (1, 2), (3, 0)])
+def test_sums_of_planes_of_odd_size_wherever_they_lie(x_off, dy_off):
+    """Both tensors alike: in pieces of four; not alike: element by element."""
+    shape = [67, 83, 3, 3, 2]
+    rng = np.random.default_rng(10 * x_off + dy_off)
+    be, C = dc.BackendDNNLib(dc.Locale(0, 1)), shape[-2]
+    x_t, dy_t = (_rank0(shape, [1] * 5, [0] * 5) for _ in range(2))
+    emu.allocate_off_boundary(x_t, x_off)
+    emu.allocate_off_boundary(dy_t, dy_off)
+    x = rng.normal(0.3, 1.5, x_t.np_real_shape()).astype(np.float32)
+    dy = rng.normal(0.1, 1, x.shape).astype(np.float32)
+    x_t.buffer.copy_(torch.from_numpy(x))
+    dy_t.buffer.copy_(torch.from_numpy(dy))
+    bn = dc.BatchNormalization(be, 5, decay=0.9, epsilon=1e-5, global_stats=False)
+    st, g = torch.zeros(2 * C, device="cuda"), torch.zeros(4 * C, device="cuda")
+    bn.forward_stage1(x_t, st[:C], st[C:], True)
+    for got, ref, name in zip(st.split(C), O.bn_sums(x), ("sums", "sqsums")):
+        emu.assert_close(got.cpu().numpy(), ref, TOL, name)
+    mean, var = x.mean(axis=(0, 2, 3, 4)), x.var(axis=(0, 2, 3, 4))
+    scale = rng.uniform(0.5, 1.5, C).astype(np.float32)
+    bn.backward_stage1(x_t, dy_t, *(torch.from_numpy(v).cuda() for v in (mean, var, scale)), *g.split(C))
+    for got, ref, name in zip(g.split(C), O.bn_backprop1(x, dy, mean, var, scale, 1e-5), ("dscale", "dbias", "dmean", "dvar")):
+        emu.assert_close(got.cpu().numpy(), ref, 2e-5, name)
+
+
 def test_ends_of_unaligned_runs_are_summed_with_their_half():
     """A plane of 1300 pieces of four and three elements: the thread that has those three, in the second half
     of its unit, has whole pieces of large values that cancel in the first."""

@@ -88,6 +88,42 @@ def test_runs_off_16_byte_boundaries(shape, sgrid, dgrid, dov):
     test_forward_and_backward(shape, sgrid, dgrid, dov)
 
 
+@pytest.mark.parametrize("src_off,dst_off", [(1, 0), (0, 2), (3, 1)])
+@pytest.mark.parametrize("shape,dgrid,dov", [
+    ([16, 8, 4, 3, 2], [2, 1, 1, 1, 1], [0, 0, 0, 0, 0]),     # runs of 8 cells
+    ([8, 8, 4, 3, 2], [2, 1, 1, 1, 1], [0, 0, 0, 0, 0]),      # of 4: cell by cell
+    ([24, 20, 6, 3, 2], [1, 2, 1, 1, 1], [0, 1, 0, 0, 0]),    # rows merged
+    ([64, 72, 6, 2, 2], [1, 1, 2, 1, 1], [0, 0, 1, 0, 0]),    # long runs
+])
+def test_tensors_off_16_byte_boundaries(shape, dgrid, dov, src_off, dst_off):
+    """Everything is a multiple of 16 bytes but the tensors' own addresses: 16-byte accesses are out, pieces are not."""
+    sgrid, g = [1, 1, 1, 1, 2], np.random.default_rng(2).normal(size=tuple(reversed(shape))).astype(np.float32)
+    srcs, dsts, backs = ([_tensor(shape, grid, ov, loc) for loc in emu.locales(2)]
+                         for grid, ov in ((sgrid, [0] * 5), (dgrid, dov), (sgrid, [0] * 5)))
+    for ts, off in ((srcs, src_off), (dsts, dst_off), (backs, src_off)):
+        for t in ts:
+            emu.allocate_off_boundary(t, off)
+            t.buffer.fill_(-7.0)
+    for t in srcs:
+        emu.scatter_owned_into(t, g)
+    shufflers = [dc.TensorShuffler(s, d, connect=False) for s, d in zip(srcs, dsts)]
+    for which, a, b in (("fwd", srcs, dsts), ("bwd", dsts, backs)):
+        blobs = [sh.export(which) for sh in shufflers]
+        for sh in shufflers:
+            sh.connect(which, blobs)
+        for sh, t in zip(shufflers, a):
+            sh.put(which, t.get_buffer())
+        for sh, t in zip(shufflers, b):
+            sh.wait_unpack(which, t.get_buffer())
+        torch.cuda.synchronize()
+        assert np.array_equal(emu.gather_owned(b, g.shape), g)
+        for t in b:  # halo cells untouched
+            own = torch.zeros_like(t.buffer, dtype=torch.bool)
+            own[t._geo().owned] = True
+            assert bool((t.buffer[~own] == -7.0).all())
+        assert all(sh.status(which) == _abi.OK for sh in shufflers)
+
+
 def test_wait_expires_with_status_when_a_sender_never_comes():
     """A rank whose peer never puts gets DCB_PEER_TIMEOUT from the bounded wait,
     not a hang, and the destination stays as it was."""

@@ -40,6 +40,8 @@ def _stats_noalloc(t):
 @pytest.mark.parametrize("shape,locale,overlap", [
     ([64, 48, 40, 16, 1], [1, 1, 1, 1, 1], [0, 0, 0, 0, 0]),   # dense, float4 path
     ([33, 9, 6, 3, 2], [1, 1, 2, 1, 1], [0, 0, 1, 0, 0]),       # halo in D, scalar path
+    ([67, 83, 3, 5, 2], [1, 1, 1, 1, 1], [0, 0, 0, 0, 0]),      # planes of odd size, in pieces of four
+    ([67, 166, 3, 2, 2], [1, 2, 1, 1, 1], [0, 1, 0, 0, 0]),     # the same, several runs a plane
 ])
 def test_noalloc_matches_planned_stats_twice(shape, locale, overlap):
     rng = np.random.default_rng(0)
