@@ -30,6 +30,8 @@ constexpr int BN_UNROLL_RED = 8;
 // 67 x 83 x 101: statistics 34.9 -> 30.7 us, backward sums 57.8 -> 54.2 us).
 template <int V>
 constexpr int bn_unroll_red = V == 1 ? 2 * BN_UNROLL_RED : BN_UNROLL_RED;
+// ... and 4 where vectors are pieces of unaligned runs (see Piece), or 8 (make_multi).
+constexpr int BN_UNROLL_PIECES = 4;
 
 struct UnitGeom
 {
@@ -200,7 +202,20 @@ struct Piece
         lo = e < 0 ? head : 0;
         hi = len - e < 4 ? (int) (len - e > 0 ? len - e : 0) : 4;
     }
-    __device__ __forceinline__ bool whole() const { return lo == 0 && hi == 4; }
+    __device__ __forceinline__ bool any() const { return lo < hi; }
+    // Element i of the four is the run's.
+    __device__ __forceinline__ bool has(int i) const { return i >= lo && i < hi; }
+    // Zeros stand for the others.  (Nothing is added up here: the loads of all of a thread's
+    // pieces are in flight together.)
+    __device__ __forceinline__ void load(const float* run, Vec<4>* v) const
+    {
+        if (lo == 0 && hi == 4)
+            v->load(run + e);
+        else
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                v->v[i] = has(i) ? run[e + i] : 0.f;
+    }
 };
 
 // Sum NV doubles across the block; result valid in thread 0.
@@ -282,13 +297,14 @@ __device__ __forceinline__ void finish_channel(double (&val)[NV],
     }
 }
 
-template <int V, bool PACKED, bool PIECES = false>
+// PIECES: the pieces of four that a thread has in flight, 0: aligned vectors
+template <int V, bool PACKED, int PIECES = 0>
 __global__ void __launch_bounds__(BN_THREADS)
     bn_stats_kernel(const float* __restrict__ x, RunStrides xs, UnitGeom ug,
                     double* partial, unsigned* tickets,
                     float* __restrict__ sums, float* __restrict__ sqsums)
 {
-    constexpr auto half = [](int k) { return PIECES && k >= bn_unroll_red<V> / 2 ? 1 : 0; };
+    constexpr int U = PIECES ? PIECES : bn_unroll_red<V>;
     wait_for_previous_kernel(x);
     const int c = blockIdx.y;
     double acc[2] = {0.0, 0.0};
@@ -297,30 +313,20 @@ __global__ void __launch_bounds__(BN_THREADS)
         const UnitPos p = decode_unit(ug, u);
         const float* xp = x + unit_offset(xs, ug.g, p, c);
         const int nv = p.count / V;
-        Vec<V> v[bn_unroll_red<V>];
-        bool on[bn_unroll_red<V>];
-        // PIECES: each half of the unit has its own, of sixteen elements at most, as element by element.
-        // (With the ends of a run added to the first half's, whichever they lie in, it was nineteen.
-        // 2 x 24 x 67 x 83 x 101, inputs in L2: 20.3 us either way, backward sums 43.3 -> 44.0.)
-        float s[2] = {0.f, 0.f}, q[2] = {0.f, 0.f};
+        Vec<V> v[U];
+        bool on[U];
+        float s = 0.f, q = 0.f;
         const float* run = xp - p.e0;
         const int head = (int) (reinterpret_cast<uintptr_t>(run) >> 2 & 3);
 #pragma unroll
-        for (int k = 0; k < bn_unroll_red<V>; ++k)
+        for (int k = 0; k < U; ++k)
         {
             if (PIECES)
             {
                 const Piece pc(p.e0 / 4 + threadIdx.x + k * BN_THREADS, head, ug.g.len);
-                on[k] = pc.whole();
-                if (on[k])
-                    v[k].load(run + pc.e);
-                else
-                    for (int i = pc.lo; i < pc.hi; ++i)
-                    {
-                        const float f = run[pc.e + i];
-                        s[half(k)] += f;
-                        q[half(k)] = fmaf(f, f, q[half(k)]);
-                    }
+                on[k] = pc.any();
+                if constexpr (PIECES)
+                    pc.load(run, &v[k]);
                 continue;
             }
             const ElemPos ep = elem_pos<PACKED>(ug, p, threadIdx.x + k * BN_THREADS, nv);
@@ -329,19 +335,22 @@ __global__ void __launch_bounds__(BN_THREADS)
                 v[k].load(xp + ep.template off<V>(xs));
         }
 #pragma unroll
-        for (int k = 0; k < bn_unroll_red<V>; ++k)
+        for (int k = 0; k < U; ++k)
+        {
             if (on[k])
 #pragma unroll
                 for (int i = 0; i < V; ++i)
                 {
-                    s[half(k)] += v[k].v[i];
-                    q[half(k)] = fmaf(v[k].v[i], v[k].v[i], q[half(k)]);
+                    s += v[k].v[i];
+                    q = fmaf(v[k].v[i], v[k].v[i], q);
                 }
-#pragma unroll
-        for (int h = 0; h < (PIECES ? 2 : 1); ++h)
-        {
-            acc[0] += (double) s[h];
-            acc[1] += (double) q[h];
+            // (pieces: sums of sixteen in fp32, as element by element)
+            if (k == U - 1 || (PIECES && k % BN_UNROLL_PIECES == BN_UNROLL_PIECES - 1))
+            {
+                acc[0] += (double) s;
+                acc[1] += (double) q;
+                s = q = 0.f;
+            }
         }
     }
     block_reduce<2>(acc);
@@ -484,7 +493,7 @@ __global__ void __launch_bounds__(BN_THREADS)
     }
 }
 
-template <int V, bool PACKED, bool PIECES = false>
+template <int V, bool PACKED, int PIECES = 0>
 __global__ void __launch_bounds__(BN_THREADS)
     bn_bwd_reduce_kernel(const float* __restrict__ x, RunStrides xs,
                          const float* __restrict__ dy, RunStrides ds,
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(BN_THREADS)
                          float* __restrict__ dscale, float* __restrict__ dbias,
                          float* __restrict__ dmean, float* __restrict__ dvar)
 {
-    constexpr auto half = [](int k) { return PIECES && k >= bn_unroll_red<V> / 2 ? 1 : 0; };
+    constexpr int U = PIECES ? PIECES : bn_unroll_red<V>;
     wait_for_previous_kernel(x, dy, mean, var, scale);
     const int c = blockIdx.y;
     const float m = mean[c];
@@ -509,35 +518,32 @@ __global__ void __launch_bounds__(BN_THREADS)
         const float* xp = x + unit_offset(xs, ug.g, p, c);
         const float* dp = dy + unit_offset(ds, ug.g, p, c);
         const int nv = p.count / V;
-        Vec<V> vx[bn_unroll_red<V>], vd[bn_unroll_red<V>];
-        bool on[bn_unroll_red<V>];
-        float a[2][4] = {}; // (see bn_stats_kernel)
-        auto add = [&](int h, float xv, float g) {
+        Vec<V> vx[U], vd[U];
+        bool on[U];
+        float a[4] = {};
+        auto add = [&](float xv, float g) {
             // backprop1 (batchnorm.cu:940-952)
             const float xhat = (xv - m) * inv_stdev;
-            a[h][0] += g * xhat;
-            a[h][1] += g;
+            a[0] += g * xhat;
+            a[1] += g;
             const float dxhat = g * sc;
-            a[h][2] += -dxhat * inv_stdev;
-            a[h][3] += -dxhat * (xv - m) * dvar_factor;
+            a[2] += -dxhat * inv_stdev;
+            a[3] += -dxhat * (xv - m) * dvar_factor;
         };
         const float *xrun = xp - p.e0, *drun = dp - p.e0;
         const int head = (int) (reinterpret_cast<uintptr_t>(xrun) >> 2 & 3);
 #pragma unroll
-        for (int k = 0; k < bn_unroll_red<V>; ++k)
+        for (int k = 0; k < U; ++k)
         {
             if (PIECES)
             {
                 const Piece pc(p.e0 / 4 + threadIdx.x + k * BN_THREADS, head, ug.g.len);
-                on[k] = pc.whole();
-                if (on[k])
+                on[k] = pc.any();
+                if constexpr (PIECES)
                 {
-                    vx[k].load(xrun + pc.e);
-                    vd[k].load(drun + pc.e);
+                    pc.load(xrun, &vx[k]);
+                    pc.load(drun, &vd[k]);
                 }
-                else
-                    for (int i = pc.lo; i < pc.hi; ++i)
-                        add(half(k), xrun[pc.e + i], drun[pc.e + i]);
                 continue;
             }
             const ElemPos ep = elem_pos<PACKED>(ug, p, threadIdx.x + k * BN_THREADS, nv);
@@ -549,16 +555,18 @@ __global__ void __launch_bounds__(BN_THREADS)
             }
         }
 #pragma unroll
-        for (int k = 0; k < bn_unroll_red<V>; ++k)
+        for (int k = 0; k < U; ++k)
             if (on[k])
+            {
+                const Piece pc(p.e0 / 4 + threadIdx.x + k * BN_THREADS, head, ug.g.len);
 #pragma unroll
                 for (int i = 0; i < V; ++i)
-                    add(half(k), vx[k].v[i], vd[k].v[i]);
+                    if (!PIECES || pc.has(i)) // (an infinite mean times a zero that stands for no element is none)
+                        add(vx[k].v[i], vd[k].v[i]);
+            }
 #pragma unroll
-        for (int h = 0; h < (PIECES ? 2 : 1); ++h)
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                acc[i] += (double) a[h][i];
+        for (int i = 0; i < 4; ++i)
+            acc[i] += (double) a[i];
     }
     block_reduce<4>(acc);
     finish_channel<4>(acc, partial, tickets, [&](const double(&t)[4]) {
@@ -684,7 +692,7 @@ struct MultiView
     UnitGeom ug;
     RunStrides s[3];
     int vec;
-    bool pieces; // reductions: aligned pieces of four (see Piece), in units of 16-byte vectors
+    int pieces; // reductions: aligned pieces of four (see Piece), so many a thread
 };
 
 // Whether all tensors' runs start equally far above a 16-byte boundary.
@@ -731,13 +739,29 @@ static int32_t make_multi(const dcb_nd_desc* const* descs,
     }
     mv->ug = make_units(g, vec, vec == 1 ? unroll1 : unroll);
     mv->vec = vec;
-    // Shorter runs are mostly their partial ends.  2 x 24 x 67 x 83 x 101, element by element / in
-    // pieces: statistics 31.4 / 22.2 us, backward sums 53.6 / 51.0.
-    mv->pieces = reduction && vec == 1 && mv->ug.vpr == 0 && g.len >= 1024 && pieces_fit(*mv, ptrs, count);
+    // Pieces, us element by element / with eight a thread / with four, with inputs that have left L2
+    // (in brackets: with those that have not):
+    //   statistics     2 x 24 x 67 x 83 x 101  38.9 / 30.7 / -    (28.0 / 19.1 / 22.8)
+    //                  8 x 128 x 41 x 67       14.4 / 14.4 / 12.3 (8.4 / 8.5 / 6.5)
+    //                  16 x 256 x 33 x 33      24.5 / 30.7 / 20.5 (14.7 / 20.2 / 15.1)
+    //   backward sums  2 x 24 x 67 x 83 x 101  60.4 / 57.3 / 53.3 (44.2 / 43.6 / 38.1)
+    //                  8 x 128 x 3 x 67 x 83   46.0 / 49.2 / 40.9 (33.1 / 39.0 / 29.1)
+    //                  16 x 32 x 3 x 67 x 83   31.6 / 32.8 / 27.7 (16.2 / 21.5 / 17.0)
+    //                  16 x 128 x 41 x 51      22.5 / 34.8 / 22.5 (13.0 / 23.8 / 13.7)
+    //                  16 x 256 x 33 x 33      26.7 / 53.2 / 29.7 (19.1 / 38.5 / 20.8)
+    // Shorter runs are mostly their ends.  The backward sums never take eight: 107 registers, two blocks
+    // an SM (four: 60).  The statistics do where two thirds of such a unit's threads have work.
+    mv->pieces = reduction && vec == 1 && mv->ug.vpr == 0 && g.len >= (count == 1 ? 1024 : 2048) && pieces_fit(*mv, ptrs, count)
+                     ? BN_UNROLL_PIECES
+                     : 0;
     if (mv->pieces)
     {
-        mv->ug.unit = BN_THREADS * unroll * 4;
-        mv->ug.upr = ((g.len + 6) / 4 + BN_THREADS * unroll - 1) / (BN_THREADS * unroll);
+        const long long n = (g.len + 6) / 4, large = BN_THREADS * 2 * BN_UNROLL_PIECES;
+        if (count == 1 && 3 * n >= 2 * large * ((n + large - 1) / large))
+            mv->pieces = 2 * BN_UNROLL_PIECES;
+        const long long unit = BN_THREADS * mv->pieces;
+        mv->ug.unit = (int) unit * 4;
+        mv->ug.upr = (n + unit - 1) / unit;
         mv->ug.upc = g.n * g.rows * mv->ug.upr;
     }
     DCB_REQUIRE(g.c <= 65535, "too many channels");
@@ -853,9 +877,13 @@ int32_t dcb_bn_stats(dcb_bn_plan* plan, const void* x, void* sums,
     DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, __VA_ARGS__>), grid, BN_THREADS, 0, as_stream(stream),           \
         static_cast<const float*>(x), mv.s[0], mv.ug, plan->partial,           \
         plan->tickets, static_cast<float*>(sums), static_cast<float*>(sqsums)))
-    if (mv.pieces)
+    if (mv.pieces == BN_UNROLL_PIECES)
     {
-        CALL(4, false, true);
+        CALL(4, false, BN_UNROLL_PIECES);
+    }
+    else if (mv.pieces)
+    {
+        CALL(4, false, 2 * BN_UNROLL_PIECES);
     }
     else
         DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
@@ -983,7 +1011,7 @@ int32_t dcb_bn_bwd_reduce(dcb_bn_plan* plan, const void* x,
         static_cast<float*>(dvar)))
     if (mv.pieces)
     {
-        CALL(4, false, true);
+        CALL(4, false, BN_UNROLL_PIECES);
     }
     else
         DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);
@@ -1156,9 +1184,13 @@ extern "C" int32_t dcb_bn_stats_noalloc(const dcb_nd_desc* xd, const void* x, vo
     DCB_CUDA_TRY(launch_overlapped((bn_stats_kernel<VV, __VA_ARGS__>), grid, BN_THREADS, 0, as_stream(stream),           \
         static_cast<const float*>(x), mv.s[0], mv.ug, partial, tickets,        \
         static_cast<float*>(sums), static_cast<float*>(sqsums)))
-    if (mv.pieces)
+    if (mv.pieces == BN_UNROLL_PIECES)
     {
-        CALL(4, false, true);
+        CALL(4, false, BN_UNROLL_PIECES);
+    }
+    else if (mv.pieces)
+    {
+        CALL(4, false, 2 * BN_UNROLL_PIECES);
     }
     else
         DCB_VEC_DISPATCH(mv.vec, mv.ug.vpr != 0, CALL);

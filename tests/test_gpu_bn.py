@@ -89,9 +89,13 @@ def test_bn_forward_backward_local(shape, locale, overlap):
 
 
 @pytest.mark.parametrize("shape", [
-    [41, 25, 1, 3, 2],   # 1025 elements a plane: just long enough for pieces of four, every start
-    [91, 89, 1, 5, 1],   # 8099: the pieces of one unit and its last, partial one
-    [91, 91, 1, 4, 2],   # 8281: a second unit of 23 pieces
+    [41, 25, 1, 3, 2],   # 1025 elements a plane: just long enough for the statistics in pieces of four, every start
+    [89, 23, 1, 3, 2],   # 2047 and 2049: on either side of what is long enough for the backward sums
+    [683, 3, 1, 3, 2],
+    [321, 17, 1, 3, 1],  # 5457 and 5459: on either side of eight pieces a thread
+    [103, 53, 1, 4, 1],
+    [91, 89, 1, 5, 1],   # 8099: the pieces of one or two units and the last, partial one
+    [91, 91, 1, 4, 2],   # 8281: a last unit of 23 pieces
     [67, 83, 3, 2, 2],
 ])
 def test_planes_of_odd_size(shape):
@@ -129,14 +133,14 @@ def test_sums_of_planes_of_odd_size_wherever_they_lie(x_off, dy_off):
 
 
 def test_ends_of_unaligned_runs_are_summed_with_their_half():
-    """A plane of 1300 pieces of four and three elements: the thread that has those three, in the second half
-    of its unit, has whole pieces of large values that cancel in the first."""
-    H, W = 43, 121  # 5203
+    """A plane of 1800 pieces of four and three elements, in one unit of the statistics: the thread that has
+    those three in the second half of its eight pieces has large values that cancel in the first."""
+    H, W = 49, 147  # 7203
     be = dc.BackendDNNLib(dc.Locale(0, 1))
     x_t, dy_t = (_rank0([W, H, 1, 1], [1] * 4, [0] * 4) for _ in range(2))
     big = np.zeros(H * W, np.float32)
     big[:4096:2], big[1:4096:2] = 2.0 ** 26, -(2.0 ** 26)
-    big[5200:] = 1.0
+    big[7200:] = 1.0
     for t in (x_t, dy_t):
         emu.upload(t, big.reshape(1, 1, H, W))
     bn = dc.BatchNormalization(be, 4, decay=0.9, epsilon=1e-5, global_stats=False)
