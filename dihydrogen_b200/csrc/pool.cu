@@ -141,17 +141,18 @@ __global__ void __launch_bounds__(POOL_THREADS)
     *yp = beta != 0.f ? alpha * r + beta * *yp : alpha * r;
 }
 
-// The same for the common windows, four neighbouring outputs a thread: a window row's cells are
-// loaded once for all four and the addresses worked out once.  Same scan order, same bits (us, an
-// output a thread before: 8 x 128^3, 3 / 1, averages 309 -> 124; 16 x 64 x 100 x 90, 2 / 2, maxima
-// 19.6 -> 12.8, 3 / 1 182 -> 155).
-template <int WD, int W, int S, bool MAXP>
+// The same for the common windows, O neighbouring outputs a thread (launch_pool_general): a window
+// row's cells are loaded once for all of them and the addresses worked out once.  Same scan order,
+// same bits.  Bound by what a thread does per cell.  (us, an output a thread with a check per cell
+// before: 8 x 128^3, 3 / 1, averages 309 -> 124; 16 x 64 x 100 x 90, maxima, 2 / 2 18.5 -> 11.8, 3 / 1 177 -> 133;
+// 4 x 16^3, maxima, 3 / 1 4.2 -> 3.9.)
+template <int WD, int W, int S, bool MAXP, int O>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_fwd_cells_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ x, float* y,
                           unsigned char* __restrict__ argmax, int tw_log2, long long rows)
 {
-    constexpr int SD = WD == 1 ? 1 : S, NC = 3 * S + W; // cells behind four outputs
-    const int ow0 = ((blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1))) * 4;
+    constexpr int SD = WD == 1 ? 1 : S, NC = (O - 1) * S + W; // cells behind O outputs
+    const int ow0 = ((blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1))) * O;
     const long long row = (long long) blockIdx.x * (POOL_THREADS >> tw_log2) + (threadIdx.x >> tw_log2);
     if (ow0 >= g.out[2] || row >= rows)
         return;
@@ -161,10 +162,11 @@ __global__ void __launch_bounds__(POOL_THREADS)
     const int d0 = od * SD - g.pad[0], h0 = oh * S - g.pad[1], w0 = ow0 * S - g.pad[2];
     const float* xp = x + (size_t) n * g.xs_n + (size_t) c * g.xs_c + (long long) d0 * g.xs[0] + (long long) h0 * g.xs[1] + w0;
     const bool all = w0 >= g.lo[2] && w0 + NC <= g.hi[2]; // every cell exists
-    float r[4];
-    int best[4];
+    float r[O];
+    int best[O];
+    bool first = true;
 #pragma unroll
-    for (int o = 0; o < 4; ++o)
+    for (int o = 0; o < O; ++o)
         r[o] = MAXP ? -FLT_MAX : 0.f, best[o] = -1;
 #pragma unroll
     for (int kd = 0; kd < WD; ++kd)
@@ -181,35 +183,49 @@ __global__ void __launch_bounds__(POOL_THREADS)
             const bool row_in = h0 + kh >= g.lo[1] && h0 + kh < g.hi[1];
 #pragma unroll
             for (int i = 0; i < NC; ++i)
-                v[kh][i] = row_in && (all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) ? __ldg(rp + i) : 0.f;
+                v[kh][i] = row_in && (all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) ? __ldg(rp + i) : (MAXP ? -INFINITY : 0.f);
         }
 #pragma unroll
         for (int kh = 0; kh < W; ++kh)
         {
             if (h0 + kh < g.lo[1] || h0 + kh >= g.hi[1])
                 continue;
+            if (MAXP && first)
+            {
+                // the first cell that exists, whatever it holds (a NaN stays the maximum)
+                first = false;
 #pragma unroll
-            for (int o = 0; o < 4; ++o)
+                for (int o = 0; o < O; ++o)
+#pragma unroll
+                    for (int kw = W - 1; kw >= 0; --kw)
+                        if (all || (w0 + o * S + kw >= g.lo[2] && w0 + o * S + kw < g.hi[2]))
+                        {
+                            r[o] = v[kh][o * S + kw];
+                            best[o] = (kd * W + kh) * W + kw;
+                        }
+            }
+#pragma unroll
+            for (int o = 0; o < O; ++o)
 #pragma unroll
                 for (int kw = 0; kw < W; ++kw)
                 {
-                    const int i = o * S + kw;
+                    // (cells that do not exist add nothing and are no greater than any)
                     if (!MAXP)
-                        r[o] += v[kh][i]; // (cells that do not exist are zeros)
-                    else if ((all || (w0 + i >= g.lo[2] && w0 + i < g.hi[2])) && (best[o] < 0 || v[kh][i] > r[o]))
+                        r[o] += v[kh][o * S + kw];
+                    else if (v[kh][o * S + kw] > r[o])
                     {
-                        r[o] = v[kh][i];
+                        r[o] = v[kh][o * S + kw];
                         best[o] = (kd * W + kh) * W + kw;
                     }
                 }
         }
     }
-    const int left = min(4, g.out[2] - ow0);
+    const int left = min(O, g.out[2] - ow0);
     if (argmax)
     {
         unsigned char* ap = argmax + ((((size_t) n * g.c + c) * g.out[0] + od) * g.out[1] + oh) * g.out[2] + ow0;
 #pragma unroll
-        for (int o = 0; o < 4; ++o)
+        for (int o = 0; o < O; ++o)
             if (o < left)
                 ap[o] = (unsigned char) best[o];
         if (!y)
@@ -217,7 +233,7 @@ __global__ void __launch_bounds__(POOL_THREADS)
     }
     float* yp = y + (size_t) n * g.ys_n + (size_t) c * g.ys_c + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1] + ow0;
 #pragma unroll
-    for (int o = 0; o < 4; ++o)
+    for (int o = 0; o < O; ++o)
         if (o < left)
         {
             const float q = MAXP ? r[o] : r[o] / fmaxf(pool_count(g, od, oh, ow0 + o), 1.f);
@@ -1142,15 +1158,43 @@ bool pool_grid(int w, long long rows, long long planes, dim3* grid)
             DCB_POOL_CALL(0, 0, 0);                                                                                   \
     } while (0)
 
+template <int WD, int W, int S, int O>
+void launch_pool_cells(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax, long long rows,
+                       unsigned planes, cudaStream_t stream)
+{
+    const int threads = (g.out[2] + O - 1) / O; // a row needs
+    int tw_log2 = 8;
+    while (tw_log2 > 2 && (1 << (tw_log2 - 1)) >= threads)
+        --tw_log2;
+    const long long rpb = POOL_THREADS >> tw_log2;
+    // (as many blocks in x and y as the caller's grid has, or fewer)
+    const dim3 grid((unsigned) ((rows + rpb - 1) / rpb), (unsigned) ((threads + (1 << tw_log2) - 1) >> tw_log2), planes);
+    (g.mode == DCB_POOL_MAX ? pool_fwd_cells_kernel<WD, W, S, true, O> : pool_fwd_cells_kernel<WD, W, S, false, O>)
+        <<<grid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, tw_log2, rows);
+}
+
 template <int WD, int W, int S>
-void launch_pool_cells(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax, dim3 qgrid,
-                       int qw_log2, dim3 grid, int tw_log2, long long rows, cudaStream_t stream)
+void launch_pool_general(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax, dim3 grid,
+                         int tw_log2, long long rows, cudaStream_t stream)
 {
     if constexpr (WD == 0)
         pool_fwd_kernel<<<grid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, tw_log2, rows);
     else
-        (g.mode == DCB_POOL_MAX ? pool_fwd_cells_kernel<WD, W, S, true> : pool_fwd_cells_kernel<WD, W, S, false>)
-            <<<qgrid, POOL_THREADS, 0, stream>>>(g, alpha, beta, x, y, argmax, qw_log2, rows);
+    {
+        // Outputs a thread, us with 1 / 2 / 4 (maxima).  Few outputs: latency, 4 x 16^3, 3 / 1 3.9 / 4.3 /
+        // 4.9, 4 x 93 x 19 x 57, 2 / 2 2.9 / 3.1 / 3.5.  Stride 1: what neighbours share, 16 x 64 x 100 x
+        // 90, 3 / 1 199 / 173 / 133.  Stride 2: they share a cell or none, and two keep twice the threads
+        // in flight, 4 x 58 x 108 x 238, 2 / 2 10.4 / 7.8 / 9.6, 3 / 2 17.6 / 13.3 / 19.9; but large tensors
+        // of rows that do not fill a warp like that, 64 x 78 x 62 x 47, 2 / 2 26.7 / 19.5 / 16.4, 3 / 2, pad 1
+        // 55.0 / 38.9 / 33.1.
+        const long long outs = rows * g.out[2] * grid.z;
+        if (outs <= 65536)
+            launch_pool_cells<WD, W, S, 1>(g, alpha, beta, x, y, argmax, rows, grid.z, stream);
+        else if (S > 1 && (outs < 300000 || g.out[2] >= 63))
+            launch_pool_cells<WD, W, S, 2>(g, alpha, beta, x, y, argmax, rows, grid.z, stream);
+        else
+            launch_pool_cells<WD, W, S, 4>(g, alpha, beta, x, y, argmax, rows, grid.z, stream);
+    }
 }
 
 int32_t launch_pool_fwd(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax,
@@ -1201,13 +1245,7 @@ int32_t launch_pool_fwd(const PoolGeom& g, float alpha, float beta, const float*
         DCB_LAUNCH_CHECK();
         return DCB_OK;
     }
-    const int quads = (g.out[2] + 3) / 4;
-    int qw_log2 = 8;
-    while (qw_log2 > 2 && (1 << (qw_log2 - 1)) >= quads)
-        --qw_log2;
-    const long long qpb = POOL_THREADS >> qw_log2;
-    const dim3 qgrid((unsigned) ((rows + qpb - 1) / qpb), (unsigned) ((quads + (1 << qw_log2) - 1) >> qw_log2), (unsigned) planes);
-#define DCB_POOL_CALL(WD, W, S) launch_pool_cells<WD, W, S>(g, alpha, beta, x, y, argmax, qgrid, qw_log2, grid, tw_log2, rows, stream)
+#define DCB_POOL_CALL(WD, W, S) launch_pool_general<WD, W, S>(g, alpha, beta, x, y, argmax, grid, tw_log2, rows, stream)
     DCB_POOL_DISPATCH(g);
 #undef DCB_POOL_CALL
     DCB_LAUNCH_CHECK();

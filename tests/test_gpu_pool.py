@@ -105,6 +105,61 @@ def test_rows_of_all_lengths(window, pad, stride, widths, mode):
                 test_kernels_against_oracle((1, 2, sp, *([v] * len(sp) for v in (window, pad, stride))), mode)
 
 
+# outputs a thread: two and four (fewer than 65537 outputs, as everywhere else here, take one)
+MANY_OUTPUTS = [
+    (1, 4, (42, 43, 81), (2, 2, 2), (0, 0, 0), (2, 2, 2)),    # two, stride 2: 70560 outputs
+    (1, 7, (21, 71, 89), (3, 3, 3), (1, 1, 1), (2, 2, 2)),    # two, rows off 16-byte boundaries
+    (2, 5, (131, 257), (3, 3), (0, 0), (2, 2)),               # two, images
+    (2, 16, (30, 50, 53), (2, 2, 2), (0, 0, 0), (2, 2, 2)),   # four, stride 2: 312000 outputs in short rows
+    (1, 3, (16, 31, 46), (3, 3, 3), (1, 1, 1), (1, 1, 1)),    # four, stride 1: 68448 outputs
+    (3, 2, (111, 101), (3, 3), (1, 1), (1, 1)),
+]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("case", MANY_OUTPUTS)
+def test_many_outputs(case, mode):
+    test_kernels_against_oracle(case, mode)
+
+
+@pytest.mark.parametrize("case", MANY_OUTPUTS + [
+    (2, 2, (5, 6, 7), (2, 2, 2), (0, 0, 0), (2, 2, 2)), (1, 2, (5, 8, 9), (3, 3, 3), (1, 1, 1), (2, 2, 2)),
+    (1, 2, (4, 9, 33), (3, 3, 3), (1, 1, 1), (1, 1, 1)), (2, 2, (13, 6), (3, 3), (1, 1), (1, 1)),
+])
+def test_maxima_of_infinities_and_nans(case):
+    """A window's cells in order: the first one, whatever it is, then every one that is greater."""
+    N, C, sp, window, pads, strides = case
+    rng = np.random.default_rng(5)
+    x = rng.integers(-3, 3, size=(N, C, *sp)).astype(np.float32)
+    u = rng.random(x.shape)
+    for lo, value in ((.1, -np.inf), (.3, np.float32(-3.4028234663852886e38)), (.5, np.nan), (.6, np.inf), (.7, -0.0)):
+        x[(u > lo) & (u < lo + .08)] = value
+    x[:, 0, :3] = -np.inf
+    nsd = len(sp)
+    w3, p3, s3 = ([a] * (3 - nsd) + list(v) for a, v in ((1, window), (0, pads), (1, strides)))
+    vals, where, out = O._pool_windows(O._as5(x), w3, p3, s3)
+    r, best = np.full(vals.shape[1:], -3.4028234663852886e38), np.full(vals.shape[1:], -1)
+    for v, at in zip(vals, where):
+        with np.errstate(invalid="ignore"):
+            take = (at >= 0) & ((best < 0) | (v > r))
+        r, best = np.where(take, v, r), np.where(take, at, best)
+    xs = torch.from_numpy(x).cuda()
+    y = torch.zeros((N, C, *out[3 - nsd:]), device="cuda")
+    dys, dx = torch.randn_like(y), torch.full_like(xs, 9.0)
+    pd, xd, yd = _pd(window, pads, strides, "MAX"), _nd(xs), _nd(y)
+    P = lambda t: ctypes.c_void_p(t.data_ptr())
+    _abi.call("dcb_pool_fwd", ctypes.byref(pd), ctypes.byref(xd), ctypes.byref(yd), 1.0, P(xs), 0.0, P(y), None)
+    ws = torch.empty(y.numel(), dtype=torch.uint8, device="cuda")
+    _abi.call("dcb_pool_bwd", ctypes.byref(pd), ctypes.byref(xd), ctypes.byref(yd), 1.0, P(y), P(dys), P(xs), 0.0, P(dx),
+              P(ws), ws.numel(), None)
+    assert np.array_equal(y.cpu().numpy().reshape(r.shape), r.astype(np.float32), equal_nan=True)
+    dx_ref = np.zeros((N, C, x[0, 0].size))
+    for i in range(N):
+        for j in range(C):
+            np.add.at(dx_ref[i, j], best[i, j].ravel(), dys[i, j].cpu().numpy().ravel())
+    emu.assert_close(dx.cpu().numpy(), dx_ref.reshape(x.shape).astype(np.float32), 2e-6, "dx")
+
+
 # window 3, stride 2: walks of several outputs along D (the last one shorter), one walk
 # per output, an odd row end, no padding along D
 @pytest.mark.parametrize("n,c,sp,pad_d", [(1, 512, (37, 31, 20), 1), (2, 512, (24, 9, 8), 0), (1, 2, (6, 5, 264), 1),
