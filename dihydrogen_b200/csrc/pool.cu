@@ -61,6 +61,8 @@ __device__ __forceinline__ int pool_extent(const PoolGeom& g, int i, int o)
 
 __device__ __forceinline__ float pool_count(const PoolGeom& g, int od, int oh, int ow)
 {
+    if (g.mode == DCB_POOL_AVERAGE)
+        return (float) (g.win[0] * g.win[1] * g.win[2]);
     return (float) (pool_extent(g, 0, od) * pool_extent(g, 1, oh) * pool_extent(g, 2, ow));
 }
 
@@ -710,35 +712,38 @@ __global__ void __launch_bounds__(POOL_THREADS)
     dx[me] = beta != 0.f ? alpha * acc + beta * dx[me] : alpha * acc;
 }
 
-// Backward for any window: averages, and maxima by the index workspace.  A thread owns four
+// Backward for any window: averages, and maxima by the index workspace.  A thread owns E
 // consecutive cells of an input row and walks the windows that hold the row, each gradient (and
-// index byte, or quotient) once for all four cells.  Short rows share a block.  Bound by
+// index byte, or quotient) once for all of them.  Short rows share a block; with UNIFORM a block is
+// one row, and what depends on the row is worked out once for all its threads (rows of more than 128
+// cells; us, rows sharing a block / like this: maxima, 3 / 2, 32 x 27 x 120 x 181 218 / 191, 8 x 112 x 59 x
+// 157 112 / 101, averages 75.7 / 67.4; the loops of a general window gain nothing).  Bound by
 // instruction issue: what a thread does per window is what counts (us, a cell a thread for averages
 // and one row a block before: 2 x 16 x 100 x 96 x 128, 3 / 2, averages 644 -> 217; 8 x 128^3, 3 / 1,
 // averages 940 -> 411; 16 x 64 x 100 x 90, 2 / 2, maxima 68 -> 54; 4 x 30 x 30 x 31, 3 / 1, 28.5 -> 9).
-template <int WD, int W, int S, bool MAXP>
+template <int WD, int W, int S, bool MAXP, int E, bool UNIFORM>
 __global__ void __launch_bounds__(POOL_THREADS)
     pool_bwd_cells_kernel(PoolGeom g, float alpha, float beta, const float* __restrict__ dy, float* dx,
                           const unsigned char* __restrict__ argmax, int tw_log2, long long rows)
 {
     const int w0_ = WD ? WD : g.win[0], w1_ = W ? W : g.win[1], w2_ = W ? W : g.win[2];
     const int s0_ = S ? (WD == 1 ? 1 : S) : g.stride[0], s1_ = S ? S : g.stride[1], s2_ = S ? S : g.stride[2];
-    const int iw0 = ((blockIdx.y << tw_log2) + (threadIdx.x & ((1 << tw_log2) - 1))) * 4;
-    const long long row = (long long) blockIdx.x * (POOL_THREADS >> tw_log2) + (threadIdx.x >> tw_log2);
+    const int iw0 = ((blockIdx.y << tw_log2) + (UNIFORM ? threadIdx.x : threadIdx.x & ((1 << tw_log2) - 1))) * E;
+    const long long row = UNIFORM ? blockIdx.x : (long long) blockIdx.x * (POOL_THREADS >> tw_log2) + (threadIdx.x >> tw_log2);
     if (iw0 >= g.in[2] || row >= rows)
         return;
     int id, ih;
     pool_split_row(row, rows, g.in[1], &id, &ih);
     const int c = blockIdx.z % g.c, n = blockIdx.z / g.c;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    float acc[E] = {};
     int dlo, dhi, hlo, hhi;
     pool_cover(id, s0_, g.pad[0], w0_, g.out[0], &dlo, &dhi);
     pool_cover(ih, s1_, g.pad[1], w1_, g.out[1], &hlo, &hhi);
     if (id < g.lo[0] || id >= g.hi[0] || ih < g.lo[1] || ih >= g.hi[1])
         dhi = dlo - 1; // a row outside the global tensor is padding
-    int wlo[4], whi[4], first = g.out[2], last = -1; // windows of each cell, of all
+    int wlo[E], whi[E], first = g.out[2], last = -1; // windows of each cell, of all
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
+    for (int e = 0; e < E; ++e)
     {
         pool_cover(iw0 + e, s2_, g.pad[2], w2_, g.out[2], &wlo[e], &whi[e]);
         if (iw0 + e < g.lo[2] || iw0 + e >= g.hi[2] || iw0 + e >= g.in[2])
@@ -749,7 +754,7 @@ __global__ void __launch_bounds__(POOL_THREADS)
     // stride 1: the loads of all windows along W go out together (maxima of 16 x 64 x 100 x 90
     // 365 -> 325 us, averages of 8 x 128^3 488 -> 411; with stride 2 there are two or three, and
     // a fixed number of them costs more: averages of 2 x 16 x 100 x 96 x 128 231 -> 320)
-    constexpr int M = S == 1 ? W + 3 : 1;
+    constexpr int M = S == 1 ? W + E - 1 : 1;
     const size_t plane = ((size_t) n * g.c + c) * g.out[0];
     const float* dyp = dy + (size_t) n * g.ys_n + (size_t) c * g.ys_c;
     for (int od = dlo; od <= dhi; ++od)
@@ -758,7 +763,8 @@ __global__ void __launch_bounds__(POOL_THREADS)
             const unsigned char* arow = argmax + ((plane + od) * g.out[1] + oh) * g.out[2];
             const float* dyrow = dyp + (size_t) od * g.ys[0] + (size_t) oh * g.ys[1];
             const int tap0 = ((id - (od * s0_ - g.pad[0])) * w1_ + (ih - (oh * s1_ - g.pad[1]))) * w2_ + g.pad[2] + iw0;
-            // (windows of 2 with stride 2: one window a cell, nothing to share; 68 us like that, 60 so)
+            // (windows of 2 with stride 2: one window a cell, nothing to share.  us like that / so: 16 x 256^3
+            // 998 / 928, 64 x 16 x 200 x 130 196 / 173, 64 x 100 x 90 x 16 34 / 33, 16 x 64 x 100 x 90 48 / 50)
             const int cells = MAXP || W == 2 ? 0 : pool_extent(g, 0, od) * pool_extent(g, 1, oh);
             for (int ow0 = first; ow0 <= last; ow0 += M)
             {
@@ -778,16 +784,16 @@ __global__ void __launch_bounds__(POOL_THREADS)
                     if (!MAXP)
                         d[k] /= fmaxf(W == 2 ? pool_count(g, od, oh, ow) : (float) (cells * pool_extent(g, 2, ow)), 1.f);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
+                    for (int e = 0; e < E; ++e)
                         if (ow >= wlo[e] && ow <= whi[e] && (!MAXP || tap[k] == e))
                             acc[e] += d[k];
                 }
             }
         }
     float* xp = dx + (size_t) n * g.xs_n + (size_t) c * g.xs_c + (size_t) id * g.xs[0] + (size_t) ih * g.xs[1] + iw0;
-    if (iw0 + 4 <= g.in[2] && (reinterpret_cast<uintptr_t>(xp) & 15) == 0)
+    if (E == 4 && iw0 + 4 <= g.in[2] && (reinterpret_cast<uintptr_t>(xp) & 15) == 0)
     {
-        float4 o = make_float4(alpha * acc[0], alpha * acc[1], alpha * acc[2], alpha * acc[3]);
+        float4 o = make_float4(alpha * acc[0], alpha * acc[E > 1 ? 1 : 0], alpha * acc[E > 2 ? 2 : 0], alpha * acc[E > 3 ? 3 : 0]);
         if (beta != 0.f)
         {
             const float4 old = *reinterpret_cast<const float4*>(xp);
@@ -801,7 +807,7 @@ __global__ void __launch_bounds__(POOL_THREADS)
     else
     {
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < E; ++e)
             if (iw0 + e < g.in[2])
                 xp[e] = beta != 0.f ? alpha * acc[e] + beta * xp[e] : alpha * acc[e];
     }
@@ -1197,6 +1203,37 @@ void launch_pool_general(const PoolGeom& g, float alpha, float beta, const float
     }
 }
 
+template <int WD, int W, int S, int E, bool UNIFORM>
+void launch_pool_bwd_cells(const PoolGeom& g, float alpha, float beta, const float* dy, float* dx, const unsigned char* idx, int tw_log2,
+                           unsigned planes, cudaStream_t stream)
+{
+    const long long rows = (long long) g.in[0] * g.in[1], rpb = UNIFORM ? 1 : POOL_THREADS >> tw_log2;
+    const int threads = (g.in[2] + E - 1) / E; // a row needs
+    // (as many blocks in x and y as pool_grid has allowed, or fewer)
+    const dim3 grid((unsigned) ((rows + rpb - 1) / rpb), (unsigned) ((threads + (1 << tw_log2) - 1) >> tw_log2), planes);
+    (idx ? pool_bwd_cells_kernel<WD, W, S, true, E, UNIFORM> : pool_bwd_cells_kernel<WD, W, S, false, E, UNIFORM>)
+        <<<grid, UNIFORM ? 1 << tw_log2 : POOL_THREADS, 0, stream>>>(g, alpha, beta, dy, dx, idx, tw_log2, rows);
+}
+
+template <int WD, int W, int S>
+void launch_pool_bwd(const PoolGeom& g, float alpha, float beta, const float* dy, float* dx, const unsigned char* idx, unsigned planes,
+                     cudaStream_t stream)
+{
+    // Few cells: one a thread, latency counts (us, one / four: averages of 4 x 32 x 32, 5 / 1 6.3 / 7.9;
+    // 4 x 16^3, 3 / 1 6.3 / 8.3, maxima 8.1 / 10.4; but 4 x 32^3 10.3 / 8.7 and 13.1 / 11.5).
+    const bool few = (long long) g.in[0] * g.in[1] * g.in[2] * planes <= 32768;
+    const int threads = few ? g.in[2] : (g.in[2] + 3) / 4; // a row needs
+    int tw_log2 = 8;
+    while (tw_log2 > 2 && (1 << (tw_log2 - 1)) >= threads)
+        --tw_log2;
+    if (few)
+        launch_pool_bwd_cells<WD, W, S, 1, false>(g, alpha, beta, dy, dx, idx, tw_log2, planes, stream);
+    else if (W != 0 && tw_log2 >= 6)
+        launch_pool_bwd_cells<WD, W, S, 4, W != 0>(g, alpha, beta, dy, dx, idx, tw_log2, planes, stream);
+    else
+        launch_pool_bwd_cells<WD, W, S, 4, false>(g, alpha, beta, dy, dx, idx, tw_log2, planes, stream);
+}
+
 int32_t launch_pool_fwd(const PoolGeom& g, float alpha, float beta, const float* x, float* y, unsigned char* argmax,
                         cudaStream_t stream)
 {
@@ -1371,17 +1408,9 @@ extern "C" int32_t dcb_pool_bwd(const dcb_pool_desc* pd, const dcb_nd_desc* xd, 
     }
     if (idx || g.mode != DCB_POOL_MAX)
     {
-        const int wcells = (g.in[2] + 3) / 4; // threads a row needs
-        int tw_log2 = 8;
-        while (tw_log2 > 2 && (1 << (tw_log2 - 1)) >= wcells)
-            --tw_log2;
-        const long long rows = (long long) g.in[0] * g.in[1], rpb = POOL_THREADS >> tw_log2;
-        // (as many blocks in x and y as pool_grid has allowed, or fewer)
-        const dim3 grid4((unsigned) ((rows + rpb - 1) / rpb), (unsigned) ((wcells + (1 << tw_log2) - 1) >> tw_log2), grid.z);
 #define DCB_POOL_CALL(WD, W, S)                                                                                       \
-    (idx ? pool_bwd_cells_kernel<WD, W, S, true> : pool_bwd_cells_kernel<WD, W, S, false>)                            \
-        <<<grid4, POOL_THREADS, 0, as_stream(stream)>>>(g, (float) alpha, (float) beta, static_cast<const float*>(dy), \
-                                                       static_cast<float*>(dx), idx, tw_log2, rows)
+    launch_pool_bwd<WD, W, S>(g, (float) alpha, (float) beta, static_cast<const float*>(dy), static_cast<float*>(dx), idx, \
+                              grid.z, as_stream(stream))
         DCB_POOL_DISPATCH(g);
 #undef DCB_POOL_CALL
         DCB_LAUNCH_CHECK();

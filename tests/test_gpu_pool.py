@@ -105,6 +105,18 @@ def test_rows_of_all_lengths(window, pad, stride, widths, mode):
                 test_kernels_against_oracle((1, 2, sp, *([v] * len(sp) for v in (window, pad, stride))), mode)
 
 
+# the same rows where there are more than 32768 cells: backward, four cells a thread, and from 129 on a row a block
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("window,pad,stride,widths", [
+    (2, 0, 2, (3, 8, 9, 129, 258)), (3, 1, 1, (4, 5, 17, 130)), (3, 1, 2, (5, 7, 18, 131, 257)), (4, 2, 2, (3, 8, 133)),
+])
+def test_rows_of_all_lengths_in_larger_tensors(window, pad, stride, widths, mode):
+    for w in widths:
+        sp = (33, -(-32769 // (2 * 33 * w)) + window, w)
+        test_kernels_against_oracle((1, 2, sp, *([v] * 3 for v in (window, pad, stride))), mode)
+    test_kernels_against_oracle((1, 2, (-(-32769 // (2 * widths[-1])) + window, widths[-1]), *([v] * 2 for v in (window, pad, stride))), mode)
+
+
 # outputs a thread: two and four (fewer than 65537 outputs, as everywhere else here, take one)
 MANY_OUTPUTS = [
     (1, 4, (42, 43, 81), (2, 2, 2), (0, 0, 0), (2, 2, 2)),    # two, stride 2: 70560 outputs
