@@ -174,9 +174,9 @@ __device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v)
 // true in the block that arrives last, which then release-stores the peers' flags.  Arriving is
 // a release at device scope: the last block's acquire orders every block's stores, also those
 // into peers' windows, before what it releases at system scope, because releases are cumulative
-// over what happens before them.  With a fence at system scope in every block, of up to 1184, the
-// pack of 32 x 106 x 72 rows of a W face took 9.9 us (now 8.6) and the put of 2 x 8 x 136 x 99 x 40
-// 14.9 (13.2).
+// over what happens before them (run with both ranks on one GPU only).  With a fence at system
+// scope in every block, of up to 1184, the pack of 32 x 106 x 72 rows of a W face took 9.9 us (now
+// 8.6) and the put of 2 x 8 x 136 x 99 x 40 14.9 (13.2).
 __device__ __forceinline__ bool last_block(uint32_t* ticket, uint32_t blocks)
 {
     uint32_t before;

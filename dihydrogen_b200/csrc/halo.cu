@@ -217,10 +217,12 @@ __global__ void __launch_bounds__(HALO_THREADS) halo_kernel(HaloArgs a)
     }
     else
     {
-        // Short runs (a W face is `width` cells of every row): every cell is a
-        // sector of its own, so what counts is how many accesses are in flight and
-        // how little arithmetic stands before them.  Exchange of two ranks, us, with one
-        // access at a time behind a 64-bit division / like this: 16 x 256^3, width 1
+        // Short runs (a W face is `width` cells of every row): a cell that is read brings its
+        // line of 128 bytes from memory (134 MB for 1.05 M rows, 544 bytes apart), one that is
+        // written its sector, there and back.  A kernel that only reads such a column takes 23 us,
+        // one that only writes it 45, with 1 to 16 accesses a thread and 148 to 4096 blocks alike; two
+        // of each are the exchange of two ranks.  What is left is arithmetic and latency: us, with
+        // one access at a time behind a 64-bit division / like this: 16 x 256^3, width 1
         // 156 / 152, width 3 168 / 159; 4 x 128^3 31 / 26.
         const long long total = j.runs * j.len_v;
         const long long step = (long long) gridDim.x * HALO_CHUNK;
