@@ -88,8 +88,9 @@ def test_kernels_against_oracle(case, mode):
     emu.assert_close(dxb.cpu().numpy(), 0.5 * dx_ref - dx0, 4e-6, "dx blend")
 
 
-# four cells a thread: rows around multiples of four and of a block's shares of rows, padding on
-# either side, gaps between windows, a window of each compiled kind and a general one
+# rows around multiples of four and of a block's shares of rows, padding on either side, gaps
+# between windows, a window of each compiled kind and a general one; tensors as small as these
+# take one output and one cell a thread (the larger ones follow)
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("window,pad,stride,widths", [
     (2, 0, 2, (2, 3, 8, 9, 10, 17, 66)),
