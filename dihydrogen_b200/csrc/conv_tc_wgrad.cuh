@@ -104,7 +104,12 @@ struct WgConvArgs
 // a time (w, w + warps; then the next two), loads one pair ahead.  A lane is four
 // positions of one channel or filter; the cells behind them are fetched as the aligned
 // 16-byte pieces they lie in, the first one AL cells below them (AL < 0: cell by cell).
-// Lanes outside the tensor store zeros (the padding).  A warp's own chain of dependent
+// Lanes outside the tensor store zeros (the padding).  Eight lanes along a row, then the
+// next channel: a quarter of a 16-byte load is then one line of 128 bytes, and a quarter of
+// a store is eight cells LBO = 16 mod 128 apart.  (With the channels side by side a quarter
+// touched the same banks of four lines: what bounds the kernel is shared memory, which the
+// instructions read their operands from, 256^3, 4 -> 16 1206 -> 1011 us, 128^3 185 -> 148,
+// 32 -> 32 on 24 x 40 x 64 119 -> 111.)  A warp's own chain of dependent
 // instructions is what bounds a stage where channels are few: hence pairs of items
 // without branches between them, and stages that follow each other along H, so that
 // most of them only move a pointer.
@@ -114,7 +119,7 @@ __device__ __forceinline__ bool wg_convert(const WgGeom& g, const WgConvArgs& c,
     constexpr int NV = ISX ? 3 * SW + KWG : 4;                  // cells behind four positions
     constexpr int AO = AL < 0 ? 0 : AL, NB = (NV + AO + 3) / 4; // their offset in the pieces, pieces
     constexpr uint32_t ALL = (1u << NV) - 1;
-    const int cl = c.lane & 3, ql = c.lane >> 2;
+    const int cl = c.lane >> 3, ql = c.lane & 7;
     const uint32_t lane_dst = (uint32_t) (ql * (ISX ? g.lbo_x : g.lbo_y) + 16 * cl);
     const uint32_t row16 = 16u * (uint32_t) (ISX ? g.cg : g.kgp);
     const int rows_in = ISX ? g.in[1] : g.out[1], step_rows = ISX ? g.B * g.stride[1] : g.B;

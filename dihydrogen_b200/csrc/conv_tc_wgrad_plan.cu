@@ -21,7 +21,7 @@ double wg_mma_cost(int n)
 }
 
 // Updates of an accumulator between flushes.  A chain of truncating updates is off by 1.7e-8
-// each (2.2e-6 with WG_CHAIN), fp32 FMAs over n positions, as the CUDA-core kernel deals them
+// each (2.0e-6 with WG_CHAIN), fp32 FMAs over n positions, as the CUDA-core kernel deals them
 // out, by 1.4e-9 sqrt(n) and more where there are many sums.  Strided layers and rows that
 // cannot be read in aligned 16-byte pieces are held to that: 16 -> 16, 24 x 40 x 67, 1.9e-6
 // with WG_CHAIN, 7.4e-7 with FMAs.  The others are only where they are small: 64 updates (1e-6)
@@ -122,14 +122,14 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
     if ((cgp - 1) / 4 * 4 * (double) cg.xs_c + (kdg - 1) * (double) cg.xs[0] + g.X * (double) cg.xs[1] + 4.0 * PW >= 4294967296.0
         || (kg - 1) / 4 * 4 * (double) cg.ys_c + B * (double) cg.ys[1] + 4.0 * PW >= 4294967296.0)
         return false;
-    // shared memory; 64 bytes behind every 128-byte multiple of cells keep the
-    // converters' stores (four rows x two cells at a time) on different banks
+    // shared memory; 16 bytes behind every 128-byte multiple of cells keep the
+    // converters' stores (eight cells of a row at a time) on different banks
     const int planes = ring ? 1 : kdg; // of x that a stage brings
     g.ring = ring;
     g.xrows = planes * g.X * g.r8;
     g.yrows = B * g.n8;
-    g.lbo_x = g.xrows * 16 + 64;
-    g.lbo_y = g.yrows * 16 + 64;
+    g.lbo_x = g.xrows * 16 + 16;
+    g.lbo_y = g.yrows * 16 + 16;
     g.y_off = (g.Q * g.lbo_x + 127) / 128 * 128;
     g.stage_bytes = g.y_off + (g.Q * g.lbo_y + 127) / 128 * 128;
     g.cq = (cgp + 3) / 4;
