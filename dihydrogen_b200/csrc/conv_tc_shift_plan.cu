@@ -276,8 +276,12 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
         g.tile_w = std::min(TC_M, align_up((g.q_w + g.tiles_w - 1) / g.tiles_w, 32));
         g.tiles_w = (g.q_w + g.tile_w - 1) / g.tile_w;
     }
-    const int used = g.npack * (g.tile_w + reach);
-    g.pt = std::max(TC_M + reach, used) + 1;
+    // what the row's outputs read: a tile is whole warps, but what lies behind a row that is its
+    // only one needs no converter item (backward data of 8 -> 24 on 2 x 67 x 83 x 101: four items
+    // instead of five, three teams of converters instead of two, 245 -> 175 us)
+    T->per = (g.tiles_w == 1 ? std::min(g.tile_w, g.q_w) : g.tile_w) + reach;
+    const int used = g.npack * T->per;
+    g.pt = std::max(TC_M + reach, g.npack * (g.tile_w + reach)) + 1;
     const int npb = (used + 31) / 32;
     g.ipr = g.st_w * npb;
     if (g.ipr > SH_MAX_ITEMS)
@@ -405,7 +409,7 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
     };
 
     // tables that do not depend on where the images live
-    const int nlanes = std::max(TC_M, (g.npack * (g.tile_w + (m_w.taps - 1) / m_w.st) + 31) / 32 * 32);
+    const int nlanes = std::max(TC_M, (g.npack * T->per + 31) / 32 * 32);
     for (int mode = 0; mode < 2; ++mode)
     {
         g.stream = mode;
@@ -476,9 +480,8 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
             for (int pb = 0; pb < npb; ++pb)
                 items.push_back((uint32_t) par | (uint32_t) (pb * 32) << 8);
         std::vector<int> lanes((size_t) nlanes, -1);
-        const int per = g.tile_w + (m_w.taps - 1) / m_w.st;
-        for (int p = 0; p < g.npack * per; ++p)
-            lanes[(size_t) p] = (p / per) << 16 | (p % per);
+        for (int p = 0; p < g.npack * T->per; ++p)
+            lanes[(size_t) p] = (p / T->per) << 16 | (p % T->per);
 
         auto put = [&](const void* src, size_t bytes) {
             const size_t at = T->blob.size();

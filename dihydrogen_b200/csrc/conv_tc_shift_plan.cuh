@@ -59,6 +59,7 @@ struct ShPack // filter-image kernel's tables
 struct ShTables
 {
     ShGeom g;
+    int per;                         // positions staged for a sub-column
     int kind, parts;
     bool wide;                       // 64-bit channel offsets
     int c_of_cell;
