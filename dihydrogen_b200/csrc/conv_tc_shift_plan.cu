@@ -261,13 +261,13 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     g.cgroups = t.cgroups;
     g.cpg = J * m_ch;
     const int reach = (m_w.taps - 1) / m_w.st; // positions to the right of an output's own
-    if (g.q_w + (g.q_w + reach) <= TC_M)
+    if (t.wt > 0)
     {
-        // narrow rows: several sub-columns side by side
+        // rows, or equal parts of them, several sub-columns side by side
         const int segs_left = m_flat ? t.nseg : (g.q_r + g.th - 1) / g.th;
-        g.npack = std::min((TC_M - g.q_w) / (g.q_w + reach) + 1, segs_left);
-        g.tile_w = g.q_w;
-        g.tiles_w = 1;
+        g.tile_w = (g.q_w + t.wt - 1) / t.wt;
+        g.tiles_w = (g.q_w + g.tile_w - 1) / g.tile_w;
+        g.npack = std::min(packed(g.tile_w), segs_left);
     }
     else
     {
@@ -327,6 +327,46 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
         e.f[d] = cg.f[i], e.stride[d] = cg.stride[i], e.pad[d] = cg.pad[i];
     }
     return true;
+}
+
+// Sub-columns of w outputs that fit the 128 lanes side by side.
+int ShBuilder::packed(int w) const
+{
+    const int reach = (m_w.taps - 1) / m_w.st;
+    return w > TC_M ? 0 : (TC_M - w) / (w + reach) + 1;
+}
+
+// Parts that rows may be cut in to lie side by side (0: whole tiles of 32, one beside no other).
+// Rows of up to 63 outputs fit whole, several of them.  A row of 64 has room for one (64 + 66
+// positions) and one of 132 is two tiles of 96, half of the lanes of either idle: 16 outputs of seven
+// rows fill 112 lanes, 22 of five 110.  Such parts are stored by registers and read their
+// neighbours' cells again, so they are only tried where they fill a good deal more of the lanes.
+// us, forward and backward data: 32 -> 32 on 2 x 24 x 40 x 64 151 -> 82 and 156 -> 82, 24 -> 28 on 40 x 100 x 132
+// 541 -> 312 and 453 -> 258, 12 -> 20 on 50 x 90 x 177 132 -> 101 and 151 -> 126, 16 -> 24 with stride 2
+// on 90 x 90 x 160 backward data 77 -> 58.
+std::vector<int> ShBuilder::row_parts() const
+{
+    if (packed(m_w.q) >= 2)
+        return {1};
+    const int tiles = (m_w.q + TC_M - 1) / TC_M;
+    const double whole = (double) m_w.q / (tiles * TC_M);
+    double most = 0;
+    std::vector<std::pair<int, double>> fill;
+    for (int parts = tiles + 1; parts <= 8 * tiles && parts <= m_w.q / 8; ++parts)
+    {
+        const int w = (m_w.q + parts - 1) / parts, n = packed(w);
+        if (n < 2 || (m_w.q + w - 1) / w != parts)
+            continue;
+        const double f = (double) n * m_w.q / (parts * TC_M);
+        fill.push_back({parts, f});
+        most = std::max(most, f);
+    }
+    std::vector<int> r = {0};
+    // the widest that come close to the best
+    for (const auto& f : fill)
+        if (r.size() < 3 && f.second > 1.15 * whole && f.second > (r.size() == 1 ? 0.85 : 0.97) * most)
+            r.push_back(f.first);
+    return r;
 }
 
 // Fills in the tables; false when something does not fit shared memory.
@@ -605,7 +645,12 @@ double ShBuilder::clocks(const ShGeom& g, double mma, int teams) const
     if (g.th == 1 && g.ns == (m_s.taps + m_s.st - 1) / m_s.st)
         plane += 0.63 * drain; // a block has to be drained before its plane slot is opened again
     const double waves = (double) ((g.units + m_sms - 1) / m_sms);
-    return waves * (((g.seglen - 1) * m_s.st + m_s.taps) * plane + 16800.0);
+    // parts of a row take more than the fit, which has none of them, says (16 -> 16 on 64^3, forward with
+    // statistics: 54 us expected and 66.7 taken, 56 and 64.3 with whole rows)
+    // and more where the statistics come out of the epilogue that stores them
+    const bool stats = !m_tr && !m_flat && g.kgroups == 1 && g.nb <= 16;
+    const double parts = g.npack > 1 && g.tiles_w > 1 ? (stats ? 1.15 : 1.08) : 1.0;
+    return parts * waves * (((g.seglen - 1) * m_s.st + m_s.taps) * plane + 16800.0);
 }
 
 // The corrections (every product but the first) are small and have a set of their own.
@@ -618,13 +663,14 @@ int ShBuilder::chain_of(int items, int lead, int cgroups) const
 bool ShBuilder::build_within(double limit, ShTables* out) const
 {
     std::vector<Try> tries;
+    const std::vector<int> parts = row_parts();
     const int live = (m_s.taps + m_s.st - 1) / m_s.st; // planes live at once
     for (int kg = 1; kg <= 16 && kg <= m_kout; ++kg)
         for (int cgroups = 1; cgroups <= 8; cgroups *= 2)
             for (int th = m_flat ? 1 : std::min(16, m_r.q); th >= 1; --th)
             {
                 ShTables T;
-                Try t = {kg, th, live, cgroups, 1, 1, 0, 0};
+                Try t = {kg, th, live, cgroups, 1, 1, parts[0], 0, 0};
                 if (!layout(t, &T))
                     continue;
                 const int J = T.g.cpg / m_ch;
@@ -666,44 +712,63 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
                             for (const auto& r : ranges(row_code(T.g, ph, i, ew)))
                                 t.mma += (double) n * sh_mma_cost(r.second) * cgroups / m_s.st;
                         }
-                double best = 0;
-                int best_ns = 0;
-                for (int ns = 1; ns <= std::min(m_s.q, 64); ++ns)
+                for (int wt : parts)
                 {
-                    Try s = t;
-                    s.nseg = ns;
-                    if (!layout(s, &T))
+                    t.wt = wt;
+                    double best = 0;
+                    int best_ns = 0;
+                    for (int ns = 1; ns <= std::min(m_s.q, 64); ++ns)
+                    {
+                        Try s = t;
+                        s.nseg = ns;
+                        if (!layout(s, &T))
+                            continue;
+                        const double c = clocks(T.g, t.mma, std::max(1, SH_CONV / T.g.ipr));
+                        if (best_ns == 0 || c < best)
+                            best = c, best_ns = ns;
+                    }
+                    if (best_ns == 0)
                         continue;
-                    const double c = clocks(T.g, t.mma, std::max(1, SH_CONV / T.g.ipr));
-                    if (best_ns == 0 || c < best)
-                        best = c, best_ns = ns;
+                    t.nseg = best_ns;
+                    t.cost = best;
+                    tries.push_back(t);
                 }
-                if (best_ns == 0)
-                    continue;
-                t.nseg = best_ns;
-                t.cost = best;
-                tries.push_back(t);
             }
     std::stable_sort(tries.begin(), tries.end(), [](const Try& a, const Try& b) { return a.cost < b.cost; });
     // how many converter teams fit shows in the finished tables only
-    int left = 24, found = 0;
-    for (const Try& t : tries)
-    {
-        if (left == 0 || found == 4 || (found > 0 && t.cost >= out->cost))
-            break;
-        ShTables T;
-        const bool fits = layout(t, &T) && finish(t, &T);
-        left -= !T.too_long; // (lower columns have shorter tables)
-        if (fits)
+    auto pick = [&](const std::vector<Try>& from) {
+        int left = 24, found = 0;
+        for (const Try& t : from)
         {
-            T.cost = clocks(T.g, t.mma, T.g.teams);
-            T.chain = T.g.nsets == 1 ? chain_of(m_parts * (m_parts + 1) / 2 * T.g.cpg / m_ch * m_w.most(), 1, T.g.cgroups)
-                                     : chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
-            if (found++ == 0 || T.cost < out->cost)
-                *out = T;
+            if (left == 0 || found == 4 || (found > 0 && t.cost >= out->cost))
+                break;
+            ShTables T;
+            const bool fits = layout(t, &T) && finish(t, &T);
+            left -= !T.too_long; // (lower columns have shorter tables)
+            if (fits)
+            {
+                T.cost = clocks(T.g, t.mma, T.g.teams);
+                T.chain = T.g.nsets == 1 ? chain_of(m_parts * (m_parts + 1) / 2 * T.g.cpg / m_ch * m_w.most(), 1, T.g.cgroups)
+                                         : chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
+                if (found++ == 0 || T.cost < out->cost)
+                    *out = T;
+            }
         }
-    }
-    return found > 0;
+        return found > 0;
+    };
+    std::vector<Try> whole;
+    for (const Try& t : tries)
+        if (t.wt == parts[0])
+            whole.push_back(t);
+    const bool found = pick(whole);
+    if (whole.size() == tries.size() || !found)
+        return found;
+    const ShTables rows = *out;
+    if (!pick(tries) || out->cost > rows.cost)
+        *out = rows;
+    // (the CUDA-core kernels are weighed against whole rows, which their rule was made with)
+    out->cost = rows.cost;
+    return true;
 }
 
 } // namespace dcb

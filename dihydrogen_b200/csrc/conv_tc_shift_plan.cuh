@@ -64,7 +64,7 @@ struct ShTables
     bool wide;                       // 64-bit channel offsets
     int c_of_cell;
     size_t smem;
-    double cost;
+    double cost;                     // of the best layout without parts of rows
     int chain;                       // longest chain of leading products in one accumulator
     std::vector<uint8_t> issue;      // issuers' tables
     bool too_long = false;           // they would not fit
@@ -153,12 +153,14 @@ private:
     }
     struct Try
     {
-        int kg, th, ns, cgroups, nsets, nseg;
+        int kg, th, ns, cgroups, nsets, nseg, wt;
         double cost, mma;
     };
     double chain_limit() const;
     double clocks(const ShGeom& g, double mma, int teams) const;
     bool one_set(int cgroups, int items) const;
+    int packed(int w) const;
+    std::vector<int> row_parts() const;
     int chain_of(int items, int lead, int cgroups) const;
     bool build_within(double limit, ShTables* out) const;
     bool layout(const Try& t, ShTables* T) const;

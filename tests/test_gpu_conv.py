@@ -926,3 +926,25 @@ def test_statistics_from_the_shift_kernel(geom, mode):
     d, over = y.double(), (0, 2, 3, 4)
     for got, ref, size in ((sums[0], d.sum(over), d.abs().sum(over)), (sums[1], d.square().sum(over), d.square().sum(over))):
         assert ((got.double() - ref).abs() <= 1e-5 * size).all()
+
+
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_BF16])
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, stride: rows that are laid side by side in parts, last parts short
+    (1, 32, 24, (9, 33, 64), (3, 3, 3), 1), (2, 24, 28, (7, 20, 132), (3, 3, 3), 1), (1, 12, 20, (9, 31, 177), (3, 3, 3), 1),
+    (1, 8, 8, (12, 40, 66), (3, 3, 3), 1), (2, 32, 16, (75, 65), (3, 3), 1), (1, 16, 24, (11, 23, 160), (3, 3, 3), 2),
+])
+def test_rows_in_parts(geom, mode):
+    N, C, K, sp, f, s = geom
+    rng = np.random.default_rng(sp[-1])
+    pads, strides = [1] * len(sp), [s] * len(sp)
+    x = rng.normal(size=(N, C, *sp)).astype(np.float32)
+    w = rng.normal(0, np.sqrt(2.0 / (C * np.prod(f))), (K, C, *f)).astype(np.float32)
+    dy = rng.normal(size=(N, K, *[O.conv_out_extent(i, 3, 1, s, 1) for i in sp])).astype(np.float32)
+    y, dx, _ = run_all(x, w, dy, pads, strides, [1] * len(sp), mode)
+    if mode == _abi.MATH_BF16:  # exact products of rounded operands, fp32 sums
+        x, w, dy = _round_bf16(x), _round_bf16(w), _round_bf16(dy)
+    dx_ref = np.zeros_like(x)
+    O.conv_bwd_data(w, dy, dx_ref, pads, strides)
+    emu.assert_close(y, O.conv_fwd(x, w, pads, strides), TOL, "y")
+    emu.assert_close(dx, dx_ref, TOL, "dx")

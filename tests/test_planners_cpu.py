@@ -162,3 +162,11 @@ def test_tables_that_do_not_fit_leave_a_lower_column(tmp_path):
             else:
                 lower += rows < full[tr][3]
     assert lower >= 8
+
+
+def test_parts_of_rows_cover_every_output_once(tmp_path):
+    """Parts of a row side by side in the lanes, each with its own row blocks or segments."""
+    r = subprocess.run([compile_check(tmp_path, "shift_parts_check")], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    passes, parts, bad = map(int, r.stdout.split())
+    assert passes > 150 and parts > 30 and bad == 0
