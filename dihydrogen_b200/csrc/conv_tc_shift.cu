@@ -273,13 +273,16 @@ int32_t sh_conv(ShPlan* p, float alpha, const float* x, const float* w, float be
     auto dispatch = [&](auto wide, auto size) -> int32_t {
         constexpr bool W = decltype(wide)::value;
         constexpr int C = decltype(size)::value;
-        if (t.kind == 0 && t.parts == 1)
-            return stats ? launch(sh_conv_kernel<0, 1, true, W, C>, size) : launch(sh_conv_kernel<0, 1, false, W, C>, size);
-        if (t.kind == 0)
-            return stats ? launch(sh_conv_kernel<0, 2, true, W, C>, size) : launch(sh_conv_kernel<0, 2, false, W, C>, size);
-        if (t.parts == 1)
-            return stats ? launch(sh_conv_kernel<1, 1, true, W, C>, size) : launch(sh_conv_kernel<1, 1, false, W, C>, size);
-        return stats ? launch(sh_conv_kernel<1, 3, true, W, C>, size) : launch(sh_conv_kernel<1, 3, false, W, C>, size);
+        auto with = [&](auto epilogue) -> int32_t {
+            constexpr int E = decltype(epilogue)::value;
+            if (t.kind == 0)
+                return t.parts == 1 ? launch(sh_conv_kernel<0, 1, E, W, C>, size) : launch(sh_conv_kernel<0, 2, E, W, C>, size);
+            return t.parts == 1 ? launch(sh_conv_kernel<1, 1, E, W, C>, size) : launch(sh_conv_kernel<1, 3, E, W, C>, size);
+        };
+        // (statistics are of plain outputs of 16 filters at most: never of blocks with two halves)
+        return stats                ? with(std::integral_constant<int, SH_STATS>())
+               : sh_shared_drain(g) ? with(std::integral_constant<int, SH_SHARED>())
+                                    : with(std::integral_constant<int, SH_PLAIN>());
     };
     using Large = std::integral_constant<int, SH_CONST>;
     using Small = std::integral_constant<int, SH_CONST_SMALL>;

@@ -58,6 +58,8 @@ constexpr int SH_THREADS = (SH_EPI + SH_CONV + SH_ISS + 1) * 32;
 constexpr int SH_MAX_ITEMS = SH_CONV; // warp-sized pieces of a staged row: never more than the warps of a team
 constexpr int SH_MAX_SLOTS = 9;   // A slots: a multiple of SH_ISS
 constexpr int SH_MAX_BLOCKS = 64; // (row, plane slot) accumulator blocks of a column
+// the epilogue's teams take blocks in turn; the same with statistics of the output; they share every block
+constexpr int SH_PLAIN = 0, SH_STATS = 1, SH_SHARED = 2;
 
 struct ShGroup // one accumulator range of a staged row
 {
@@ -375,6 +377,16 @@ __host__ __device__ __forceinline__ int sh_columns(const ShGeom& g)
     return g.set_off * g.nsets + (g.nb % 16 ? 16 - g.nb % 16 : 0);
 }
 
+// Columns without a spare plane slot, of one row: a block has to be drained before its slot is
+// opened again, by the next plane, so that nothing else goes on meanwhile. Both epilogue teams
+// then share every block where it has two halves (cells of either parity along W, or pieces of 16
+// filters): 32 -> 16, stride 2, backward data on 256^3 944 -> 804 us, 24 -> 28 forward on 40 x 100 x 132
+// 311 -> 300. (A kernel of its own: with the choice at run time all others lost 1 %.)
+inline bool sh_shared_drain(const ShGeom& g)
+{
+    return g.th == 1 && g.ns * g.st_s < g.fs + g.st_s && (g.e_w == 2 || (g.e_s * g.e_r == 1 && g.nb > 16));
+}
+
 __device__ __forceinline__ bool sh_number(float v)
 {
     return fabsf(v) <= 3.402823466e+38f;
@@ -578,13 +590,15 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 
 // WIDE: channels lie too far apart for 32-bit offsets.  (64-bit offsets throughout, or two
 // pointers per channel pair, make every other layer 1 to 2 % slower.)
-template <int KIND, int PARTS, bool STATS, bool WIDE, int CONST>
+template <int KIND, int PARTS, int EPILOGUE, bool WIDE, int CONST>
 __global__ void __launch_bounds__(SH_THREADS, 1)
     sh_conv_kernel(const __grid_constant__ ShGeom g, const __grid_constant__ ShExact ex, float beta, const __grid_constant__ ShConst<CONST> ct,
                    const float* __restrict__ x, const uint4* __restrict__ bimg, const uint8_t* __restrict__ tables, float* y, int* status,
                    float* __restrict__ stat_part, const __grid_constant__ CUtensorMap ymap, int use_ymap)
 {
     constexpr int CH = KIND == 0 ? 4 : 8;
+    constexpr bool STATS = EPILOGUE == SH_STATS, SHARED = EPILOGUE == SH_SHARED;
+    constexpr int HALVES = SHARED ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     const uint2* sets = reinterpret_cast<const uint2*>(smem + g.so_sets);
@@ -623,7 +637,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         for (int b = lane; b < g.th * g.ns; b += 32)
         {
             mbar_init(&ev_full[b], SH_ISS);
-            mbar_init(&ev_empty[b], 4);
+            mbar_init(&ev_empty[b], SHARED ? SH_EPI : 4);
         }
         if (lane == 0)
         {
@@ -690,7 +704,9 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
         const uint32_t stage_s = smem_u32(smem + g.so_stage) + (uint32_t) (warp * g.stage);
         const uint32_t stage_lane = stage_s + 4u * lane;
         const bool store_w = quad * 32 < g.tile_w;
-        int j = team < teams ? team : 0x40000000;
+        static_assert(SH_EPI == 8, "two teams, a half each");
+        const int half = SHARED ? team : 0; // of every block
+        int j = SHARED ? 0 : team < teams ? team : 0x40000000;
 #pragma unroll 1
         for (uint32_t unit = blockIdx.x; unit < g.units && ok; unit += gridDim.x)
         {
@@ -706,7 +722,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                 const int q = u.qb + qi + add_s;
                 // this team's blocks of the plane; the count goes on into the next one
 #pragma unroll 1
-                for (; j < g.th; j += teams)
+                for (; j < g.th; j += SHARED ? 1 : teams)
                 {
                     const int b = j * g.ns + (int) slot;
                     ok = mbar_wait(&ev_full[b], lap & 1, abort_flag);
@@ -716,7 +732,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                     const int r = u.row0 + j + add_r;
                     const bool on = lane_w && live && q < g.q_s && r < g.q_r;
                     const uint32_t block = lane_addr + (uint32_t) (j * g.rowst + (int) slot * g.blk);
-                    if (use_ymap)
+                    if (!SHARED && use_ymap)
                     {
                         // one bulk tensor store per warp: 32 positions of every filter
                         float v[16];
@@ -758,16 +774,16 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                         continue;
                     }
                     float* yp = y + (long long) u.n * g.ys_n + (long long) kbase * g.ys_c;
-                    if (g.e_s * g.e_r * g.e_w == 1)
+                    if (STATS || g.e_s * g.e_r * g.e_w == 1)
                     {
                         yp += (long long) q * g.ys_s + (long long) r * g.ys_r + qw;
 #pragma unroll 1
-                        for (int k0 = 0; k0 < in_loop(g.nb); k0 += 16)
+                        for (int k0 = 16 * half; k0 < in_loop(g.nb); k0 += 16 * HALVES)
                         {
                             float v[16];
                             const int piece = min(16, g.nb - k0);
                             sh_drain(block + (uint32_t) k0, piece, g.nsets, g.set_off, v);
-                            if (k0 + 16 >= g.nb)
+                            if (k0 + 16 * HALVES >= g.nb)
                             {
                                 // last columns of the block: hand it back before the stores
                                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -798,7 +814,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                         // is four quarters, each of one cell (4 -> 16, stride 2, 64 x 128 x 128: 79 us
                         // with a fetch per cell, 48 like this; of 16 filters 992 per cell, 1275).
 #pragma unroll 1
-                        for (int ew = 0; ew < in_loop(g.e_w); ++ew)
+                        for (int ew = half; ew < in_loop(g.e_w); ew += HALVES)
                         {
                             const int ow = qw * g.e_w + ew, cols = g.e_s * g.e_r * g.nb;
                             int es = 0, er = 0, k0 = 0; // of the next quarter
@@ -835,7 +851,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
 #pragma unroll 1
                             for (int er = 0; er < in_loop(g.e_r); ++er)
 #pragma unroll 1
-                                for (int ew = 0; ew < in_loop(g.e_w); ++ew)
+                                for (int ew = half; ew < in_loop(g.e_w); ew += HALVES)
                                 {
                                     const uint32_t cell = block + (uint32_t) (ew * g.woff + (es * g.e_r + er) * g.nb);
                                     const int os = q * g.e_s + es, orow = r * g.e_r + er, ow = qw * g.e_w + ew;

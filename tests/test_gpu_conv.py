@@ -948,3 +948,30 @@ def test_rows_in_parts(geom, mode):
     O.conv_bwd_data(w, dy, dx_ref, pads, strides)
     emu.assert_close(y, O.conv_fwd(x, w, pads, strides), TOL, "y")
     emu.assert_close(dx, dx_ref, TOL, "dx")
+
+
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, stride: columns of one row without a spare plane slot, blocks with two halves:
+    # parities along W of 4 filters a cell, 16 + 12 and 16 + 16 filters (last part of a row short), W odd
+    (1, 16, 32, (9, 24, 64), (3, 3, 3), 2), (1, 28, 32, (9, 20, 50), (3, 3, 3), 1), (2, 24, 28, (7, 20, 131), (3, 3, 3), 1),
+    (1, 16, 32, (9, 24, 61), (3, 3, 3), 2),
+])
+def test_epilogue_teams_that_share_a_block(geom, beta):
+    N, C, K, sp, f, s = geom
+    rng = np.random.default_rng(sp[-1] + 1)
+    pads, strides = [1] * len(sp), [s] * len(sp)
+    out = [O.conv_out_extent(i, 3, 1, s, 1) for i in sp]
+    x, dy, y0, dx0 = (rng.normal(size=(N, c, *e)).astype(np.float32) for c, e in ((C, sp), (K, out), (K, out), (C, sp)))
+    w = rng.normal(0, np.sqrt(2.0 / (C * np.prod(f))), (K, C, *f)).astype(np.float32)
+    y, dx, _ = run_all(x, w, dy, pads, strides, [1] * len(sp), _abi.MATH_FP32, 1.0, beta, y0.copy(), dx0.copy(), np.zeros_like(w))
+    dx_ref = np.zeros_like(x)
+    O.conv_bwd_data(w, dy, dx_ref, pads, strides)
+    emu.assert_close(y, O.conv_fwd(x, w, pads, strides) + beta * y0, TOL, "y")
+    emu.assert_close(dx, dx_ref + beta * dx0, TOL, "dx")
+
+
+def test_epilogue_teams_that_share_a_block_of_16_filters_a_cell():
+    """Large enough for all filters in one group; chains of 16 updates, 2^-25 of the result each, as much
+    again for the rounding of the sums, 2^-22 for the split."""
+    assert max(_relative_errors(1, 16, 32, (64, 128, 256), (3, 3, 3), 2, _abi.MATH_FP32)) <= 16 * 2.0 ** -25 + 2.0 ** -22
