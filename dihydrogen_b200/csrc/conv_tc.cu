@@ -7,6 +7,7 @@
 #include "conv_tc_wgrad_api.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 namespace dcb
@@ -335,7 +336,6 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
     long long grid = (long long) num_sms();
     if (grid > g.units)
         grid = g.units;
-    const bool c4f3 = g.c == 4 && g.f[2] == 3 && g.pad[2] <= 1 && g.split;
     const bool stats = sums != nullptr;
     // second issuers (and the second A slot of every group) for the plain variant only
     const bool xiss = !stats && g.a_slots == 2 * g.groups;
@@ -349,13 +349,23 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
                                        status, map, ymap, use_ymap, p->stat_part));
         return DCB_OK;
     };
-    int32_t st;
-    if (stats)
-        st = c4f3 ? launch(sw_conv_kernel<true, true, 0>, 0) : launch(sw_conv_kernel<false, true, 0>, 0);
-    else if (xiss)
-        st = c4f3 ? launch(sw_conv_kernel<true, false, 1>, 1) : launch(sw_conv_kernel<false, false, 1>, 1);
-    else
-        st = c4f3 ? launch(sw_conv_kernel<true, false, 0>, 0) : launch(sw_conv_kernel<false, false, 0>, 0);
+    auto variant = [&](auto channels, auto split) -> int32_t {
+        constexpr int C = decltype(channels)::value;
+        constexpr bool S = decltype(split)::value;
+        return stats ? launch(sw_conv_kernel<C, S, true, 0>, 0)
+                     : (xiss ? launch(sw_conv_kernel<C, S, false, 1>, 1) : launch(sw_conv_kernel<C, S, false, 0>, 0));
+    };
+    auto channels = [&](auto split) -> int32_t {
+        switch (g.f[2] == 3 && g.pad[2] <= 1 ? g.c : 0)
+        {
+        case 1: return variant(std::integral_constant<int, 1>(), split);
+        case 2: return variant(std::integral_constant<int, 2>(), split);
+        case 3: return variant(std::integral_constant<int, 3>(), split);
+        case 4: return variant(std::integral_constant<int, 4>(), split);
+        default: return variant(std::integral_constant<int, 0>(), std::true_type()); // (looks at g.split)
+        }
+    };
+    const int32_t st = g.split ? channels(std::true_type()) : channels(std::false_type());
     if (st != DCB_OK || !stats)
         return st;
     DCB_CUDA_TRY(launch_overlapped(sw_stats_fold_kernel, dim3(1), SW_FOLD_WARPS * 32, 0, stream, p->stat_part,

@@ -257,25 +257,46 @@ __global__ void __launch_bounds__(SW_FOLD_WARPS * 32)
         sqsums[t - SW_NBK] = (float) acc;
 }
 
-// 4 channels x 3 taps, split: A columns 0..11 hi, 12..23 lo.
-__device__ __forceinline__ void sw_convert_c4f3(uint32_t raw_lane, uint32_t pitch, uint32_t (&v)[3][8])
+// A columns of a slot for C channels x 3 taps: hi parts, then (SPLIT) lo parts, then zeros up to
+// a multiple of 8.
+__host__ __device__ constexpr int sw_f3_columns(int c, bool split)
 {
-    uint32_t xv[12];
+    return (c * 3 * (split ? 2 : 1) + 7) / 8 * 8;
+}
+
+// Converts them without a table, all loads at once, and before the slot has to be free (the general
+// converter walks the columns in eights behind that wait). us, with the general converter and like this:
+// 128^3, 4 -> 16 in bf16 71 and 58, 3 -> 12 103 and 81; 64 x 80 x 200, 1 -> 16 40.7 and 37.1, 2 -> 16 54.0 and 47.8.
+template <int C, bool SPLIT>
+__device__ __forceinline__ void sw_convert_f3(uint32_t raw_lane, uint32_t pitch, uint32_t rnd_add, uint32_t rnd_mask,
+                                              uint32_t (&v)[sw_f3_columns(C, SPLIT) / 8][8])
+{
+    constexpr int N = 3 * C, COLUMNS = sw_f3_columns(C, SPLIT);
+    uint32_t xv[N];
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < C; ++c)
 #pragma unroll
         for (int kw = 0; kw < 3; ++kw)
             xv[c * 3 + kw] = lds_u32(raw_lane + 4u * ((uint32_t) c * pitch + 3u + (uint32_t) kw));
 #pragma unroll
-    for (int r = 0; r < 12; ++r)
+    for (int r = SPLIT ? 2 * N : N; r < COLUMNS; ++r)
+        v[r / 8][r % 8] = 0u;
+#pragma unroll
+    for (int r = 0; r < N; ++r)
     {
         const float xe = __uint_as_float(xv[r]);
+        if (!SPLIT)
+        {
+            v[r / 8][r % 8] = round_fast(xe, rnd_add) & rnd_mask;
+            continue;
+        }
         const uint32_t hi = tf32_rna(xe);
         // x - hi is exact in fp32 and below 2^-11 |x|; the tensor pipe reads the
-        // upper 19 bits of it, an error below 2^-21 |x|: no rounding of its own
-        const uint32_t lo = __float_as_uint(xe - __uint_as_float(hi));
+        // upper 19 bits of it, an error below 2^-21 |x|: with four channels no rounding of its own
+        const int rest = __float_as_int(xe - __uint_as_float(hi));
+        const uint32_t lo = C == 4 ? (uint32_t) rest : (uint32_t) min(rest, 0x7fffefff) + 0x1000u;
         v[r / 8][r % 8] = hi;
-        v[(12 + r) / 8][(12 + r) % 8] = lo;
+        v[(N + r) / 8][(N + r) % 8] = lo;
     }
 }
 
@@ -310,7 +331,8 @@ __host__ __device__ constexpr int sw_threads(int xiss)
     return (TC_TMA_WARP + 1 + SW_EPI + (xiss ? TC_GROUPS_MAX : 0)) * 32;
 }
 
-template <bool C4F3, bool STATS, int XISS>
+// F3C: channels of a filter that is 3 wide, with a converter for them (SPLIT: 3xTF32); 0: any.
+template <int F3C, bool SPLIT, bool STATS, int XISS>
 __global__ void __launch_bounds__(sw_threads(XISS), 1)
     sw_conv_kernel(SwGeom g, float alpha, const float* __restrict__ bimg, float* y, int* status,
                    const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap ymap, int use_ymap,
@@ -432,18 +454,19 @@ __global__ void __launch_bounds__(sw_threads(XISS), 1)
                                            + (i - lo) * TC_RAW_W;
                         const uint32_t a_addr = lane_addr + a_col0 + (uint32_t) (a_slot * g.kr);
                         const uint32_t raw_s = smem_u32(raw) + 4u * (uint32_t) mcol;
-                        if (C4F3)
+                        if (F3C > 0)
                         {
-                            uint32_t v[3][8];
+                            constexpr int PIECES = sw_f3_columns(F3C > 0 ? F3C : 1, SPLIT) / 8;
+                            uint32_t v[PIECES][8];
                             // the converter is written for taps that start 3 cells into the staged row
-                            sw_convert_c4f3(raw_s + 4u * (uint32_t) (g.rx - 3), pitch, v);
+                            sw_convert_f3<(F3C > 0 ? F3C : 1), SPLIT>(raw_s + 4u * (uint32_t) (g.rx - 3), pitch, g.rnd_add, g.rnd_mask, v);
                             if (!a_first)
                                 ok = mbar_wait(&a_empty[a_slot], a_phase, abort_flag);
                             if (!ok)
                                 break;
                             tc_fence_after();
 #pragma unroll
-                            for (int ck = 0; ck < 3; ++ck)
+                            for (int ck = 0; ck < PIECES; ++ck)
                                 tmem_st8(a_addr + (uint32_t) (ck * 8), v[ck]);
                         }
                         else
