@@ -324,7 +324,9 @@ __device__ __forceinline__ void sw_convert_f3(uint32_t raw_lane, uint32_t pitch,
 // shard, ~140 clocks per tcgen05.mma or commit, seven per staged row); with six the
 // kernel takes 0.378 ms instead of 0.433.  The variant with statistics is
 // held by its epilogue warps and by registers (the extra warps lower the cap to 66
-// per thread, its epilogue then spills): it keeps three issuers and one slot per group.
+// per thread, its epilogue then spills): it keeps three issuers. They go through both slots of
+// their group in turn, so that a row is written while the one before it is multiplied: 256^3
+// 449 -> 440 us, 128^3 89 -> 86, 5 -> 16 on 64 x 80 x 128 64 -> 58 with one slot and with two.
 constexpr int SW_EPI = 12;
 __host__ __device__ constexpr int sw_threads(int xiss)
 {
@@ -606,7 +608,7 @@ __global__ void __launch_bounds__(sw_threads(XISS), 1)
                     // away.  The first issuer waits for every row's hand-back in every step,
                     // so once both have finished a step the barriers this group looks at are
                     // at most one completion behind what either expects next.
-                    if (laps_a > 1 && step != 0)
+                    if (XISS && laps_a > 1 && step != 0)
                         ok = mbar_wait_t<0>(&iss_sync[mq], (step - 1) & 1, abort_flag);
                     const bool real = sw_real(g, t, d);
                     const uint32_t par = step & 1;
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(sw_threads(XISS), 1)
                     {
                         // a real row belongs to the issuer of the slot it was written to,
                         // a virtual one (nothing to multiply) to the group's first issuer
-                        if (real ? (laps_a > 1 && lap_a != mh) : mh != 0)
+                        if (XISS && (real ? (laps_a > 1 && lap_a != mh) : mh != 0))
                         {
                             if (real && ++lap_a == laps_a)
                             {
@@ -674,7 +676,7 @@ __global__ void __launch_bounds__(sw_threads(XISS), 1)
                             __syncwarp();
                         }
                     }
-                    if (laps_a > 1)
+                    if (XISS && laps_a > 1)
                     {
                         __syncwarp();
                         if (lane == 0)
