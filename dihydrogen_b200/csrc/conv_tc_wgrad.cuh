@@ -398,16 +398,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                                              : g.y_off + q0 * g.lbo_y + 16 * (r * g.n8 + ch)),
                              (uint32_t) off, 0u); // (elements, below 2^32: wg_layout)
     }
-    // matrix rows that no item writes (filters up to a multiple of 8) stay zero
-    for (int i = tid; i < g.nstages * g.stage_bytes / 16; i += WG_THREADS)
-        reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // Matrix rows that no item writes (filters up to a multiple of 8, rows past a tile's) hold what an
+    // earlier kernel left: they only reach accumulators that nobody reads.
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    const uint32_t columns = (uint32_t) (g.sum_col + g.kdg * g.nblocks * g.kgp); // accumulators, running sums
     if (warp < 4)
-        for (uint32_t c = 0; c < TC_TMEM_COLS; c += 16)
+        for (uint32_t c = 0; c < columns; c += 16)
             tmem_st16_zero(tmem + ((uint32_t) (warp * 32) << 16) + c);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     tc_fence_before();

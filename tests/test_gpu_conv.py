@@ -975,3 +975,23 @@ def test_epilogue_teams_that_share_a_block_of_16_filters_a_cell():
     """Large enough for all filters in one group; chains of 16 updates, 2^-25 of the result each, as much
     again for the rounding of the sums, 2^-22 for the split."""
     assert max(_relative_errors(1, 16, 32, (64, 128, 256), (3, 3, 3), 2, _abi.MATH_FP32)) <= 16 * 2.0 ** -25 + 2.0 ** -22
+
+
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, stride: operands whose rows do not fill a multiple of 8, or a tile's 128
+    (1, 3, 13, (9, 11, 37), (3, 3, 3), 1), (2, 5, 3, (30, 41), (5, 5), 1), (1, 4, 16, (16, 24, 32), (3, 3, 3), 1), (1, 7, 9, (8, 9, 34), (3, 3, 3), 2),
+])
+def test_backward_filter_behind_one_of_nans(geom):
+    """What an earlier kernel left in shared and tensor memory reaches no output."""
+    N, C, K, sp, f, s = geom
+    rng = np.random.default_rng(K)
+    pads, strides = [(e - 1) // 2 for e in f], [s] * len(sp)
+    x = rng.normal(size=(N, C, *sp)).astype(np.float32)
+    dy = rng.normal(size=(N, K, *[O.conv_out_extent(i, e, p, s, 1) for i, e, p in zip(sp, f, pads)])).astype(np.float32)
+    xs, dys, dw = torch.from_numpy(x).cuda(), torch.from_numpy(dy).cuda(), torch.zeros(K, C, *f, device="cuda")
+    p = Plan(xs, dw, dys, pads, strides, [1] * len(sp), _abi.MATH_FP32)
+    assert _abi.lib().dcb_conv_plan_kernel_kind(p.p, 2) == 1
+    p.bwd_filter(1.0, torch.full_like(xs, float("nan")), torch.full_like(dys, float("nan")), 0.0, dw)
+    assert bool(torch.isnan(dw).all())
+    p.bwd_filter(1.0, xs, dys, 0.0, dw)
+    emu.assert_close(dw.cpu().numpy(), O.conv_bwd_filter(x, dy, f, pads, strides), TOL, "dw")
