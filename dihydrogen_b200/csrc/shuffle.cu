@@ -82,6 +82,12 @@ struct ShfJob
     FastDiv by_run[3], by_ext[4];
 };
 
+// Windows of this many cells and more are unpacked from their end, where what was written last may
+// still be in L2, by streaming stores, which leave it there: us there and back of 2 x 16 x 128^3 387 -> 376,
+// 16 x 100^3 216 -> 206. (Either alone is 1 to 3 % slower than neither. Below 32 MB the tensor itself
+// stays in L2 otherwise: 16 x 56 x 189 x 38 149 us, 153 from the end; pieces lose as much.)
+constexpr long long SHF_BACK = 8ll << 20;
+
 struct ShfArgs
 {
     const ShfJob* jobs;
@@ -169,6 +175,7 @@ struct ShfPiece
                 v[i] = from[i];
     }
     __device__ __forceinline__ void none() { lo = hi = 0; }
+    template <bool>
     __device__ __forceinline__ void put() const
     {
         if (lo == 0 && hi == 4)
@@ -194,14 +201,19 @@ struct ShfCell
         v = __ldcs(reinterpret_cast<const T*>(run.from) + e);
     }
     __device__ __forceinline__ void none() { to = nullptr; }
+    template <bool STREAM>
     __device__ __forceinline__ void put() const
     {
-        if (to != nullptr)
+        if (to == nullptr)
+            return;
+        if (STREAM)
+            __stcs(to, v);
+        else
             *to = v;
     }
 };
 
-template <int WAY, class T>
+template <int WAY, bool STREAM, class T>
 __device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, const float* from, float* to, const long long* fs,
                                          const long long* ts)
 {
@@ -241,7 +253,7 @@ __device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, const flo
     }
 #pragma unroll
     for (int k = 0; k < shf_unroll<WAY>; ++k)
-        a[k].put();
+        a[k].template put<STREAM>();
 }
 
 // PUT: tensor (strided) -> peers' windows (dense).  !PUT: own window -> tensor.
@@ -250,7 +262,8 @@ __device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, const flo
 // 100 us for 134 MB.
 // PIECES: some job of the call takes them (a kernel of its own: with their registers the others took
 // 5 us more of 50).
-template <bool PUT, bool PIECES>
+// BACK: see SHF_BACK.
+template <bool PUT, bool PIECES, bool BACK>
 __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
 {
     if (!PUT)
@@ -272,8 +285,9 @@ __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
     }
     __shared__ ShfJob j;
     long long u = blockIdx.x;
-    for (int q = 0; q < a.njobs; ++q)
+    for (int n = 0; n < a.njobs; ++n)
     {
+        const int q = BACK ? a.njobs - 1 - n : n;
         __syncthreads();
         for (int i = threadIdx.x; i < (int) (sizeof(ShfJob) / 4); i += SHF_THREADS)
             reinterpret_cast<uint32_t*>(&j)[i] = reinterpret_cast<const uint32_t*>(&a.jobs[q])[i];
@@ -286,12 +300,13 @@ __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
         float* to = (PUT ? w : a.tensor) + (PUT ? j.b_off : j.a_off);
         for (; u < j.units[way]; u += gridDim.x)
         {
+            const long long unit = BACK ? j.units[way] - 1 - u : u;
             if (way == SHF_VEC)
-                shf_unit<SHF_VEC, ShfCell<float4>>(j, u, from, to, fs, ts);
+                shf_unit<SHF_VEC, BACK, ShfCell<float4>>(j, unit, from, to, fs, ts);
             else if (PIECES && way == SHF_PIECE)
-                shf_unit<SHF_PIECE, ShfPiece>(j, u, from, to, fs, ts);
+                shf_unit<SHF_PIECE, BACK, ShfPiece>(j, unit, from, to, fs, ts);
             else
-                shf_unit<SHF_CELL, ShfCell<float>>(j, u, from, to, fs, ts);
+                shf_unit<SHF_CELL, BACK, ShfCell<float>>(j, unit, from, to, fs, ts);
         }
         u -= j.units[way];
     }
@@ -703,7 +718,7 @@ int32_t dcb_shuffle_put(dcb_shuffle_plan* p, const void* src, void* stream)
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    (p->put_pieces[a.aligned] ? shuffle_kernel<true, true> : shuffle_kernel<true, false>)<<<shf_grid(p->put_units), SHF_THREADS, 0,
+    (p->put_pieces[a.aligned] ? shuffle_kernel<true, true, false> : shuffle_kernel<true, false, false>)<<<shf_grid(p->put_units), SHF_THREADS, 0,
                                                                                         as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;
@@ -731,8 +746,10 @@ int32_t dcb_shuffle_wait_unpack(dcb_shuffle_plan* p, void* dst, void* stream)
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    (p->wait_pieces[a.aligned] ? shuffle_kernel<false, true> : shuffle_kernel<false, false>)<<<shf_grid(p->wait_units),
-                                                                                           SHF_THREADS, 0, as_stream(stream)>>>(a);
+    auto kernel = p->wait_pieces[a.aligned]                   ? shuffle_kernel<false, true, false>
+                  : (long long) p->parity_floats >= SHF_BACK ? shuffle_kernel<false, false, true>
+                                                              : shuffle_kernel<false, false, false>;
+    kernel<<<shf_grid(p->wait_units), SHF_THREADS, 0, as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;
 }
