@@ -188,10 +188,6 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
     const double harvest = kdg * (g.nblocks * g.n8 * 35.0 + kg * cgp * kwg * 5.5);
     const double flush = n / g.flush_stages * (kdg * g.nblocks * (g.kgp / 8)) * 280.0;
     *cost = g.nkw * (waves * ((n + lead + 0.3) * per + flush + harvest) + 24000.0);
-    // walks as they are now, against plain layouts: 61 layers, the best of either by the cost above timed
-    // (8 -> 24 on 2 x 67 x 83 x 101, where the two costs are alike: 257 us against 286)
-    if (ring)
-        *cost = 0.97 * *cost + 6600.0;
     return true;
 }
 
