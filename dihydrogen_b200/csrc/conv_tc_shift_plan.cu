@@ -564,6 +564,12 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
                 if (t > g.teams)
                     g.teams = t, slots = n;
             }
+            // Three teams of four warps are better than two where conversion bounds: one pass of products
+            // (16 -> 16 in TF32 on 100 x 100 x 75 77 / 94 us), parts of rows (16 -> 4 on 100 x 100 x 160 119 / 125), or
+            // no room for two slots a team. Elsewhere they get in the way of the other roles (24 -> 24 on
+            // 2 x 700 x 118 31.2 / 29.3, 16 -> 24 on 4 x 300 x 30 16.2 / 15.3, backward data 18.3 / 16.7).
+            if (g.ipr == 4 && fit >= 6 && m_parts > 1 && (g.npack == 1 || g.tiles_w == 1))
+                g.teams = 2, slots = 6;
         }
         if (slots == 0)
             continue;
@@ -747,7 +753,7 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
             left -= !T.too_long; // (lower columns have shorter tables)
             if (fits)
             {
-                T.cost = clocks(T.g, t.mma, T.g.teams);
+                T.cost = clocks(T.g, t.mma, T.g.ipr == 4 && T.g.teams == 2 ? 3 : T.g.teams);
                 T.chain = T.g.nsets == 1 ? chain_of(m_parts * (m_parts + 1) / 2 * T.g.cpg / m_ch * m_w.most(), 1, T.g.cgroups)
                                          : chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
                 if (found++ == 0 || T.cost < out->cost)
