@@ -50,9 +50,9 @@ bool sw_geom(const ConvGeom& cg, int math_mode, SwGeom* out)
     g.ys_c = cg.ys_c;
     if (g.f[0] < 2 || g.f[0] > 4 || g.k > SW_NBK)
         return false;
-    // Its tiles are 128 outputs of a row; the shift kernel packs narrow rows side by
-    // side.  Measured (4 -> 16 channels, us, this kernel / shift kernel): rows of 64
-    // 29 / 38, of 56 40 / 31, of 32 22 / 18, of 148 96 / 116.
+    // Its tiles are 128 outputs of a row; the shift kernel lays narrow rows, or parts of rows, side by
+    // side.  Measured (4 -> 16 channels, 64 x 80 rows, with statistics, us, this kernel / shift kernel): rows
+    // of 100 43.1 / 48.6, of 128 43.0 / 48.7, of 200 59.6 / 75.5; with whole rows only, rows of 56 40 / 31, of 32 22 / 18.
     if (2 * g.out[2] < (g.out[2] + TC_M - 1) / TC_M * TC_M)
         return false;
     g.split = (math_mode == DCB_MATH_TF32 || math_mode == DCB_MATH_BF16) ? 0 : 1;
