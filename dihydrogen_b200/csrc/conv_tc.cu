@@ -337,7 +337,7 @@ int32_t tc_sweep_fwd(TcPlan* p, float alpha, const float* x, const float* w, flo
     if (grid > g.units)
         grid = g.units;
     const bool stats = sums != nullptr;
-    // second issuers (and the second A slot of every group) for the plain variant only
+    // second issuers for the plain variant only
     const bool xiss = !stats && g.a_slots == 2 * g.groups;
     auto launch = [&](auto kernel, int xi) -> int32_t {
         const int32_t set = allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 224 * 1024);
