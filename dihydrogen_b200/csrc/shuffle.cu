@@ -25,6 +25,8 @@
 #include <cstring>
 #include <vector>
 
+#include <unistd.h>
+
 namespace dcb
 {
 namespace
@@ -82,11 +84,18 @@ struct ShfJob
     FastDiv by_run[3], by_ext[4];
 };
 
-// Windows of this many cells and more are unpacked from their end, where what was written last may
-// still be in L2, by streaming stores, which leave it there: us there and back of 2 x 16 x 128^3 387 -> 376,
-// 16 x 100^3 216 -> 206. (Either alone is 1 to 3 % slower than neither. Below 32 MB the tensor itself
-// stays in L2 otherwise: 16 x 56 x 189 x 38 149 us, 153 from the end; pieces lose as much.)
-constexpr long long SHF_BACK = 8ll << 20;
+// Windows are unpacked from their end, where what was written last may still be in L2, by streaming
+// stores, which leave it there, if the windows of this device's ranks together take three quarters of L2
+// or more. Below, a window that is read from its start by plain stores leaves the tensor in L2 for its next
+// reader. us, one way and a pass over the tensor behind it, rank's window from the start / from the end
+// (B200, L2 of 126 MB; 2 x 16 x D x 128 x 128 split along D):
+//   one rank on the device   34 MB 36.3 / 37.8, 67 MB 61.8 / 65.0, 84 MB 78.0 / 79.7, 101 MB 98.9 / 94.5, 134 MB 136.9 / 126.1
+//   two ranks, of each       34 MB 85.8 / 91.9, 42 MB 101.2 / 108.2, 50 MB 121.7 / 121.6, 59 MB 142.9 / 138.0, 134 MB 281.6 / 276.8
+// Either alone is 1 to 3 % slower than neither; pieces lose with both.
+inline bool shf_from_the_end(double window_bytes, double l2_bytes)
+{
+    return window_bytes >= 0.75 * l2_bytes;
+}
 
 struct ShfArgs
 {
@@ -262,7 +271,7 @@ __device__ __forceinline__ void shf_unit(const ShfJob& j, long long u, const flo
 // 100 us for 134 MB.
 // PIECES: some job of the call takes them (a kernel of its own: with their registers the others took
 // 5 us more of 50).
-// BACK: see SHF_BACK.
+// BACK: see shf_from_the_end.
 template <bool PUT, bool PIECES, bool BACK>
 __global__ void __launch_bounds__(SHF_THREADS) shuffle_kernel(ShfArgs a)
 {
@@ -465,6 +474,7 @@ struct dcb_shuffle_plan
     int n_put = 0, n_wait = 0;
     long long put_units = 0, wait_units = 0;
     bool put_pieces[2] = {}, wait_pieces[2] = {}; // whether a job takes pieces; by whether the tensor is 16-byte aligned
+    bool from_the_end = false;
     uint32_t epoch = 0;
     bool connected = false;
 
@@ -673,6 +683,18 @@ int32_t dcb_shuffle_plan_connect(dcb_shuffle_plan* p, const void* blobs, int32_t
         p->put_pieces[aligned] = std::any_of(put.begin(), put.end(), pieces);
         p->wait_pieces[aligned] = std::any_of(wait.begin(), wait.end(), pieces);
     }
+    // (ranks that share a device share this process, or are not known to share it)
+    double windows = 0;
+    for (int r = 0; r < nranks; ++r)
+    {
+        ShfBlob b;
+        std::memcpy(&b, static_cast<const char*>(blobs) + (size_t) r * DCB_SHUFFLE_BLOB_BYTES, sizeof(b));
+        if (r == p->rank || (b.win.pid == (int32_t) getpid() && b.win.device == p->win.device))
+            windows += 4.0 * (double) ((p->dst_boxes[r].volume() + 3) / 4 * 4);
+    }
+    int l2_bytes = 0;
+    DCB_CUDA_TRY(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, p->win.device));
+    p->from_the_end = shf_from_the_end(windows, l2_bytes);
     p->n_put = (int) put.size();
     p->n_wait = (int) wait.size();
     if (p->n_put)
@@ -746,9 +768,9 @@ int32_t dcb_shuffle_wait_unpack(dcb_shuffle_plan* p, void* dst, void* stream)
     a.ticket = p->ticket();
     a.status = p->status();
     a.budget_ns = wait_budget_ns();
-    auto kernel = p->wait_pieces[a.aligned]                   ? shuffle_kernel<false, true, false>
-                  : (long long) p->parity_floats >= SHF_BACK ? shuffle_kernel<false, false, true>
-                                                              : shuffle_kernel<false, false, false>;
+    auto kernel = p->wait_pieces[a.aligned] ? shuffle_kernel<false, true, false>
+                  : p->from_the_end        ? shuffle_kernel<false, false, true>
+                                           : shuffle_kernel<false, false, false>;
     kernel<<<shf_grid(p->wait_units), SHF_THREADS, 0, as_stream(stream)>>>(a);
     DCB_LAUNCH_CHECK();
     return DCB_OK;

@@ -88,6 +88,17 @@ def test_runs_off_16_byte_boundaries(shape, sgrid, dgrid, dov):
     test_forward_and_backward(shape, sgrid, dgrid, dov)
 
 
+@pytest.mark.parametrize("shape,dgrid,dov", [
+    ([128, 128, 104, 8, 2], [1, 1, 2, 1, 1], [0, 0, 1, 0, 0]),   # whole planes: 16-byte accesses, jobs of several units
+    ([10, 127, 128, 84, 2], [2, 1, 1, 1, 1], [0, 0, 0, 0, 0]),   # runs of 5 cells, one by one; the last unit is short
+    ([8, 130, 126, 105, 2], [2, 1, 1, 1, 1], [1, 0, 0, 0, 0]),   # of 4, rows off a boundary by the halo
+])
+def test_large_windows(shape, dgrid, dov):
+    """Unpacked from their end (no pieces in them)."""
+    assert 4 * np.prod(shape) >= 0.75 * torch.cuda.get_device_properties(0).L2_cache_size
+    test_forward_and_backward(shape, [1, 1, 1, 1, 2], dgrid, dov)
+
+
 @pytest.mark.parametrize("src_off,dst_off", [(1, 0), (0, 2), (3, 1)])
 @pytest.mark.parametrize("shape,dgrid,dov", [
     ([16, 8, 4, 3, 2], [2, 1, 1, 1, 1], [0, 0, 0, 0, 0]),     # runs of 8 cells
