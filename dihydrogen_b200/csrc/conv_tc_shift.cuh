@@ -130,7 +130,7 @@ struct ShUnit
 };
 
 // Not inlined: several divisions, called at a handful of places once per unit.
-static __device__ __noinline__ ShUnit sh_unit(const ShGeom& g, uint32_t u)
+static __host__ __device__ __noinline__ ShUnit sh_unit(const ShGeom& g, uint32_t u)
 {
     ShUnit t;
     const uint32_t tw = u % (uint32_t) g.tiles_w;
@@ -385,6 +385,15 @@ __host__ __device__ __forceinline__ int sh_columns(const ShGeom& g)
 inline bool sh_shared_drain(const ShGeom& g)
 {
     return g.th == 1 && g.ns * g.st_s < g.fs + g.st_s && (g.e_w == 2 || (g.e_s * g.e_r == 1 && g.nb > 16));
+}
+
+// An issuer reports a block as complete when its next row, SH_ISS further on, is past the block's last one. Where
+// a plane's blocks are opened and closed in the same step (one tap along the sweep), those are only the
+// blocks up to its own row: it has waited for no others to be free, and a report of one that is still in
+// use counts for that use.
+__host__ __device__ __forceinline__ int sh_reports_ahead(const ShGeom& g)
+{
+    return g.fs > 1 ? SH_ISS : min(SH_ISS, g.fr);
 }
 
 __device__ __forceinline__ bool sh_number(float v)
@@ -1143,7 +1152,7 @@ __global__ void __launch_bounds__(SH_THREADS, 1)
                         }
                         // blocks whose last row comes before this issuer's next one
 #pragma unroll 1
-                        for (; j_close * g.st_r + g.fr - 1 < i + SH_ISS && j_close < g.th; ++j_close)
+                        for (; j_close * g.st_r + g.fr - 1 < i + sh_reports_ahead(g) && j_close < g.th; ++j_close)
                             if (elected)
                                 mma_commit(&ev_full[j_close * g.ns + (int) last_slot]);
                     }

@@ -928,6 +928,31 @@ def test_statistics_from_the_shift_kernel(geom, mode):
         assert ((got.double() - ref).abs() <= 1e-5 * size).all()
 
 
+def _round_tf32(a):
+    return ((a.view(np.uint32) + np.uint32(0x1000)) & np.uint32(0xFFFFE000)).view(np.float32)
+
+
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_TF32, _abi.MATH_BF16])
+@pytest.mark.parametrize("geom", [
+    # N, C, K, spatial, filter, padding, stride: one tap along D, columns of several rows, several planes a CTA
+    (3, 4, 3, (56, 51, 132), (1, 1, 1), (0, 0, 0), 1), (1, 8, 32, (40, 64, 64), (1, 2, 2), (0, 0, 0), 1),
+    (1, 8, 8, (40, 64, 64), (1, 3, 3), (0, 1, 1), 2), (2, 16, 8, (60, 80, 64), (2, 2, 2), (0, 0, 0), 2),
+])
+def test_planes_that_open_and_close_in_one_step(geom, mode):
+    N, C, K, sp, f, pads, s = geom
+    rng = np.random.default_rng(K)
+    rnd = {_abi.MATH_FP32: lambda a: a, _abi.MATH_TF32: _round_tf32, _abi.MATH_BF16: _round_bf16}[mode]
+    x = rnd(rng.normal(size=(N, C, *sp)).astype(np.float32))
+    w = rnd(rng.normal(0, np.sqrt(2.0 / (C * np.prod(f))), (K, C, *f)).astype(np.float32))
+    dy = rnd(rng.normal(size=(N, K, *[O.conv_out_extent(i, e, p, s, 1) for i, e, p in zip(sp, f, pads)])).astype(np.float32))
+    for _ in range(3):
+        y, dx, dw = run_all(x, w, dy, pads, [s] * 3, [1] * 3, mode)
+        emu.assert_close(y, O.conv_fwd(x, w, pads, [s] * 3), TOL, "y")
+        dx_ref = np.zeros_like(x)
+        O.conv_bwd_data(w, dy, dx_ref, pads, [s] * 3)
+        emu.assert_close(dx, dx_ref, TOL, "dx")
+
+
 @pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_BF16])
 @pytest.mark.parametrize("geom", [
     # N, C, K, spatial, filter, stride: rows that are laid side by side in parts, last parts short

@@ -180,3 +180,11 @@ def test_windows_that_stay_in_l2_are_unpacked_from_their_start(tmp_path):
     r = subprocess.run([exe], input=" ".join(map(str, start + end)), capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split() == ["0"] * len(start) + ["1"] * len(end)
+
+
+def test_no_report_of_a_block_counts_for_another_use_of_it(tmp_path):
+    """Filters with one tap along D and one or two along H: an issuer reported blocks that it had not waited for."""
+    r = subprocess.run([compile_check(tmp_path, "shift_protocol_check")], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    passes, same_step, bad = map(int, r.stdout.split())
+    assert passes > 80 and same_step > 30 and bad == 0, r.stdout
