@@ -33,13 +33,36 @@ static ConvGeom geom(int c, int k, int d, int h, int w, int f, int s)
     return g;
 }
 
+// Positions to the right of an output's own (or of its group's, backward with stride s) that it reads, of the tensor
+// along W: forward a position is s cells, backward one cell of dy.
+static int reach_of(int f, int s, bool transposed)
+{
+    if (!transposed)
+        return (f - 1) / s;
+    const int pad = (f - 1) / 2;
+    int lo = f, hi = -f;
+    for (int o = 0; o < s; ++o) // cells of a group
+        for (int tap = 0; tap < f; ++tap)
+            if ((o + pad - tap) % s == 0)
+            {
+                lo = std::min(lo, (o + pad - tap) / s);
+                hi = std::max(hi, (o + pad - tap) / s);
+            }
+    return hi - lo;
+}
+
 // The kernel's walk: units, sub-columns, planes, rows, lanes.
-static bool once(const ShTables& t)
+static bool once(const ShTables& t, int f, int s, bool transposed)
 {
     const ShGeom& g = t.g;
-    const int reach = t.per - std::min(g.tile_w, g.q_w);
-    if (g.npack * t.per > g.pt || g.ipr < g.st_w * ((g.npack * t.per + 31) / 32) || (g.npack - 1) * t.per + g.tile_w > TC_M || reach < 0)
+    const int reach = reach_of(f, s, transposed), row = std::min(g.tile_w, g.q_w), staged = g.ipr / g.st_w * 32;
+    if (g.npack * t.per > g.pt || (g.npack - 1) * t.per + g.tile_w > TC_M)
         return false;
+    // what an output reads lies in its own sub-column and is staged by an item
+    for (int sub = 0; sub < g.npack; ++sub)
+        for (int xx = 0; xx < row; ++xx)
+            if ((sub * t.per + xx + reach) / t.per != sub || sub * t.per + xx + reach >= staged)
+                return false;
     std::vector<unsigned char> seen((size_t) g.q_s * g.q_r * g.q_w, 0);
     const int sub_s = g.pack_s > 0 ? g.npack : 1, sub_r = g.pack_r > 0 ? g.npack : 1;
     for (unsigned u = 0; u < g.units / (unsigned) (g.n * g.kgroups); ++u)
@@ -72,7 +95,7 @@ int main()
                             continue;
                         ++passes;
                         parts += t.g.npack > 1 && t.g.tiles_w > 1;
-                        bad += !once(t);
+                        bad += !once(t, f, s, tr == 1);
                     }
     std::printf("%d %d %d\n", passes, parts, bad);
     return 0;

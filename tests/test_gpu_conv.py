@@ -13,6 +13,7 @@ from dihydrogen_b200 import _abi
 from oracle import oracle as O
 
 import emu
+import layers
 from conftest import GOLDEN, conv_fixtures
 
 pytestmark = pytest.mark.gpu
@@ -807,7 +808,9 @@ def test_layers_of_few_products_on_either_kernel(geom):
 NAN_ALL_ONES = np.uint32(0x7FFFFFFF).view(np.float32)  # what CUDA's arithmetic returns
 NON_FINITE_GEOMS = [
     (1, 4, 16, (6, 9, 140), (3, 3, 3), 1),   # sweep kernel
-    (1, 2, 8, (6, 9, 132), (3, 3, 3), 1),    # ... without its special case of 4 channels
+    (1, 2, 8, (6, 9, 132), (3, 3, 3), 1),    # ... with fewer channels
+    (1, 1, 8, (6, 9, 132), (3, 3, 3), 1),
+    (1, 5, 16, (6, 9, 132), (3, 3, 3), 1),   # ... with its general converter
     (1, 4, 16, (6, 9, 33), (3, 3, 3), 1),    # shift kernel, TF32 cells
     (1, 16, 16, (12, 37), (3, 3), 1),        # ... bf16 cells
     (2, 8, 16, (7, 9, 20), (3, 3, 3), 2),
@@ -843,7 +846,7 @@ def test_what_is_not_a_number_stays_that(geom, mode):
 
 @pytest.mark.parametrize("value", [np.float32(np.inf), NAN_ALL_ONES])
 @pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_TF32, _abi.MATH_BF16])
-@pytest.mark.parametrize("geom", NON_FINITE_GEOMS[2:] + [
+@pytest.mark.parametrize("geom", NON_FINITE_GEOMS[4:] + [
     (1, 4, 4, (8, 9, 64), (3, 3, 3), 2),     # backward data: cells of four columns drained together
     (1, 8, 16, (20, 64), (3, 3), 1),         # bulk stores
     (1, 16, 24, (5, 6, 40), (3, 3, 3), 1),
@@ -895,13 +898,44 @@ def test_statistics_of_an_output_with_an_infinity():
     assert float(sums[0][0]) == float("inf") and float(sums[1][0]) == float("inf")
 
 
+def _round_tf32(a):
+    return ((a.view(np.uint32) + np.uint32(0x1000)) & np.uint32(0xFFFFE000)).view(np.float32)
+
+
+@pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_TF32, _abi.MATH_BF16])
+@pytest.mark.parametrize("geom", [g for g, _ in layers.SWEEP])
+def test_converters_of_the_sweep_kernel(geom, mode):
+    """Every converter, alone and with statistics (to fp32 rounding of partial sums); one pass: the product of the rounded operands."""
+    N, C, K, sp, f, pads = geom
+    rng = np.random.default_rng(C + sp[-1])
+    x = rng.normal(0.3, 1, (N, C, *sp)).astype(np.float32)
+    w = rng.normal(0, np.sqrt(2.0 / (C * np.prod(f))), (K, C, *f)).astype(np.float32)
+    xs, ws = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    y = torch.full((N, K, *[O.conv_out_extent(i, e, p, 1, 1) for i, e, p in zip(sp, f, pads)]), float("nan"), device="cuda")
+    sums = torch.full((2, K), float("nan"), device="cuda")
+    p = Plan(xs, ws, y, pads, [1] * 3, [1] * 3, mode)
+    rnd = {_abi.MATH_FP32: lambda a: a, _abi.MATH_TF32: _round_tf32, _abi.MATH_BF16: _round_bf16}[mode]
+    ref = O.conv_fwd(rnd(x), rnd(w), pads, [1] * 3)
+    p.fwd(1.0, xs, ws, 0.0, y)
+    emu.assert_close(y.cpu().numpy(), ref, TOL, "y")
+    y.fill_(float("nan"))
+    assert _abi.lib().dcb_conv_fwd_stats(p.p, 1.0, xs.data_ptr(), ws.data_ptr(), y.data_ptr(), sums[0].data_ptr(),
+                                         sums[1].data_ptr(), None) == _abi.OK
+    emu.assert_close(y.cpu().numpy(), ref, TOL, "y with statistics")
+    assert _abi.lib().dcb_conv_plan_status(p.p, None) == _abi.OK
+    d, over = y.double(), (0, 2, 3, 4)
+    for got, exact, size in ((sums[0], d.sum(over), d.abs().sum(over)), (sums[1], d.square().sum(over), d.square().sum(over))):
+        assert ((got.double() - exact).abs() <= 1e-5 * size).all()
+
+
 @pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_BF16])
 @pytest.mark.parametrize("geom", [
     (1, 4, 16, (6, 9, 9), (3, 3, 3), 1),      # sub-columns side by side
     (2, 8, 7, (5, 11, 31), (3, 3, 3), 1),     # two samples, filters padded
     (1, 16, 16, (7, 9, 101), (3, 3, 3), 1),   # ragged rows: plain stores
     (1, 16, 4, (8, 9, 132), (3, 3, 3), 2),    # stride 2
-    (1, 32, 16, (64, 64, 64), (3, 3, 3), 1),  # channel groups, bulk stores
+    (1, 32, 16, (64, 64, 64), (3, 3, 3), 1),  # channel groups, in fp32 parts of rows
+    layers.STATISTICS_BY_BULK_STORES,
 ])
 def test_statistics_from_the_shift_kernel(geom, mode):
     """Sums and sums of squares of the output that it wrote, to fp32 rounding of partial sums:
@@ -928,10 +962,6 @@ def test_statistics_from_the_shift_kernel(geom, mode):
         assert ((got.double() - ref).abs() <= 1e-5 * size).all()
 
 
-def _round_tf32(a):
-    return ((a.view(np.uint32) + np.uint32(0x1000)) & np.uint32(0xFFFFE000)).view(np.float32)
-
-
 @pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_TF32, _abi.MATH_BF16])
 @pytest.mark.parametrize("geom", [
     # N, C, K, spatial, filter, padding, stride: one tap along D, columns of several rows, several planes a CTA
@@ -954,11 +984,7 @@ def test_planes_that_open_and_close_in_one_step(geom, mode):
 
 
 @pytest.mark.parametrize("mode", [_abi.MATH_FP32, _abi.MATH_BF16])
-@pytest.mark.parametrize("geom", [
-    # N, C, K, spatial, filter, stride: rows that are laid side by side in parts, last parts short
-    (1, 32, 24, (9, 33, 64), (3, 3, 3), 1), (2, 24, 28, (7, 20, 132), (3, 3, 3), 1), (1, 12, 20, (9, 31, 177), (3, 3, 3), 1),
-    (1, 8, 8, (12, 40, 66), (3, 3, 3), 1), (2, 32, 16, (75, 65), (3, 3), 1), (1, 16, 24, (11, 23, 160), (3, 3, 3), 2),
-])
+@pytest.mark.parametrize("geom", [g for g, _ in layers.ROWS_IN_PARTS])
 def test_rows_in_parts(geom, mode):
     N, C, K, sp, f, s = geom
     rng = np.random.default_rng(sp[-1])

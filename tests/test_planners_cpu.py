@@ -8,10 +8,13 @@ import pytest
 
 import dihydrogen_b200.build as build
 
+import layers
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 pytestmark = pytest.mark.skipif(not os.path.exists(build._nvcc()) and shutil.which(build._nvcc()) is None,
                                 reason="no nvcc")
 FP32, TF32 = 0, 1
+MODES = {"fp32": 0, "tf32": 1, "bf16": 3}
 
 
 def compile_check(folder, name):
@@ -165,7 +168,7 @@ def test_tables_that_do_not_fit_leave_a_lower_column(tmp_path):
 
 
 def test_parts_of_rows_cover_every_output_once(tmp_path):
-    """Parts of a row side by side in the lanes, each with its own row blocks or segments."""
+    """Parts of a row side by side in the lanes, each with its own row blocks or segments; what their outputs read is staged."""
     r = subprocess.run([compile_check(tmp_path, "shift_parts_check")], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     passes, parts, bad = map(int, r.stdout.split())
@@ -180,6 +183,32 @@ def test_windows_that_stay_in_l2_are_unpacked_from_their_start(tmp_path):
     r = subprocess.run([exe], input=" ".join(map(str, start + end)), capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split() == ["0"] * len(start) + ["1"] * len(end)
+
+
+def test_layers_have_the_layouts_that_the_tests_on_the_gpu_mean(tmp_path):
+    exe = compile_check(tmp_path, "conv_layout_check")
+
+    def layout(n, c, k, sp, f, pads, stride, mode):
+        flat = len(sp) == 2
+        v = [n, c, k, *([0] if flat else []), *sp, *([1] if flat else []), *f, *([0] if flat else []), *pads, stride, MODES[mode]]
+        r = subprocess.run([exe], input=" ".join(map(str, v)), capture_output=True, text=True, timeout=60)
+        assert r.returncode == 0, r.stderr
+        return {l.split()[0]: [int(a) for a in l.split()[1:]] for l in r.stdout.splitlines()}
+
+    for (n, c, k, sp, f, pads), slots in layers.SWEEP:
+        for mode in MODES:
+            want = slots["fp32" if mode == "fp32" else "bf16"]
+            assert layout(n, c, k, sp, f, pads, 1, mode)["sweep"] == [int(want > 0), want], (n, c, k, sp, f, mode)
+    for (n, c, k, sp, f, s), passes in layers.ROWS_IN_PARTS:
+        for mode in ("fp32", "bf16"):
+            got = layout(n, c, k, sp, f, [1] * len(sp), s, mode)
+            assert got["sweep"][0] == 0
+            in_parts = tuple(p for p in ("fwd", "bwd_data") if got[p][0] and got[p][1] > 1 and got[p][2] > 1)
+            assert in_parts == passes[mode], (n, c, k, sp, mode, got)
+    n, c, k, sp, f, s = layers.STATISTICS_BY_BULK_STORES
+    for mode in ("fp32", "bf16"):
+        got = layout(n, c, k, sp, f, [1] * 3, s, mode)
+        assert got["sweep"][0] == 0 and got["fwd"][:3] == [1, 1, 1] and got["fwd"][3] > 0, got
 
 
 def test_no_report_of_a_block_counts_for_another_use_of_it(tmp_path):
