@@ -851,6 +851,8 @@ def test_what_is_not_a_number_stays_that(geom, mode):
     (1, 8, 16, (20, 64), (3, 3), 1),         # bulk stores
     (1, 16, 24, (5, 6, 40), (3, 3, 3), 1),
     (1, 4, 8, (9, 33), (1, 1), 2),           # one tap: its k-step's other half is the neighbour's cell
+    (1, 8, 8, (12, 40, 66), (3, 3, 3), 1),   # rows in parts
+    (1, 16, 32, (9, 24, 64), (3, 3, 3), 2),  # epilogue teams that share a block
 ])
 def test_infinities_and_nans_come_out_as_from_fp32_fma(geom, mode, value):
     """... and only where they are a term: the cells around keep their values (strides 2:
