@@ -121,7 +121,8 @@ bool sw_geom(const ConvGeom& cg, int math_mode, SwGeom* out)
     g.nseg = best_ns;
     g.rows = g.th + g.f[1] - 1;
     // Two A slots per group (and with them a second issuer per group in the plain
-    // kernel) where the chosen column height leaves the tensor-memory columns for them.
+    // kernel) where the chosen column height leaves the tensor-memory columns for them:
+    // the height is chosen first, by staged rows alone.
     if (2 * g.groups * g.kr <= 256
         && 2 * g.groups * g.kr + g.th * g.f[0] * SW_NBK <= (int) TC_TMEM_COLS)
         g.a_slots = 2 * g.groups;

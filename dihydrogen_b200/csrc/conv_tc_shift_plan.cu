@@ -278,7 +278,7 @@ bool ShBuilder::layout(const Try& t, ShTables* T) const
     }
     // what the row's outputs read: a tile is whole warps, but what lies behind a row that is its
     // only one needs no converter item (backward data of 8 -> 24 on 2 x 67 x 83 x 101: four items
-    // instead of five, three teams of converters instead of two, 245 -> 175 us)
+    // instead of five, three teams of converters instead of one, 245 -> 175 us)
     T->per = (g.tiles_w == 1 ? std::min(g.tile_w, g.q_w) : g.tile_w) + reach;
     const int used = g.npack * T->per;
     g.pt = std::max(TC_M + reach, g.npack * (g.tile_w + reach)) + 1;
@@ -343,7 +343,9 @@ int ShBuilder::packed(int w) const
 // neighbours' cells again, so they are only tried where they fill a good deal more of the lanes.
 // us, forward and backward data: 32 -> 32 on 2 x 24 x 40 x 64 151 -> 82 and 156 -> 82, 24 -> 28 on 40 x 100 x 132
 // 541 -> 312 and 453 -> 258, 12 -> 20 on 50 x 90 x 177 132 -> 101 and 151 -> 126, 16 -> 24 with stride 2
-// on 90 x 90 x 160 backward data 77 -> 58.
+// on 90 x 90 x 160 backward data 77 -> 58. Of 260 layers drawn over the range, 2 % less time for all together forward
+// and 3 % backward; the worst is 8 -> 32 with stride 2 on 4 images of 40 x 200, 10.2 -> 10.8. (The shares of the
+// lanes below which parts are not tried are set by hand, to keep the search short; the clocks decide.)
 std::vector<int> ShBuilder::row_parts() const
 {
     if (packed(m_w.q) >= 2)
@@ -567,7 +569,9 @@ bool ShBuilder::finish(const Try& t, ShTables* T) const
             // Three teams of four warps are better than two where conversion bounds: one pass of products
             // (16 -> 16 in TF32 on 100 x 100 x 75 77 / 94 us), parts of rows (16 -> 4 on 100 x 100 x 160 119 / 125), or
             // no room for two slots a team. Elsewhere they get in the way of the other roles (24 -> 24 on
-            // 2 x 700 x 118 31.2 / 29.3, 16 -> 24 on 4 x 300 x 30 16.2 / 15.3, backward data 18.3 / 16.7).
+            // 2 x 700 x 118 31.2 / 29.3, 16 -> 24 on 4 x 300 x 30 16.2 / 15.3, backward data 18.3 / 16.7). Over 32 forward
+            // passes and 62 of backward data, 27 of them with stride 2, two teams take 0.6 and 1.2 % less (9 % at
+            // best; 1.6 % more at worst, 24 -> 4 on 4 x 16 x 72 x 27).
             if (g.ipr == 4 && fit >= 6 && m_parts > 1 && (g.npack == 1 || g.tiles_w == 1))
                 g.teams = 2, slots = 6;
         }
@@ -638,9 +642,11 @@ bool ShBuilder::one_set(int cgroups, int items) const
 }
 
 // Clocks of the busiest SM.  A fit to the times of 730 layouts of 56 passes (the layout that it
-// picks of a pass is 1.7 % slower than the best of it; a maximum of products, conversion and
+// picked of a pass was 1.7 % slower than the best of it; a maximum of products, conversion and
 // draining instead of their sum: 4 %): the roles wait for one another row by row, so that
-// what each of them takes adds up.
+// what each of them takes adds up. The fit is older than the tables in the constant bank, blocks that both
+// epilogue teams drain, and rows in parts, and has not been made again. Over passes of 40 us and more in fp32
+// the time taken is 0.91 of the estimate (median; 0.62 to 1.21 for eight of ten), 0.86 where blocks are shared.
 double ShBuilder::clocks(const ShGeom& g, double mma, int teams) const
 {
     const double rows = (double) g.rows * g.cgroups, cells = g.cpg / m_ch * (m_kind == 0 ? 1.0 : 2.0);
@@ -651,9 +657,9 @@ double ShBuilder::clocks(const ShGeom& g, double mma, int teams) const
     if (g.th == 1 && g.ns == (m_s.taps + m_s.st - 1) / m_s.st)
         plane += 0.63 * drain; // a block has to be drained before its plane slot is opened again
     const double waves = (double) ((g.units + m_sms - 1) / m_sms);
-    // parts of a row take more than the fit, which has none of them, says (16 -> 16 on 64^3, forward with
-    // statistics: 54 us expected and 66.7 taken, 56 and 64.3 with whole rows)
-    // and more where the statistics come out of the epilogue that stores them
+    // Parts of a row take more, beside whole rows, than the fit, which has none of them, says (16 -> 16 on 64^3,
+    // forward with statistics: 54 us expected and 66.7 taken, 56 and 64.3 with whole rows), and more where the
+    // statistics come out of the epilogue that stores them. Set by hand from a few such layers.
     const bool stats = !m_tr && !m_flat && g.kgroups == 1 && g.nb <= 16;
     const double parts = g.npack > 1 && g.tiles_w > 1 ? (stats ? 1.15 : 1.08) : 1.0;
     return parts * waves * (((g.seglen - 1) * m_s.st + m_s.taps) * plane + 16800.0);
@@ -753,6 +759,8 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
             left -= !T.too_long; // (lower columns have shorter tables)
             if (fits)
             {
+                // two teams of four are taken where three would be slower (finish), which the fit does not know:
+                // priced as the three that it would have liked better
                 T.cost = clocks(T.g, t.mma, T.g.ipr == 4 && T.g.teams == 2 ? 3 : T.g.teams);
                 T.chain = T.g.nsets == 1 ? chain_of(m_parts * (m_parts + 1) / 2 * T.g.cpg / m_ch * m_w.most(), 1, T.g.cgroups)
                                          : chain_of(T.g.cpg / m_ch * m_w.most(), T.g.nsets - (m_parts > 1 ? 1 : 0), T.g.cgroups);
@@ -772,7 +780,8 @@ bool ShBuilder::build_within(double limit, ShTables* out) const
     const ShTables rows = *out;
     if (!pick(tries) || out->cost > rows.cost)
         *out = rows;
-    // (the CUDA-core kernels are weighed against whole rows, which their rule was made with)
+    // The CUDA-core kernels are weighed against whole rows, which their rule was made with. (Layers in parts
+    // take 0.63 of that, so that a layer near the line may be on the CUDA cores that would be faster here.)
     out->cost = rows.cost;
     return true;
 }

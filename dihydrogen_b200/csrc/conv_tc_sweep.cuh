@@ -324,9 +324,10 @@ __device__ __forceinline__ void sw_convert_f3(uint32_t raw_lane, uint32_t pitch,
 // shard, ~140 clocks per tcgen05.mma or commit, seven per staged row); with six the
 // kernel takes 0.378 ms instead of 0.433.  The variant with statistics is
 // held by its epilogue warps and by registers (the extra warps lower the cap to 66
-// per thread, its epilogue then spills): it keeps three issuers. They go through both slots of
-// their group in turn, so that a row is written while the one before it is multiplied: 256^3
-// 449 -> 440 us, 128^3 89 -> 86, 5 -> 16 on 64 x 80 x 128 64 -> 58 with one slot and with two.
+// per thread, its epilogue then spills): it keeps three issuers. Where their group has two
+// slots they go through them in turn, so that a row is written while the one before it is multiplied: with one
+// slot and with two 256^3 449 and 440 us, in bf16 467 and 433, 5 -> 16 on 64 x 80 x 128 64 and 58. A column of
+// eight rows and 24 k-rows a slot (4 -> 16 in fp32 on 128^3, 64 x 80 x 200, 128 x 128 x 256) leaves room for one.
 constexpr int SW_EPI = 12;
 __host__ __device__ constexpr int sw_threads(int xiss)
 {

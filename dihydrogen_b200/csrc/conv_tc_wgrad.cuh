@@ -107,8 +107,7 @@ struct WgConvArgs
 // Lanes outside the tensor store zeros (the padding).  Eight lanes along a row, then the
 // next channel: a quarter of a 16-byte load is then one line of 128 bytes, and a quarter of
 // a store is eight cells LBO = 16 mod 128 apart.  (With the channels side by side a quarter
-// touched the same banks of four lines: what bounds the kernel is shared memory, which the
-// instructions read their operands from, 256^3, 4 -> 16 1206 -> 1011 us, 128^3 185 -> 148,
+// touched the same banks of four lines: 256^3, 4 -> 16 1206 -> 1011 us, 128^3 185 -> 148,
 // 32 -> 32 on 24 x 40 x 64 119 -> 111.)  A warp's own chain of dependent
 // instructions is what bounds a stage where channels are few: hence pairs of items
 // without branches between them, and stages that follow each other along H, so that
@@ -404,7 +403,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t columns = (uint32_t) (g.sum_col + g.kdg * g.nblocks * g.kgp); // accumulators, running sums
+    // accumulators, running sums (all 512 columns in a loop that is not unrolled: two registers fewer spilled with
+    // three taps, large layers the same, small ones 10 % slower)
+    const uint32_t columns = (uint32_t) (g.sum_col + g.kdg * g.nblocks * g.kgp);
     if (warp < 4)
         for (uint32_t c = 0; c < columns; c += 16)
             tmem_st16_zero(tmem + ((uint32_t) (warp * 32) << 16) + c);

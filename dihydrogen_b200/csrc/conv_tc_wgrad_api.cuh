@@ -14,7 +14,7 @@ constexpr int WG_ISSUE_WARP = WG_FLUSH + WG_CONV;
 constexpr int WG_THREADS = (WG_FLUSH + WG_CONV + 1) * 32;
 constexpr int WG_MAX_STAGES = 8;
 constexpr int WG_MAX_TILES = 24;
-constexpr int WG_CHAIN = 120; // updates of an accumulator: 2.4e-6 of the result on the longest sums
+constexpr int WG_CHAIN = 120; // updates of an accumulator: 2.5e-6 of the result on the longest sums (128^3)
 
 struct WgTile
 {

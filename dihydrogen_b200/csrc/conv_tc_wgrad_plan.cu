@@ -20,12 +20,12 @@ double wg_mma_cost(int n)
     return a > b ? (a > 45.5 ? a : 45.5) : (b > 45.5 ? b : 45.5);
 }
 
-// Updates of an accumulator between flushes.  A chain of truncating updates is off by 1.7e-8
-// each (2.0e-6 with WG_CHAIN), fp32 FMAs over n positions, as the CUDA-core kernel deals them
+// Updates of an accumulator between flushes.  A chain of truncating updates is off by 1.5e-8 to
+// 2e-8 each (1.8e-6 to 2.5e-6 with WG_CHAIN), fp32 FMAs over n positions, as the CUDA-core kernel deals them
 // out, by 1.4e-9 sqrt(n) and more where there are many sums.  Strided layers and rows that
-// cannot be read in aligned 16-byte pieces are held to that: 16 -> 16, 24 x 40 x 67, 1.9e-6
-// with WG_CHAIN, 7.4e-7 with FMAs.  The others are only where they are small: 64 updates (1e-6)
-// cost a few percent there, on 256^3 4 -> 16 would take 1457 us instead of 1180.
+// cannot be read in aligned 16-byte pieces are held to that: 16 -> 16, 24 x 40 x 67, 1.8e-6
+// with WG_CHAIN, 6.4e-7 like this, 7.4e-7 with FMAs.  The others are only where they are small: with 64 updates
+// (1.2e-6) 4 -> 16 would take 1125 us instead of 1053 on 256^3, 162 instead of 149 on 128^3.
 int wg_chain(const ConvGeom& cg)
 {
     const bool aligned = ((cg.xs[0] | cg.xs[1] | cg.xs_c | cg.xs_n | cg.ys[0] | cg.ys[1] | cg.ys_c | cg.ys_n) & 3) == 0;
@@ -176,9 +176,12 @@ bool wg_layout(const ConvGeom& cg, WgGeom* out, int cgp, int kwg, int kdg, int k
             best = score, lat = m, g.warps_x = wx;
     }
     // The terms' weights are a fit to the times of 1200 layouts of 33 layers (8 % rms; the layout
-    // that it picks of a layer is 1 % slower than the best of it, with all weights 1 it was 9 %):
+    // that it picked of a layer was 1 % slower than the best of it, with all weights 1 it was 9 %):
     // pipe and converters overlap in part, stages narrower than 32 positions fetch parts of lines,
-    // a walk's lead steps bring a plane each, a piece of eight columns costs a flush 280.
+    // a walk's lead steps bring a plane each, a piece of eight columns costs a flush 280. The fit is older
+    // than the converters' lanes along the row. Of the best walk and the best plain layout of 61 layers,
+    // both timed with those, it picks one that is 0.7 % slower than the other (geometric mean; 22 % at worst,
+    // 6 -> 32 on 90 x 160 x 16); 8 -> 24 on 2 x 67 x 83 x 101 takes 285 us and would take 256 as a walk.
     const double feed = std::max(instr, lat);
     const double narrow = 1.0 + 0.285 * std::max(0, 32 - PW) / 32.0;
     const double per = (1.2 * std::max(pipe, feed) + 0.64 * std::min(pipe, feed) + 530.0) * narrow;

@@ -91,7 +91,8 @@ struct ShfJob
 // (B200, L2 of 126 MB; 2 x 16 x D x 128 x 128 split along D):
 //   one rank on the device   34 MB 36.3 / 37.8, 67 MB 61.8 / 65.0, 84 MB 78.0 / 79.7, 101 MB 98.9 / 94.5, 134 MB 136.9 / 126.1
 //   two ranks, of each       34 MB 85.8 / 91.9, 42 MB 101.2 / 108.2, 50 MB 121.7 / 121.6, 59 MB 142.9 / 138.0, 134 MB 281.6 / 276.8
-// Either alone is 1 to 3 % slower than neither; pieces lose with both.
+// Either alone is 1 to 3 % slower than neither; pieces lose with both. (Not timed with a device per rank: one rank
+// with a window of its own stands for it.)
 inline bool shf_from_the_end(double window_bytes, double l2_bytes)
 {
     return window_bytes >= 0.75 * l2_bytes;
