@@ -266,7 +266,8 @@ __host__ __device__ constexpr int sw_f3_columns(int c, bool split)
 
 // Converts them without a table, all loads at once, and before the slot has to be free (the general
 // converter walks the columns in eights behind that wait). us, with the general converter and like this:
-// 128^3, 4 -> 16 in bf16 71 and 58, 3 -> 12 103 and 81; 64 x 80 x 200, 1 -> 16 40.7 and 37.1, 2 -> 16 54.0 and 47.8.
+// 128^3, 4 -> 16 in bf16 71 and 58, 3 -> 12 103 and 81, in bf16 69 and 57; 64 x 80 x 200, 1 -> 16 40.7 and 37.1, in
+// bf16 38.8 and 35.7, 2 -> 16 54.0 and 47.8, in bf16 38.9 and 36.2.
 template <int C, bool SPLIT>
 __device__ __forceinline__ void sw_convert_f3(uint32_t raw_lane, uint32_t pitch, uint32_t rnd_add, uint32_t rnd_mask,
                                               uint32_t (&v)[sw_f3_columns(C, SPLIT) / 8][8])
