@@ -20,8 +20,9 @@ SWEEP = [
     ((1, 4, 12, (7, 9, 136), (4, 3, 3), (1, 1, 1)), {"fp32": 0, "bf16": 2}),
 ]
 
-# N, C, K, spatial, filter, stride: rows that the shift kernel lays side by side in parts, last parts short;
-# the passes that do so per mode (the others are layers next to those)
+# N, C, K, spatial, filter, stride: rows that the shift kernel lays side by side in parts, last parts short
+STRIDED_ROWS_IN_PARTS = [(1, 8, 24, (40, 60, 132), (3, 3, 3), 2), (1, 16, 8, (40, 60, 131), (3, 3, 3), 2)]
+# ... with the passes that do so per mode (some layers are next to such ones)
 ROWS_IN_PARTS = [
     ((1, 32, 24, (9, 33, 64), (3, 3, 3), 1), {"fp32": ("fwd", "bwd_data"), "bf16": ("fwd",)}),
     ((2, 24, 28, (7, 20, 132), (3, 3, 3), 1), {"fp32": ("fwd", "bwd_data"), "bf16": ("fwd", "bwd_data")}),
@@ -29,8 +30,8 @@ ROWS_IN_PARTS = [
     ((1, 8, 8, (12, 40, 66), (3, 3, 3), 1), {"fp32": ("fwd", "bwd_data"), "bf16": ("fwd", "bwd_data")}),
     ((2, 32, 16, (75, 65), (3, 3), 1), {"fp32": ("bwd_data",), "bf16": ()}),
     ((1, 16, 24, (11, 23, 160), (3, 3, 3), 2), {"fp32": (), "bf16": ()}),
-    ((1, 8, 24, (40, 60, 132), (3, 3, 3), 2), {"fp32": ("fwd", "bwd_data"), "bf16": ("fwd", "bwd_data")}),
-    ((1, 16, 8, (40, 60, 131), (3, 3, 3), 2), {"fp32": ("fwd", "bwd_data"), "bf16": ("bwd_data",)}),
+    (STRIDED_ROWS_IN_PARTS[0], {"fp32": ("fwd", "bwd_data"), "bf16": ("fwd", "bwd_data")}),
+    (STRIDED_ROWS_IN_PARTS[1], {"fp32": ("fwd", "bwd_data"), "bf16": ("bwd_data",)}),
 ]
 
 # N, C, K, spatial, filter, stride: forward by whole rows and bulk stores
